@@ -33,7 +33,9 @@ def _ptr(t) -> int:
 
 def _stream(stream=None) -> int:
     if stream is None:
-        return torch.cuda.current_stream().cuda_stream
+        # the current stream's handle without a Stream object around it (0.1 us instead of 3.4 us a call, which a
+        # small projection's launch would wait for)
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     return stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
 
 
