@@ -226,7 +226,7 @@ gw_status gw_nvfp4_plan_create(uint32_t rows, uint32_t input_width, uint32_t out
   // by the plan and room for FP32 partial tiles in the scratch.  Without a usable device
   // (or memory for the counters) the plan falls back to whole tiles per CTA.
   p->total_bytes = p->split_offset;
-  const cudaError_t counters = p->descriptors.allocate_split_counters(rows, output_width);
+  const cudaError_t counters = p->descriptors.allocate_split_counters(GemmKind::nvfp4, rows, input_width, output_width);
   if (counters != cudaSuccess) {
     (void)cudaGetLastError();
     // Without any device the plan is only a shape record (it cannot run); every other failure is an error,
@@ -236,7 +236,7 @@ gw_status gw_nvfp4_plan_create(uint32_t rows, uint32_t input_width, uint32_t out
       return fail(GW_CUDA_ERROR, std::string("plan: tile counters of the K split: ") + cudaGetErrorString(counters));
     }
   }
-  if (p->descriptors.split_counters) p->total_bytes += align_up(dense_split_bytes(p->descriptors.tuning, rows, output_width), 256);
+  p->total_bytes += p->descriptors.split_bytes(rows, output_width);
   *plan = p;
   return GW_OK;
 }
@@ -262,6 +262,22 @@ gw_status gw_nvfp4_plan_run(gw_nvfp4_plan* plan, const void* input_bf16, const u
   cudaStream_t s = as_stream(stream);
   auto* packed = static_cast<uint8_t*>(scratch);
   uint8_t* scales = packed + plan->scale_offset;
+  {
+    StreamProblem q{StreamKind::w4a4, plan->rows, plan->input_width, plan->output_width, input_bf16};
+    q.gelu = transform == GW_TRANSFORM_GELU_TANH_MULTIPLY;
+    q.inverse_scale = 1.0F / input_scale;
+    q.packed = packed;
+    q.packed_scales = scales;
+    q.first = StreamMatrix{weight_data, weight_scales, alpha, nullptr};
+    q.output = output_bf16;
+    q.ld_out = plan->output_width;
+    q.workspace = packed + plan->split_offset;
+    q.counters = plan->descriptors.split_counters;
+    q.error = device_error_word();
+    bool done = false;
+    const gw_status status = launch_dense_stream(q, &plan->descriptors, s, &done);
+    if (status != GW_OK || done) return status;
+  }
   GW_CUDA_CHECK(launch_nvfp4_quantize(input_bf16, plan->rows, plan->input_width, 1.0F / input_scale,
                                       transform == GW_TRANSFORM_GELU_TANH_MULTIPLY, packed, scales, s),
                 "NVFP4 quantize activations");
@@ -326,7 +342,7 @@ gw_status gw_fp8_plan_create(uint32_t rows, uint32_t input_width, uint32_t outpu
   // by the plan and room for FP32 partial tiles in the scratch.  Without a usable device
   // (or memory for the counters) the plan falls back to whole tiles per CTA.
   p->total_bytes = p->split_offset;
-  const cudaError_t counters = p->descriptors.allocate_split_counters(rows, output_width);
+  const cudaError_t counters = p->descriptors.allocate_split_counters(GemmKind::fp8, rows, input_width, output_width);
   if (counters != cudaSuccess) {
     (void)cudaGetLastError();
     // Without any device the plan is only a shape record (it cannot run); every other failure is an error,
@@ -336,7 +352,7 @@ gw_status gw_fp8_plan_create(uint32_t rows, uint32_t input_width, uint32_t outpu
       return fail(GW_CUDA_ERROR, std::string("plan: tile counters of the K split: ") + cudaGetErrorString(counters));
     }
   }
-  if (p->descriptors.split_counters) p->total_bytes += align_up(dense_split_bytes(p->descriptors.tuning, rows, output_width), 256);
+  p->total_bytes += p->descriptors.split_bytes(rows, output_width);
   *plan = p;
   return GW_OK;
 }
@@ -361,6 +377,20 @@ gw_status gw_fp8_plan_run(gw_fp8_plan* plan, const void* input_bf16, const uint8
                 "scales with a finite positive product and finite input-scale reciprocal");
   cudaStream_t s = as_stream(stream);
   auto* packed = static_cast<uint8_t*>(scratch);
+  if (plan->gemv_rows == 0) {
+    StreamProblem q{StreamKind::w8a8, plan->rows, plan->input_width, plan->output_width, input_bf16};
+    q.gelu = transform == GW_TRANSFORM_GELU_TANH_MULTIPLY;
+    q.inverse_scale = 1.0F / input_scale;
+    q.first = StreamMatrix{weight_data, nullptr, alpha, plan->channel_scales ? channel_scales : nullptr};
+    q.output = output_bf16;
+    q.ld_out = plan->output_width;
+    q.workspace = packed + plan->split_offset;
+    q.counters = plan->descriptors.split_counters;
+    q.error = device_error_word();
+    bool done = false;
+    const gw_status status = launch_dense_stream(q, &plan->descriptors, s, &done);
+    if (status != GW_OK || done) return status;
+  }
   // Optional CUDA-core path for 1..4 rows (weight streaming with warp reductions, activations
   // quantised inside the kernel).  Measured on B200 it is slower than the tensor-core path
   // (55 us against 50 us for one row of the 43008 x 5376 projection, 82 us for two), so it is
@@ -404,9 +434,9 @@ gw_status gw_bf16_plan_create(uint32_t rows, uint32_t input_width, uint32_t outp
   p->output_width = output_width;
   // Decode shapes split the K loop evenly over the SMs (FP32 partial tiles in the scratch).
   p->total_bytes = 0;
-  const cudaError_t status = p->descriptors.allocate_split_counters(rows, output_width);
-  if (status == cudaSuccess && p->descriptors.split_counters) {
-    p->total_bytes = align_up(dense_split_bytes(p->descriptors.tuning, rows, output_width), 256);
+  const cudaError_t status = p->descriptors.allocate_split_counters(GemmKind::bf16, rows, input_width, output_width);
+  if (status == cudaSuccess) {
+    p->total_bytes = p->descriptors.split_bytes(rows, output_width);
   } else if (status != cudaSuccess) {
     (void)cudaGetLastError();
     if (status != cudaErrorNoDevice && status != cudaErrorInsufficientDriver) {
@@ -430,6 +460,18 @@ gw_status gw_bf16_plan_run(gw_bf16_plan* plan, const void* input_bf16, const voi
       !aligned(output_bf16, 16) || (scratch && plan->total_bytes != 0 && (!aligned(scratch, 256) ||
                                                                            scratch_capacity < plan->total_bytes)))
     return fail(GW_INVALID_ARGUMENT, "BF16 run requires 16-byte aligned device buffers and aligned sufficient scratch");
+  if (scratch || !plan->descriptors.stream.needs_workspace()) {
+    StreamProblem q{StreamKind::w16a16, plan->rows, plan->input_width, plan->output_width, input_bf16};
+    q.first.data = weight_bf16;
+    q.output = output_bf16;
+    q.ld_out = plan->output_width;
+    q.workspace = scratch;
+    q.counters = plan->descriptors.split_counters;
+    q.error = device_error_word();
+    bool done = false;
+    const gw_status status = launch_dense_stream(q, &plan->descriptors, as_stream(stream), &done);
+    if (status != GW_OK || done) return status;
+  }
   DenseProblem problem{GemmKind::bf16, plan->rows, plan->input_width, plan->output_width, weight_bf16, nullptr,
                        input_bf16, nullptr, 1.0F, nullptr, output_bf16, device_error_word()};
   if (plan->total_bytes != 0 && scratch) problem.split_workspace = scratch;

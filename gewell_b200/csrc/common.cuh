@@ -77,11 +77,12 @@ __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.
 // its predecessor in the stream drains; it must call griddep_wait() before it touches global
 // memory (every kernel launched through this helper does so first thing).
 template <typename... Params, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t stream, Args&&... args) {
+inline cudaError_t launch_pdl_shared(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
+                                     Args&&... args) {
   cudaLaunchConfig_t config{};
   config.gridDim = grid;
   config.blockDim = block;
-  config.dynamicSmemBytes = 0;
+  config.dynamicSmemBytes = shared_bytes;
   config.stream = stream;
   cudaLaunchAttribute attribute{};
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -90,6 +91,10 @@ inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, 
   config.numAttrs = 1;
   note_launch();
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t stream, Args&&... args) {
+  return launch_pdl_shared(kernel, grid, block, 0, stream, static_cast<Args&&>(args)...);
 }
 
 #ifdef __CUDACC__

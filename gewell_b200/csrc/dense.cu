@@ -1,6 +1,7 @@
 #include "dense.h"
 #include "gemm_pair.h"
 
+#include <algorithm>
 #include <cstdlib>
 #include <string>
 
@@ -35,15 +36,42 @@ size_t split_counter_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n)
 }
 }  // namespace
 
+// Where the weight-streaming kernel is the faster one for rows <= 16 (B200, both timed back to back, us; old = activation
+// quantiser + tcgen05 swap form): NVFP4 16x2816x2816 15.3 -> 9.3, 8x5376x43008 32.6 -> 33, 1x21504x5376 24.1 -> 20.9; FP8
+// 8x5376x43008 46.3 -> 42.6.  It saves the quantiser's launch and the tensor-memory prologue; what it pays is that every SM
+// reads and quantises all of the activations: about 1 us per 16K values, which meets the gain at 64K.  Nine and more
+// rows need a second token group (half as many instructions again per weight byte), which only small matrices hide.
+// W4A16 has no other kernel that reads the packed weights.
+bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
+  if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
+  const size_t values = size_t(rows) * k;
+  const size_t bytes = n * k * (kind == StreamKind::w4a4 ? 9 : kind == StreamKind::w8a8 ? 16 : 32) / 16;
+  if (values > 65536) return false;
+  if (plan.tiles == 2 && values > 46 * 1024 && bytes > (size_t(20) << 20)) return false;
+  // BF16 tokens of more than 8192 values need several slabs: twice the sums
+  return kind != StreamKind::w16a16 || plan.slabs == 1 || bytes <= (size_t(48) << 20);
+}
+
 size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n) {
   (void)n;
   if (!dense_uses_swap_form(tuning, rows) || tuning.no_split) return 0;
   return size_t(2) * sm_count() * 128 * dense_block_n(tuning, rows) * sizeof(float);
 }
 
-cudaError_t DenseDescriptors::allocate_split_counters(uint32_t rows, uint32_t n) {
+size_t DenseDescriptors::split_bytes(uint32_t rows, uint32_t n) const {
+  if (split_counters == nullptr) return 0;
+  return align_up(std::max(dense_split_bytes(tuning, rows, n), stream.usable ? stream.workspace_bytes : 0), 256);
+}
+
+cudaError_t DenseDescriptors::allocate_split_counters(GemmKind kind, uint32_t rows, uint32_t k, uint32_t n) {
   if (dense_split_bytes(tuning, rows, n) == 0) return cudaSuccess;
-  const size_t bytes = split_counter_bytes(tuning, rows, n);
+  size_t bytes = split_counter_bytes(tuning, rows, n);
+  if (tuning.streams()) {
+    const StreamKind as = kind == GemmKind::nvfp4 ? StreamKind::w4a4 : kind == GemmKind::fp8 ? StreamKind::w8a8 : StreamKind::w16a16;
+    stream = plan_stream(as, rows, k, n, false, sm_count());
+    stream.usable = stream_pays(as, stream, rows, k, n);
+    if (stream.usable) bytes = std::max(bytes, align_up(stream.counter_count * sizeof(int32_t), 256));
+  }
   cudaError_t status = cudaMalloc(&split_counters, bytes);
   if (status == cudaSuccess) status = cudaMemset(split_counters, 0, bytes);
   return status;
@@ -51,6 +79,16 @@ cudaError_t DenseDescriptors::allocate_split_counters(uint32_t rows, uint32_t n)
 
 DenseDescriptors::~DenseDescriptors() {
   if (split_counters != nullptr) cudaFree(split_counters);
+}
+
+gw_status launch_dense_stream(const StreamProblem& q, DenseDescriptors* cache, cudaStream_t stream, bool* done) {
+  *done = cache->stream.usable && stream_aligned(q);
+  if (!*done) return GW_OK;
+  std::string error;
+  if (!cache->stream_maps.get(q.kind, q.first, cache->stream.physical_n, q.k, &error))
+    return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
+  GW_CUDA_CHECK(launch_stream(q, cache->stream, cache->stream_maps, cache->stream_maps, stream), "weight-streaming projection");
+  return GW_OK;
 }
 
 gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStream_t stream) {

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "decode_stream.h"
 #include "gemm_tc.cuh"
 
 namespace gw {
@@ -13,10 +14,12 @@ namespace gw {
 //   GW_DENSE_FORM=swap|direct, GW_DENSE_BLOCK_N=128|256   operand roles / column tile
 //   GW_DENSE_NO_PAIR=1    NVFP4 projections with >= 256 rows stay on the single-CTA kernel
 //   GW_DENSE_NO_SPLIT=1   decode-shaped plans run whole tiles per CTA
+// Each of them but the third also keeps small row counts off the weight-streaming kernel.
 struct DenseTuning {
   char form = 0;            // 's', 'd' or 0
   int block_n = 0;
   bool no_pair = false, no_split = false;
+  bool streams() const { return form == 0 && block_n == 0 && !no_split; }
   static DenseTuning from_environment();
 };
 
@@ -31,7 +34,12 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   // Split mode: one arrival counter per weight tile, owned by the plan (device memory,
   // zeroed at creation; the kernel leaves every counter at zero again).
   int32_t* split_counters = nullptr;
-  cudaError_t allocate_split_counters(uint32_t rows, uint32_t n);
+  // Small row counts: how the weight-streaming kernel divides the work (its counters are split_counters).
+  StreamPlan stream;
+  StreamMaps stream_maps;
+  cudaError_t allocate_split_counters(GemmKind kind, uint32_t rows, uint32_t k, uint32_t n);
+  // Scratch for FP32 partial sums of either form (0: none), once the counters exist.
+  size_t split_bytes(uint32_t rows, uint32_t n) const;
   ~DenseDescriptors();
 };
 
@@ -58,6 +66,12 @@ int dense_block_n(const DenseTuning& tuning, uint32_t rows);
 
 // Bytes of split workspace a projection of this shape can use (0: none).
 size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n);
+
+// Whether the weight-streaming kernel is the faster one for this shape (n: output channels of all matrices together).
+bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n);
+
+// The problem on the weight-streaming kernel; *done = false when its pointers keep it off that kernel.
+gw_status launch_dense_stream(const StreamProblem& problem, DenseDescriptors* cache, cudaStream_t stream, bool* done);
 
 gw_status launch_dense(const DenseProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 

@@ -9,6 +9,8 @@
 //               FP8 with per-channel scales, or BF16; otherwise two separate projections
 //   GeGLU       fused into the activation quantiser of the down projection when that one runs
 //               quantised on a joined [rows, gate | up] tensor; an element-wise kernel otherwise
+//               (rows <= 16: gate, up and GeGLU are one launch of the weight-streaming kernel, and W4A16
+//               reads the packed weights, rows <= 48)
 //   down        FP8, NVFP4 (W4A4) or BF16 GEMM; NVFP4 weights with BF16 activations are
 //               dequantised into the chain's scratch first (W4A16)
 //
@@ -31,6 +33,8 @@
 #include <vector>
 
 #include "common.cuh"
+#include "decode_stream.h"
+#include "dense.h"
 #include "kernels.h"
 
 using namespace gw;
@@ -46,6 +50,9 @@ struct Buffer {
   }
   ~Buffer() { if (data) cudaFree(data); }
 };
+
+// Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each.
+constexpr uint32_t kW4a16Rows = 48;
 
 enum Kind { kNvfp4 = 0, kFp8 = 1, kFp8Channel = 2, kBf16 = 3 };
 using Key = std::tuple<int, uint32_t, uint32_t>;   // kind, K, N
@@ -92,6 +99,12 @@ struct PlanBook {
   int policy = GW_POLICY_ALWAYS;
   std::map<Key, PlanSet> plans;
   Buffer scratch, dequantized;
+  // Small row counts on the weight-streaming kernel: the plans of prepare()'s row count by (kind, K, N, two matrices), the
+  // counters they share (they run one after another) and the tensor maps of the last matrices by the same key.
+  using StreamKey = std::tuple<int, uint32_t, uint32_t, bool>;
+  struct Streaming { StreamPlan plan; StreamMaps maps[2]; };
+  std::map<StreamKey, Streaming> streaming;
+  Buffer counters;
   ~PlanBook() { for (auto& entry : plans) entry.second.reset(); }
 
   // shapes: (K, N) pairs; scratch for the widest of them, the dequantised buffer for the largest
@@ -131,6 +144,92 @@ struct PlanBook {
     for (auto& entry : plans) entry.second.reset();
     plans = std::move(next);
     rows = new_rows;
+    return prepare_streaming(shapes);
+  }
+
+  gw_status prepare_streaming(const std::vector<std::pair<uint32_t, uint32_t>>& shapes) {
+    streaming.clear();
+    size_t most = 0;
+    const bool allowed = DenseTuning::from_environment().streams();
+    for (const auto& [k, n] : shapes)
+      for (StreamKind kind : {StreamKind::w4a4, StreamKind::w4a16, StreamKind::w8a8, StreamKind::w16a16})
+        for (bool pair : {false, true}) {
+          // W4A16 beyond one launch's rows: several launches, each of them reads the packed weights once
+          const uint32_t tile = kind == StreamKind::w4a16 && rows <= kW4a16Rows ? std::min(rows, kStreamMaxRows) : rows;
+          Streaming s;
+          s.plan = plan_stream(kind, tile, k, n, pair, sm_count());
+          s.plan.usable = allowed && stream_pays(kind, s.plan, tile, k, pair ? 2 * size_t(n) : n);
+          if (!s.plan.usable || s.plan.workspace_bytes > scratch.bytes) continue;
+          most = std::max(most, s.plan.counter_count);
+          streaming[StreamKey{int(kind), k, n, pair}] = s;
+        }
+    if (most * sizeof(int32_t) > counters.bytes) {
+      Buffer larger;
+      cudaError_t status = larger.allocate(most * sizeof(int32_t));
+      if (status == cudaSuccess) status = cudaMemset(larger.data, 0, larger.bytes);
+      if (status != cudaSuccess) {
+        streaming.clear();
+        return fail(GW_CUDA_ERROR, std::string("counters of the weight-streaming kernel: ") + cudaGetErrorString(status));
+      }
+      std::swap(larger.data, counters.data);
+      std::swap(larger.bytes, counters.bytes);
+    }
+    return GW_OK;
+  }
+
+  // The projection `first` -- or, with `second`, GeGLU of both -- on the weight-streaming kernel; *done = false when the
+  // shape, the storage or the pointers keep it off that kernel.
+  gw_status stream(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4, cudaStream_t s,
+                   bool* done) {
+    *done = false;
+    if (second && (second->storage != first.storage || second->input != first.input || second->output != first.output)) return GW_OK;
+    StreamKind kind = StreamKind::w16a16;
+    float input_scale = 1.0F;
+    if (first.storage == GW_STORAGE_NVFP4_W4A4) {
+      kind = fp4 ? StreamKind::w4a4 : StreamKind::w4a16;
+      if (fp4) {
+        input_scale = first.nvfp4_input_scale;
+        if (second && second->nvfp4_input_scale != input_scale) return GW_OK;
+      }
+    } else if (first.storage == GW_STORAGE_FP8_W8A8) {
+      kind = StreamKind::w8a8;
+      input_scale = first.fp8_input_scale;
+      if (second && second->fp8_input_scale != input_scale) return GW_OK;
+    }
+    const auto found = streaming.find(StreamKey{int(kind), first.input, first.output, second != nullptr});
+    if (found == streaming.end() || !std::isfinite(1.0F / input_scale) || !(input_scale > 0.0F)) return GW_OK;
+    Streaming& with = found->second;
+    StreamProblem q{kind, std::min(rows, kStreamMaxRows), first.input, first.output, input};
+    q.inverse_scale = 1.0F / input_scale;
+    const gw_projection* projection[2] = {&first, second};
+    StreamMatrix* matrix[2] = {&q.first, &q.second};
+    std::string error;
+    for (int i = 0; i < (second ? 2 : 1); ++i) {
+      const gw_projection& p = *projection[i];
+      StreamMatrix& m = *matrix[i];
+      if (p.storage == GW_STORAGE_NVFP4_W4A4)
+        m = StreamMatrix{p.nvfp4_data, p.nvfp4_scales, fp4 ? p.nvfp4_input_scale * p.nvfp4_weight_scale : p.nvfp4_weight_scale, nullptr};
+      else if (p.storage == GW_STORAGE_FP8_W8A8)
+        m = StreamMatrix{p.fp8_data, nullptr, p.fp8_input_scale * p.fp8_weight_scale, p.fp8_channel_scales};
+      else
+        m.data = p.bf16;
+      if (!m.data || !(m.alpha > 0.0F) || !std::isfinite(m.alpha)) return GW_OK;      // the plans report what is wrong
+    }
+    if (!stream_aligned(q)) return GW_OK;
+    for (int i = 0; i < (second ? 2 : 1); ++i)
+      if (!with.maps[i].get(kind, *matrix[i], with.plan.physical_n, q.k, &error))
+        return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
+    q.ld_out = first.output;
+    q.workspace = scratch.data;
+    q.counters = static_cast<int32_t*>(counters.data);
+    q.error = device_error_word();
+    for (uint32_t row = 0; row < rows; row += kStreamMaxRows) {
+      q.rows = std::min(rows - row, kStreamMaxRows);
+      q.input = static_cast<const bf16*>(input) + size_t(row) * q.k;
+      q.output = static_cast<bf16*>(output) + size_t(row) * q.ld_out;
+      GW_CUDA_CHECK(launch_stream(q, with.plan, with.maps[0], with.maps[1], s), "weight-streaming projection");
+    }
+    *done = true;
     return GW_OK;
   }
 };
@@ -237,6 +336,11 @@ namespace {
 gw_status run_linear(PlanBook& book, const gw_projection& p, const void* input, void* output, bool fp4, int transform,
                      cudaStream_t s) {
   const uint32_t n = p.storage == GW_STORAGE_NVFP4_W4A4 ? p.physical_output : p.output;
+  if (p.storage == GW_STORAGE_NVFP4_W4A4 && !fp4 && transform == GW_TRANSFORM_IDENTITY && n == p.output) {
+    bool done = false;
+    const gw_status status = book.stream(p, nullptr, input, output, fp4, s, &done);
+    if (status != GW_OK || done) return status;
+  }
   const auto plan = [&](int kind) -> const PlanSet* {
     const auto found = book.plans.find(Key{kind, p.input, n});
     return found == book.plans.end() ? nullptr : &found->second;
@@ -295,6 +399,10 @@ gw_status gw_mlp_chain_run(gw_mlp_chain* c, const gw_projection* gate, const gw_
   const bool fp4 = gw_nvfp4_fp4_activations(c->book.policy, phase) != 0;
   auto* gate_out = static_cast<bf16*>(gate_up_bf16);
   gw_status status = GW_OK;
+  bool paired = false;
+  if (status = c->book.stream(*gate, up, input_bf16, product_bf16, fp4, s, &paired); status != GW_OK) return status;
+  if (paired)                    // one launch: gate, up and GeGLU
+    return run_linear(c->book, *down, product_bf16, output_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
   bool interleaved = true;       // gate_up holds [rows, gate | up]; otherwise gate rows, then up rows
   if ((nvfp4_joined(*gate, *up) && fp4) || fp8_joined(*gate, *up) || bf16_joined(*gate, *up)) {
     status = run_linear(c->book, widened(*gate, 2 * m), input_bf16, gate_out, fp4, GW_TRANSFORM_IDENTITY, s);

@@ -79,4 +79,41 @@ bool encode_tensor_map_scales(CUtensorMap* map, const void* base, uint64_t k_ato
   return true;
 }
 
+// Matrix [rows, row_bytes] as {bytes, row % 32, row / 32} (rows % 32 == 0) with a box of 128 bytes of eight rows of
+// four 32-row groups, 128-byte swizzle.
+bool encode_tensor_map_piece(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t rows, std::string* error) {
+  auto fn = encode_fn();
+  if (fn == nullptr) {
+    if (error) *error = "cuTensorMapEncodeTiled is not available from this driver";
+    return false;
+  }
+  const cuuint64_t dims[3] = {row_bytes, 32, rows / 32};
+  const cuuint64_t strides[2] = {row_bytes, row_bytes * 32};
+  const cuuint32_t box[3] = {128, 8, 4};
+  const cuuint32_t element_strides[3] = {1, 1, 1};
+  const CUresult status = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, element_strides,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (status != CUDA_SUCCESS && error) *error = "cuTensorMapEncodeTiled (piece) failed with CUresult " + std::to_string(int(status));
+  return status == CUDA_SUCCESS;
+}
+
+// Tiled NVFP4 scale storage as {byte of the atom, atom} with a box of 128 bytes of four atoms.
+bool encode_tensor_map_atoms(CUtensorMap* map, const void* base, uint64_t atoms, std::string* error) {
+  auto fn = encode_fn();
+  if (fn == nullptr) {
+    if (error) *error = "cuTensorMapEncodeTiled is not available from this driver";
+    return false;
+  }
+  const cuuint64_t dims[2] = {512, atoms};
+  const cuuint64_t strides[1] = {512};
+  const cuuint32_t box[2] = {128, 4};
+  const cuuint32_t element_strides[2] = {1, 1};
+  const CUresult status = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, element_strides,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (status != CUDA_SUCCESS && error) *error = "cuTensorMapEncodeTiled (scale atoms) failed with CUresult " + std::to_string(int(status));
+  return status == CUDA_SUCCESS;
+}
+
 }  // namespace gw
