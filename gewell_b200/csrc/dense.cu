@@ -1,5 +1,6 @@
 #include "dense.h"
 #include "gemm_pair.h"
+#include "gemm_pair_wide.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -91,6 +92,44 @@ gw_status launch_dense_stream(const StreamProblem& q, DenseDescriptors* cache, c
   return GW_OK;
 }
 
+namespace {
+
+// FP8 and BF16 with more rows than the swap form takes: channels on the lanes of a CTA pair.
+gw_status launch_dense_pair_wide(const DenseProblem& q, uint64_t row_bytes, DenseDescriptors* cache, cudaStream_t stream) {
+  std::string error;
+  if (cache->token_tile == 0) cache->token_tile = pair_wide_tile_rows(q.rows, q.n, sm_count());
+  if (cache->weight_half != q.weight) {
+    if (!encode_tensor_map_2d(&cache->weight_half_map, q.weight, row_bytes, q.n, 128, &error))
+      return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
+    cache->weight_half = q.weight;
+  }
+  if (cache->activations != q.activations) {
+    if (!encode_tensor_map_2d(&cache->activation_map, q.activations, row_bytes, q.rows, uint32_t(cache->token_tile / 2), &error))
+      return fail(GW_CUDA_ERROR, "activation descriptor: " + error);
+    cache->activations = q.activations;
+  }
+  PairWideParams pair{};
+  pair.map_weights = cache->weight_half_map;
+  pair.map_tokens = cache->activation_map;
+  pair.k_stages = int32_t((row_bytes + 127) / 128);
+  pair.last_kb = int32_t((row_bytes - uint64_t(pair.k_stages - 1) * 128 + 31) / 32);
+  pair.rows = int32_t(q.rows);
+  pair.n = int32_t(q.n);
+  pair.channel_tiles = int32_t((q.n + 255) / 256);
+  pair.token_tiles = int32_t((q.rows + cache->token_tile - 1) / cache->token_tile);
+  pair.tile_rows = cache->token_tile;
+  pair.out = q.output;
+  pair.ld_out = q.n;
+  pair.alpha = q.alpha;
+  pair.channel_alpha = q.channel_alpha;
+  pair.error = q.error;
+  GW_CUDA_CHECK(launch_gemm_pair_wide(q.kind == GemmKind::fp8, pair, sm_count(), stream),
+                q.kind == GemmKind::fp8 ? "FP8 CTA-pair tensor-core GEMM" : "BF16 CTA-pair tensor-core GEMM");
+  return GW_OK;
+}
+
+}  // namespace
+
 gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
   const DenseTuning& tuning = cache->tuning;
   const bool swap = dense_uses_swap_form(tuning, q.rows);
@@ -98,6 +137,9 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
   const bool fp4 = q.kind == GemmKind::nvfp4;
   const uint64_t row_bytes = fp4 ? q.k / 2 : (q.kind == GemmKind::bf16 ? uint64_t(2) * q.k : q.k);
   std::string error;
+  // Outputs of these kinds are 16-byte aligned and a multiple of 8 wide (plan creation and the run check it).
+  if (!fp4 && !swap && tuning.form == 0 && tuning.block_n == 0 && !tuning.no_pair)
+    return launch_dense_pair_wide(q, row_bytes, cache, stream);
   const bool single_box = !swap && block_n == 256;   // both column halves come from the one weight matrix
   if (cache->weight != q.weight) {
     if (!encode_tensor_map_2d(&cache->weight_map, q.weight, row_bytes, q.n, single_box ? 256 : 128, &error))

@@ -12,7 +12,7 @@ namespace gw {
 // Tuning overrides of the dense projections, read from the environment once per plan (when its
 // descriptors are first used), not at every call:
 //   GW_DENSE_FORM=swap|direct, GW_DENSE_BLOCK_N=128|256   operand roles / column tile
-//   GW_DENSE_NO_PAIR=1    NVFP4 projections with >= 256 rows stay on the single-CTA kernel
+//   GW_DENSE_NO_PAIR=1    projections of many rows stay on the single-CTA kernel
 //   GW_DENSE_NO_SPLIT=1   decode-shaped plans run whole tiles per CTA
 // Each of them but the third also keeps small row counts off the weight-streaming kernel.
 struct DenseTuning {
@@ -31,6 +31,7 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   CUtensorMap weight_map{}, activation_map{}, weight_scale_map{};
   const void* weight_half = nullptr;
   CUtensorMap weight_half_map{};     // 128-row box over the weights (CTA-pair kernel: each CTA stages half a tile)
+  int token_tile = 0;                // FP8 / BF16 CTA-pair kernel: token columns per tile
   // Split mode: one arrival counter per weight tile, owned by the plan (device memory,
   // zeroed at creation; the kernel leaves every counter at zero again).
   int32_t* split_counters = nullptr;

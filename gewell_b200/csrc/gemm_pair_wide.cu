@@ -1,0 +1,306 @@
+// FP8 and BF16 prefill GEMM on CTA pairs (tcgen05 cta_group::2, kind::f8f6f4 / kind::f16) for sm_100a.
+//
+// What bounds it: the tensor pipe, if it can be fed.  A single CTA with a 128 x 256 tile brings 48 KB through
+// L2 -> shared memory for 512 cycles of MMA; two CTAs that share the token tile (each stages its own 128 weight rows
+// and half of the tokens, the pair's tensor cores read both halves) need 32 KB each.  Without block scales tensor
+// memory has room for two 256-column accumulators, so a tile's epilogue runs under the next tile's MMAs.  Channels
+// are on the lanes because their number is a multiple of 128 while the tokens are not: the column width of a tile
+// goes in steps of 32, so that 1025 tokens cost 1120 (5 x 224) and not 1280.
+// Measured (us, with the activation quantiser): FP8 2048x5376x43008 653 -> 341 (with half of the loads left out 301),
+// 1025x5376x16384 113 -> 81; BF16 4096x2816x4096 84 -> 68, 200x2816x8192 26.2 -> 15.3.
+//
+// Roles per CTA: warp 0 = producer (one lane), warp 1 = MMA issuer (one lane, only in the pair's leader), warps
+// 4..11 = epilogue.
+// Cross-CTA protocol (barriers at the same offsets in both CTAs):
+//   full[s]   in the leader; the operand tiles of both CTAs complete on it (the peer's copies into the peer's own
+//             shared memory may count there before the leader expects them: only its arrival closes the phase)
+//   empty[s], acc_full[a]   local; signalled in both CTAs at once by the leader's tcgen05.commit
+//   acc_empty[a]   in the leader, 16 arrivals (epilogue warps of both CTAs)
+// Every wait is bounded; the kernel ends with a cluster barrier before tensor memory is released.  No load fans
+// out to other CTAs.
+#include "common.cuh"
+#include "gemm_pair_wide.h"
+#include "pair.cuh"
+#include "ptx.cuh"
+
+namespace gw {
+namespace {
+
+using namespace pair;
+
+constexpr int kMaxStages = 12;
+constexpr int kWgtBytes = 128 * 128;
+constexpr int kEpilogueWarps = 8, kFirstEpilogueWarp = 4;
+constexpr int kThreads = 32 * (kFirstEpilogueWarp + kEpilogueWarps);
+constexpr int kAccCols = 256, kTmemCols = 512;
+constexpr int kRingBytes = 221 * 1024;
+constexpr int kSmemBytes = kRingBytes + 1024;
+constexpr int kGroupTiles = 8;                     // token tiles that are walked together
+constexpr uint32_t kDescHiSw128 = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);   // SBO 1024 B, version 1, SWIZZLE_128B
+
+__device__ __forceinline__ uint64_t make_desc(uint32_t lo16) { return (uint64_t(kDescHiSw128) << 32) | lo16; }
+
+// copy into this CTA's shared memory that completes on a barrier of the pair's leader
+__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, int32_t x, int32_t y, uint32_t leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(ptx::smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(leader_bar) : "memory");
+}
+
+template <bool FP8>
+__device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  if constexpr (FP8)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// Work item -> tile.  Eight token tiles at a time go through all channels, token tile fastest: the pairs that run
+// together (74) then read 8 token tiles and about 9 weight tiles, whatever the larger side of the problem is.
+struct Tile { int channel, token; };
+__device__ __forceinline__ Tile tile_of(const PairWideParams& p, int w) {
+  const int group = w / (kGroupTiles * p.channel_tiles);
+  const int rest = w - group * kGroupTiles * p.channel_tiles;
+  const int width = min(kGroupTiles, p.token_tiles - group * kGroupTiles);
+  return {rest / width, group * kGroupTiles + rest % width};
+}
+
+// 8 tokens of one channel per lane (w[i] = tokens 2i, 2i+1) -> 8 channels of one token per lane, inside groups of
+// eight lanes: afterwards lane j of a group holds token j of the group's eight channels.
+__device__ __forceinline__ void transpose_8x8(uint32_t* w, int lane) {
+  {
+    const bool hi = (lane & 4) != 0;
+    const uint32_t a = __shfl_xor_sync(0xffffffffu, hi ? w[0] : w[2], 4), b = __shfl_xor_sync(0xffffffffu, hi ? w[1] : w[3], 4);
+    if (hi) { w[0] = a; w[1] = b; } else { w[2] = a; w[3] = b; }
+  }
+  {
+    const bool hi = (lane & 2) != 0;
+    const uint32_t a = __shfl_xor_sync(0xffffffffu, hi ? w[0] : w[1], 2), b = __shfl_xor_sync(0xffffffffu, hi ? w[2] : w[3], 2);
+    if (hi) { w[0] = a; w[2] = b; } else { w[1] = a; w[3] = b; }
+  }
+  const bool odd = (lane & 1) != 0;
+  const uint32_t give = odd ? 0x5410u : 0x7632u;       // odd lanes give the first token of each pair, even ones the second
+  const uint32_t a = __shfl_xor_sync(0xffffffffu, __byte_perm(w[0], w[1], give), 1);
+  const uint32_t b = __shfl_xor_sync(0xffffffffu, __byte_perm(w[2], w[3], give), 1);
+  w[0] = odd ? __byte_perm(a, w[0], 0x7610u) : __byte_perm(w[0], a, 0x5410u);
+  w[1] = odd ? __byte_perm(a, w[1], 0x7632u) : __byte_perm(w[1], a, 0x7610u);
+  w[2] = odd ? __byte_perm(b, w[2], 0x7610u) : __byte_perm(w[2], b, 0x5410u);
+  w[3] = odd ? __byte_perm(b, w[3], 0x7632u) : __byte_perm(w[3], b, 0x7610u);
+}
+
+template <bool FP8>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_full_bar[2], acc_empty_bar[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int abort_flag;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
+  const uint32_t rank = cluster_rank();           // 0 = leader of the pair
+  griddep_launch();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kMaxStages; ++s) {
+      ptx::mbar_init(full_bar + s, 1);
+      ptx::mbar_init(empty_bar + s, 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      ptx::mbar_init(acc_full_bar + a, 1);
+      ptx::mbar_init(acc_empty_bar + a, 2 * kEpilogueWarps);
+    }
+    abort_flag = 0;
+    ptx::fence_barrier_init();
+    ptx::fence_proxy_async_smem();
+  }
+  if (warp == 1) {
+    tmem_alloc_pair(&tmem_slot, kTmemCols);
+    tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();                               // both CTAs' barriers exist before anybody signals them
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
+  griddep_wait();
+  const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
+  const int total_work = p.channel_tiles * p.token_tiles;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer (one lane)
+    if (ptx::elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      const int token_half = p.tile_rows / 2;
+      const uint32_t bytes = 2 * (kWgtBytes + uint32_t(token_half) * 128);      // of both CTAs
+      const uint32_t leader_full = leader_address(full_bar);
+      for (int w = pair; w < total_work && !abort_flag; w += pairs) {
+        const Tile tile = tile_of(p, w);
+        const int weight_row = (tile.channel * 2 + int(rank)) * 128;
+        const int token_row = tile.token * p.tile_rows + int(rank) * token_half;
+        bool failed = false;
+        for (int ks = 0; ks < p.k_stages; ++ks) {
+          if (!ptx::mbar_wait_bounded(empty_bar + stage, phase ^ 1)) {
+            report(p.error, 0x15000000u | (blockIdx.x << 8) | stage, &abort_flag);
+            failed = true;
+            break;
+          }
+          uint8_t* base = smem + stage * p.stage_bytes;
+          if (rank == 0) ptx::mbar_expect_tx(full_bar + stage, bytes);       // rows beyond a matrix arrive as zeros
+          tma_load_pair(base, &p.map_weights, ks * 128, weight_row, leader_full + stage * 8);
+          tma_load_pair(base + kWgtBytes, &p.map_tokens, ks * 128, token_row, leader_full + stage * 8);
+          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        }
+        if (failed) break;
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer (leader CTA, whole warp)
+    if (rank == 0) {
+      int stage = 0, turn = 0;
+      uint32_t phase = 0;
+      // FP32 accumulator, E4M3 or BF16 operands, M = 256 across the pair
+      const uint32_t idesc = (1u << 4) | (FP8 ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t(p.tile_rows) >> 3) << 17) | ((256u >> 4) << 24);
+      const uint32_t smem_base16 = ptx::smem_u32(smem) >> 4;
+      bool failed = false;
+      for (int w = pair; w < total_work && !failed; w += pairs, ++turn) {
+        const int acc = turn & 1;
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(acc_empty_bar + acc, (uint32_t(turn >> 1) & 1u) ^ 1u))) {
+          report(p.error, 0x25000000u | (blockIdx.x << 8) | acc, &abort_flag);
+          break;
+        }
+        ptx::tc_fence_after_sync();
+        const uint32_t d = tmem_base + acc * kAccCols;
+        for (int ks = 0; ks < p.k_stages; ++ks) {
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(full_bar + stage, phase))) {
+            report(p.error, 0x35000000u | (blockIdx.x << 8) | stage, &abort_flag);
+            failed = true;
+            break;
+          }
+          ptx::tc_fence_after_sync();
+          const uint32_t base16 = smem_base16 + uint32_t(stage) * (uint32_t(p.stage_bytes) >> 4);
+          if (ptx::elect_one()) {
+            const int nkb = ks + 1 == p.k_stages ? p.last_kb : 4;
+            const uint64_t a = make_desc(base16), b = make_desc(base16 + (kWgtBytes >> 4));
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb)
+              if (kb < nkb) mma_pair<FP8>(d, a + 2 * kb, b + 2 * kb, idesc, (ks | kb) != 0 ? 1u : 0u);
+            commit_pair(empty_bar + stage);
+          }
+          __syncwarp();
+          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        }
+        if (!failed && ptx::elect_one()) commit_pair(acc_full_bar + acc);;
+      }
+    }
+    __syncwarp();
+  } else if (warp >= kFirstEpilogueWarp) {
+    // ------------------------------------------------------------------ epilogue (own 128 channels x tile_rows tokens)
+    const int quad = warp % 4;
+    const int half = (warp - kFirstEpilogueWarp) / 4;            // takes every other 32-token chunk
+    const uint32_t leader_acc_empty = leader_address(acc_empty_bar);
+    bf16* out = static_cast<bf16*>(p.out);
+    int turn = 0;
+    for (int w = pair; w < total_work && !abort_flag; w += pairs, ++turn) {
+      const int acc = turn & 1;
+      const Tile tile = tile_of(p, w);
+      const int channel0 = (tile.channel * 2 + int(rank)) * 128 + quad * 32;
+      const float scale = p.channel_alpha == nullptr ? p.alpha : channel0 + lane < p.n ? __ldg(p.channel_alpha + channel0 + lane) : 0.0F;
+      if (!ptx::mbar_wait_warp(acc_full_bar + acc, uint32_t(turn >> 1) & 1u)) {
+        report(p.error, 0x45000000u | (blockIdx.x << 8) | acc, &abort_flag);
+        break;
+      }
+      ptx::tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + acc * kAccCols + (uint32_t(quad * 32) << 16);
+      const int c = channel0 + (lane & ~7);                         // n % 8 == 0: eight channels are inside or outside
+      for (int t0 = half * 32; t0 < p.tile_rows; t0 += 64) {
+        const int token0 = tile.token * p.tile_rows + t0;
+        if (token0 >= p.rows) break;                                // warp-uniform
+        uint32_t r[32];
+        ptx::tmem_load16(taddr + t0, r);
+        ptx::tmem_load16(taddr + t0 + 16, r + 16);
+        ptx::tmem_load_wait();
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint32_t v[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            v[i] = pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * g + 2 * i]), scale), __fmul_rn(__uint_as_float(r[8 * g + 2 * i + 1]), scale));
+          transpose_8x8(v, lane);
+          const int token = token0 + 8 * g + (lane & 7);
+          if (token < p.rows && c < p.n) *reinterpret_cast<uint4*>(out + size_t(token) * p.ld_out + c) = make_uint4(v[0], v[1], v[2], v[3]);
+        }
+      }
+      ptx::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) arrive_cluster(leader_acc_empty + acc * 8);
+    }
+  }
+
+  ptx::tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();                               // the peer no longer reads this CTA's shared or tensor memory
+  if (warp == 1) {
+    ptx::tc_fence_after_sync();
+    tmem_dealloc_pair(tmem_base, kTmemCols);
+  }
+}
+
+template <bool FP8>
+cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStream_t stream) {
+  static bool configured_on[kMaxDeviceSlots] = {};   // the attribute is per GPU
+  bool& configured = configured_on[current_device_slot()];
+  if (!configured) {
+    const cudaError_t status = cudaFuncSetAttribute(gemm_pair_wide_kernel<FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (status != cudaSuccess) return status;
+    configured = true;
+  }
+  const int work = params.channel_tiles * params.token_tiles;
+  const int pairs = work < sm_count / 2 ? work : sm_count / 2;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(2 * pairs);
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kSmemBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attributes[2]{};
+  attributes[0].id = cudaLaunchAttributeClusterDimension;
+  attributes[0].val.clusterDim.x = 2;
+  attributes[0].val.clusterDim.y = 1;
+  attributes[0].val.clusterDim.z = 1;
+  attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attributes[1].val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = attributes;
+  config.numAttrs = 2;
+  note_launch();
+  return cudaLaunchKernelEx(&config, gemm_pair_wide_kernel<FP8>, params);
+}
+
+}  // namespace
+
+int pair_wide_tile_rows(uint32_t rows, uint32_t n, int sm_count) {
+  // A tile takes as long as its weight rows and MMA issue cost whatever its width (about 136 columns) plus its columns:
+  // measured on FP8 K=5376, per wave of tiles of 64 / 128 / 192 / 256 tokens 8.9 / 11.3 / 14.3 / 17.4 us.
+  const uint64_t channel_tiles = (n + 255) / 256, pairs = uint64_t(sm_count / 2);
+  int best = 256;
+  uint64_t best_cost = ~0ull;
+  for (int tile = 256; tile >= 64; tile -= 32) {
+    const uint64_t tiles = channel_tiles * ((rows + tile - 1) / tile);
+    const uint64_t cost = (tiles + pairs - 1) / pairs * uint64_t(tile + 136);
+    if (cost < best_cost) { best_cost = cost; best = tile; }
+  }
+  return best;
+}
+
+cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& given, int sm_count, cudaStream_t stream) {
+  PairWideParams params = given;
+  params.stage_bytes = kWgtBytes + given.tile_rows * 64;
+  params.stages = kRingBytes / params.stage_bytes < kMaxStages ? kRingBytes / params.stage_bytes : kMaxStages;
+
+  return fp8 ? launch_instance<true>(params, sm_count, stream) : launch_instance<false>(params, sm_count, stream);
+}
+
+}  // namespace gw

@@ -1,0 +1,32 @@
+// Launch description of the CTA-pair prefill GEMM for FP8 and BF16 weights (gemm_pair_wide.cu):
+// Y[rows, n] = bf16(alpha * X . W^T), output channels on the lanes (256 per pair tile), tokens on the columns
+// (tile_rows per tile, half of them staged by each CTA of the pair).
+#pragma once
+
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <cstdint>
+
+namespace gw {
+
+struct PairWideParams {
+  CUtensorMap map_weights;         // weights [n, k], box 128 rows x 128 bytes, 128-byte swizzle
+  CUtensorMap map_tokens;          // activations [rows, k], box tile_rows / 2 rows
+  int32_t k_stages;                // 128-byte slabs of K
+  int32_t last_kb;                 // 32-byte K blocks in the last one
+  int32_t rows, n;
+  int32_t channel_tiles, token_tiles, tile_rows;
+  int32_t stages, stage_bytes;     // of the operand ring (set by the launch)
+  void* out;                       // BF16 [rows, ld_out], 16-byte aligned rows
+  int64_t ld_out;
+  float alpha;
+  const float* channel_alpha;      // optional multiplier per output channel instead of alpha
+  uint32_t* error;
+};
+
+// Tokens per tile for this shape: the number whose whole waves of pair tiles take least.
+int pair_wide_tile_rows(uint32_t rows, uint32_t n, int sm_count);
+
+cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& params, int sm_count, cudaStream_t stream);
+
+}  // namespace gw

@@ -51,16 +51,29 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return done != 0;
 }
 
+// One lane of a converged warp.  The single-lane roles branch on this and not on the lane number: the compiler then
+// knows that one thread runs the branch and keeps descriptors in uniform registers (four MMAs behind `lane == 0`
+// took 430 cycles to issue, whatever their width).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+
 // Wait for a phase with an upper bound: gives up after `limit_ns` of wall time
 // (checked every 256 polls) and returns false; the caller records the failure
 // and unwinds, so a protocol bug shows up as an error code instead of a hang.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   uint64_t limit_ns = 2000000000ull) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t start = global_timer_ns();
+  // the timer is read only after many polls
+  uint64_t start = 0;
   for (uint32_t spin = 1;; ++spin) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 255u) == 0 && global_timer_ns() - start > limit_ns) return false;
+    if ((spin & 255u) == 0) {
+      const uint64_t now = global_timer_ns();
+      if (start == 0) start = now;
+      else if (now - start > limit_ns) return false;
+    }
   }
 }
 
@@ -72,11 +85,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
   uint32_t ok = 1;
   if ((threadIdx.x & 31) == 0) {
     if (!mbar_try_wait(bar, parity)) {
-      const uint64_t start = global_timer_ns();
+      uint64_t start = 0;
       for (uint32_t spin = 1;; ++spin) {
         if (backoff_ns) __nanosleep(backoff_ns);
         if (mbar_try_wait(bar, parity)) break;
-        if ((spin & 63u) == 0 && global_timer_ns() - start > limit_ns) { ok = 0; break; }
+        if ((spin & 63u) == 0) {
+          const uint64_t now = global_timer_ns();
+          if (start == 0) start = now;
+          else if (now - start > limit_ns) { ok = 0; break; }
+        }
       }
     }
   }
