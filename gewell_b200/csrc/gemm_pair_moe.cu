@@ -163,7 +163,7 @@ pair_moe_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   WorkTable* table = reinterpret_cast<WorkTable*>(tmem_slot + 4);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
   const uint32_t rank = cluster_rank();           // 0 = leader of the pair
   griddep_launch();
   if (threadIdx.x == 0) {
@@ -187,7 +187,7 @@ pair_moe_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
   __syncthreads();
   cluster_sync_all();                               // both CTAs' barriers exist before anybody signals them
   ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_wait();                                   // the offsets and the quantised rows come from earlier kernels
   build_work_table(p, table, kCTiles);
 
@@ -197,7 +197,7 @@ pair_moe_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       Unit u{-1, 0, 0, 0, 0};
@@ -267,7 +267,7 @@ pair_moe_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA, one lane)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0, acc_phase = 0;
       const uint32_t idesc = idesc_pair_nvfp4(256);
@@ -563,7 +563,7 @@ pair_moe_down_kernel(const __grid_constant__ PairMoeParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   WorkTable* table = reinterpret_cast<WorkTable*>(tmem_slot + 4);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
   const uint32_t rank = cluster_rank();
   griddep_launch();
   if (threadIdx.x == 0) {
@@ -592,7 +592,7 @@ pair_moe_down_kernel(const __grid_constant__ PairMoeParams p) {
   __syncthreads();
   cluster_sync_all();
   ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_wait();
   build_work_table(p, table, kChunks);
 
@@ -601,7 +601,7 @@ pair_moe_down_kernel(const __grid_constant__ PairMoeParams p) {
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       // request the rows (and their scale atoms) of the unit with running number `number`
       auto request_rows = [&](int w, int number) -> bool {
         Unit v{-1, 0, 0, 0, 0};
@@ -668,7 +668,7 @@ pair_moe_down_kernel(const __grid_constant__ PairMoeParams p) {
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA, one lane)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && ptx::elect_one()) {
       int stage = 0, number = 0, tiles = 0;
       uint32_t phase = 0;
       const uint32_t idesc = idesc_pair_nvfp4(kTileCols);

@@ -174,7 +174,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   int32_t* prefix = reinterpret_cast<int32_t*>(tmem_slot + 4);   // work_begin of every group (+ sentinel)
   griddep_launch();
 
-  const int warp = threadIdx.x / 32;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0);
   const int lane = threadIdx.x % 32;
 
   if (threadIdx.x == 0) {
@@ -198,7 +198,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // Everything above is independent of earlier kernels in the stream and may overlap
   // them (programmatic dependent launch); from here on their results are read.
   const bool early_weights = EPI == GemmEpilogue::swap_store && p.groups == nullptr && p.early_weights != 0;
@@ -239,7 +239,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
     // ------------------------------------------------------------------ producer
     // One thread runs the whole role (no per-stage warp votes or shuffles); the other lanes
     // wait at the end of the branch.
-    if (lane == 0) {
+    if (ptx::elect_one()) {
     int stage = 0;
     uint32_t phase = 0;
     bool waited = !early_weights;        // this warp defers its wait for the previous kernel (see below)
@@ -334,12 +334,10 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
         // activations, so the first ring of weight copies is issued before waiting for it;
         // the token-side copies of those stages follow once it has finished.
         const int ahead = min(C::kStages, ks1 - ks0);
-        if (lane == 0)
-          for (int i = 0; i < ahead; ++i) issue(ks0 + i, i, true, false);
+        for (int i = 0; i < ahead; ++i) issue(ks0 + i, i, true, false);
         griddep_wait();
         waited = true;
-        if (lane == 0)
-          for (int i = 0; i < ahead; ++i) issue(ks0 + i, i, false, true);
+        for (int i = 0; i < ahead; ++i) issue(ks0 + i, i, false, true);
         stage = ahead == C::kStages ? 0 : ahead;
         phase = ahead == C::kStages ? 1 : 0;
         ks_begin = ks0 + ahead;
@@ -351,7 +349,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
           break;
         }
         if (prof) prof_wait += clock64() - t0;
-        if (lane == 0) issue(ks, stage, true, true);
+        issue(ks, stage, true, true);
         if (++stage == C::kStages) { stage = 0; phase ^= 1; }
       }
     }
@@ -360,7 +358,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (one thread, as above)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     WorkItem item, next;
@@ -405,7 +403,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
         const long long t1 = prof ? clock64() : 0;
         if (prof) prof_wait += t1 - t0;
         ptx::tc_fence_after_sync();
-        if (lane == 0) {
+        {
           // Single in-order instruction stream: descriptors are a constant plus
           // stage * (kStageBytes >> 4) in their low word, the loop is unrolled.
           const int nkb = min(kKbPerStage, total_kb - ks * kKbPerStage);
@@ -436,7 +434,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
         if (++stage == C::kStages) { stage = 0; phase ^= 1; }
       }
       if (failed) break;
-      if (lane == 0) ptx::tc_commit(acc_full_bar + acc);
+      ptx::tc_commit(acc_full_bar + acc);
       if (++acc == C::kAccStages) { acc = 0; acc_phase ^= 1; }
     }
     }
