@@ -13,10 +13,13 @@
 // squares by ascending i, a lane's total is ((a0 + a1) + a2) + a3, and lanes
 // fold in a halving tree.  `lanes` depends on the row count and the width.
 //
-// Here a row is read from HBM once (it stays in shared memory between the
-// reduction and the output), and the block's tail -- two post norms, add, the
-// third norm, residual add, layer scalar: seven launches in the reference --
-// is one kernel with one block per row.
+// Here a row is read from HBM once: every thread keeps its eight (or 16, 32) values and their weights in
+// registers between the reduction and the output, and the row sits in shared memory for the fixed-order sums
+// only.  What bounds these kernels at decode sizes is the chain of memory latency, barriers and adds, not
+// bytes: all loads of a thread are 16 bytes wide and issued before the first barrier (2816 wide, 8 rows, weights
+// not in L2: norm 16.9 -> 3.9 us, tail 18.8 -> 4.5 us, with the launch, against element-wise loads in the output loop and a
+// block barrier for every level of the sum).  The block's tail -- two post norms, add, the third norm, residual
+// add, layer scalar: seven launches in the reference -- is one kernel with one block per row.
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -31,7 +34,7 @@ using namespace gw;
 
 namespace {
 
-constexpr int kNormThreads = 256;
+constexpr int kNormThreads = 512;                // at most; a block has a thread for every eight values of a row
 constexpr float kRmsEpsilon = 1e-6F;   // include/gewell/models/gemma4/26b_a4b/model.h:26
 
 uint32_t floor_power_of_two(uint32_t value) {
@@ -52,42 +55,51 @@ uint32_t reduction_lanes(uint32_t rows, uint32_t width) {
 __device__ __forceinline__ float as_float(bf16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ bf16 rounded(float v) { return __float2bfloat16_rn(v); }
 
-// Copies one row of `width` BF16 values (width % 8 == 0, 16-byte aligned) into shared memory.
-__device__ __forceinline__ void stage_row(const bf16* __restrict__ source, bf16* row, uint32_t width) {
-  const uint4* in = reinterpret_cast<const uint4*>(source);
-  uint4* out = reinterpret_cast<uint4*>(row);
-  for (uint32_t i = threadIdx.x; i < width / 8; i += blockDim.x) out[i] = __ldg(in + i);
-}
-
-// 1 / sqrt(mean(row^2) + eps) of the row in shared memory, in the reference's order (see the head of
-// this file).  `partial` holds 5 * lanes floats.  Every thread returns the same value.  No fused
-// multiply-add anywhere: the reference's translation unit is built with --fmad=false.
-__device__ float inverse_rms(const bf16* row, uint32_t width, uint32_t lanes, float inverse_width, float* partial) {
-  __syncthreads();                                     // the row is complete; `partial` is free
-  const uint32_t accumulators = 4 * lanes;
-  for (uint32_t p = threadIdx.x; p < accumulators; p += blockDim.x) {
-    float sum = 0.F;
-    for (uint32_t i = p; i < width; i += accumulators) {
-      const float v = as_float(row[i]);
-      sum = __fadd_rn(sum, __fmul_rn(v, v));
+// Eight BF16 values as a thread loads and keeps them; thread t has vectors t, t + blockDim.x, ... of a row.
+union Vec {
+  uint4 bits;
+  bf16 v[8];
+};
+template <int NV>
+struct RowPart {
+  Vec part[NV];
+  __device__ __forceinline__ void load(const bf16* __restrict__ row, uint32_t vectors) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const uint32_t i = threadIdx.x + j * blockDim.x;
+      part[j].bits = i < vectors ? *(reinterpret_cast<const uint4*>(row) + i) : make_uint4(0, 0, 0, 0);
     }
-    partial[p] = sum;
   }
-  __syncthreads();
-  float* totals = partial + accumulators;            // lane totals live beside the accumulators
-  for (uint32_t lane = threadIdx.x; lane < lanes; lane += blockDim.x) {
-    const float4 a = reinterpret_cast<const float4*>(partial)[lane];
-    totals[lane] = __fadd_rn(__fadd_rn(__fadd_rn(a.x, a.y), a.z), a.w);
+  // 16-bit loads for a row that is not 16-byte aligned (a weight vector inside a larger buffer)
+  __device__ __forceinline__ void load_any(const bf16* __restrict__ row, uint32_t vectors) {
+    if (reinterpret_cast<uintptr_t>(row) % 16 == 0) return load(row, vectors);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const uint32_t i = threadIdx.x + j * blockDim.x;
+      part[j].bits = make_uint4(0, 0, 0, 0);
+      if (i < vectors)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) part[j].v[e] = row[size_t(i) * 8 + e];
+    }
   }
-  __syncthreads();
-  for (uint32_t stride = lanes / 2; stride; stride /= 2) {
-    for (uint32_t lane = threadIdx.x; lane < stride; lane += blockDim.x)
-      totals[lane] = __fadd_rn(totals[lane], totals[lane + stride]);
-    __syncthreads();
+  __device__ __forceinline__ void store(bf16* row, uint32_t vectors) const {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const uint32_t i = threadIdx.x + j * blockDim.x;
+      if (i < vectors) *(reinterpret_cast<uint4*>(row) + i) = part[j].bits;
+    }
   }
-  const float mean = __fadd_rn(__fmul_rn(totals[0], inverse_width), kRmsEpsilon);
-  return rsqrtf(mean);
-}
+  __device__ __forceinline__ void store_any(bf16* row, uint32_t vectors) const {
+    if (reinterpret_cast<uintptr_t>(row) % 16 == 0) return store(row, vectors);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const uint32_t i = threadIdx.x + j * blockDim.x;
+      if (i < vectors)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) row[size_t(i) * 8 + e] = part[j].v[e];
+    }
+  }
+};
 
 struct NormArgs {
   const bf16* input;
@@ -95,19 +107,73 @@ struct NormArgs {
   float inverse_width;
 };
 
+// 1 / sqrt(mean(row^2) + eps) of ROWS rows in shared memory, in the reference's order (see the head of this file).
+// A thread takes whole logical lanes (four accumulators, eight bytes a step); warp r folds the lane totals of row r,
+// the levels inside a warp by shuffles.  `totals` holds ROWS * lanes floats.  Every thread gets the results.  No
+// fused multiply-add anywhere: the reference's translation unit is built with --fmad=false.
+template <int ROWS>
+__device__ __forceinline__ void inverse_rms(const NormArgs& a, const bf16* const (&rows)[ROWS], float* totals, float (&inverse)[ROWS]) {
+  __shared__ float result[ROWS];
+  __syncthreads();                                     // the rows are complete; `totals` is free
+  const uint32_t lanes = a.lanes;                      // a power of two; 4 * lanes <= width
+  for (uint32_t item = threadIdx.x; item < ROWS * lanes; item += blockDim.x) {
+    const uint32_t which = ROWS == 1 ? 0 : item / lanes, l = ROWS == 1 ? item : item % lanes;
+    const bf16* row = rows[0];
+#pragma unroll
+    for (int r = 1; r < ROWS; ++r)
+      if (which == r) row = rows[r];
+    float sum[4] = {0.F, 0.F, 0.F, 0.F};
+#pragma unroll 4
+    for (uint32_t i = 4 * l; i < a.width; i += 4 * lanes) {
+      const uint2 bits = *reinterpret_cast<const uint2*>(row + i);
+      const float v[4] = {bf16_bits_to_float(bits.x & 0xffff), bf16_bits_to_float(bits.x >> 16), bf16_bits_to_float(bits.y & 0xffff),
+                          bf16_bits_to_float(bits.y >> 16)};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) sum[e] = __fadd_rn(sum[e], __fmul_rn(v[e], v[e]));
+    }
+    totals[item] = __fadd_rn(__fadd_rn(__fadd_rn(sum[0], sum[1]), sum[2]), sum[3]);
+  }
+  __syncthreads();
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, warps = blockDim.x / 32;
+  for (uint32_t r = warp; r < uint32_t(ROWS); r += warps) {
+    float* mine = totals + r * lanes;
+    for (uint32_t stride = lanes / 2; stride >= 32; stride /= 2) {
+      for (uint32_t l = lane; l < stride; l += 32) mine[l] = __fadd_rn(mine[l], mine[l + stride]);
+      __syncwarp();
+    }
+    float sum = lane < lanes ? mine[lane] : 0.F;
+    for (uint32_t stride = (lanes < 32 ? lanes : 32) / 2; stride; stride /= 2)
+      sum = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, stride));
+    if (lane == 0) result[r] = rsqrtf(__fadd_rn(__fmul_rn(sum, a.inverse_width), kRmsEpsilon));
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) inverse[r] = result[r];
+}
+
 // y = bf16(x * inv * w)   (w == nullptr: no weight)       -- NormOutput, bf16_math.cuh:18-24
-__global__ void __launch_bounds__(kNormThreads) rms_norm_kernel(NormArgs a, const bf16* __restrict__ weight,
-                                                               bf16* __restrict__ output) {
+template <int NV>
+__global__ void __launch_bounds__(kNormThreads) rms_norm_kernel(NormArgs a, const bf16* __restrict__ weight, bf16* __restrict__ output) {
   extern __shared__ __align__(16) unsigned char norm_smem[];
   bf16* row = reinterpret_cast<bf16*>(norm_smem);
-  float* partial = reinterpret_cast<float*>(norm_smem + size_t(a.width) * sizeof(bf16));
-  stage_row(a.input + size_t(blockIdx.x) * a.width, row, a.width);
-  const float inv = inverse_rms(row, a.width, a.lanes, a.inverse_width, partial);
-  bf16* out = output + size_t(blockIdx.x) * a.width;
-  for (uint32_t i = threadIdx.x; i < a.width; i += blockDim.x) {
-    const float x = __fmul_rn(as_float(row[i]), inv);
-    out[i] = rounded(weight ? __fmul_rn(x, as_float(weight[i])) : x);
-  }
+  float* totals = reinterpret_cast<float*>(norm_smem + size_t(a.width) * sizeof(bf16));
+  const uint32_t vectors = a.width / 8;
+  griddep_launch();
+  RowPart<NV> x, w;
+  if (weight) w.load_any(weight, vectors);
+  griddep_wait();
+  x.load(a.input + size_t(blockIdx.x) * a.width, vectors);
+  x.store(row, vectors);
+  float inv[1];
+  inverse_rms<1>(a, {row}, totals, inv);
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float v = __fmul_rn(as_float(x.part[j].v[e]), inv[0]);
+      x.part[j].v[e] = rounded(weight ? __fmul_rn(v, as_float(w.part[j].v[e])) : v);
+    }
+  x.store_any(output + size_t(blockIdx.x) * a.width, vectors);
 }
 
 struct FeedForwardNormArgs {
@@ -118,20 +184,36 @@ struct FeedForwardNormArgs {
 
 // FeedForwardNormOutput (bf16_math.cuh:25-37): one RMS, three outputs; the router input keeps its three
 // separate roundings (unweighted norm, weighted product, final scale).
+template <int NV>
 __global__ void __launch_bounds__(kNormThreads) rms_norm_feedforward_kernel(NormArgs a, FeedForwardNormArgs f) {
   extern __shared__ __align__(16) unsigned char norm_smem[];
   bf16* row = reinterpret_cast<bf16*>(norm_smem);
-  float* partial = reinterpret_cast<float*>(norm_smem + size_t(a.width) * sizeof(bf16));
-  stage_row(a.input + size_t(blockIdx.x) * a.width, row, a.width);
-  const float inv = inverse_rms(row, a.width, a.lanes, a.inverse_width, partial);
+  float* totals = reinterpret_cast<float*>(norm_smem + size_t(a.width) * sizeof(bf16));
+  const uint32_t vectors = a.width / 8;
+  griddep_launch();
+  RowPart<NV> x, shared, expert, router;
+  shared.load_any(f.shared_weight, vectors);
+  expert.load_any(f.expert_weight, vectors);
+  router.load_any(f.router_weight, vectors);
+  griddep_wait();
+  x.load(a.input + size_t(blockIdx.x) * a.width, vectors);
+  x.store(row, vectors);
+  float inv[1];
+  inverse_rms<1>(a, {row}, totals, inv);
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float v = __fmul_rn(as_float(x.part[j].v[e]), inv[0]);
+      shared.part[j].v[e] = rounded(__fmul_rn(v, as_float(shared.part[j].v[e])));
+      expert.part[j].v[e] = rounded(__fmul_rn(v, as_float(expert.part[j].v[e])));
+      const bf16 weighted = rounded(__fmul_rn(as_float(rounded(v)), as_float(router.part[j].v[e])));
+      router.part[j].v[e] = rounded(__fmul_rn(as_float(weighted), f.router_scale));
+    }
   const size_t base = size_t(blockIdx.x) * a.width;
-  for (uint32_t i = threadIdx.x; i < a.width; i += blockDim.x) {
-    const float x = __fmul_rn(as_float(row[i]), inv);
-    f.shared[base + i] = rounded(__fmul_rn(x, as_float(f.shared_weight[i])));
-    f.expert[base + i] = rounded(__fmul_rn(x, as_float(f.expert_weight[i])));
-    const bf16 weighted = rounded(__fmul_rn(as_float(rounded(x)), as_float(f.router_weight[i])));
-    f.router[base + i] = rounded(__fmul_rn(as_float(weighted), f.router_scale));
-  }
+  shared.store_any(f.shared + base, vectors);
+  expert.store_any(f.expert + base, vectors);
+  router.store_any(f.router + base, vectors);
 }
 
 struct TailArgs {
@@ -143,40 +225,84 @@ struct TailArgs {
 
 // shared = norm1(shared_mlp); branch = norm2(routed); sum = bf16(shared + branch); branch = norm3(sum);
 // hidden = bf16(hidden + branch); hidden = bf16(hidden * scalar)        (batched_executor.cu:260,278-285)
+template <int NV>
 __global__ void __launch_bounds__(kNormThreads) ffn_tail_kernel(NormArgs a, TailArgs t) {
   extern __shared__ __align__(16) unsigned char norm_smem[];
   bf16* first = reinterpret_cast<bf16*>(norm_smem);
   bf16* second = first + a.width;
-  float* partial = reinterpret_cast<float*>(norm_smem + size_t(2) * a.width * sizeof(bf16));
+  float* totals = reinterpret_cast<float*>(norm_smem + size_t(2) * a.width * sizeof(bf16));
   const size_t base = size_t(blockIdx.x) * a.width;
-  stage_row(t.shared_mlp + base, first, a.width);
-  stage_row(t.routed + base, second, a.width);
-  const float inv_shared = inverse_rms(first, a.width, a.lanes, a.inverse_width, partial);
-  const float inv_routed = inverse_rms(second, a.width, a.lanes, a.inverse_width, partial);
-  for (uint32_t i = threadIdx.x; i < a.width; i += blockDim.x) {
-    const bf16 shared = rounded(__fmul_rn(__fmul_rn(as_float(first[i]), inv_shared), as_float(t.norm_shared[i])));
-    const bf16 branch = rounded(__fmul_rn(__fmul_rn(as_float(second[i]), inv_routed), as_float(t.norm_routed[i])));
-    first[i] = rounded(__fadd_rn(as_float(shared), as_float(branch)));
-  }
-  const float inv_sum = inverse_rms(first, a.width, a.lanes, a.inverse_width, partial);
+  const uint32_t vectors = a.width / 8;
+  griddep_launch();
+  RowPart<NV> shared, branch, norm_shared, norm_routed, norm_sum, hidden;
+  norm_shared.load_any(t.norm_shared, vectors);
+  norm_routed.load_any(t.norm_routed, vectors);
+  norm_sum.load_any(t.norm_sum, vectors);
   const float scalar = as_float(*t.layer_scalar);
-  for (uint32_t i = threadIdx.x; i < a.width; i += blockDim.x) {
-    const bf16 branch = rounded(__fmul_rn(__fmul_rn(as_float(first[i]), inv_sum), as_float(t.norm_sum[i])));
-    const bf16 updated = rounded(__fadd_rn(as_float(t.hidden[base + i]), as_float(branch)));
-    t.hidden[base + i] = rounded(__fmul_rn(as_float(updated), scalar));
-  }
+  griddep_wait();
+  shared.load(t.shared_mlp + base, vectors);
+  branch.load(t.routed + base, vectors);
+  hidden.load_any(t.hidden + base, vectors);
+  shared.store(first, vectors);
+  branch.store(second, vectors);
+  float inv[2], inv_sum[1];
+  inverse_rms<2>(a, {first, second}, totals, inv);
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const bf16 x = rounded(__fmul_rn(__fmul_rn(as_float(shared.part[j].v[e]), inv[0]), as_float(norm_shared.part[j].v[e])));
+      const bf16 y = rounded(__fmul_rn(__fmul_rn(as_float(branch.part[j].v[e]), inv[1]), as_float(norm_routed.part[j].v[e])));
+      shared.part[j].v[e] = rounded(__fadd_rn(as_float(x), as_float(y)));
+    }
+  shared.store(first, vectors);
+  inverse_rms<1>(a, {first}, totals, inv_sum);
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const bf16 x = rounded(__fmul_rn(__fmul_rn(as_float(shared.part[j].v[e]), inv_sum[0]), as_float(norm_sum.part[j].v[e])));
+      const bf16 updated = rounded(__fadd_rn(as_float(hidden.part[j].v[e]), as_float(x)));
+      hidden.part[j].v[e] = rounded(__fmul_rn(as_float(updated), scalar));
+    }
+  hidden.store_any(t.hidden + base, vectors);
 }
 
 // y = bf16(a + b)                                                       (bf16_math.cuh:109-112)
-__global__ void add_kernel(const bf16* __restrict__ a, const bf16* __restrict__ b, bf16* __restrict__ y, size_t n) {
-  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) y[i] = rounded(__fadd_rn(as_float(a[i]), as_float(b[i])));
+// VECTOR: every buffer 16-byte aligned, a thread has eight values
+template <bool VECTOR>
+__global__ void add_kernel(const bf16* a, const bf16* b, bf16* y, size_t n) {
+  griddep_launch();
+  griddep_wait();
+  const size_t i = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * (VECTOR ? 8 : 1);
+  if (VECTOR && i + 8 <= n) {
+    Vec u, v;
+    u.bits = *reinterpret_cast<const uint4*>(a + i);
+    v.bits = *reinterpret_cast<const uint4*>(b + i);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) u.v[e] = rounded(__fadd_rn(as_float(u.v[e]), as_float(v.v[e])));
+    *reinterpret_cast<uint4*>(y + i) = u.bits;
+  } else {
+    for (size_t j = i; j < n && j < i + (VECTOR ? 8 : 1); ++j) y[j] = rounded(__fadd_rn(as_float(a[j]), as_float(b[j])));
+  }
 }
 
 // x = bf16(x * scalar[0])                                               (batched_executor.cu:30-33)
-__global__ void scale_kernel(bf16* __restrict__ x, const bf16* __restrict__ scalar, size_t n) {
-  const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) x[i] = rounded(__fmul_rn(as_float(x[i]), as_float(*scalar)));
+template <bool VECTOR>
+__global__ void scale_kernel(bf16* x, const bf16* scalar, size_t n) {
+  griddep_launch();
+  griddep_wait();
+  const float s = as_float(*scalar);
+  const size_t i = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * (VECTOR ? 8 : 1);
+  if (VECTOR && i + 8 <= n) {
+    Vec u;
+    u.bits = *reinterpret_cast<const uint4*>(x + i);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) u.v[e] = rounded(__fmul_rn(as_float(u.v[e]), s));
+    *reinterpret_cast<uint4*>(x + i) = u.bits;
+  } else {
+    for (size_t j = i; j < n && j < i + (VECTOR ? 8 : 1); ++j) x[j] = rounded(__fmul_rn(as_float(x[j]), s));
+  }
 }
 
 __global__ void rsqrt_kernel(const float* in, float* out, uint32_t n) {
@@ -197,7 +323,17 @@ NormArgs norm_args(const void* input, uint32_t rows, uint32_t width) {
 }
 
 size_t norm_shared_bytes(uint32_t width, uint32_t lanes, int staged_rows) {
-  return size_t(staged_rows) * width * sizeof(bf16) + size_t(5) * lanes * sizeof(float);
+  return size_t(staged_rows) * (width * sizeof(bf16) + lanes * sizeof(float));
+}
+
+// A thread for every eight values of a row up to 512, then two or four vectors a thread.
+uint32_t norm_vectors(uint32_t width) {
+  const uint32_t per_thread = (width / 8 + kNormThreads - 1) / kNormThreads;
+  return per_thread <= 2 ? per_thread : 4;
+}
+uint32_t norm_threads(uint32_t width) {
+  const uint32_t nv = norm_vectors(width);
+  return ((width / 8 + nv - 1) / nv + 31) / 32 * 32;
 }
 
 struct DeviceBuffer {
@@ -239,10 +375,11 @@ gw_status gw_rms_norm_bf16(const void* input_bf16, const void* weight_bf16, void
   if (!input_bf16 || !output_bf16 || !aligned16(input_bf16))
     return fail(GW_INVALID_ARGUMENT, "RMS norm requires a 16-byte aligned input and an output");
   const NormArgs a = norm_args(input_bf16, rows, width);
-  rms_norm_kernel<<<rows, kNormThreads, norm_shared_bytes(width, a.lanes, 1), as_stream(stream)>>>(
-      a, static_cast<const bf16*>(weight_bf16), static_cast<bf16*>(output_bf16));
-  note_launch();
-  GW_CUDA_CHECK(cudaGetLastError(), "RMS norm");
+  const uint32_t nv = norm_vectors(width);
+  GW_CUDA_CHECK(launch_pdl_shared(nv == 1 ? rms_norm_kernel<1> : nv == 2 ? rms_norm_kernel<2> : rms_norm_kernel<4>, rows, norm_threads(width),
+                                  norm_shared_bytes(width, a.lanes, 1), as_stream(stream), a, static_cast<const bf16*>(weight_bf16),
+                                  static_cast<bf16*>(output_bf16)),
+                "RMS norm");
   return GW_OK;
 }
 
@@ -260,9 +397,12 @@ gw_status gw_rms_norm_feedforward_bf16(const void* input_bf16, const void* share
                               static_cast<const bf16*>(expert_weight), static_cast<bf16*>(shared_bf16),
                               static_cast<bf16*>(router_bf16), static_cast<bf16*>(expert_bf16),
                               1.F / std::sqrt(float(width))};
-  rms_norm_feedforward_kernel<<<rows, kNormThreads, norm_shared_bytes(width, a.lanes, 1), as_stream(stream)>>>(a, f);
-  note_launch();
-  GW_CUDA_CHECK(cudaGetLastError(), "feed-forward norm");
+  const uint32_t nv = norm_vectors(width);
+  GW_CUDA_CHECK(launch_pdl_shared(nv == 1   ? rms_norm_feedforward_kernel<1>
+                                  : nv == 2 ? rms_norm_feedforward_kernel<2>
+                                            : rms_norm_feedforward_kernel<4>,
+                                  rows, norm_threads(width), norm_shared_bytes(width, a.lanes, 1), as_stream(stream), a, f),
+                "feed-forward norm");
   return GW_OK;
 }
 
@@ -282,15 +422,15 @@ gw_status gw_ffn_tail_bf16(const void* shared_mlp_bf16, const void* routed_bf16,
                    static_cast<const bf16*>(norm_sum_weight), static_cast<const bf16*>(layer_scalar_bf16),
                    static_cast<bf16*>(hidden_bf16)};
   const size_t shared_bytes = norm_shared_bytes(width, a.lanes, 2);
+  const uint32_t nv = norm_vectors(width);
+  const auto kernel = nv == 1 ? ffn_tail_kernel<1> : nv == 2 ? ffn_tail_kernel<2> : ffn_tail_kernel<4>;
   static bool raised[kMaxDeviceSlots] = {};
-  if (shared_bytes > 48 * 1024 && !raised[current_device_slot()]) {
-    GW_CUDA_CHECK(cudaFuncSetAttribute(ffn_tail_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024),
+  if (shared_bytes > 48 * 1024 && !raised[current_device_slot()]) {   // only rows of more than 12000 values: four vectors a thread
+    GW_CUDA_CHECK(cudaFuncSetAttribute(ffn_tail_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024),
                   "feed-forward tail shared memory");
     raised[current_device_slot()] = true;
   }
-  ffn_tail_kernel<<<rows, kNormThreads, shared_bytes, as_stream(stream)>>>(a, t);
-  note_launch();
-  GW_CUDA_CHECK(cudaGetLastError(), "feed-forward tail");
+  GW_CUDA_CHECK(launch_pdl_shared(kernel, rows, norm_threads(width), shared_bytes, as_stream(stream), a, t), "feed-forward tail");
   return GW_OK;
 }
 
@@ -298,10 +438,11 @@ gw_status gw_add_bf16(const void* a_bf16, const void* b_bf16, void* output_bf16,
   clear_error();
   if (count == 0) return GW_OK;
   if (!a_bf16 || !b_bf16 || !output_bf16) return fail(GW_INVALID_ARGUMENT, "add requires three buffers");
-  add_kernel<<<unsigned((count + 255) / 256), 256, 0, as_stream(stream)>>>(
-      static_cast<const bf16*>(a_bf16), static_cast<const bf16*>(b_bf16), static_cast<bf16*>(output_bf16), count);
-  note_launch();
-  GW_CUDA_CHECK(cudaGetLastError(), "add");
+  const bool vector = aligned16(a_bf16) && aligned16(b_bf16) && aligned16(output_bf16);
+  const uint64_t per_block = vector ? 2048 : 256;
+  GW_CUDA_CHECK(launch_pdl(vector ? add_kernel<true> : add_kernel<false>, unsigned((count + per_block - 1) / per_block), 256, as_stream(stream),
+                           static_cast<const bf16*>(a_bf16), static_cast<const bf16*>(b_bf16), static_cast<bf16*>(output_bf16), size_t(count)),
+                "add");
   return GW_OK;
 }
 
@@ -309,10 +450,11 @@ gw_status gw_scale_bf16(void* values_bf16, const void* scalar_bf16, uint64_t cou
   clear_error();
   if (count == 0) return GW_OK;
   if (!values_bf16 || !scalar_bf16) return fail(GW_INVALID_ARGUMENT, "scale requires values and a device scalar");
-  scale_kernel<<<unsigned((count + 255) / 256), 256, 0, as_stream(stream)>>>(static_cast<bf16*>(values_bf16),
-                                                                            static_cast<const bf16*>(scalar_bf16), count);
-  note_launch();
-  GW_CUDA_CHECK(cudaGetLastError(), "scale");
+  const bool vector = aligned16(values_bf16);
+  const uint64_t per_block = vector ? 2048 : 256;
+  GW_CUDA_CHECK(launch_pdl(vector ? scale_kernel<true> : scale_kernel<false>, unsigned((count + per_block - 1) / per_block), 256, as_stream(stream),
+                           static_cast<bf16*>(values_bf16), static_cast<const bf16*>(scalar_bf16), size_t(count)),
+                "scale");
   return GW_OK;
 }
 
