@@ -42,7 +42,7 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float* out) {
 // kernel (models/gemma4/26b_a4b/sm120/moe.cu:104-157), so ids and FP32 weights match it bit for bit.
 __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales,
                                             uint32_t row, uint32_t local, unsigned lane, int32_t* __restrict__ keys,
-                                            float* __restrict__ weights, uint32_t (*bitmap)[2]) {
+                                            float* __restrict__ weights, uint32_t (*bitmap)[2], int32_t* shared_keys) {
   // Softmax over the token's 128 logits; this lane owns experts lane, lane + 32, lane + 64, lane + 96.
   // The FP32 additions keep the order the reference's weights depend on: the lane's four terms in
   // ascending expert order first, then the xor butterfly 16, 8, 4, 2, 1 over the lanes.
@@ -64,51 +64,43 @@ __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, con
   }
 #pragma unroll
   for (int step = 16; step > 0; step >>= 1) denominator += __shfl_xor_sync(0xffffffffu, denominator, step);
-  // Eight winners, one 64-bit maximum per round: the probability's bit pattern (probabilities are
-  // not negative, so their patterns order like unsigned integers) in the high word and 128 - id
-  // in the low word, so that the larger probability wins and, among equal ones, the smaller id.
-  // A candidate that has won is replaced by key 0, below every live key.
-  unsigned long long candidate[4];
+  // Eight winners, two hardware maxima a round: the largest probability (probabilities are not negative, so their bit
+  // patterns order like unsigned integers), then the smallest id among those that have it.  A candidate that has won
+  // drops to pattern 0, and its id out of the running.  Lane r keeps round r's winner.  The rounds stay a loop: decode
+  // steps run this code cold, and unrolled it was fetched from memory for longer than it ran (route of 64 tokens 18 us).
+  uint32_t pattern[4];
+  uint32_t live = 0xF;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    prob[q] = __fdiv_rn(prob[q], denominator);
-    candidate[q] = (static_cast<unsigned long long>(__float_as_uint(prob[q])) << 32) | uint32_t(kExperts - (lane + 32 * q));
-  }
-  int ids[kTopK];
-  float chosen[kTopK];
+  for (int q = 0; q < 4; ++q) pattern[q] = __float_as_uint(__fdiv_rn(prob[q], denominator));
+  int my_id = 0;
+  float my_p = 0.0F;
+#pragma unroll 1
+  for (unsigned round = 0; round < unsigned(kTopK); ++round) {
+    uint32_t best = 0;
 #pragma unroll
-  for (int round = 0; round < kTopK; ++round) {
-    unsigned long long winner = candidate[0];
+    for (int q = 0; q < 4; ++q) best = (live >> q & 1u) ? max(best, pattern[q]) : best;
+    best = __reduce_max_sync(0xffffffffu, best);
+    uint32_t id = kExperts;
 #pragma unroll
-    for (int q = 1; q < 4; ++q) winner = candidate[q] > winner ? candidate[q] : winner;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-      const unsigned long long theirs = __shfl_xor_sync(0xffffffffu, winner, step);
-      winner = theirs > winner ? theirs : winner;
-    }
-    const int id = kExperts - int(uint32_t(winner));
-    ids[round] = id;
-    chosen[round] = __uint_as_float(uint32_t(winner >> 32));
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (id == int(lane) + 32 * q) candidate[q] = 0;
+    for (int q = 3; q >= 0; --q)
+      if ((live >> q & 1u) && pattern[q] == best) id = lane + 32 * q;
+    id = __reduce_min_sync(0xffffffffu, id);
+    if (id % 32 == lane) live &= ~(1u << (id / 32));
+    if (lane == round) { my_id = int(id); my_p = __uint_as_float(best); }
   }
   // renormalisation: ((p0+p4)+(p2+p6)) + ((p1+p5)+(p3+p7)), the pairwise order of a stride-4/2/1 fold
-  float fold[4];
+  float sum = my_p + __shfl_down_sync(0xffffffffu, my_p, 4);
+  sum += __shfl_down_sync(0xffffffffu, sum, 2);
+  sum += __shfl_down_sync(0xffffffffu, sum, 1);
+  sum = __shfl_sync(0xffffffffu, sum, 0);
+  int rank = 0;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) fold[q] = chosen[q] + chosen[q + 4];
-  const float sum = (fold[0] + fold[2]) + (fold[1] + fold[3]);
-  int my_id = 0;
-  float my_p = 0;
-#pragma unroll
-  for (int i = 0; i < kTopK; ++i) if (lane == unsigned(i)) { my_id = ids[i]; my_p = chosen[i]; }
-  if (lane < kTopK) {
-    int rank = 0;
-#pragma unroll
-    for (int i = 0; i < kTopK; ++i) rank += ids[i] < my_id;
+  for (int i = 0; i < kTopK; ++i) rank += __shfl_sync(0xffffffffu, my_id, i) < my_id;
+  if (lane < unsigned(kTopK)) {
     const float weight = __fmul_rn(__fdiv_rn(my_p, sum), __bfloat162float(expert_scales[my_id]));
     keys[size_t(row) * kTopK + rank] = my_id;
     weights[size_t(row) * kTopK + rank] = weight;
+    if (shared_keys != nullptr) shared_keys[local * kTopK + rank] = my_id;
     atomicOr(&bitmap[my_id][local / 32], 1u << (local % 32));
   }
 }
@@ -137,11 +129,13 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
   __syncthreads();
   const uint32_t chunk = blockIdx.x;
   const int tokens_per_warp = kChunkTokens / int(blockDim.x / 32);     // 8 warps: 8 tokens each; 32 warps: 2
+  __shared__ int32_t shared_keys[kChunkTokens * kTopK];
+#pragma unroll 1
   for (int t = 0; t < tokens_per_warp; ++t) {
-    const uint32_t local = warp * tokens_per_warp + t;
+    const uint32_t local = warp + t * (blockDim.x / 32);
     const uint32_t row = chunk * kChunkTokens + local;
     if (row >= rows) break;
-    route_token(scores, expert_scales, row, local, lane, keys, weights, bitmap);
+    route_token(scores, expert_scales, row, local, lane, keys, weights, bitmap, shared_keys);
   }
   __syncthreads();
   if (threadIdx.x < kExperts) {
@@ -176,12 +170,10 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
     }
     if (lane == 31) offsets[kExperts] = acc;
   }
-  __syncthreads();                       // also orders this block's writes of `keys` before the reads below
-  for (uint32_t i = threadIdx.x; i < kChunkTokens * kTopK; i += blockDim.x) {
-    const uint32_t local = i / kTopK;
-    if (local >= rows) continue;
-    const uint32_t assignment = local * kTopK + i % kTopK;
-    const int32_t e = keys[assignment];
+  __syncthreads();
+  for (uint32_t assignment = threadIdx.x; assignment < rows * kTopK; assignment += blockDim.x) {
+    const uint32_t local = assignment / kTopK;
+    const int32_t e = shared_keys[assignment];
     const uint32_t w0 = bitmap[e][0], w1 = bitmap[e][1];
     const int rank = local < 32 ? __popc(w0 & ((1u << local) - 1u))
                                 : __popc(w0) + __popc(w1 & ((1u << (local - 32)) - 1u));
@@ -255,11 +247,11 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
   for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
     if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
     __syncthreads();
-#pragma unroll
+#pragma unroll 1
     for (int t = 0; t < kTokensPerWarp; ++t) {
       const uint32_t local = warp * kTokensPerWarp + t;
       const uint32_t row = chunk * kChunkTokens + local;
-      if (row < rows) route_token(scores, expert_scales, row, local, lane, keys, weights, bitmap);
+      if (row < rows) route_token(scores, expert_scales, row, local, lane, keys, weights, bitmap, nullptr);
     }
     __syncthreads();
     if (threadIdx.x < kExperts) {
@@ -574,25 +566,38 @@ moe_prepare_groups_kernel(MoeGroupPlan plan, GemmGroup* __restrict__ first_group
     items_down[e] = grp.l_tiles * grp.c_tiles;
     down_groups[e] = grp;
   }
+  // work_begin: exclusive sums of the work items, by warp shuffles (one thread adding them up took 5 us)
+  __shared__ int32_t warp_sums[2][8];
   __syncthreads();
-  if (g == 0) {
-    const int count_first = plan.form == kMoeFormFused ? kExperts : 2 * kExperts;
-    int32_t acc = 0;
-    for (int i = 0; i < count_first; ++i) {
-      first_groups[i].work_begin = acc;
-      acc += plan.form == kMoeFormFused ? items_first[2 * i] : items_first[i];
+  const unsigned lane = g % 32, warp = g / 32;
+  const bool fused = plan.form == kMoeFormFused;
+  const int32_t mine[2] = {items_first[g], g < unsigned(kExperts) ? items_down[g] : 0};
+  int32_t below[2];
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    int32_t scan = mine[which];
+#pragma unroll
+    for (int step = 1; step < 32; step *= 2) {
+      const int32_t other = __shfl_up_sync(0xffffffffu, scan, step);
+      if (lane >= unsigned(step)) scan += other;
     }
-    GemmGroup sentinel{};
-    sentinel.work_begin = acc;
-    sentinel.l_tiles = sentinel.c_tiles = 1;
-    first_groups[count_first] = sentinel;
+    below[which] = scan - mine[which];
+    if (lane == 31) warp_sums[which][warp] = scan;
   }
-  if (g == 1) {
-    int32_t acc = 0;
-    for (int i = 0; i < kExperts; ++i) { down_groups[i].work_begin = acc; acc += items_down[i]; }
+  __syncthreads();
+#pragma unroll
+  for (int which = 0; which < 2; ++which)
+    for (unsigned v = 0; v < warp; ++v) below[which] += warp_sums[which][v];
+  // fused: items_first counts at the even entries only, one group per expert
+  if (!fused) first_groups[g].work_begin = below[0];
+  else if (part == 0) first_groups[e].work_begin = below[0];
+  if (g < unsigned(kExperts)) down_groups[g].work_begin = below[1];
+  if (g == 255) {
     GemmGroup sentinel{};
-    sentinel.work_begin = acc;
+    sentinel.work_begin = below[0] + mine[0];
     sentinel.l_tiles = sentinel.c_tiles = 1;
+    first_groups[fused ? kExperts : 2 * kExperts] = sentinel;
+    sentinel.work_begin = below[1] + mine[1];
     down_groups[kExperts] = sentinel;
   }
 }
