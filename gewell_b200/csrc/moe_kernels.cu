@@ -606,7 +606,9 @@ moe_prepare_groups_kernel(MoeGroupPlan plan, GemmGroup* __restrict__ first_group
 // 5. NVFP4 quantisation of sorted rows with the destination expert's input
 //    scale (recipe of moe.cu:254-304 == src/nvfp4_linear.cu:61-116), reading
 //    either through the permutation (fused gather, moe.cu:183-186) or in place.
-//    One thread per K16 block.  Scales go to the expert's 128-row aligned
+//    Two threads per K16 block, each with eight values: at decode sizes the kernel is bound by latency and by
+//    fetching its own code (sixteen unrolled tanh), so more and smaller threads are faster; at large sizes by
+//    memory either way.  Scales go to the expert's 128-row aligned
 //    region ((first/128 + e) * 128, moe.cu:296-300) in the tiled layout.
 //    Source modes: plain rows of width K, or [rows, 2K] gate|up with GeGLU
 //    (moe.cu:439-445) whose BF16 result is also stored for the capture accessor.
@@ -616,57 +618,64 @@ __global__ void __launch_bounds__(256)
 moe_quantize_kernel(const uint4* __restrict__ input, const int32_t* __restrict__ gather_index,
                     const int32_t* __restrict__ sorted_keys, const int32_t* __restrict__ offsets,
                     const MoeExpertInfo* __restrict__ experts, uint32_t n, uint32_t scale_rows, int projection,
-                    uint32_t gather_divisor, uint2* __restrict__ packed, uint8_t* __restrict__ scales,
+                    uint32_t gather_divisor, uint32_t* __restrict__ packed, uint8_t* __restrict__ scales,
                     uint4* __restrict__ activated) {
   griddep_launch();
   griddep_wait();     // results of earlier kernels in the stream are read from here on
-  constexpr uint32_t kBlocks = K / 16;
+  constexpr uint32_t kVectors = K / 8;          // even: the two threads of a block are neighbours in a warp
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   const uint32_t part = blockIdx.y;             // gate/up copy (0 unless the scales differ)
-  if (index >= size_t(n) * kBlocks) return;
-  const uint32_t row = index / kBlocks, kb = index % kBlocks;
-  if (row >= uint32_t(offsets[kExperts])) return;       // n may be an upper bound (expert parallelism)
-  const int32_t e = sorted_keys[row];
-  const int32_t first = offsets[e];
-  const float inverse_scale = experts[e].inverse_input_scale[projection + part];
-  float values[16];
-  if constexpr (Gelu) {
-    const size_t gate = size_t(row) * (2 * kBlocks) + kb;
-    float g[16], u[16];
-    unpack8(input[2 * gate], g);
-    unpack8(input[2 * gate + 1], g + 8);
-    unpack8(input[2 * (gate + kBlocks)], u);
-    unpack8(input[2 * (gate + kBlocks) + 1], u + 8);
-    uint32_t words[8];
+  const uint32_t row = uint32_t(index / kVectors), vector = uint32_t(index % kVectors);
+  // n may be an upper bound (expert parallelism); threads without a row stay for the exchange below
+  const bool active = index < size_t(n) * kVectors && row < uint32_t(offsets[kExperts]);
+  float values[8];
+  float inverse_scale = 1.0F;
+  int32_t e = 0, first = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) values[i] = gelu_tanh_multiply_bf16(g[i], u[i]);
+  for (int i = 0; i < 8; ++i) values[i] = 0.0F;
+  if (active) {
+    e = sorted_keys[row];
+    if constexpr (Gelu) {
+      const size_t gate = size_t(row) * (2 * kVectors) + vector;
+      const uint4 raw_gate = input[gate], raw_up = input[gate + kVectors];
+      first = offsets[e];
+      inverse_scale = experts[e].inverse_input_scale[projection + part];
+      float g[8], u[8];
+      unpack8(raw_gate, g);
+      unpack8(raw_up, u);
+      uint32_t words[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      words[i] = (__float_as_uint(values[2 * i]) >> 16) | (__float_as_uint(values[2 * i + 1]) & 0xFFFF0000u);
-    if (activated != nullptr) {
-      activated[2 * index] = make_uint4(words[0], words[1], words[2], words[3]);
-      activated[2 * index + 1] = make_uint4(words[4], words[5], words[6], words[7]);
+      for (int i = 0; i < 8; ++i) values[i] = gelu_tanh_multiply_bf16(g[i], u[i]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        words[i] = (__float_as_uint(values[2 * i]) >> 16) | (__float_as_uint(values[2 * i + 1]) & 0xFFFF0000u);
+      if (activated != nullptr) activated[index] = make_uint4(words[0], words[1], words[2], words[3]);
+    } else {
+      const size_t source_row = gather_index ? size_t(uint32_t(gather_index[row]) / gather_divisor) : row;
+      const uint4 raw = input[source_row * kVectors + vector];
+      first = offsets[e];
+      inverse_scale = experts[e].inverse_input_scale[projection + part];
+      unpack8(raw, values);
     }
-  } else {
-    const size_t source_row = gather_index ? size_t(uint32_t(gather_index[row]) / gather_divisor) : row;
-    const size_t block = source_row * kBlocks + kb;
-    unpack8(input[2 * block], values);
-    unpack8(input[2 * block + 1], values + 8);
   }
   float amax = 0.0F;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(values[i]));
+  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(values[i]));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  if (!active) return;
   const uint8_t scale_code = float_to_e4m3(inverse_scale * (amax * rcp_approx_ftz(6.0F)));
   const float block_scale = e4m3_to_float(scale_code);
   const float factor =
       block_scale == 0.0F ? 0.0F : rcp_approx_ftz(block_scale * rcp_approx_ftz(inverse_scale));
-  uint32_t out[2] = {0, 0};
+  uint32_t out = 0;
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-    out[i / 4] |= uint32_t(float2_to_e2m1x2(values[2 * i] * factor, values[2 * i + 1] * factor)) << (8 * (i % 4));
-  packed[(size_t(part) * n + row) * kBlocks + kb] = make_uint2(out[0], out[1]);
-  const size_t region = (size_t(part) * scale_rows + size_t(first / 128 + e) * 128) * kBlocks;
-  scales[region + scale_offset(row - first, kb, K)] = scale_code;
+  for (int i = 0; i < 4; ++i)
+    out |= uint32_t(float2_to_e2m1x2(values[2 * i] * factor, values[2 * i + 1] * factor)) << (8 * i);
+  packed[(size_t(part) * n + row) * kVectors + vector] = out;
+  if (vector % 2 == 0) {
+    const size_t region = (size_t(part) * scale_rows + size_t(first / 128 + e) * 128) * (K / 16);
+    scales[region + scale_offset(row - first, vector / 2, K)] = scale_code;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1327,10 +1336,10 @@ cudaError_t launch_moe_quantize_input(const void* input, const int32_t* gather_i
                                       const int32_t* sorted_keys, const int32_t* offsets,
                                       const MoeExpertInfo* experts, uint32_t n, uint32_t scale_rows, int parts,
                                       uint8_t* packed, uint8_t* scales, cudaStream_t stream) {
-  const dim3 grid(blocks_for(size_t(n) * (kHidden / 16)), parts);
+  const dim3 grid(blocks_for(size_t(n) * (kHidden / 8)), parts);
   launch_pdl(moe_quantize_kernel<kHidden, false>, grid, 256, stream, 
       static_cast<const uint4*>(input), gather_index, sorted_keys, offsets, experts, n, scale_rows, 0,
-      gather_divisor ? gather_divisor : 1, reinterpret_cast<uint2*>(packed), scales, nullptr);
+      gather_divisor ? gather_divisor : 1, reinterpret_cast<uint32_t*>(packed), scales, nullptr);
   return cudaGetLastError();
 }
 
@@ -1347,10 +1356,10 @@ cudaError_t launch_moe_quantize_tokens(const void* input, const int32_t* keys, c
 cudaError_t launch_moe_activate_quantize(const void* gate_up, const int32_t* sorted_keys, const int32_t* offsets,
                                          const MoeExpertInfo* experts, uint32_t n, uint32_t scale_rows, uint8_t* packed,
                                          uint8_t* scales, void* activated, cudaStream_t stream) {
-  const dim3 grid(blocks_for(size_t(n) * (kInter / 16)), 1);
+  const dim3 grid(blocks_for(size_t(n) * (kInter / 8)), 1);
   launch_pdl(moe_quantize_kernel<kInter, true>, grid, 256, stream, 
       static_cast<const uint4*>(gate_up), nullptr, sorted_keys, offsets, experts, n, scale_rows, 2, 1,
-      reinterpret_cast<uint2*>(packed), scales, static_cast<uint4*>(activated));
+      reinterpret_cast<uint32_t*>(packed), scales, static_cast<uint4*>(activated));
   return cudaGetLastError();
 }
 
