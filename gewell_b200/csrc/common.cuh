@@ -60,6 +60,21 @@ __host__ __device__ __forceinline__ size_t scale_offset(size_t row, size_t block
          block % 4;
 }
 
+// Division by a launch constant (dividends below 2^31): a multiplication instead of the 20 to 100 instructions of an
+// integer division.
+struct Divisor {
+  uint32_t value, multiplier, shift;
+  static Divisor of(uint32_t d) {
+    uint32_t s = 0;
+    while ((1ull << s) < d) ++s;                         // 2^(s-1) < d <= 2^s
+    return Divisor{d, uint32_t(((1ull << (31 + s)) + d - 1) / d), s};
+  }
+  // multiplier = ceil(2^(31 + s) / d) < 2^32, exact for n < 2^31
+#ifdef __CUDACC__
+  __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return shift == 0 ? n : __umulhi(n, multiplier) >> (shift - 1); }
+#endif
+};
+
 #ifdef __CUDACC__
 // Programmatic dependent launch.  A kernel launched with the programmatic-
 // serialisation attribute may start while its predecessor in the stream still

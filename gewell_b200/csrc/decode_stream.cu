@@ -29,18 +29,6 @@ namespace {
 
 using namespace stream;
 
-// Division by a launch constant (dividends below 2^31): the index arithmetic is in front of a warp's first copy.
-struct Divisor {
-  uint32_t value, multiplier, shift;
-  static Divisor of(uint32_t d) {
-    uint32_t s = 0;
-    while ((1ull << s) < d) ++s;                         // 2^(s-1) < d <= 2^s
-    return Divisor{d, uint32_t(((1ull << (31 + s)) + d - 1) / d), s};
-  }
-  // multiplier = ceil(2^(31 + s) / d) < 2^32, exact for n < 2^31
-  __device__ uint32_t quotient(uint32_t n) const { return shift == 0 ? n : __umulhi(n, multiplier) >> (shift - 1); }
-};
-
 struct StreamArgs {
   CUtensorMap weights[2], scales[2];
   float alpha[2];

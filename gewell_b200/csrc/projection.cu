@@ -17,6 +17,7 @@
 #include <memory>
 #include <new>
 #include <string>
+#include <algorithm>
 #include <tuple>
 #include <vector>
 
@@ -27,12 +28,19 @@ using namespace gw;
 
 namespace {
 
+// strip the padding columns: output[r, c] = input[r, c] for c < logical   (projection.cu:25-28)
+// VECTOR: both widths multiples of 8 and an aligned output, eight values a thread; one block row of the grid per row
+template <bool VECTOR>
 __global__ void __launch_bounds__(256)
-compact_rows_kernel(const bf16* __restrict__ input, bf16* __restrict__ output, uint32_t rows, uint32_t logical,
-                    uint32_t physical) {
-  // strip the padding columns: output[r, c] = input[r, c] for c < logical   (projection.cu:25-28)
-  const size_t i = size_t(blockIdx.x) * 256 + threadIdx.x;
-  if (i < size_t(rows) * logical) output[i] = input[(i / logical) * physical + i % logical];
+compact_rows_kernel(const bf16* __restrict__ input, bf16* __restrict__ output, uint32_t rows, uint32_t logical, uint32_t physical) {
+  griddep_launch();
+  griddep_wait();
+  const uint32_t c = (blockIdx.x * 256 + threadIdx.x) * (VECTOR ? 8 : 1);
+  if (c >= logical) return;
+  for (size_t row = blockIdx.y; row < rows; row += gridDim.y) {
+    if constexpr (VECTOR) *reinterpret_cast<uint4*>(output + row * logical + c) = *reinterpret_cast<const uint4*>(input + row * physical + c);
+    else output[row * logical + c] = input[row * physical + c];
+  }
 }
 
 struct Buffer {
@@ -321,11 +329,12 @@ gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_proje
   }
   if (status != GW_OK) return status;
   if (padded) {
-    const size_t count = size_t(w->rows) * p.output;
-    compact_rows_kernel<<<unsigned((count + 255) / 256), 256, 0, w->stream>>>(
-        static_cast<const bf16*>(destination), static_cast<bf16*>(output_bf16), w->rows, p.output, p.physical_output);
-    note_launch();
-    GW_CUDA_CHECK(cudaGetLastError(), "compact 26B projection output");
+    const bool vector = p.output % 8 == 0 && p.physical_output % 8 == 0 && reinterpret_cast<uintptr_t>(output_bf16) % 16 == 0;
+    const uint32_t per_block = vector ? 2048 : 256;
+    GW_CUDA_CHECK(launch_pdl(vector ? compact_rows_kernel<true> : compact_rows_kernel<false>,
+                             dim3((p.output + per_block - 1) / per_block, std::min<uint32_t>(w->rows, 65535)), 256, w->stream,
+                             static_cast<const bf16*>(destination), static_cast<bf16*>(output_bf16), w->rows, p.output, p.physical_output),
+                  "compact 26B projection output");
   }
   return GW_OK;
 }
