@@ -3,6 +3,7 @@
 #include "gemm_pair_wide.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <string>
 
@@ -51,6 +52,21 @@ bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_
   if (plan.tiles == 2 && values > 46 * 1024 && bytes > (size_t(20) << 20)) return false;
   // BF16 tokens of more than 8192 values need several slabs: twice the sums
   return kind != StreamKind::w16a16 || plan.slabs == 1 || bytes <= (size_t(48) << 20);
+}
+
+// Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each.
+constexpr uint32_t kW4a16Rows = 48;
+
+// Gate, up and GeGLU as one streaming launch (n: channels of each) against the joined GEMM whose GeGLU rides in the next
+// quantiser.  Of the large quantised pairs only one or two tokens win (chain 5376 -> 21504 -> 5376, us, streamed against
+// joined: NVFP4 1 row 55.5 / 59.2, 2 rows 58.3 / 58.1, 8 rows 61.5 / 58.0; FP8 71.1 / 74.2, 4 rows 75.8 / 74.8): every SM
+// quantises all activations and does the GeGLU of its own channels after its last byte.  BF16 has nothing to quantise
+// (8 rows 121.7 / 122.9).
+bool stream_pair_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
+  if (!stream_pays(kind, plan, rows, k, 2 * n)) return false;
+  if (kind != StreamKind::w4a4 && kind != StreamKind::w8a8) return true;
+  const size_t bytes = 2 * n * k * (kind == StreamKind::w4a4 ? 9 : 16) / 16;
+  return bytes <= (size_t(40) << 20) || size_t(rows) * k <= 8192;
 }
 
 size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n) {
@@ -129,6 +145,99 @@ gw_status launch_dense_pair_wide(const DenseProblem& q, uint64_t row_bytes, Dens
 }
 
 }  // namespace
+
+StreamBook::~StreamBook() {
+  if (counters != nullptr) cudaFree(counters);
+}
+
+gw_status StreamBook::prepare(uint32_t new_rows, const std::vector<std::pair<uint32_t, uint32_t>>& shapes, size_t workspace_bytes) {
+  rows = new_rows;
+  entries.clear();
+  size_t most = 0;
+  const bool allowed = DenseTuning::from_environment().streams();
+  for (const auto& [k, n] : shapes)
+    for (StreamKind kind : {StreamKind::w4a4, StreamKind::w4a16, StreamKind::w8a8, StreamKind::w16a16})
+      for (bool pair : {false, true}) {
+        // W4A16 beyond one launch's rows: several launches, each of them reads the packed weights once
+        const uint32_t tile = kind == StreamKind::w4a16 && rows <= kW4a16Rows ? std::min(rows, kStreamMaxRows) : rows;
+        Entry s;
+        s.plan = plan_stream(kind, tile, k, n, pair, sm_count());
+        s.plan.usable = allowed && (pair ? stream_pair_pays(kind, s.plan, tile, k, n) : stream_pays(kind, s.plan, tile, k, n));
+        if (!s.plan.usable || s.plan.workspace_bytes > workspace_bytes) continue;
+        most = std::max(most, s.plan.counter_count);
+        entries[Key{int(kind), k, n, pair}] = s;
+      }
+  if (most * sizeof(int32_t) > counter_bytes) {
+    int32_t* larger = nullptr;
+    cudaError_t status = cudaMalloc(&larger, most * sizeof(int32_t));
+    if (status == cudaSuccess) status = cudaMemset(larger, 0, most * sizeof(int32_t));
+    if (status != cudaSuccess) {
+      if (larger != nullptr) cudaFree(larger);
+      entries.clear();
+      return fail(GW_CUDA_ERROR, std::string("counters of the weight-streaming kernel: ") + cudaGetErrorString(status));
+    }
+    if (counters != nullptr) cudaFree(counters);
+    counters = larger;
+    counter_bytes = most * sizeof(int32_t);
+  }
+  return GW_OK;
+}
+
+gw_status StreamBook::run(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4,
+                          void* workspace, cudaStream_t s, bool* done) {
+  *done = false;
+  if (second && (second->storage != first.storage || second->input != first.input || second->output != first.output ||
+                 second->physical_output != first.physical_output)) return GW_OK;
+  const uint32_t physical = first.storage == GW_STORAGE_NVFP4_W4A4 ? first.physical_output : first.output;
+  StreamKind kind = StreamKind::w16a16;
+  float input_scale = 1.0F;
+  if (first.storage == GW_STORAGE_NVFP4_W4A4) {
+    kind = fp4 ? StreamKind::w4a4 : StreamKind::w4a16;
+    if (fp4) {
+      input_scale = first.nvfp4_input_scale;
+      if (second && second->nvfp4_input_scale != input_scale) return GW_OK;
+    }
+  } else if (first.storage == GW_STORAGE_FP8_W8A8) {
+    kind = StreamKind::w8a8;
+    input_scale = first.fp8_input_scale;
+    if (second && second->fp8_input_scale != input_scale) return GW_OK;
+  }
+  const auto found = entries.find(Key{int(kind), first.input, physical, second != nullptr});
+  if (found == entries.end() || !std::isfinite(1.0F / input_scale) || !(input_scale > 0.0F)) return GW_OK;
+  Entry& with = found->second;
+  StreamProblem q{kind, std::min(rows, kStreamMaxRows), first.input, first.output, input};
+  q.inverse_scale = 1.0F / input_scale;
+  const gw_projection* projection[2] = {&first, second};
+  StreamMatrix* matrix[2] = {&q.first, &q.second};
+  std::string error;
+  for (int i = 0; i < (second ? 2 : 1); ++i) {
+    const gw_projection& p = *projection[i];
+    StreamMatrix& m = *matrix[i];
+    if (p.storage == GW_STORAGE_NVFP4_W4A4)
+      m = StreamMatrix{p.nvfp4_data, p.nvfp4_scales, fp4 ? p.nvfp4_input_scale * p.nvfp4_weight_scale : p.nvfp4_weight_scale, nullptr};
+    else if (p.storage == GW_STORAGE_FP8_W8A8)
+      m = StreamMatrix{p.fp8_data, nullptr, p.fp8_input_scale * p.fp8_weight_scale, p.fp8_channel_scales};
+    else
+      m.data = p.bf16;
+    if (!m.data || !(m.alpha > 0.0F) || !std::isfinite(m.alpha)) return GW_OK;      // the plans report what is wrong
+  }
+  if (!stream_aligned(q)) return GW_OK;
+  for (int i = 0; i < (second ? 2 : 1); ++i)
+    if (!with.maps[i].get(kind, *matrix[i], with.plan.physical_n, q.k, &error))
+      return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
+  q.ld_out = first.output;
+  q.workspace = workspace;
+  q.counters = counters;
+  q.error = device_error_word();
+  for (uint32_t row = 0; row < rows; row += kStreamMaxRows) {
+    q.rows = std::min(rows - row, kStreamMaxRows);
+    q.input = static_cast<const bf16*>(input) + size_t(row) * q.k;
+    q.output = static_cast<bf16*>(output) + size_t(row) * q.ld_out;
+    GW_CUDA_CHECK(launch_stream(q, with.plan, with.maps[0], with.maps[1], s), "weight-streaming projection");
+  }
+  *done = true;
+  return GW_OK;
+}
 
 gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
   const DenseTuning& tuning = cache->tuning;

@@ -3,6 +3,11 @@
 // descriptors (cached per plan) and launches.
 #pragma once
 
+#include <map>
+#include <tuple>
+#include <utility>
+#include <vector>
+
 #include "common.cuh"
 #include "decode_stream.h"
 #include "gemm_tc.cuh"
@@ -74,6 +79,33 @@ bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_
 // The problem on the weight-streaming kernel; *done = false when its pointers keep it off that kernel.
 gw_status launch_dense_stream(const StreamProblem& problem, DenseDescriptors* cache, cudaStream_t stream, bool* done);
 
+// The weight-streaming launches of an object whose projections run one after another: plans by (kind, K, physical N,
+// two matrices) for the row count of the last prepare(), the counters they share, and the tensor maps of the last
+// matrices under each key.
+struct StreamBook {
+  using Key = std::tuple<int, uint32_t, uint32_t, bool>;
+  struct Entry { StreamPlan plan; StreamMaps maps[2]; };
+  std::map<Key, Entry> entries;
+  int32_t* counters = nullptr;
+  size_t counter_bytes = 0;
+  uint32_t rows = 0;
+  StreamBook() = default;
+  StreamBook(const StreamBook&) = delete;
+  StreamBook& operator=(const StreamBook&) = delete;
+  ~StreamBook();
+  // shapes: (K, physical N); `workspace_bytes`: of the workspace that run() will be given
+  gw_status prepare(uint32_t rows, const std::vector<std::pair<uint32_t, uint32_t>>& shapes, size_t workspace_bytes);
+  // The projection `first` -- or, with `second`, GeGLU of both -- into [rows, first.output]; *done = false when the shape,
+  // the storage or the pointers keep it off the kernel.
+  gw_status run(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4, void* workspace,
+                cudaStream_t stream, bool* done);
+};
+
 gw_status launch_dense(const DenseProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
+
+// product = GeGLU of both projections of a prepared workspace in one launch (projection.cu); *done = false when that is
+// not the faster way here.
+gw_status projection_workspace_run_geglu(gw_projection_workspace* workspace, const gw_projection& gate, const gw_projection& up,
+                                         const void* input, void* product, bool* done);
 
 }  // namespace gw

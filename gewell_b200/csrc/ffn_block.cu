@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "dense.h"
 #include "kernels.h"
 
 using namespace gw;
@@ -563,9 +564,13 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
                                                   b->expert_input, rows, kHidden, s);
   if (status != GW_OK) return status;
   // shared MLP (batched_executor.cu:256-259)
-  if ((status = gw_projection_workspace_run(b->projections, &w.gate, b->normalized, b->gate)) != GW_OK) return status;
-  if ((status = gw_projection_workspace_run(b->projections, &w.up, b->normalized, b->up)) != GW_OK) return status;
-  if ((status = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, s)) != GW_OK) return status;
+  bool product_done = false;
+  if ((status = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, &product_done)) != GW_OK) return status;
+  if (!product_done) {
+    if ((status = gw_projection_workspace_run(b->projections, &w.gate, b->normalized, b->gate)) != GW_OK) return status;
+    if ((status = gw_projection_workspace_run(b->projections, &w.up, b->normalized, b->up)) != GW_OK) return status;
+    if ((status = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, s)) != GW_OK) return status;
+  }
   if ((status = gw_projection_workspace_run(b->projections, &w.down, b->product, b->shared_mlp)) != GW_OK) return status;
   // router logits and the experts (batched_executor.cu:262-266)
   gw_projection router{};

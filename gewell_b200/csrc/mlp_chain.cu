@@ -51,9 +51,6 @@ struct Buffer {
   ~Buffer() { if (data) cudaFree(data); }
 };
 
-// Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each.
-constexpr uint32_t kW4a16Rows = 48;
-
 enum Kind { kNvfp4 = 0, kFp8 = 1, kFp8Channel = 2, kBf16 = 3 };
 using Key = std::tuple<int, uint32_t, uint32_t>;   // kind, K, N
 
@@ -99,12 +96,7 @@ struct PlanBook {
   int policy = GW_POLICY_ALWAYS;
   std::map<Key, PlanSet> plans;
   Buffer scratch, dequantized;
-  // Small row counts on the weight-streaming kernel: the plans of prepare()'s row count by (kind, K, N, two matrices), the
-  // counters they share (they run one after another) and the tensor maps of the last matrices by the same key.
-  using StreamKey = std::tuple<int, uint32_t, uint32_t, bool>;
-  struct Streaming { StreamPlan plan; StreamMaps maps[2]; };
-  std::map<StreamKey, Streaming> streaming;
-  Buffer counters;
+  StreamBook streaming;            // small row counts
   ~PlanBook() { for (auto& entry : plans) entry.second.reset(); }
 
   // shapes: (K, N) pairs; scratch for the widest of them, the dequantised buffer for the largest
@@ -144,93 +136,13 @@ struct PlanBook {
     for (auto& entry : plans) entry.second.reset();
     plans = std::move(next);
     rows = new_rows;
-    return prepare_streaming(shapes);
+    return streaming.prepare(rows, shapes, scratch.bytes);
   }
 
-  gw_status prepare_streaming(const std::vector<std::pair<uint32_t, uint32_t>>& shapes) {
-    streaming.clear();
-    size_t most = 0;
-    const bool allowed = DenseTuning::from_environment().streams();
-    for (const auto& [k, n] : shapes)
-      for (StreamKind kind : {StreamKind::w4a4, StreamKind::w4a16, StreamKind::w8a8, StreamKind::w16a16})
-        for (bool pair : {false, true}) {
-          // W4A16 beyond one launch's rows: several launches, each of them reads the packed weights once
-          const uint32_t tile = kind == StreamKind::w4a16 && rows <= kW4a16Rows ? std::min(rows, kStreamMaxRows) : rows;
-          Streaming s;
-          s.plan = plan_stream(kind, tile, k, n, pair, sm_count());
-          s.plan.usable = allowed && stream_pays(kind, s.plan, tile, k, pair ? 2 * size_t(n) : n);
-          if (!s.plan.usable || s.plan.workspace_bytes > scratch.bytes) continue;
-          most = std::max(most, s.plan.counter_count);
-          streaming[StreamKey{int(kind), k, n, pair}] = s;
-        }
-    if (most * sizeof(int32_t) > counters.bytes) {
-      Buffer larger;
-      cudaError_t status = larger.allocate(most * sizeof(int32_t));
-      if (status == cudaSuccess) status = cudaMemset(larger.data, 0, larger.bytes);
-      if (status != cudaSuccess) {
-        streaming.clear();
-        return fail(GW_CUDA_ERROR, std::string("counters of the weight-streaming kernel: ") + cudaGetErrorString(status));
-      }
-      std::swap(larger.data, counters.data);
-      std::swap(larger.bytes, counters.bytes);
-    }
-    return GW_OK;
-  }
-
-  // The projection `first` -- or, with `second`, GeGLU of both -- on the weight-streaming kernel; *done = false when the
-  // shape, the storage or the pointers keep it off that kernel.
+  // `first` or GeGLU of `first` and `second` on the weight-streaming kernel, if that is the faster one here
   gw_status stream(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4, cudaStream_t s,
                    bool* done) {
-    *done = false;
-    if (second && (second->storage != first.storage || second->input != first.input || second->output != first.output)) return GW_OK;
-    StreamKind kind = StreamKind::w16a16;
-    float input_scale = 1.0F;
-    if (first.storage == GW_STORAGE_NVFP4_W4A4) {
-      kind = fp4 ? StreamKind::w4a4 : StreamKind::w4a16;
-      if (fp4) {
-        input_scale = first.nvfp4_input_scale;
-        if (second && second->nvfp4_input_scale != input_scale) return GW_OK;
-      }
-    } else if (first.storage == GW_STORAGE_FP8_W8A8) {
-      kind = StreamKind::w8a8;
-      input_scale = first.fp8_input_scale;
-      if (second && second->fp8_input_scale != input_scale) return GW_OK;
-    }
-    const auto found = streaming.find(StreamKey{int(kind), first.input, first.output, second != nullptr});
-    if (found == streaming.end() || !std::isfinite(1.0F / input_scale) || !(input_scale > 0.0F)) return GW_OK;
-    Streaming& with = found->second;
-    StreamProblem q{kind, std::min(rows, kStreamMaxRows), first.input, first.output, input};
-    q.inverse_scale = 1.0F / input_scale;
-    const gw_projection* projection[2] = {&first, second};
-    StreamMatrix* matrix[2] = {&q.first, &q.second};
-    std::string error;
-    for (int i = 0; i < (second ? 2 : 1); ++i) {
-      const gw_projection& p = *projection[i];
-      StreamMatrix& m = *matrix[i];
-      if (p.storage == GW_STORAGE_NVFP4_W4A4)
-        m = StreamMatrix{p.nvfp4_data, p.nvfp4_scales, fp4 ? p.nvfp4_input_scale * p.nvfp4_weight_scale : p.nvfp4_weight_scale, nullptr};
-      else if (p.storage == GW_STORAGE_FP8_W8A8)
-        m = StreamMatrix{p.fp8_data, nullptr, p.fp8_input_scale * p.fp8_weight_scale, p.fp8_channel_scales};
-      else
-        m.data = p.bf16;
-      if (!m.data || !(m.alpha > 0.0F) || !std::isfinite(m.alpha)) return GW_OK;      // the plans report what is wrong
-    }
-    if (!stream_aligned(q)) return GW_OK;
-    for (int i = 0; i < (second ? 2 : 1); ++i)
-      if (!with.maps[i].get(kind, *matrix[i], with.plan.physical_n, q.k, &error))
-        return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
-    q.ld_out = first.output;
-    q.workspace = scratch.data;
-    q.counters = static_cast<int32_t*>(counters.data);
-    q.error = device_error_word();
-    for (uint32_t row = 0; row < rows; row += kStreamMaxRows) {
-      q.rows = std::min(rows - row, kStreamMaxRows);
-      q.input = static_cast<const bf16*>(input) + size_t(row) * q.k;
-      q.output = static_cast<bf16*>(output) + size_t(row) * q.ld_out;
-      GW_CUDA_CHECK(launch_stream(q, with.plan, with.maps[0], with.maps[1], s), "weight-streaming projection");
-    }
-    *done = true;
-    return GW_OK;
+    return streaming.run(first, second, input, output, fp4, scratch.data, s, done);
   }
 };
 

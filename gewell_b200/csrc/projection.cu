@@ -79,6 +79,7 @@ struct gw_projection_workspace {
   int policy = GW_POLICY_ALWAYS;
   bool fp4 = false;
   cudaStream_t stream = nullptr;
+  StreamBook streaming;                // small row counts
   ~gw_projection_workspace() { for (auto& entry : plans) entry.second.reset(); }
 };
 
@@ -252,6 +253,11 @@ gw_status gw_projection_workspace_prepare(gw_projection_workspace* w, uint32_t r
     return fail(GW_INVALID_ARGUMENT, "invalid 26B projection rows/phase");
   const bool fp4 = gw_nvfp4_fp4_activations(w->policy, phase) != 0;
   if (w->rows == rows && w->fp4 == fp4) return GW_OK;
+  if (w->streaming.rows != rows) {
+    std::vector<std::pair<uint32_t, uint32_t>> shapes;
+    for (const auto& entry : w->plans) shapes.emplace_back(std::get<1>(entry.first), std::get<2>(entry.first));
+    if (const gw_status status = w->streaming.prepare(rows, shapes, w->scratch.bytes); status != GW_OK) return status;
+  }
   // Keep a plan when only the phase changes; rebuild on a new row count, outside the layer loop.
   // Every requested plan is built first and published only when all of them exist.
   std::map<Shape, Plans> replacements;
@@ -296,6 +302,12 @@ gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_proje
   const bool padded = p.output != p.physical_output;
   if (padded && (!w->padded.data || size_t(w->rows) * p.physical_output * sizeof(bf16) > w->padded.bytes))
     return fail(GW_INVALID_ARGUMENT, "projection was not among the workspace's bindings");
+  // NVFP4 at small row counts: into the caller's rows at once, and with BF16 activations from the packed weights
+  if (p.storage == GW_STORAGE_NVFP4_W4A4 && (padded || !w->fp4)) {
+    bool done = false;
+    const gw_status status = w->streaming.run(p, nullptr, input_bf16, output_bf16, w->fp4, w->scratch.data, w->stream, &done);
+    if (status != GW_OK || done) return status;
+  }
   void* destination = padded ? w->padded.data : output_bf16;
   const int kind = p.storage == GW_STORAGE_FP8_W8A8 ? kPlanFp8
                    : (p.storage == GW_STORAGE_NVFP4_W4A4 && w->fp4) ? kPlanNvfp4 : kPlanBf16;
@@ -340,3 +352,14 @@ gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_proje
 }
 
 }  // extern "C"
+
+namespace gw {
+
+gw_status projection_workspace_run_geglu(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up, const void* input,
+                                         void* product, bool* done) {
+  *done = false;
+  if (w->rows == 0) return GW_OK;
+  return w->streaming.run(gate, &up, input, product, w->fp4, w->scratch.data, w->stream, done);
+}
+
+}  // namespace gw
