@@ -40,6 +40,7 @@ struct StreamArgs {
   int32_t* counters;
   uint8_t *packed, *packed_scales;       // w4a4: where the quantised activations are left as well, or nullptr
   uint32_t* error;
+  uint32_t reread;                       // a launch after this one reads the same weights
   float inverse_scale;
   uint32_t rows, k, n, gelu;
   uint32_t blocks, chunks, chunks_per_slab, slabs, max_units;
@@ -232,7 +233,7 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
     ptx::prefetch_tensormap(&a.weights[0]);
     if (nvfp4_weights(KIND)) ptx::prefetch_tensormap(&a.scales[0]);
   }
-  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32;
   const uint32_t piece_begin = range_begin(a, blockIdx.x), piece_end = range_begin(a, blockIdx.x + 1);
   const uint32_t unit_first = unit_of(a, piece_begin);
   if (lane == 0) {                        // the ring's barriers are this warp's own
@@ -242,6 +243,7 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
   }
   __syncwarp();
 
+  const uint64_t policy = a.reread ? ptx::l2_evict_normal() : ptx::l2_evict_first();
   uint32_t slab_unit = unit_first, turn = 0;                // turn: pieces this warp has multiplied
   for (uint32_t slab_begin = piece_begin; slab_begin < piece_end;) {
     // ---- the pieces of one slab, divided among the warps
@@ -255,16 +257,16 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
     uint32_t next = begin, next_block = block, next_chunk = chunk, next_slot = turn % kSlots, next_matrix = 0;      // the piece to ask for next
     auto request = [&]() {
       const uint32_t matrix = PAIR ? next_matrix : 0;
-      if (next < end && lane == 0) {
+      if (next < end && ptx::elect_one()) {
         const uint32_t place = warp * kSlots + next_slot;
         uint64_t* bar = full_bar + place;
         const BlockPlace at(next_block);
         ptx::mbar_expect_tx(bar, kPieceBytes + L::kScaleBytes);
         ptx::tma_load_3d(ring + place * kPieceBytes, &a.weights[matrix], int32_t((chunk0 + next_chunk) * 128), int32_t(at.row8 * 8),
-                         int32_t(at.group), bar);
+                         int32_t(at.group), bar, policy);
         if constexpr (nvfp4_weights(KIND))
           ptx::tma_load_2d(ring_scales + place * L::kScaleBytes, &a.scales[matrix], int32_t(at.row8 * 128),
-                           int32_t(at.group / 4 * (a.k / 64) + (chunk0 + next_chunk) * 4), bar);
+                           int32_t(at.group / 4 * (a.k / 64) + (chunk0 + next_chunk) * 4), bar, policy);
       }
       if (++next_slot == kSlots) next_slot = 0;
       if (PAIR && (next_matrix ^= 1) != 0) return;
@@ -457,6 +459,7 @@ cudaError_t launch_stream(const StreamProblem& q, const StreamPlan& plan, const 
   a.packed = q.packed;
   a.packed_scales = q.packed_scales;
   a.error = q.error;
+  a.reread = q.reread ? 1 : 0;
   a.inverse_scale = q.inverse_scale;
   a.rows = q.rows;
   a.k = q.k;

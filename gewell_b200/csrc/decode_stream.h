@@ -38,6 +38,7 @@ struct StreamProblem {
   size_t ld_out;
   void* workspace = nullptr;   // StreamPlan::workspace_bytes, 16-byte aligned
   int32_t* counters = nullptr; // StreamPlan::counter_count zeroed ints; left zero
+  bool reread = false;         // another launch reads the same weights soon
   uint32_t* error = nullptr;   // device error word
 };
 

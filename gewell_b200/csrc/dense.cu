@@ -231,6 +231,7 @@ gw_status StreamBook::run(const gw_projection& first, const gw_projection* secon
   q.error = device_error_word();
   for (uint32_t row = 0; row < rows; row += kStreamMaxRows) {
     q.rows = std::min(rows - row, kStreamMaxRows);
+    q.reread = rows - row > kStreamMaxRows;
     q.input = static_cast<const bf16*>(input) + size_t(row) * q.k;
     q.output = static_cast<bf16*>(output) + size_t(row) * q.ld_out;
     GW_CUDA_CHECK(launch_stream(q, with.plan, with.maps[0], with.maps[1], s), "weight-streaming projection");

@@ -242,6 +242,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
     if (ptx::elect_one()) {
     int stage = 0;
     uint32_t phase = 0;
+    const uint64_t evict_first = ptx::l2_evict_first(), evict_normal = ptx::l2_evict_normal();
     bool waited = !early_weights;        // this warp defers its wait for the previous kernel (see below)
     WorkItem item, next;
     SegmentWalk walk(int(blockIdx.x), int(gridDim.x), split, total_work, k_stages, p.work_chunk);
@@ -264,6 +265,8 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
       // copy engine; no proxy fence is needed per use (one system-scope fence per work item
       // cost more than the item's copies).
       const int l_row = item.g.l_row0 + item.l_tile * kTileL;
+      // weights on the lanes are read once when there is one column tile
+      const uint64_t l_policy = EPI == GemmEpilogue::swap_store && item.g.c_tiles == 1 ? evict_first : evict_normal;
       const int c_local = item.c_tile * p.c_rows_per_tile;   // row inside each matrix of the C operand
       const int halves = item.halves;
       // per-item source addresses; per stage they advance by a constant
@@ -295,7 +298,10 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
           // a slab past the end of K is filled with zeros by the copy engine (and skipped by the MMAs)
 #pragma unroll
           for (int slab = 0; slab < kSlabs; ++slab)
-            ptx::tma_load_2d(base + slab * C::kLSlabBytes, map_l, (ks * kSlabs + slab) * kStageRowBytes, l_row, bar);
+            if constexpr (EPI == GemmEpilogue::swap_store)
+              ptx::tma_load_2d(base + slab * C::kLSlabBytes, map_l, (ks * kSlabs + slab) * kStageRowBytes, l_row, bar, l_policy);
+            else
+              ptx::tma_load_2d(base + slab * C::kLSlabBytes, map_l, (ks * kSlabs + slab) * kStageRowBytes, l_row, bar);
           if constexpr (kNvfp4)
             ptx::bulk_load(base + C::kLBytes + C::kCBytes, sfl_src + size_t(ks) * kKBlocksPerStage * kAtomBytes,
                            nkb * kAtomBytes, bar);
