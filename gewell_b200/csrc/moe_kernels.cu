@@ -37,10 +37,16 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float* out) {
   }
 }
 
+// The scales of this lane's experts (lane, lane + 32, ...): weights, so they are read while the kernel before still runs.
+__device__ __forceinline__ void load_expert_scales(const bf16* __restrict__ expert_scales, unsigned lane, float (&scale)[4]) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) scale[q] = __bfloat162float(expert_scales[lane + 32 * q]);
+}
+
 // One token (one warp): FP32 softmax over its 128 logits, eight winners, renormalised weights, and the
 // winners' bits in the chunk's bitmaps.  The FP32 operation order is that of the reference's select
 // kernel (models/gemma4/26b_a4b/sm120/moe.cu:104-157), so ids and FP32 weights match it bit for bit.
-__device__ __forceinline__ void route_token(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales,
+__device__ __forceinline__ void route_token(const bf16* __restrict__ scores, const float (&expert_scale)[4],
                                             uint32_t row, uint32_t local, unsigned lane, int32_t* __restrict__ keys,
                                             float* __restrict__ weights, uint32_t (*bitmap)[2], int32_t* shared_keys) {
   // Softmax over the token's 128 logits; this lane owns experts lane, lane + 32, lane + 64, lane + 96.
@@ -96,8 +102,14 @@ __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, con
   int rank = 0;
 #pragma unroll
   for (int i = 0; i < kTopK; ++i) rank += __shfl_sync(0xffffffffu, my_id, i) < my_id;
+  float scale = 0.0F;                  // of my_id, from the lane that holds it
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float theirs = __shfl_sync(0xffffffffu, expert_scale[q], my_id & 31);
+    if (my_id / 32 == q) scale = theirs;
+  }
   if (lane < unsigned(kTopK)) {
-    const float weight = __fmul_rn(__fdiv_rn(my_p, sum), __bfloat162float(expert_scales[my_id]));
+    const float weight = __fmul_rn(__fdiv_rn(my_p, sum), scale);
     keys[size_t(row) * kTopK + rank] = my_id;
     weights[size_t(row) * kTopK + rank] = weight;
     if (shared_keys != nullptr) shared_keys[local * kTopK + rank] = my_id;
@@ -122,9 +134,11 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
                  int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
                  int32_t* __restrict__ inverse) {
   griddep_launch();
+  const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  float expert_scale[4];
+  load_expert_scales(expert_scales, lane, expert_scale);
   griddep_wait();     // results of earlier kernels in the stream are read from here on
   __shared__ uint32_t bitmap[kExperts][2];
-  const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
   __syncthreads();
   const uint32_t chunk = blockIdx.x;
@@ -135,7 +149,7 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
     const uint32_t local = warp + t * (blockDim.x / 32);
     const uint32_t row = chunk * kChunkTokens + local;
     if (row >= rows) break;
-    route_token(scores, expert_scales, row, local, lane, keys, weights, bitmap, shared_keys);
+    route_token(scores, expert_scale, row, local, lane, keys, weights, bitmap, shared_keys);
   }
   __syncthreads();
   if (threadIdx.x < kExperts) {
@@ -235,13 +249,15 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
                       int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
                       int32_t* __restrict__ inverse, uint32_t* __restrict__ barrier_state, uint32_t* __restrict__ error) {
   griddep_launch();
+  const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  float expert_scale[4];
+  load_expert_scales(expert_scales, lane, expert_scale);
   griddep_wait();     // results of earlier kernels in the stream are read from here on
   __shared__ uint32_t bitmap[kExperts][2];
   __shared__ int32_t own_base[kRouteOwnChunks][kExperts];
   __shared__ int32_t part_sum[kRouteParts][kExperts];
   __shared__ int32_t expert_offset[kExperts];
   __shared__ int32_t warp_totals[4];
-  const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   constexpr int kTokensPerWarp = kChunkTokens / (kRouteGridThreads / 32);     // 2
   // ---- phase 1: 32 warps, two tokens each, per chunk
   for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
@@ -251,7 +267,7 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
     for (int t = 0; t < kTokensPerWarp; ++t) {
       const uint32_t local = warp * kTokensPerWarp + t;
       const uint32_t row = chunk * kChunkTokens + local;
-      if (row < rows) route_token(scores, expert_scales, row, local, lane, keys, weights, bitmap, nullptr);
+      if (row < rows) route_token(scores, expert_scale, row, local, lane, keys, weights, bitmap, nullptr);
     }
     __syncthreads();
     if (threadIdx.x < kExperts) {
@@ -435,10 +451,11 @@ moe_keys_from_offsets_kernel(const int32_t* __restrict__ offsets, uint32_t first
 __global__ void __launch_bounds__(256)
 moe_prepare_groups_kernel(MoeGroupPlan plan, GemmGroup* __restrict__ first_groups, GemmGroup* __restrict__ down_groups) {
   griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
   __shared__ int32_t items_first[2 * kExperts], items_down[kExperts];
   const unsigned g = threadIdx.x;            // 0..255: expert = g/2, part = g%2
   const unsigned e = g / 2, part = g % 2;
+  const MoeExpertInfo info = plan.experts[e];   // of the expert table, written when it was created
+  griddep_wait();     // results of earlier kernels in the stream are read from here on
   // Offsets that come from other ranks' histograms (expert parallelism) may describe more rows than
   // the buffers hold: clamp every group to the capacity and report, so that no tile is scheduled
   // over rows that do not exist.
@@ -449,7 +466,6 @@ moe_prepare_groups_kernel(MoeGroupPlan plan, GemmGroup* __restrict__ first_group
     first = min(max(first, 0), capacity);
     last = min(max(last, first), capacity);
   }
-  const MoeExpertInfo info = plan.experts[e];
   // A projection gets work in this launch only if it runs as the launch's kind.
   const bool nv = plan.kind == kMoeKindNvfp4;
   auto runs_here = [&](int proj) { return moe_effective_kind(info.storage[proj], plan.fp4) == plan.kind; };
