@@ -445,8 +445,10 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
     first.num_groups = form == kMoeFormFused ? kExperts : 2 * kExperts;
     first.k = kHidden;
     first.c_rows_per_tile = form == kMoeFormFused ? 128 : block_n_first;
-    // two consecutive tiles per CTA (same token tile, same expert) before it strides on: measured best
-    first.work_chunk = tune.chunk_first > 0 ? tune.chunk_first : (swap ? 1 : 2);
+    // Direct forms: two consecutive tiles per CTA (same token tile, same expert) before it strides on, measured best.
+    // Swap form: one contiguous range, because its tiles are as short as a group's descriptor is late (64 tokens, down
+    // GEMM: CHUNK_US).
+    first.work_chunk = tune.chunk_first > 0 ? tune.chunk_first : (swap ? -1 : 2);
     first.error = device_error_word();
     if (form == kMoeFormFused) {
       first.out = w->packed_act.data;
@@ -494,7 +496,7 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
     down.num_groups = kExperts;
     down.k = kInter;
     down.c_rows_per_tile = block_n_down;
-    down.work_chunk = tune.chunk_down > 0 ? tune.chunk_down : (swap ? 1 : 2);
+    down.work_chunk = tune.chunk_down > 0 ? tune.chunk_down : (swap ? -1 : 2);
     down.out = down_out;
     down.ld_out = kHidden;
     down.row_dest = row_home;   // rows go to their homes (possibly on other GPUs) instead of down_out
@@ -580,7 +582,7 @@ gw_status run_experts_general(gw_moe_workspace* w, const void* input, uint32_t n
     first.num_groups = 2 * kExperts;
     first.k = kHidden;
     first.c_rows_per_tile = block_n;
-    first.work_chunk = swap ? 1 : 2;
+    first.work_chunk = swap ? -1 : 2;
     first.out = w->gate_up.data;
     first.ld_out = 2 * kInter;
     first.error = device_error_word();
@@ -608,7 +610,7 @@ gw_status run_experts_general(gw_moe_workspace* w, const void* input, uint32_t n
     down.num_groups = kExperts;
     down.k = kInter;
     down.c_rows_per_tile = block_n;
-    down.work_chunk = swap ? 1 : 2;
+    down.work_chunk = swap ? -1 : 2;
     down.out = w->down.data;
     down.ld_out = kHidden;
     down.error = device_error_word();

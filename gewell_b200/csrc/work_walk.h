@@ -4,7 +4,9 @@
 //
 // Normal mode: whole work items in chunks of `chunk` consecutive items; CTA b takes
 // chunks b, b + grid, b + 2 * grid, ...  (consecutive items of a grouped launch share
-// the token tile and the expert, so their descriptors stay hot).
+// the token tile and the expert, so their descriptors stay hot).  chunk < 0: the items in `grid` contiguous ranges that
+// differ by one item at most -- for launches whose tiles are short, where fetching the descriptor of another group
+// (a search and a dependent read of about 1 us) for every tile takes as long as the tile.
 // Split mode (decode shapes): the launch's (item, K-stage) units are cut into `grid`
 // equal contiguous ranges, so a CTA may start and end in the middle of an item's K
 // loop; every SM then streams the same number of weight bytes whatever the number of
@@ -28,6 +30,11 @@ struct SegmentWalk {
       : split(split_), w(0), step(grid), total_work(total_work_), k_stages(k_stages_),
         chunk(chunk_ > 1 ? chunk_ : 1), in_chunk(0) {
     w = cta * chunk;
+    if (chunk_ < 0) {
+      w = int((long long)total_work * cta / grid);
+      total_work = int((long long)total_work * (cta + 1) / grid);
+      chunk = total_work + 1;                          // never left
+    }
     total_units = (long long)total_work * k_stages;
     u_begin = u = total_units * cta / grid;
     u_end = total_units * (cta + 1) / grid;
