@@ -80,22 +80,24 @@ struct Config {
   static_assert(kSmemBytes > 116 * 1024, "one CTA per SM is assumed by the TMEM allocation");
 };
 
+// The descriptor stays where it is (a copy of its 152 bytes per role and tile took longer than a short tile): in global
+// memory, whose lines the producer, which runs ahead, brings into L1, or in the launch's parameters.
 struct WorkItem {
-  GemmGroup g;
+  const GemmGroup* g = nullptr;
   int l_tile, c_tile;
   int l_valid;   // valid lanes (rows of L) in this tile
   int c_valid;   // swap form: valid columns (tokens) in this tile
   int halves;    // boxes of the C operand that hold valid rows in this tile
   int mma_n;     // MMA N for this tile
   int group = -1;   // index of g in the launch's group table (grouped launches)
+  int first = 0;    // the group's first work item
 };
 
 template <int BLOCK_N, GemmEpilogue EPI>
 __device__ __forceinline__ void decode_work(const GemmParams& p, const int32_t* prefix, int w, WorkItem& item) {
   using C = Config<true, BLOCK_N>;
   if (p.groups != nullptr) {
-    // The item decoded into this slot before is usually of the same group: keep its descriptor then
-    // (no search, no global load).  prefix[] holds work_begin of every group plus the total.
+    // The item before is usually of the same group.  prefix[] holds work_begin of every group plus the total.
     if (item.group < 0 || w < prefix[item.group] || w >= prefix[item.group + 1]) {
       // largest gi with work_begin[gi] <= w; the prefix sums were staged in shared memory
       int lo = 0, hi = p.num_groups;
@@ -103,30 +105,32 @@ __device__ __forceinline__ void decode_work(const GemmParams& p, const int32_t* 
         const int mid = (lo + hi) / 2;
         if (prefix[mid] <= w) lo = mid; else hi = mid;
       }
-      item.g = p.groups[lo];
+      item.g = p.groups + lo;
       item.group = lo;
     }
+    item.first = prefix[item.group];
   } else {
-    item.g = p.single;
+    item.g = &p.single;
+    item.first = p.single.work_begin;
   }
-  const int local = w - item.g.work_begin;
+  const int local = w - item.first;
   if constexpr (EPI == GemmEpilogue::swap_store) {
     // consecutive work items share the token tile and sweep the weight tiles
-    item.l_tile = local % item.g.l_tiles;
-    item.c_tile = local / item.g.l_tiles;
+    item.l_tile = local % item.g->l_tiles;
+    item.c_tile = local / item.g->l_tiles;
   } else {
     // consecutive work items share the token tile (L) and sweep the weight tiles (C)
-    item.c_tile = local % item.g.c_tiles;
-    item.l_tile = local / item.g.c_tiles;
+    item.c_tile = local % item.g->c_tiles;
+    item.l_tile = local / item.g->c_tiles;
   }
-  const int l_left = item.g.l_rows - item.l_tile * kTileL;
+  const int l_left = item.g->l_rows - item.l_tile * kTileL;
   item.l_valid = l_left < kTileL ? l_left : kTileL;
-  const int c_left = item.g.c_rows - item.c_tile * p.c_rows_per_tile;
+  const int c_left = item.g->c_rows - item.c_tile * p.c_rows_per_tile;
   item.c_valid = c_left < C::kHalfRows ? c_left : C::kHalfRows;
   // a dense projection whose row count is not a multiple of BLOCK_N leaves the
   // second half of its last column tile empty
   item.halves = C::kHalves;
-  if (C::kHalves == 2 && item.g.c_half_stride != 0 && c_left <= C::kHalfRows) item.halves = 1;
+  if (C::kHalves == 2 && item.g->c_half_stride != 0 && c_left <= C::kHalfRows) item.halves = 1;
   if constexpr (EPI == GemmEpilogue::swap_store) item.mma_n = (item.c_valid + 15) & ~15;   // kHalves == 1
   else item.mma_n = item.halves * C::kHalfRows;
 }
@@ -242,43 +246,44 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
     if (ptx::elect_one()) {
     int stage = 0;
     uint32_t phase = 0;
+    int fetched = -1;                    // group whose descriptor has been asked for
     const uint64_t evict_first = ptx::l2_evict_first(), evict_normal = ptx::l2_evict_normal();
     bool waited = !early_weights;        // this warp defers its wait for the previous kernel (see below)
-    WorkItem item, next;
+    WorkItem item;
     SegmentWalk walk(int(blockIdx.x), int(gridDim.x), split, total_work, k_stages, p.work_chunk);
-    int tile, ks0, ks1, next_tile, next_ks0, next_ks1;
-    bool at_start, next_at_start;
-    bool more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-    if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
-    while (more && !*abort_flag) {
-      item = next; tile = next_tile; ks0 = next_ks0; ks1 = next_ks1; at_start = next_at_start;
-      // the next item's descriptor is fetched while this one is processed
-      more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-      if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
+    int tile, ks0, ks1;
+    bool at_start;
+    while (walk.next(tile, ks0, ks1, at_start) && !*abort_flag) {
+      decode_work<BLOCK_N, EPI>(p, prefix, tile, item);
       (void)tile; (void)at_start;
-      const CUtensorMap* map_l = item.g.map_l >= 0 ? p.map_table + item.g.map_l : &p.map_l;
+      if (p.groups != nullptr && item.group != fetched) {
+        fetched = item.group;
+        ptx::prefetch_l1(item.g);
+        ptx::prefetch_l1(reinterpret_cast<const uint8_t*>(item.g) + 128);
+      }
+      const CUtensorMap* map_l = item.g->map_l >= 0 ? p.map_table + item.g->map_l : &p.map_l;
       const CUtensorMap* map_c[2];
 #pragma unroll
-      for (int h = 0; h < C::kHalves; ++h) map_c[h] = item.g.map_c[h] >= 0 ? p.map_table + item.g.map_c[h] : &p.map_c;
+      for (int h = 0; h < C::kHalves; ++h) map_c[h] = item.g->map_c[h] >= 0 ? p.map_table + item.g->map_c[h] : &p.map_c;
       // The descriptors in map_table were written by the host before any launch that uses
       // them (expert table creation), so ordinary launch ordering makes them visible to the
       // copy engine; no proxy fence is needed per use (one system-scope fence per work item
       // cost more than the item's copies).
-      const int l_row = item.g.l_row0 + item.l_tile * kTileL;
+      const int l_row = item.g->l_row0 + item.l_tile * kTileL;
       // weights on the lanes are read once when there is one column tile
-      const uint64_t l_policy = EPI == GemmEpilogue::swap_store && item.g.c_tiles == 1 ? evict_first : evict_normal;
+      const uint64_t l_policy = EPI == GemmEpilogue::swap_store && item.g->c_tiles == 1 ? evict_first : evict_normal;
       const int c_local = item.c_tile * p.c_rows_per_tile;   // row inside each matrix of the C operand
       const int halves = item.halves;
       // per-item source addresses; per stage they advance by a constant
       const uint8_t* sfl_src = nullptr;
       const uint8_t* sfc_src[2] = {nullptr, nullptr};
       int c_row[2] = {0, 0};
-      if constexpr (kNvfp4) sfl_src = item.g.sf_l + size_t(item.l_tile) * k_atoms * kAtomBytes;
+      if constexpr (kNvfp4) sfl_src = item.g->sf_l + size_t(item.l_tile) * k_atoms * kAtomBytes;
 #pragma unroll
       for (int h = 0; h < C::kHalves; ++h) {
-        c_row[h] = item.g.c_row0 + c_local + h * item.g.c_half_stride;
+        c_row[h] = item.g->c_row0 + c_local + h * item.g->c_half_stride;
         if constexpr (kNvfp4)
-          sfc_src[h] = item.g.sf_c[h] + size_t((c_local + h * item.g.c_half_stride) / 128) * k_atoms * kAtomBytes;
+          sfc_src[h] = item.g->sf_c[h] + size_t((c_local + h * item.g->c_half_stride) / 128) * k_atoms * kAtomBytes;
       }
       // dense direct form: both column halves are consecutive rows of one matrix, so one
       // 256-row box and one two-row box of scale atoms replace four copies (the copy
@@ -367,16 +372,12 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
     if (ptx::elect_one()) {
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
-    WorkItem item, next;
+    WorkItem item;
     SegmentWalk walk(int(blockIdx.x), int(gridDim.x), split, total_work, k_stages, p.work_chunk);
-    int tile, ks0, ks1, next_tile, next_ks0, next_ks1;
-    bool at_start, next_at_start;
-    bool more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-    if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
-    while (more && !*abort_flag) {
-      item = next; tile = next_tile; ks0 = next_ks0; ks1 = next_ks1; at_start = next_at_start;
-      more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-      if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
+    int tile, ks0, ks1;
+    bool at_start;
+    while (walk.next(tile, ks0, ks1, at_start) && !*abort_flag) {
+      decode_work<BLOCK_N, EPI>(p, prefix, tile, item);
       (void)tile; (void)at_start;
       const long long ta = prof ? clock64() : 0;
       if (!ptx::mbar_wait_bounded(acc_empty_bar + acc, acc_phase ^ 1)) {
@@ -456,16 +457,12 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
       const uint32_t quad_lane = uint32_t((warp % 4) * 32) << 16;
       int stage = 0;
       uint32_t phase = 0;
-      WorkItem item, next;
+      WorkItem item;
       SegmentWalk walk(int(blockIdx.x), int(gridDim.x), split, total_work, k_stages, p.work_chunk);
-      int tile, ks0, ks1, next_tile, next_ks0, next_ks1;
-      bool at_start, next_at_start;
-      bool more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-      if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
-      while (more && !*abort_flag) {
-        item = next; tile = next_tile; ks0 = next_ks0; ks1 = next_ks1; at_start = next_at_start;
-        more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-        if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
+      int tile, ks0, ks1;
+      bool at_start;
+      while (walk.next(tile, ks0, ks1, at_start) && !*abort_flag) {
+        decode_work<BLOCK_N, EPI>(p, prefix, tile, item);
         (void)tile; (void)at_start;
         const int halves = item.halves;
         const uint32_t sfc_sub = BLOCK_N < 128 ? uint32_t((item.c_tile * p.c_rows_per_tile) % 128) / 32 : 0;
@@ -533,17 +530,16 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
     const int col_half = (warp - kFirstEpilogueWarp) / 4;  // which half of the accumulator columns this warp drains
     int acc = 0;
     uint32_t acc_phase = 0;
-    WorkItem item, next;
+    WorkItem item;
     SegmentWalk walk(int(blockIdx.x), int(gridDim.x), split, total_work, k_stages, p.work_chunk);
-    int tile, ks0, ks1, next_tile, next_ks0, next_ks1;
-    bool at_start, next_at_start;
-    bool more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-    if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
-    while (more && !*abort_flag) {
-      item = next; tile = next_tile; ks0 = next_ks0; ks1 = next_ks1; at_start = next_at_start;
-      more = walk.next(next_tile, next_ks0, next_ks1, next_at_start);
-      if (more) decode_work<BLOCK_N, EPI>(p, prefix, next_tile, next);
+    int tile, ks0, ks1;
+    bool at_start;
+    while (walk.next(tile, ks0, ks1, at_start) && !*abort_flag) {
+      decode_work<BLOCK_N, EPI>(p, prefix, tile, item);
       (void)tile; (void)at_start;
+      // read while the tile is still being multiplied
+      const float alpha0 = item.g->alpha[0], *channel_alpha = item.g->channel_alpha;
+      const int out_row0 = item.g->out_row0, out_col0 = item.g->out_col0;
       const long long te0 = prof ? clock64() : 0;
       if (!ptx::mbar_wait_warp(acc_full_bar + acc, acc_phase)) {
         report(p.error, 0x40000000u | (blockIdx.x << 8) | acc, abort_flag);
@@ -559,9 +555,8 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
       if constexpr (EPI == GemmEpilogue::swap_store) {
         // lanes = output channels, columns = tokens: out[token][channel]
         bf16* out = static_cast<bf16*>(p.out);
-        float alpha = item.g.alpha[0];
-        if (item.g.channel_alpha != nullptr && l_ok) alpha = item.g.channel_alpha[l_index];
-        bf16* dst = out + (size_t(item.g.out_row0) + size_t(item.c_tile) * BLOCK_N) * p.ld_out + item.g.out_col0 + l_index;
+        const float alpha = channel_alpha != nullptr && l_ok ? channel_alpha[l_index] : alpha0;
+        bf16* dst = out + (size_t(out_row0) + size_t(item.c_tile) * BLOCK_N) * p.ld_out + out_col0 + l_index;
         const bool partial = ks1 - ks0 < k_stages;      // only in split mode
         if (!partial) {
           for (int c0 = col_half * 16; c0 < item.mma_n; c0 += 32) {
@@ -574,9 +569,9 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
                 if (c0 + i < item.c_valid) {
                   bf16* token_dst = dst + size_t(c0 + i) * p.ld_out;
                   if (p.row_dest != nullptr) {   // per-row destinations: the token's row may live on another GPU
-                    const uint64_t home = p.row_dest[size_t(item.g.out_row0) + item.c_tile * BLOCK_N + c0 + i];
+                    const uint64_t home = p.row_dest[size_t(out_row0) + item.c_tile * BLOCK_N + c0 + i];
                     if (home == 0) continue;     // a row without a home (reported when the table was built)
-                    token_dst = reinterpret_cast<bf16*>(home) + item.g.out_col0 + l_index;
+                    token_dst = reinterpret_cast<bf16*>(home) + out_col0 + l_index;
                   }
                   *token_dst = __float2bfloat16_rn(__fmul_rn(__uint_as_float(r[i]), alpha));
                 }
@@ -637,17 +632,17 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
         // 64 contiguous bytes of one row (8 cache lines per store instruction, not 32).
         bf16* out = static_cast<bf16*>(p.out);
         const int c_base = item.c_tile * p.c_rows_per_tile;           // first channel of the tile
-        const int c_end = item.g.c_rows;                              // valid channels of the matrix
+        const int c_end = item.g->c_rows;                              // valid channels of the matrix
         const int group_row = item.l_tile * kTileL + quad * 32 + (lane & ~3);   // first row of this lane group
-        bf16* dst = out + (size_t(item.g.out_row0) + group_row) * p.ld_out + item.g.out_col0 + c_base + 8 * (lane & 3);
+        bf16* dst = out + (size_t(out_row0) + group_row) * p.ld_out + out_col0 + c_base + 8 * (lane & 3);
         const int rows_left = item.l_valid - (quad * 32 + (lane & ~3));          // valid rows from group_row on
         // optional per-row destinations (expert parallelism: a row goes straight to its home)
         uint64_t my_row_dest = 0;
-        if (p.row_dest != nullptr && l_ok) my_row_dest = p.row_dest[size_t(item.g.out_row0) + l_index];
+        if (p.row_dest != nullptr && l_ok) my_row_dest = p.row_dest[size_t(out_row0) + l_index];
         uint64_t group_dest[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) group_dest[i] = __shfl_sync(0xffffffffu, my_row_dest, (lane & ~3) + i);
-        const float alpha = item.g.alpha[0];
+        const float alpha = alpha0;
         const bool hi = (lane & 2) != 0, lo = (lane & 1) != 0;
         constexpr int kColsPerWarp = BLOCK_N / 2;
         constexpr int kChunks = kColsPerWarp / 32;
@@ -664,11 +659,11 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
           ptx::tmem_load_wait();
           if (prof) prof_wait2 += clock64() - td0;
           float v[32];
-          if (item.g.channel_alpha != nullptr) {
+          if (channel_alpha != nullptr) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const int c = c_base + c0 + i;
-              v[i] = __fmul_rn(__uint_as_float(r[i]), c < c_end ? item.g.channel_alpha[c] : 0.0F);
+              v[i] = __fmul_rn(__uint_as_float(r[i]), c < c_end ? channel_alpha[c] : 0.0F);
             }
           } else {
 #pragma unroll
@@ -699,7 +694,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
             if (p.row_dest != nullptr && group_dest[i] == 0) continue;   // a row without a home (reported earlier)
             bf16* row_dst = p.row_dest == nullptr
                                 ? dst + size_t(i) * p.ld_out + c0
-                                : reinterpret_cast<bf16*>(group_dest[i]) + item.g.out_col0 + c_base + 8 * (lane & 3) + c0;
+                                : reinterpret_cast<bf16*>(group_dest[i]) + out_col0 + c_base + 8 * (lane & 3) + c0;
             if (c + 8 <= c_end) {
               *reinterpret_cast<uint4*>(row_dst) = u[i];
             } else {
@@ -753,10 +748,10 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
             ptx::tmem_load_wait();
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              gate_words[8 * j + i] = pack_bf16x2(__fmul_rn(__uint_as_float(g[2 * i]), item.g.alpha[0]),
-                                                  __fmul_rn(__uint_as_float(g[2 * i + 1]), item.g.alpha[0]));
-              up_words[8 * j + i] = pack_bf16x2(__fmul_rn(__uint_as_float(u[2 * i]), item.g.alpha[1]),
-                                                __fmul_rn(__uint_as_float(u[2 * i + 1]), item.g.alpha[1]));
+              gate_words[8 * j + i] = pack_bf16x2(__fmul_rn(__uint_as_float(g[2 * i]), alpha0),
+                                                  __fmul_rn(__uint_as_float(g[2 * i + 1]), alpha0));
+              up_words[8 * j + i] = pack_bf16x2(__fmul_rn(__uint_as_float(u[2 * i]), item.g->alpha[1]),
+                                                __fmul_rn(__uint_as_float(u[2 * i + 1]), item.g->alpha[1]));
             }
           }
         }
@@ -764,10 +759,10 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(acc_empty_bar + acc);        // the next tile's MMAs may start
         if (active) {
-          const size_t row = size_t(item.g.out_row0) + l_index;
+          const size_t row = size_t(out_row0) + l_index;
           uint32_t packed_words[8];
           uint32_t scale_word = 0;
-          const float inverse_scale = item.g.quant_inverse_scale;
+          const float inverse_scale = item.g->quant_inverse_scale;
           bf16* cap_gu = static_cast<bf16*>(p.capture_gate_up);
           bf16* cap_act = static_cast<bf16*>(p.capture_activated);
 #pragma unroll
@@ -815,7 +810,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
             uint4* dst = reinterpret_cast<uint4*>(packed_out);
             dst[0] = make_uint4(packed_words[0], packed_words[1], packed_words[2], packed_words[3]);
             dst[1] = make_uint4(packed_words[4], packed_words[5], packed_words[6], packed_words[7]);
-            const size_t region = size_t(item.g.sf_out_row0) * (width / 16);
+            const size_t region = size_t(item.g->sf_out_row0) * (width / 16);
             *reinterpret_cast<uint32_t*>(p.out_scales + region + scale_offset(l_index, channel0 / 16, width)) = scale_word;
           }
         }

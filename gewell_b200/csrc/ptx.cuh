@@ -150,6 +150,7 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, 
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
       : "memory");
 }
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 // Untiled bulk copy global -> shared; both addresses 16-byte aligned, size a
 // multiple of 16 bytes.
 __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
