@@ -258,6 +258,8 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
   __shared__ int32_t part_sum[kRouteParts][kExperts];
   __shared__ int32_t expert_offset[kExperts];
   __shared__ int32_t warp_totals[4];
+  __shared__ int32_t shared_keys[kChunkTokens * kTopK];
+  const bool one_chunk = chunks <= gridDim.x;       // then the block's bitmaps and keys are still in shared memory in phase 3
   constexpr int kTokensPerWarp = kChunkTokens / (kRouteGridThreads / 32);     // 2
   // ---- phase 1: 32 warps, two tokens each, per chunk
   for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
@@ -267,7 +269,7 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
     for (int t = 0; t < kTokensPerWarp; ++t) {
       const uint32_t local = warp * kTokensPerWarp + t;
       const uint32_t row = chunk * kChunkTokens + local;
-      if (row < rows) route_token(scores, expert_scale, row, local, lane, keys, weights, bitmap, nullptr);
+      if (row < rows) route_token(scores, expert_scale, row, local, lane, keys, weights, bitmap, shared_keys);
     }
     __syncthreads();
     if (threadIdx.x < kExperts) {
@@ -300,6 +302,7 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
       for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x, ++own) {
         const uint32_t q = chunk / per_part;
         int32_t base = before[q];
+#pragma unroll 8
         for (uint32_t c = q * per_part; c < chunk; ++c) base += __ldcg(chunk_counts + size_t(c) * kExperts + e);
         own_base[own][e] = base;
       }
@@ -328,7 +331,7 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
   // ---- phase 3
   uint32_t own = 0;
   for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x, ++own) {
-    if (threadIdx.x < kExperts) {
+    if (!one_chunk && threadIdx.x < kExperts) {
       bitmap[threadIdx.x][0] = __ldcg(bitmaps + (size_t(chunk) * kExperts + threadIdx.x) * 2);
       bitmap[threadIdx.x][1] = __ldcg(bitmaps + (size_t(chunk) * kExperts + threadIdx.x) * 2 + 1);
     }
@@ -338,7 +341,7 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
       const uint32_t row = chunk * kChunkTokens + local;
       if (row >= rows) continue;
       const uint32_t assignment = row * kTopK + i % kTopK;
-      const int32_t e = keys[assignment];
+      const int32_t e = one_chunk ? shared_keys[i] : keys[assignment];
       const uint32_t w0 = bitmap[e][0], w1 = bitmap[e][1];
       const int rank = local < 32 ? __popc(w0 & ((1u << local) - 1u))
                                   : __popc(w0) + __popc(w1 & ((1u << (local - 32)) - 1u));
