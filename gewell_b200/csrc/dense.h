@@ -103,9 +103,12 @@ struct StreamBook {
 
 gw_status launch_dense(const DenseProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
-// product = GeGLU of both projections of a prepared workspace in one launch (projection.cu); *done = false when that is
-// not the faster way here.
+// gw_projection_workspace_run on a stream of the caller's choice (projection.cu).
+gw_status projection_workspace_run_on(gw_projection_workspace* workspace, const gw_projection* projection, const void* input, void* output,
+                                      cudaStream_t stream);
+// product = GeGLU of both projections of a prepared workspace in one launch; *done = false when that is not the faster
+// way here.
 gw_status projection_workspace_run_geglu(gw_projection_workspace* workspace, const gw_projection& gate, const gw_projection& up,
-                                         const void* input, void* product, bool* done);
+                                         const void* input, void* product, cudaStream_t stream, bool* done);
 
 }  // namespace gw

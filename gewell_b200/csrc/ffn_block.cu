@@ -347,6 +347,9 @@ struct DeviceBuffer {
   ~DeviceBuffer() { if (data) cudaFree(data); }
 };
 
+// Rows up to which the shared MLP runs beside the router and the routing; beyond, its GEMMs fill the GPU.
+constexpr uint32_t kForkRows = 128;
+
 constexpr uint32_t kHidden = 2816, kSharedMlp = 2112, kExperts = 128;   // model.h:12-13
 
 }  // namespace
@@ -357,12 +360,22 @@ struct gw_ffn_block {
   cudaStream_t stream = nullptr;
   gw_projection_workspace* projections = nullptr;
   gw_moe_workspace* moe = nullptr;
+  // Small row counts: the shared MLP on a stream of its own beside the router, the routing and the experts' input,
+  // which leave most of the GPU idle.  The router then needs a plan and scratch apart from the shared MLP's.
+  cudaStream_t side = nullptr;
+  cudaEvent_t forked = nullptr, joined = nullptr;
+  gw_bf16_plan* router_plan = nullptr;
+  DeviceBuffer router_scratch;
   DeviceBuffer buffers;                  // one allocation, carved below
   bf16 *normalized = nullptr, *router_input = nullptr, *expert_input = nullptr, *gate = nullptr, *up = nullptr,
        *product = nullptr, *shared_mlp = nullptr, *logits = nullptr, *routed = nullptr;
   ~gw_ffn_block() {
     if (projections) gw_projection_workspace_destroy(projections);
     if (moe) gw_moe_destroy(moe);
+    if (router_plan) gw_bf16_plan_destroy(router_plan);
+    if (forked) cudaEventDestroy(forked);
+    if (joined) cudaEventDestroy(joined);
+    if (side) cudaStreamDestroy(side);
   }
 };
 
@@ -513,6 +526,11 @@ gw_status gw_ffn_block_create(const gw_ffn_block_weights* layers, uint32_t count
   const size_t narrow = align_up(size_t(max_rows) * kSharedMlp * sizeof(bf16), 256);
   const size_t scores = align_up(size_t(max_rows) * kExperts * sizeof(bf16), 256);
   GW_CUDA_CHECK(b->buffers.allocate(5 * wide + 3 * narrow + scores), "feed-forward block buffers");
+  // FP32 partial tiles of the router's K split (<= 128 rows, 128-wide tiles)
+  GW_CUDA_CHECK(b->router_scratch.allocate(size_t(2) * size_t(sm_count()) * 128 * 128 * sizeof(float) + 256), "feed-forward block buffers");
+  GW_CUDA_CHECK(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "feed-forward block stream");
+  GW_CUDA_CHECK(cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming), "feed-forward block event");
+  GW_CUDA_CHECK(cudaEventCreateWithFlags(&b->joined, cudaEventDisableTiming), "feed-forward block event");
   auto* cursor = static_cast<unsigned char*>(b->buffers.data);
   auto carve = [&cursor](size_t bytes) {
     bf16* p = reinterpret_cast<bf16*>(cursor);
@@ -535,7 +553,7 @@ gw_status gw_ffn_block_create(const gw_ffn_block_weights* layers, uint32_t count
 void gw_ffn_block_destroy(gw_ffn_block* block) { delete block; }
 
 size_t gw_ffn_block_bytes(const gw_ffn_block* b) {
-  return b ? b->buffers.bytes + gw_projection_workspace_bytes(b->projections) + gw_moe_bytes(b->moe) : 0;
+  return b ? b->buffers.bytes + b->router_scratch.bytes + gw_projection_workspace_bytes(b->projections) + gw_moe_bytes(b->moe) : 0;
 }
 
 gw_status gw_ffn_block_prepare(gw_ffn_block* b, uint32_t rows, int phase) {
@@ -543,6 +561,15 @@ gw_status gw_ffn_block_prepare(gw_ffn_block* b, uint32_t rows, int phase) {
   if (!b || rows == 0 || rows > b->capacity) return fail(GW_INVALID_ARGUMENT, "feed-forward block: invalid rows");
   const gw_status status = gw_projection_workspace_prepare(b->projections, rows, phase);
   if (status != GW_OK) return status;
+  if (b->rows != rows) {
+    gw_bf16_plan* plan = nullptr;
+    if (rows <= kForkRows) {
+      const gw_status created = gw_bf16_plan_create(rows, kHidden, kExperts, &plan);
+      if (created != GW_OK) return created;
+    }
+    if (b->router_plan) gw_bf16_plan_destroy(b->router_plan);
+    b->router_plan = plan;
+  }
   b->rows = rows;
   b->phase = phase;
   return GW_OK;
@@ -564,23 +591,49 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
                                                   b->expert_input, rows, kHidden, s);
   if (status != GW_OK) return status;
   // shared MLP (batched_executor.cu:256-259)
-  bool product_done = false;
-  if ((status = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, &product_done)) != GW_OK) return status;
-  if (!product_done) {
-    if ((status = gw_projection_workspace_run(b->projections, &w.gate, b->normalized, b->gate)) != GW_OK) return status;
-    if ((status = gw_projection_workspace_run(b->projections, &w.up, b->normalized, b->up)) != GW_OK) return status;
-    if ((status = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, s)) != GW_OK) return status;
+  const bool fork = b->router_plan != nullptr;
+  cudaStream_t shared = as_stream(s);
+  if (fork) {
+    GW_CUDA_CHECK(cudaEventRecord(b->forked, as_stream(s)), "feed-forward block fork");
+    GW_CUDA_CHECK(cudaStreamWaitEvent(b->side, b->forked, 0), "feed-forward block fork");
+    shared = b->side;
   }
-  if ((status = gw_projection_workspace_run(b->projections, &w.down, b->product, b->shared_mlp)) != GW_OK) return status;
+  const auto shared_mlp = [&]() {
+    bool product_done = false;
+    gw_status st = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, shared, &product_done);
+    if (st == GW_OK && !product_done) {
+      st = projection_workspace_run_on(b->projections, &w.gate, b->normalized, b->gate, shared);
+      if (st == GW_OK) st = projection_workspace_run_on(b->projections, &w.up, b->normalized, b->up, shared);
+      if (st == GW_OK) st = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, shared);
+    }
+    return st == GW_OK ? projection_workspace_run_on(b->projections, &w.down, b->product, b->shared_mlp, shared) : st;
+  };
+  status = shared_mlp();
+  // a failed call still brings its side stream back
+  if (fork) {
+    const cudaError_t recorded = cudaEventRecord(b->joined, b->side);
+    if (status != GW_OK) {
+      (void)cudaStreamWaitEvent(as_stream(s), b->joined, 0);
+      return status;
+    }
+    GW_CUDA_CHECK(recorded, "feed-forward block join");
+  }
+  if (status != GW_OK) return status;
   // router logits and the experts (batched_executor.cu:262-266)
-  gw_projection router{};
-  router.storage = GW_STORAGE_BF16;
-  router.input = kHidden;
-  router.output = router.physical_output = kExperts;
-  router.bf16 = w.router_proj;
-  if ((status = gw_projection_workspace_run(b->projections, &router, b->router_input, b->logits)) != GW_OK) return status;
-  status = gw_moe_run(b->moe, b->expert_input, b->logits, w.router_per_expert_scale, w.experts, b->routed, rows,
-                      w.has_bf16, w.has_fp8, w.has_nvfp4, gw_nvfp4_fp4_activations(b->policy, b->phase), s);
+  if (fork) {
+    status = gw_bf16_plan_run(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes, s);
+  } else {
+    gw_projection router{};
+    router.storage = GW_STORAGE_BF16;
+    router.input = kHidden;
+    router.output = router.physical_output = kExperts;
+    router.bf16 = w.router_proj;
+    status = gw_projection_workspace_run(b->projections, &router, b->router_input, b->logits);
+  }
+  if (status == GW_OK)
+    status = gw_moe_run(b->moe, b->expert_input, b->logits, w.router_per_expert_scale, w.experts, b->routed, rows,
+                        w.has_bf16, w.has_fp8, w.has_nvfp4, gw_nvfp4_fp4_activations(b->policy, b->phase), s);
+  if (fork) GW_CUDA_CHECK(cudaStreamWaitEvent(as_stream(s), b->joined, 0), "feed-forward block join");
   if (status != GW_OK) return status;
   return gw_ffn_tail_bf16(b->shared_mlp, b->routed, w.post_feedforward_norm_1, w.post_feedforward_norm_2,
                           w.post_feedforward_norm, w.layer_scalar, hidden_bf16, rows, kHidden, s);

@@ -295,6 +295,15 @@ gw_status gw_projection_workspace_prepare(gw_projection_workspace* w, uint32_t r
 
 gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_projection* projection,
                                       const void* input_bf16, void* output_bf16) {
+  return gw::projection_workspace_run_on(w, projection, input_bf16, output_bf16, w ? w->stream : nullptr);
+}
+
+}  // extern "C"
+
+namespace gw {
+
+gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_projection* projection, const void* input_bf16,
+                                      void* output_bf16, cudaStream_t stream) {
   clear_error();
   if (!w || !projection || w->rows == 0 || !input_bf16 || !output_bf16)
     return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
@@ -305,7 +314,7 @@ gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_proje
   // NVFP4 at small row counts: into the caller's rows at once, and with BF16 activations from the packed weights
   if (p.storage == GW_STORAGE_NVFP4_W4A4 && (padded || !w->fp4)) {
     bool done = false;
-    const gw_status status = w->streaming.run(p, nullptr, input_bf16, output_bf16, w->fp4, w->scratch.data, w->stream, &done);
+    const gw_status status = w->streaming.run(p, nullptr, input_bf16, output_bf16, w->fp4, w->scratch.data, stream, &done);
     if (status != GW_OK || done) return status;
   }
   void* destination = padded ? w->padded.data : output_bf16;
@@ -318,11 +327,11 @@ gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_proje
   if (kind == kPlanFp8) {
     if (!plans.fp8) return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
     status = gw_fp8_plan_run(plans.fp8, input_bf16, p.fp8_data, p.fp8_input_scale, p.fp8_weight_scale, nullptr,
-                             destination, w->scratch.data, w->scratch.bytes, w->stream, GW_TRANSFORM_IDENTITY);
+                             destination, w->scratch.data, w->scratch.bytes, stream, GW_TRANSFORM_IDENTITY);
   } else if (kind == kPlanNvfp4) {
     if (!plans.nvfp4) return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
     status = gw_nvfp4_plan_run(plans.nvfp4, input_bf16, p.nvfp4_data, p.nvfp4_scales, p.nvfp4_input_scale,
-                               p.nvfp4_weight_scale, destination, w->scratch.data, w->scratch.bytes, w->stream,
+                               p.nvfp4_weight_scale, destination, w->scratch.data, w->scratch.bytes, stream,
                                GW_TRANSFORM_IDENTITY);
   } else {
     if (!plans.bf16) return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
@@ -331,35 +340,31 @@ gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_proje
       if (!w->dequantized.data || size_t(p.physical_output) * p.input * sizeof(bf16) > w->dequantized.bytes)
         return fail(GW_INVALID_ARGUMENT, "projection was not among the workspace's bindings");
       status = gw_nvfp4_dequantize(p.nvfp4_data, p.nvfp4_scales, p.nvfp4_weight_scale, p.input, p.physical_output,
-                                   w->dequantized.data, w->stream);
+                                   w->dequantized.data, stream);
       if (status != GW_OK) return status;
       weights = w->dequantized.data;
     }
     const bool split = w->scratch.data && w->scratch.bytes >= gw_bf16_plan_scratch_bytes(plans.bf16);
     status = gw_bf16_plan_run(plans.bf16, input_bf16, weights, destination, split ? w->scratch.data : nullptr,
-                              split ? w->scratch.bytes : 0, w->stream);
+                              split ? w->scratch.bytes : 0, stream);
   }
   if (status != GW_OK) return status;
   if (padded) {
     const bool vector = p.output % 8 == 0 && p.physical_output % 8 == 0 && reinterpret_cast<uintptr_t>(output_bf16) % 16 == 0;
     const uint32_t per_block = vector ? 2048 : 256;
     GW_CUDA_CHECK(launch_pdl(vector ? compact_rows_kernel<true> : compact_rows_kernel<false>,
-                             dim3((p.output + per_block - 1) / per_block, std::min<uint32_t>(w->rows, 65535)), 256, w->stream,
+                             dim3((p.output + per_block - 1) / per_block, std::min<uint32_t>(w->rows, 65535)), 256, stream,
                              static_cast<const bf16*>(destination), static_cast<bf16*>(output_bf16), w->rows, p.output, p.physical_output),
                   "compact 26B projection output");
   }
   return GW_OK;
 }
 
-}  // extern "C"
-
-namespace gw {
-
 gw_status projection_workspace_run_geglu(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up, const void* input,
-                                         void* product, bool* done) {
+                                         void* product, cudaStream_t stream, bool* done) {
   *done = false;
   if (w->rows == 0) return GW_OK;
-  return w->streaming.run(gate, &up, input, product, w->fp4, w->scratch.data, w->stream, done);
+  return w->streaming.run(gate, &up, input, product, w->fp4, w->scratch.data, stream, done);
 }
 
 }  // namespace gw
