@@ -609,12 +609,23 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
               float sum[16];
 #pragma unroll
               for (int i = 0; i < 16; ++i) sum[i] = 0.0F;
-              for (int cta = cta_first; cta <= cta_last; ++cta) {
-                // the tile is the first segment of every CTA but (possibly) the first one
-                const int which = (cta == cta_first && walk.range_begin(cta) < tile_first_unit) ? 1 : 0;
-                const float* theirs = p.split_partials + (size_t(cta) * 2 + which) * size_t(kTileL * BLOCK_N);
+              // four CTAs' partials are in flight at a time; they are added one by one, in order
+              for (int cta0 = cta_first; cta0 <= cta_last; cta0 += 4) {
+                float part[4][16];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) sum[i] += __ldcg(theirs + (c0 + i) * kTileL + row);
+                for (int j = 0; j < 4; ++j) {
+                  const int cta = min(cta0 + j, cta_last);
+                  // the tile is the first segment of every CTA but (possibly) the first one
+                  const int which = (cta == cta_first && walk.range_begin(cta) < tile_first_unit) ? 1 : 0;
+                  const float* theirs = p.split_partials + (size_t(cta) * 2 + which) * size_t(kTileL * BLOCK_N);
+#pragma unroll
+                  for (int i = 0; i < 16; ++i) part[j][i] = __ldcg(theirs + (c0 + i) * kTileL + row);
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  if (cta0 + j <= cta_last)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) sum[i] += part[j][i];
               }
               if (l_ok) {
 #pragma unroll

@@ -639,8 +639,9 @@ moe_quantize_kernel(const uint4* __restrict__ input, const int32_t* __restrict__
                     const MoeExpertInfo* __restrict__ experts, uint32_t n, uint32_t scale_rows, int projection,
                     uint32_t gather_divisor, uint32_t* __restrict__ packed, uint8_t* __restrict__ scales,
                     uint4* __restrict__ activated) {
-  griddep_launch();
   griddep_wait();     // results of earlier kernels in the stream are read from here on
+  // Only now: the GEMM that follows fills every SM, and its blocks would keep out other streams' kernels while they wait.
+  griddep_launch();
   constexpr uint32_t kVectors = K / 8;          // even: the two threads of a block are neighbours in a warp
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   const uint32_t part = blockIdx.y;             // gate/up copy (0 unless the scales differ)
@@ -710,8 +711,9 @@ moe_quantize_tokens_kernel(const uint4* __restrict__ input, const int32_t* __res
                            const int32_t* __restrict__ inverse, const int32_t* __restrict__ offsets,
                            const MoeExpertInfo* __restrict__ experts, uint32_t tokens, uint32_t scale_rows, int parts,
                            uint2* __restrict__ packed, uint8_t* __restrict__ scales) {
-  griddep_launch();
   griddep_wait();     // results of earlier kernels in the stream are read from here on
+  // Only now: the GEMM that follows fills every SM, and its blocks would keep out other streams' kernels while they wait.
+  griddep_launch();
   // Two warps per token, each with one half of the row (88 K16 blocks, three per lane): half the
   // registers of a whole row per warp, so twice as many warps are resident to cover the loads.
   constexpr uint32_t kBlocks = kHidden / 16;            // 176
