@@ -69,6 +69,27 @@ bool stream_pair_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, ui
   return bytes <= (size_t(40) << 20) || size_t(rows) * k <= 8192;
 }
 
+namespace {
+// CTAs of a swap-form launch that divides the K loops of its `tiles` among them, or 0: whole tiles are faster.
+// Dividing costs about 3.4 us (32 token columns; 4.3 with 64, 8 with 128) for the partial sums, the fence, the counter and
+// the reading back, and more with more than four CTAs a tile; it gains what an uneven or nearly empty wave of tiles
+// leaves idle.  A K stage takes 0.28 (NVFP4) / 0.5 (FP8, two slabs) / 0.2 us (BF16) of latency, and no less than its bytes
+// at 5.2 TB/s over the CTAs that run.  Measured, divided over all SMs -> whole tiles (us): NVFP4 32x2816x2816 12.8 -> 7.6,
+// 64x2816x2816 16.3 -> 8.9, 24x5376x8192 14.4 -> 10.4, FP8 64x2816x2816 15.3 -> 8.9; BF16 64x2816x128 stays divided, by
+// four: 12.4 -> 9.9.
+int swap_split_grid(GemmKind kind, int tiles, int stages, int block_n) {
+  const int sms = sm_count();
+  const double latency = kind == GemmKind::nvfp4 ? 0.28 : kind == GemmKind::fp8 ? 0.5 : 0.2;
+  const double bytes = kind == GemmKind::nvfp4 ? 18e3 : kind == GemmKind::fp8 ? 32e3 : 16e3;
+  const auto stage_us = [&](int ctas) { return std::max(latency, bytes * ctas / 5.2e6); };
+  const int whole_grid = std::min(tiles, sms);
+  const double whole = double((tiles + whole_grid - 1) / whole_grid) * stages * stage_us(whole_grid);
+  const int grid = int(std::min<long long>({(long long)(tiles) * stages, (long long)(sms), 4ll * tiles}));
+  const double divided = double(tiles) * stages / grid * stage_us(grid) + (block_n <= 32 ? 3.4 : block_n <= 64 ? 4.3 : 8.0);
+  return divided < whole ? grid : 0;
+}
+}  // namespace
+
 size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n) {
   (void)n;
   if (!dense_uses_swap_form(tuning, rows) || tuning.no_split) return 0;
@@ -334,12 +355,13 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
   params.total_work = g.l_tiles * g.c_tiles;
   int grid = params.total_work < sm_count() ? params.total_work : sm_count();
   if (swap && q.split_workspace != nullptr && cache->split_counters != nullptr) {
-    params.split_counters = cache->split_counters;
-    params.split_partials = static_cast<float*>(q.split_workspace);
-    const long long stages = (long long)gemm_tc_k_stages(q.kind, GemmEpilogue::swap_store, row_bytes) * params.total_work;
-    // A tile's partial sums are added by one CTA, about 0.25 us for each that has some, and a K stage takes 0.4 us: of a
-    // matrix of few tiles no more than eight CTAs share one (router 64x2816x128, BF16: 44 CTAs 40 us, 8 CTAs 10.4 us).
-    grid = int(std::min<long long>({stages, (long long)(sm_count()), 8ll * params.total_work}));
+    const int stages = gemm_tc_k_stages(q.kind, GemmEpilogue::swap_store, row_bytes);
+    const int split_grid = swap_split_grid(q.kind, params.total_work, stages, block_n);
+    if (split_grid > 0) {
+      params.split_counters = cache->split_counters;
+      params.split_partials = static_cast<float*>(q.split_workspace);
+      grid = split_grid;
+    }
   }
   GW_CUDA_CHECK(launch_gemm_tc(q.kind, swap ? GemmEpilogue::swap_store : GemmEpilogue::direct_store, block_n, params,
                                grid, stream),
