@@ -38,35 +38,30 @@ size_t split_counter_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n)
 }
 }  // namespace
 
-// Where the weight-streaming kernel is the faster one for rows <= 16 (B200, both timed back to back, us; old = activation
-// quantiser + tcgen05 swap form): NVFP4 16x2816x2816 15.3 -> 9.3, 8x5376x43008 32.6 -> 33, 1x21504x5376 24.1 -> 20.9; FP8
-// 8x5376x43008 46.3 -> 42.6.  It saves the quantiser's launch and the tensor-memory prologue; what it pays is that every SM
-// reads and quantises all of the activations: about 1 us per 16K values, which meets the gain at 64K.  Nine and more
-// rows need a second token group (half as many instructions again per weight byte), which only small matrices hide.
+// Where the weight-streaming kernel is the faster one (B200, cold weights, us; streamed against activation quantiser +
+// tcgen05 swap form): NVFP4 1x2816x2816 5.4 / 7.1, 8x2816x2816 6.8 / 7.3, 2x8192x5376 13.1 / 14.4, but 16x2816x2816 9.6 / 7.3,
+// 4x2816x8192 9.8 / 8.2, 8x5376x4096 10.1 / 10.4, 1x21504x5376 22.1 / 19.9; FP8 8x2816x2816 6.4 / 8.1, 16x4096x2816 10.1 / 8.6;
+// BF16 8x2816x2816 7.0 / 8.7, 4x5376x16384 33.0 / 30.2.  It saves the quantiser's launch and the tensor-memory prologue and
+// uses every SM where there are few tiles; what it pays is that every SM reads and quantises all of the activations.
 // W4A16 has no other kernel that reads the packed weights.
 bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
   if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
-  const size_t values = size_t(rows) * k;
-  const size_t bytes = n * k * (kind == StreamKind::w4a4 ? 9 : kind == StreamKind::w8a8 ? 16 : 32) / 16;
-  if (values > 65536) return false;
-  if (plan.tiles == 2 && values > 46 * 1024 && bytes > (size_t(20) << 20)) return false;
-  // BF16 tokens of more than 8192 values need several slabs: twice the sums
-  return kind != StreamKind::w16a16 || plan.slabs == 1 || bytes <= (size_t(48) << 20);
+  return plan.tiles == 1 && n <= 5376 && k <= 16384 && size_t(rows) * k <= 24 * 1024;
 }
 
 // Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each.
 constexpr uint32_t kW4a16Rows = 48;
 
 // Gate, up and GeGLU as one streaming launch (n: channels of each) against the joined GEMM whose GeGLU rides in the next
-// quantiser.  Of the large quantised pairs only one or two tokens win (chain 5376 -> 21504 -> 5376, us, streamed against
-// joined: NVFP4 1 row 55.5 / 59.2, 2 rows 58.3 / 58.1, 8 rows 61.5 / 58.0; FP8 71.1 / 74.2, 4 rows 75.8 / 74.8): every SM
-// quantises all activations and does the GeGLU of its own channels after its last byte.  BF16 has nothing to quantise
-// (8 rows 121.7 / 122.9).
+// quantiser (whole chains of hidden -> n -> hidden, us, streamed / joined): NVFP4 4 rows 1408 -> 4096 18.0 / 20.7, 8 rows of
+// the feed-forward block (2816 -> 2112) 94 / 97.5, 4 rows 2816 -> 8192 28.4 / 23.0; 5376 -> 21504 1 row 51.6 / 53.9, 8 rows
+// 55.1 / 54.2; FP8 1 row 68.4 / 69.0, 8 rows 71.5 / 69.8.  So: small matrices, whose joined GEMM leaves SMs idle, and
+// large ones for one token, where the launches it saves are all there is to gain.
 bool stream_pair_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
-  if (!stream_pays(kind, plan, rows, k, 2 * n)) return false;
-  if (kind != StreamKind::w4a4 && kind != StreamKind::w8a8) return true;
-  const size_t bytes = 2 * n * k * (kind == StreamKind::w4a4 ? 9 : 16) / 16;
-  return bytes <= (size_t(40) << 20) || size_t(rows) * k <= 8192;
+  if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
+  const size_t bytes = 2 * n * k * (kind == StreamKind::w4a4 ? 9 : kind == StreamKind::w8a8 ? 16 : 32) / 16;
+  const size_t values = size_t(rows) * k;
+  return plan.tiles == 1 && (n <= 4224 ? values <= 24 * 1024 : bytes >= (size_t(96) << 20) && values <= 8192);
 }
 
 namespace {
