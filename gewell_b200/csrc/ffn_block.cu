@@ -27,9 +27,11 @@
 #include <string>
 #include <vector>
 
+#include "combine.cuh"
 #include "common.cuh"
 #include "dense.h"
 #include "kernels.h"
+#include "moe_kernels.h"
 
 using namespace gw;
 
@@ -218,16 +220,23 @@ __global__ void __launch_bounds__(kNormThreads) rms_norm_feedforward_kernel(Norm
 }
 
 struct TailArgs {
-  const bf16 *shared_mlp, *routed;                    // [rows, width]: shared MLP output, MoE output
+  const bf16* shared_mlp;                             // [rows, width]: shared MLP output
+  bf16* routed;                                       // MoE output
   const bf16 *norm_shared, *norm_routed, *norm_sum;   // post_feedforward_norm_1, _2, post_feedforward_norm
   const bf16* layer_scalar;                           // [1]
   bf16* hidden;                                       // [rows, width], updated in place
+  // COMBINE: `routed` is this kernel's output as well, the weighted sum of the token's eight expert rows
+  const uint4* down;
+  const int32_t* inverse;
+  const float* weights;
 };
+constexpr int kTopK = 8;
 
 // shared = norm1(shared_mlp); branch = norm2(routed); sum = bf16(shared + branch); branch = norm3(sum);
 // hidden = bf16(hidden + branch); hidden = bf16(hidden * scalar)        (batched_executor.cu:260,278-285)
-template <int NV>
+template <int NV, bool COMBINE>
 __global__ void __launch_bounds__(kNormThreads) ffn_tail_kernel(NormArgs a, TailArgs t) {
+  static_assert(!COMBINE || NV == 1, "one vector a thread");
   extern __shared__ __align__(16) unsigned char norm_smem[];
   bf16* first = reinterpret_cast<bf16*>(norm_smem);
   bf16* second = first + a.width;
@@ -242,7 +251,20 @@ __global__ void __launch_bounds__(kNormThreads) ffn_tail_kernel(NormArgs a, Tail
   const float scalar = as_float(*t.layer_scalar);
   griddep_wait();
   shared.load(t.shared_mlp + base, vectors);
-  branch.load(t.routed + base, vectors);
+  if constexpr (COMBINE) {
+    __shared__ int32_t slot_row[kTopK];
+    __shared__ float slot_weight[kTopK];
+    if (threadIdx.x < kTopK) {
+      slot_row[threadIdx.x] = t.inverse[size_t(blockIdx.x) * kTopK + threadIdx.x];
+      slot_weight[threadIdx.x] = t.weights[size_t(blockIdx.x) * kTopK + threadIdx.x];
+    }
+    __syncthreads();
+    branch.part[0].bits = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < vectors) branch.part[0].bits = combine_rows<kTopK>(t.down, slot_row, slot_weight, vectors, threadIdx.x);
+    branch.store(t.routed + base, vectors);
+  } else {
+    branch.load(t.routed + base, vectors);
+  }
   hidden.load_any(t.hidden + base, vectors);
   shared.store(first, vectors);
   branch.store(second, vectors);
@@ -431,16 +453,16 @@ gw_status gw_ffn_tail_bf16(const void* shared_mlp_bf16, const void* routed_bf16,
     return fail(GW_INVALID_ARGUMENT, "feed-forward tail requires two 16-byte aligned inputs, three norm weights, "
                                      "the layer scalar and the hidden state");
   const NormArgs a = norm_args(shared_mlp_bf16, rows, width);
-  const TailArgs t{static_cast<const bf16*>(shared_mlp_bf16), static_cast<const bf16*>(routed_bf16),
+  const TailArgs t{static_cast<const bf16*>(shared_mlp_bf16), static_cast<bf16*>(const_cast<void*>(routed_bf16)),
                    static_cast<const bf16*>(norm_shared_weight), static_cast<const bf16*>(norm_routed_weight),
                    static_cast<const bf16*>(norm_sum_weight), static_cast<const bf16*>(layer_scalar_bf16),
-                   static_cast<bf16*>(hidden_bf16)};
+                   static_cast<bf16*>(hidden_bf16), nullptr, nullptr, nullptr};
   const size_t shared_bytes = norm_shared_bytes(width, a.lanes, 2);
   const uint32_t nv = norm_vectors(width);
-  const auto kernel = nv == 1 ? ffn_tail_kernel<1> : nv == 2 ? ffn_tail_kernel<2> : ffn_tail_kernel<4>;
+  const auto kernel = nv == 1 ? ffn_tail_kernel<1, false> : nv == 2 ? ffn_tail_kernel<2, false> : ffn_tail_kernel<4, false>;
   static bool raised[kMaxDeviceSlots] = {};
   if (shared_bytes > 48 * 1024 && !raised[current_device_slot()]) {   // only rows of more than 12000 values: four vectors a thread
-    GW_CUDA_CHECK(cudaFuncSetAttribute(ffn_tail_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024),
+    GW_CUDA_CHECK(cudaFuncSetAttribute(ffn_tail_kernel<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024),
                   "feed-forward tail shared memory");
     raised[current_device_slot()] = true;
   }
@@ -630,13 +652,23 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
     router.bf16 = w.router_proj;
     status = gw_projection_workspace_run(b->projections, &router, b->router_input, b->logits);
   }
+  MoeCombineInput combine;
   if (status == GW_OK)
-    status = gw_moe_run(b->moe, b->expert_input, b->logits, w.router_per_expert_scale, w.experts, b->routed, rows,
-                        w.has_bf16, w.has_fp8, w.has_nvfp4, gw_nvfp4_fp4_activations(b->policy, b->phase), s);
+    status = moe_run_to_down(b->moe, b->expert_input, b->logits, w.router_per_expert_scale, w.experts, rows, w.has_bf16, w.has_fp8,
+                             w.has_nvfp4, gw_nvfp4_fp4_activations(b->policy, b->phase), as_stream(s), &combine);
   if (fork) GW_CUDA_CHECK(cudaStreamWaitEvent(as_stream(s), b->joined, 0), "feed-forward block join");
   if (status != GW_OK) return status;
-  return gw_ffn_tail_bf16(b->shared_mlp, b->routed, w.post_feedforward_norm_1, w.post_feedforward_norm_2,
-                          w.post_feedforward_norm, w.layer_scalar, hidden_bf16, rows, kHidden, s);
+  // the experts' weighted sum and the block's tail in one launch
+  const NormArgs a = norm_args(b->shared_mlp, rows, kHidden);
+  const TailArgs t{b->shared_mlp, b->routed, static_cast<const bf16*>(w.post_feedforward_norm_1),
+                   static_cast<const bf16*>(w.post_feedforward_norm_2), static_cast<const bf16*>(w.post_feedforward_norm),
+                   static_cast<const bf16*>(w.layer_scalar), static_cast<bf16*>(hidden_bf16), static_cast<const uint4*>(combine.down),
+                   combine.inverse, combine.weights};
+  static_assert(kHidden / 8 <= kNormThreads, "one vector a thread");
+  GW_CUDA_CHECK(launch_pdl_shared(ffn_tail_kernel<1, true>, rows, norm_threads(kHidden), norm_shared_bytes(kHidden, a.lanes, 2), as_stream(s), a, t),
+                "feed-forward tail");
+  moe_mark_combined(b->moe, as_stream(s));
+  return GW_OK;
 }
 
 const void* gw_ffn_block_buffer(const gw_ffn_block* b, int which) {

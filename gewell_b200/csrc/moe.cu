@@ -319,6 +319,59 @@ gw_status gw_moe_create_ex(uint32_t max_rows, uint32_t flags, gw_moe_workspace**
 
 void gw_moe_destroy(gw_moe_workspace* workspace) { delete workspace; }
 
+}  // extern "C"
+
+namespace {
+
+GemmGroup* first_groups_of(gw_moe_workspace* w) { return w->groups.as<GemmGroup>(); }
+GemmGroup* down_groups_of(gw_moe_workspace* w) { return w->groups.as<GemmGroup>() + 2 * kExperts + 1; }
+
+// `plan` != nullptr: the routing launch of a small batch writes the plan's group descriptors too
+gw_status dispatch(gw_moe_workspace* w, const void* scores, const void* expert_scales, uint32_t rows, const MoeGroupPlan* plan, cudaStream_t s) {
+  GW_CUDA_CHECK(launch_moe_dispatch(scores, expert_scales, rows, w->keys, w->weights, w->bitmaps.as<uint32_t>(),
+                                    w->chunk_counts, w->offsets, w->sorted_assignments, w->sorted_keys, w->inverse,
+                                    w->route_barrier.as<uint32_t>(), device_error_word(), sm_count(),
+                                    !w->tuning.route_three_launches, s, plan, first_groups_of(w), down_groups_of(w)),
+                "MoE dispatch");
+  return GW_OK;
+}
+
+// How the expert GEMMs of an NVFP4 table run over n sorted rows.
+struct ExpertPlan {
+  int form;
+  bool pair_first, pair_down;
+  MoeGroupPlan groups;
+  bool needs_groups() const { return !(pair_first && pair_down); }
+};
+ExpertPlan plan_experts(gw_moe_workspace* w, const gw_expert_table* table, const int32_t* offsets, uint32_t n) {
+  const MoeTuning& tune = w->tuning;
+  int form = n <= 8 * 512 ? kMoeFormSwap : (table->shared_gate_up ? kMoeFormFused : kMoeFormDirect);
+  if (tune.form == 's') form = kMoeFormSwap;
+  if (tune.form == 'd') form = kMoeFormDirect;
+  if (tune.form == 'f' && table->shared_gate_up) form = kMoeFormFused;
+  // Large batches run on CTA pairs: the gate/up GEMM when one quantised copy of a row serves both
+  // projections (the fused plan), the down GEMM whenever tokens sit on the lanes.
+  const bool pair_first = form == kMoeFormFused && !tune.no_pair;
+  const bool pair_down = form != kMoeFormSwap && !tune.no_pair;
+  int block_n_first, block_n_down;
+  if (form == kMoeFormSwap) {
+    block_n_first = n <= 8 * 64 ? 32 : (n <= 8 * 256 ? 64 : 128);
+    if (tune.block_n == 32 || tune.block_n == 64 || tune.block_n == 128) block_n_first = tune.block_n;
+    block_n_down = block_n_first;
+  } else {
+    block_n_first = form == kMoeFormFused ? 256 : (tune.block_n == 256 ? 256 : 128);
+    block_n_down = tune.block_n_down == 256 ? 256 : 128;
+  }
+  return ExpertPlan{form, pair_first, pair_down,
+                    MoeGroupPlan{offsets, table->info.as<MoeExpertInfo>(), w->scales_in.as<uint8_t>(), w->scales_act.as<uint8_t>(), n,
+                                 w->scale_rows, form, block_n_first, block_n_down, table->shared_gate_up ? 1 : 0, device_error_word(),
+                                 kMoeKindNvfp4, 1}};
+}
+
+}  // namespace
+
+extern "C" {
+
 gw_status gw_moe_dispatch(gw_moe_workspace* w, const void* scores_bf16, const void* expert_scales_bf16, uint32_t rows,
                           void* stream) {
   clear_error();
@@ -326,12 +379,7 @@ gw_status gw_moe_dispatch(gw_moe_workspace* w, const void* scores_bf16, const vo
   if (rows > w->max_rows) return fail(GW_INVALID_ARGUMENT, "MoE rows exceed workspace");
   if (!rows) return GW_OK;
   if (!scores_bf16 || !expert_scales_bf16) return fail(GW_INVALID_ARGUMENT, "MoE dispatch requires scores and expert scales");
-  GW_CUDA_CHECK(launch_moe_dispatch(scores_bf16, expert_scales_bf16, rows, w->keys, w->weights, w->bitmaps.as<uint32_t>(),
-                                    w->chunk_counts, w->offsets, w->sorted_assignments, w->sorted_keys, w->inverse,
-                                    w->route_barrier.as<uint32_t>(), device_error_word(), sm_count(),
-                                    !w->tuning.route_three_launches, as_stream(stream)),
-                "MoE dispatch");
-  return GW_OK;
+  return dispatch(w, scores_bf16, expert_scales_bf16, rows, nullptr, as_stream(stream));
 }
 
 }  // extern "C"
@@ -359,37 +407,21 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
                       const int32_t* offsets, uint32_t n, const gw_expert_table* table, void* down_out, cudaStream_t s,
                       const void* records = nullptr, const uint64_t* row_home = nullptr,
                       int stages = kStageFirst | kStageDown, void* activation_records = nullptr,
-                      bool* exported = nullptr) {
+                      bool* exported = nullptr, bool groups_ready = false) {
   if (!table->all_nvfp4)
     return fail(GW_UNSUPPORTED, "this entry point runs NVFP4 (W4A4) expert tables only; mixed tables run through gw_moe_run");
   const auto* info = table->info.as<MoeExpertInfo>();
-  auto* first_groups = w->groups.as<GemmGroup>();
-  auto* down_groups = first_groups + 2 * kExperts + 1;
+  auto* first_groups = first_groups_of(w);
+  auto* down_groups = down_groups_of(w);
   const MoeTuning& tune = w->tuning;
-  int form = n <= 8 * 512 ? kMoeFormSwap : (table->shared_gate_up ? kMoeFormFused : kMoeFormDirect);
-  if (tune.form == 's') form = kMoeFormSwap;
-  if (tune.form == 'd') form = kMoeFormDirect;
-  if (tune.form == 'f' && table->shared_gate_up) form = kMoeFormFused;
-  // Large batches run on CTA pairs: the gate/up GEMM when one quantised copy of a row serves both
-  // projections (the fused plan), the down GEMM whenever tokens sit on the lanes.
-  const bool pair_first = form == kMoeFormFused && !tune.no_pair;
-  const bool pair_down = form != kMoeFormSwap && !tune.no_pair;
-  int block_n_first, block_n_down;
-  if (form == kMoeFormSwap) {
-    block_n_first = n <= 8 * 64 ? 32 : (n <= 8 * 256 ? 64 : 128);
-    if (tune.block_n == 32 || tune.block_n == 64 || tune.block_n == 128) block_n_first = tune.block_n;
-    block_n_down = block_n_first;
-  } else {
-    block_n_first = form == kMoeFormFused ? 256 : (tune.block_n == 256 ? 256 : 128);
-    block_n_down = tune.block_n_down == 256 ? 256 : 128;
-  }
+  const ExpertPlan plan = plan_experts(w, table, offsets, n);
+  const int form = plan.form;
+  const bool pair_first = plan.pair_first, pair_down = plan.pair_down;
+  const int block_n_first = plan.groups.block_n_first, block_n_down = plan.groups.block_n_down;
   const int parts = table->shared_gate_up ? 1 : 2;
   w->mark(1, s);
-  if (!(pair_first && pair_down)) {
-    MoeGroupPlan plan{offsets, info, w->scales_in.as<uint8_t>(), w->scales_act.as<uint8_t>(), n, w->scale_rows, form,
-                      block_n_first, block_n_down, table->shared_gate_up ? 1 : 0, device_error_word(), kMoeKindNvfp4, 1};
-    GW_CUDA_CHECK(launch_moe_prepare_groups(plan, first_groups, down_groups, s), "MoE group descriptors");
-  }
+  if (plan.needs_groups() && !groups_ready)
+    GW_CUDA_CHECK(launch_moe_prepare_groups(plan.groups, first_groups, down_groups, s), "MoE group descriptors");
   if (!(stages & kStageFirst)) {
     // the down input is in place already
   } else if (records != nullptr) {
@@ -624,15 +656,16 @@ gw_status run_experts_general(gw_moe_workspace* w, const void* input, uint32_t n
 
 extern "C" {
 
-gw_status gw_moe_run(gw_moe_workspace* w, const void* input_bf16, const void* scores_bf16,
-                     const void* expert_scales_bf16, const gw_expert_table* table, void* output_bf16, uint32_t rows,
-                     int has_bf16, int has_fp8, int has_nvfp4, int fp4, void* stream) {
-  clear_error();
+}  // extern "C"
+
+namespace gw {
+
+gw_status moe_run_to_down(gw_moe_workspace* w, const void* input_bf16, const void* scores_bf16, const void* expert_scales_bf16,
+                          const gw_expert_table* table, uint32_t rows, int has_bf16, int has_fp8, int has_nvfp4, int fp4, cudaStream_t s,
+                          MoeCombineInput* combine) {
   if (!w) return fail(GW_INVALID_ARGUMENT, "MoE run requires a workspace");
   if (rows > w->max_rows) return fail(GW_INVALID_ARGUMENT, "MoE rows exceed workspace");
-  if (!rows) return GW_OK;
-  if (!input_bf16 || !scores_bf16 || !expert_scales_bf16 || !table || !output_bf16 ||
-      reinterpret_cast<uintptr_t>(input_bf16) % 16 || reinterpret_cast<uintptr_t>(output_bf16) % 16)
+  if (!input_bf16 || !scores_bf16 || !expert_scales_bf16 || !table || reinterpret_cast<uintptr_t>(input_bf16) % 16)
     return fail(GW_INVALID_ARGUMENT, "MoE run requires 16-byte aligned input/output, scores, expert scales and a bound expert table");
   // The storage flags say which kinds of expert weights the caller's table holds (the reference launches
   // one set of kernels per flag); fp4 == 0 runs NVFP4 weights with BF16 activations (W4A16).
@@ -651,16 +684,45 @@ gw_status gw_moe_run(gw_moe_workspace* w, const void* input_bf16, const void* sc
     if (run_fp8 && !w->fp8_in.data)
       return fail(GW_UNSUPPORTED, "FP8 experts need a workspace created with GW_MOE_FP8_EXPERTS (gw_moe_create_ex)");
   }
-  cudaStream_t s = as_stream(stream);
   w->mark(0, s);
-  gw_status status = gw_moe_dispatch(w, scores_bf16, expert_scales_bf16, rows, stream);
+  gw_status status;
+  if (fast) {
+    const ExpertPlan plan = plan_experts(w, table, w->offsets, 8 * rows);
+    const bool with_groups = plan.needs_groups() && moe_chunks(rows) == 1;
+    status = dispatch(w, scores_bf16, expert_scales_bf16, rows, with_groups ? &plan.groups : nullptr, s);
+    if (status == GW_OK)
+      status = run_experts(w, input_bf16, w->sorted_assignments, 8, w->offsets, 8 * rows, table, w->down.data, s, nullptr, nullptr,
+                           kStageFirst | kStageDown, nullptr, nullptr, with_groups);
+  } else {
+    status = dispatch(w, scores_bf16, expert_scales_bf16, rows, nullptr, s);
+    if (status == GW_OK) status = run_experts_general(w, input_bf16, 8 * rows, table, run_nvfp4, run_bf16, run_fp8, fp4, s);
+  }
+  *combine = MoeCombineInput{w->down.data, w->inverse, w->weights};
+  return status;
+}
+
+void moe_mark_combined(gw_moe_workspace* w, cudaStream_t s) { w->mark(6, s); }
+
+}  // namespace gw
+
+extern "C" {
+
+gw_status gw_moe_run(gw_moe_workspace* w, const void* input_bf16, const void* scores_bf16,
+                     const void* expert_scales_bf16, const gw_expert_table* table, void* output_bf16, uint32_t rows,
+                     int has_bf16, int has_fp8, int has_nvfp4, int fp4, void* stream) {
+  clear_error();
+  if (!w) return fail(GW_INVALID_ARGUMENT, "MoE run requires a workspace");
+  if (rows > w->max_rows) return fail(GW_INVALID_ARGUMENT, "MoE rows exceed workspace");
+  if (!rows) return GW_OK;
+  if (!input_bf16 || !scores_bf16 || !expert_scales_bf16 || !table || !output_bf16 ||
+      reinterpret_cast<uintptr_t>(input_bf16) % 16 || reinterpret_cast<uintptr_t>(output_bf16) % 16)
+    return fail(GW_INVALID_ARGUMENT, "MoE run requires 16-byte aligned input/output, scores, expert scales and a bound expert table");
+  cudaStream_t s = as_stream(stream);
+  MoeCombineInput combine;
+  const gw_status status = moe_run_to_down(w, input_bf16, scores_bf16, expert_scales_bf16, table, rows, has_bf16, has_fp8, has_nvfp4, fp4, s,
+                                           &combine);
   if (status != GW_OK) return status;
-  if (fast)
-    status = run_experts(w, input_bf16, w->sorted_assignments, 8, w->offsets, 8 * rows, table, w->down.data, s);
-  else
-    status = run_experts_general(w, input_bf16, 8 * rows, table, run_nvfp4, run_bf16, run_fp8, fp4, s);
-  if (status != GW_OK) return status;
-  GW_CUDA_CHECK(launch_moe_combine(w->down.data, w->inverse, w->weights, rows, kHidden, output_bf16, s), "MoE combine");
+  GW_CUDA_CHECK(launch_moe_combine(combine.down, combine.inverse, combine.weights, rows, kHidden, output_bf16, s), "MoE combine");
   w->mark(6, s);
   return GW_OK;
 }

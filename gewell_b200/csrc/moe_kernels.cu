@@ -9,6 +9,7 @@
 // computed here with per-64-token bitmaps and popcounts: kernel 1 routes and
 // builds the bitmaps, kernel 2 scans the per-chunk counts, kernel 3 scatters.
 #include "common.cuh"
+#include "combine.cuh"
 #include "moe_kernels.h"
 #include "ptx.cuh"
 
@@ -34,6 +35,186 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float* out) {
   for (int i = 0; i < 4; ++i) {
     out[2 * i] = __uint_as_float(w[i] << 16);
     out[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// 4. group descriptors of the grouped GEMMs, from the offsets (the role of
+//    grouped_nvfp4::prepare, moe_nvfp4.cuh:51-78).  Three plans:
+//      swap    weights on the lane operand, an expert's tokens on the column operand
+//              (small batches): 256 gate/up groups + 128 down groups
+//      direct  tokens on the lane operand, weights on the column operand, plain BF16
+//              output: 256 gate/up groups + 128 down groups
+//      fused   direct form with gate and up as the two halves of the column operand
+//              and GeGLU + FP4 quantisation in the epilogue: 128 groups (+128 down)
+// ---------------------------------------------------------------------------
+// The barrier of the 256 threads that run prepare_groups (a block of their own, or the first 256 of the routing block).
+__device__ __forceinline__ void group_barrier() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
+
+// 256 threads: thread g has part g % 2 of expert g / 2, whose sorted rows are [first, last).
+__device__ __forceinline__ void prepare_groups(const MoeGroupPlan& plan, const MoeExpertInfo& info, int32_t first, int32_t last,
+                                               GemmGroup* __restrict__ first_groups, GemmGroup* __restrict__ down_groups) {
+  __shared__ int32_t items_first[2 * kExperts], items_down[kExperts];
+  const unsigned g = threadIdx.x;            // 0..255: expert = g/2, part = g%2
+  const unsigned e = g / 2, part = g % 2;
+  // Offsets that come from other ranks' histograms (expert parallelism) may describe more rows than
+  // the buffers hold: clamp every group to the capacity and report, so that no tile is scheduled
+  // over rows that do not exist.
+  const int32_t capacity = int32_t(plan.n);
+  if (first < 0 || last < first || last > capacity) {
+    if (plan.error != nullptr && part == 0) atomicCAS(plan.error, 0u, 0x70000100u | e);
+    first = min(max(first, 0), capacity);
+    last = min(max(last, first), capacity);
+  }
+  // A projection gets work in this launch only if it runs as the launch's kind.
+  const bool nv = plan.kind == kMoeKindNvfp4;
+  auto runs_here = [&](int proj) { return moe_effective_kind(info.storage[proj], plan.fp4) == plan.kind; };
+  const int map_base = int32_t(e) * kMapsPerExpert + (nv ? 0 : 4);
+  // BF16 operands carry no scales (the info's alpha belongs to the NVFP4 form of a W4A16 projection)
+  auto alpha_of = [&](int proj) { return plan.kind == kMoeKindBf16 ? 1.0F : info.alpha[proj]; };
+  const int32_t count = last - first;
+  const int32_t token_tiles_swap = (count + plan.block_n_first - 1) / plan.block_n_first;
+  const int32_t token_tiles_direct = (count + 127) / 128;
+  const int32_t padded_first = (first / 128 + int32_t(e)) * 128;
+  // which copy of the quantised input a gate/up projection reads: NVFP4 keeps one copy when gate and up
+  // share their input scale, FP8 always keeps two, BF16 rows are not quantised at all
+  const int src_part = nv ? (plan.shared_gate_up ? 0 : int(part)) : (plan.kind == kMoeKindFp8 ? int(part) : 0);
+  const uint8_t* in_scales = nv ? plan.scales_in + (size_t(src_part) * plan.scale_rows + padded_first) * (kHidden / 16) : nullptr;
+  const uint8_t* act_scales = nv ? plan.scales_act + size_t(padded_first) * (kInter / 16) : nullptr;
+  {
+    GemmGroup grp{};
+    if (plan.form == kMoeFormFused) {
+      // one group per expert (threads with part == 1 write nothing); NVFP4 only
+      const bool active = runs_here(0) && runs_here(1);
+      grp.sf_l = in_scales;
+      grp.map_l = -1;
+      grp.l_row0 = first;
+      grp.l_rows = count;
+      grp.l_tiles = active ? token_tiles_direct : 0;
+      grp.sf_c[0] = info.scales[0];
+      grp.sf_c[1] = info.scales[1];
+      grp.map_c[0] = map_base;
+      grp.map_c[1] = map_base + 1;
+      grp.c_row0 = 0;
+      grp.c_rows = kInter;
+      grp.c_tiles = (kInter + 127) / 128;
+      grp.c_half_stride = 0;
+      grp.alpha[0] = info.alpha[0];
+      grp.alpha[1] = info.alpha[1];
+      grp.quant_inverse_scale = info.inverse_input_scale[2];
+      grp.out_row0 = first;
+      grp.out_col0 = 0;
+      grp.sf_out_row0 = padded_first;
+      items_first[g] = part == 0 ? grp.l_tiles * grp.c_tiles : 0;
+      if (part == 0) first_groups[e] = grp;
+    } else if (plan.form == kMoeFormDirect) {
+      const int proj = part;
+      grp.sf_l = in_scales;
+      grp.map_l = -1;
+      grp.l_row0 = src_part * int32_t(plan.n) + first;
+      grp.l_rows = count;
+      grp.l_tiles = runs_here(proj) ? token_tiles_direct : 0;
+      grp.sf_c[0] = grp.sf_c[1] = info.scales[proj];
+      grp.map_c[0] = grp.map_c[1] = map_base + proj;
+      grp.c_row0 = 0;
+      grp.c_rows = kInter;
+      grp.c_tiles = (kInter + plan.block_n_first - 1) / plan.block_n_first;
+      grp.c_half_stride = plan.block_n_first > 128 ? 128 : 0;
+      grp.alpha[0] = grp.alpha[1] = alpha_of(proj);
+      grp.channel_alpha = nv ? nullptr : info.channel_alpha[proj];
+      grp.out_row0 = first;
+      grp.out_col0 = proj * kInter;
+      items_first[g] = grp.l_tiles * grp.c_tiles;
+      first_groups[g] = grp;
+    } else {
+      const int proj = part;
+      grp.sf_l = info.scales[proj];
+      grp.map_l = map_base + proj;
+      grp.l_row0 = 0;
+      grp.l_rows = kInter;
+      grp.l_tiles = runs_here(proj) ? (kInter + 127) / 128 : 0;
+      grp.sf_c[0] = grp.sf_c[1] = in_scales;
+      grp.map_c[0] = grp.map_c[1] = -1;
+      grp.c_row0 = src_part * int32_t(plan.n) + first;
+      grp.c_rows = count;
+      grp.c_tiles = token_tiles_swap;
+      grp.c_half_stride = 0;
+      grp.alpha[0] = grp.alpha[1] = alpha_of(proj);
+      grp.channel_alpha = nv ? nullptr : info.channel_alpha[proj];
+      grp.out_row0 = first;
+      grp.out_col0 = proj * kInter;
+      items_first[g] = grp.l_tiles * grp.c_tiles;
+      first_groups[g] = grp;
+    }
+  }
+  if (part == 0) {
+    GemmGroup grp{};
+    const bool active = runs_here(2);
+    if (plan.form == kMoeFormSwap) {
+      grp.sf_l = info.scales[2];
+      grp.map_l = map_base + 2;
+      grp.l_row0 = 0;
+      grp.l_rows = kHidden;
+      grp.l_tiles = active ? kHidden / 128 : 0;
+      grp.sf_c[0] = grp.sf_c[1] = act_scales;
+      grp.map_c[0] = grp.map_c[1] = -1;
+      grp.c_row0 = first;
+      grp.c_rows = count;
+      grp.c_tiles = (count + plan.block_n_down - 1) / plan.block_n_down;
+      grp.c_half_stride = 0;
+    } else {
+      grp.sf_l = act_scales;
+      grp.map_l = -1;
+      grp.l_row0 = first;
+      grp.l_rows = count;
+      grp.l_tiles = active ? token_tiles_direct : 0;
+      grp.sf_c[0] = grp.sf_c[1] = info.scales[2];
+      grp.map_c[0] = grp.map_c[1] = map_base + 2;
+      grp.c_row0 = 0;
+      grp.c_rows = kHidden;
+      grp.c_tiles = kHidden / plan.block_n_down;
+      grp.c_half_stride = plan.block_n_down > 128 ? 128 : 0;
+    }
+    grp.alpha[0] = grp.alpha[1] = alpha_of(2);
+    grp.channel_alpha = nv ? nullptr : info.channel_alpha[2];
+    grp.out_row0 = first;
+    grp.out_col0 = 0;
+    items_down[e] = grp.l_tiles * grp.c_tiles;
+    down_groups[e] = grp;
+  }
+  // work_begin: exclusive sums of the work items, by warp shuffles (one thread adding them up took 5 us)
+  __shared__ int32_t warp_sums[2][8];
+  group_barrier();
+  const unsigned lane = g % 32, warp = g / 32;
+  const bool fused = plan.form == kMoeFormFused;
+  const int32_t mine[2] = {items_first[g], g < unsigned(kExperts) ? items_down[g] : 0};
+  int32_t below[2];
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    int32_t scan = mine[which];
+#pragma unroll
+    for (int step = 1; step < 32; step *= 2) {
+      const int32_t other = __shfl_up_sync(0xffffffffu, scan, step);
+      if (lane >= unsigned(step)) scan += other;
+    }
+    below[which] = scan - mine[which];
+    if (lane == 31) warp_sums[which][warp] = scan;
+  }
+  group_barrier();
+#pragma unroll
+  for (int which = 0; which < 2; ++which)
+    for (unsigned v = 0; v < warp; ++v) below[which] += warp_sums[which][v];
+  // fused: items_first counts at the even entries only, one group per expert
+  if (!fused) first_groups[g].work_begin = below[0];
+  else if (part == 0) first_groups[e].work_begin = below[0];
+  if (g < unsigned(kExperts)) down_groups[g].work_begin = below[1];
+  if (g == 255) {
+    GemmGroup sentinel{};
+    sentinel.work_begin = below[0] + mine[0];
+    sentinel.l_tiles = sentinel.c_tiles = 1;
+    first_groups[fused ? kExperts : 2 * kExperts] = sentinel;
+    sentinel.work_begin = below[1] + mine[1];
+    down_groups[kExperts] = sentinel;
   }
 }
 
@@ -132,7 +313,8 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
                  int32_t* __restrict__ keys, float* __restrict__ weights, uint32_t* __restrict__ bitmaps,
                  int32_t* __restrict__ chunk_counts, int32_t* __restrict__ offsets,
                  int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
-                 int32_t* __restrict__ inverse) {
+                 int32_t* __restrict__ inverse, const __grid_constant__ MoeGroupPlan plan, GemmGroup* __restrict__ first_groups,
+                 GemmGroup* __restrict__ down_groups) {
   griddep_launch();
   const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   float expert_scale[4];
@@ -195,6 +377,12 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
     sorted_assignments[position] = int32_t(assignment);
     sorted_keys[position] = e;
     inverse[assignment] = position;
+  }
+  // the expert GEMMs' descriptors as well: one dependent launch less
+  if (first_groups != nullptr && threadIdx.x < 2 * kExperts) {
+    const unsigned e = threadIdx.x / 2;
+    const int32_t first = base[e];
+    prepare_groups(plan, plan.experts[e], first, e + 1 < unsigned(kExperts) ? base[e + 1] : int32_t(rows * kTopK), first_groups, down_groups);
   }
 }
 
@@ -441,184 +629,12 @@ moe_keys_from_offsets_kernel(const int32_t* __restrict__ offsets, uint32_t first
   sorted_keys[i] = int32_t(first_expert + lo);
 }
 
-// ---------------------------------------------------------------------------
-// 4. group descriptors of the grouped GEMMs, from the offsets (the role of
-//    grouped_nvfp4::prepare, moe_nvfp4.cuh:51-78).  Three plans:
-//      swap    weights on the lane operand, an expert's tokens on the column operand
-//              (small batches): 256 gate/up groups + 128 down groups
-//      direct  tokens on the lane operand, weights on the column operand, plain BF16
-//              output: 256 gate/up groups + 128 down groups
-//      fused   direct form with gate and up as the two halves of the column operand
-//              and GeGLU + FP4 quantisation in the epilogue: 128 groups (+128 down)
-// ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 moe_prepare_groups_kernel(MoeGroupPlan plan, GemmGroup* __restrict__ first_groups, GemmGroup* __restrict__ down_groups) {
   griddep_launch();
-  __shared__ int32_t items_first[2 * kExperts], items_down[kExperts];
-  const unsigned g = threadIdx.x;            // 0..255: expert = g/2, part = g%2
-  const unsigned e = g / 2, part = g % 2;
-  const MoeExpertInfo info = plan.experts[e];   // of the expert table, written when it was created
+  const MoeExpertInfo info = plan.experts[threadIdx.x / 2];   // of the expert table, written when it was created
   griddep_wait();     // results of earlier kernels in the stream are read from here on
-  // Offsets that come from other ranks' histograms (expert parallelism) may describe more rows than
-  // the buffers hold: clamp every group to the capacity and report, so that no tile is scheduled
-  // over rows that do not exist.
-  int32_t first = plan.offsets[e], last = plan.offsets[e + 1];
-  const int32_t capacity = int32_t(plan.n);
-  if (first < 0 || last < first || last > capacity) {
-    if (plan.error != nullptr && part == 0) atomicCAS(plan.error, 0u, 0x70000100u | e);
-    first = min(max(first, 0), capacity);
-    last = min(max(last, first), capacity);
-  }
-  // A projection gets work in this launch only if it runs as the launch's kind.
-  const bool nv = plan.kind == kMoeKindNvfp4;
-  auto runs_here = [&](int proj) { return moe_effective_kind(info.storage[proj], plan.fp4) == plan.kind; };
-  const int map_base = int32_t(e) * kMapsPerExpert + (nv ? 0 : 4);
-  // BF16 operands carry no scales (the info's alpha belongs to the NVFP4 form of a W4A16 projection)
-  auto alpha_of = [&](int proj) { return plan.kind == kMoeKindBf16 ? 1.0F : info.alpha[proj]; };
-  const int32_t count = last - first;
-  const int32_t token_tiles_swap = (count + plan.block_n_first - 1) / plan.block_n_first;
-  const int32_t token_tiles_direct = (count + 127) / 128;
-  const int32_t padded_first = (first / 128 + int32_t(e)) * 128;
-  // which copy of the quantised input a gate/up projection reads: NVFP4 keeps one copy when gate and up
-  // share their input scale, FP8 always keeps two, BF16 rows are not quantised at all
-  const int src_part = nv ? (plan.shared_gate_up ? 0 : int(part)) : (plan.kind == kMoeKindFp8 ? int(part) : 0);
-  const uint8_t* in_scales = nv ? plan.scales_in + (size_t(src_part) * plan.scale_rows + padded_first) * (kHidden / 16) : nullptr;
-  const uint8_t* act_scales = nv ? plan.scales_act + size_t(padded_first) * (kInter / 16) : nullptr;
-  {
-    GemmGroup grp{};
-    if (plan.form == kMoeFormFused) {
-      // one group per expert (threads with part == 1 write nothing); NVFP4 only
-      const bool active = runs_here(0) && runs_here(1);
-      grp.sf_l = in_scales;
-      grp.map_l = -1;
-      grp.l_row0 = first;
-      grp.l_rows = count;
-      grp.l_tiles = active ? token_tiles_direct : 0;
-      grp.sf_c[0] = info.scales[0];
-      grp.sf_c[1] = info.scales[1];
-      grp.map_c[0] = map_base;
-      grp.map_c[1] = map_base + 1;
-      grp.c_row0 = 0;
-      grp.c_rows = kInter;
-      grp.c_tiles = (kInter + 127) / 128;
-      grp.c_half_stride = 0;
-      grp.alpha[0] = info.alpha[0];
-      grp.alpha[1] = info.alpha[1];
-      grp.quant_inverse_scale = info.inverse_input_scale[2];
-      grp.out_row0 = first;
-      grp.out_col0 = 0;
-      grp.sf_out_row0 = padded_first;
-      items_first[g] = part == 0 ? grp.l_tiles * grp.c_tiles : 0;
-      if (part == 0) first_groups[e] = grp;
-    } else if (plan.form == kMoeFormDirect) {
-      const int proj = part;
-      grp.sf_l = in_scales;
-      grp.map_l = -1;
-      grp.l_row0 = src_part * int32_t(plan.n) + first;
-      grp.l_rows = count;
-      grp.l_tiles = runs_here(proj) ? token_tiles_direct : 0;
-      grp.sf_c[0] = grp.sf_c[1] = info.scales[proj];
-      grp.map_c[0] = grp.map_c[1] = map_base + proj;
-      grp.c_row0 = 0;
-      grp.c_rows = kInter;
-      grp.c_tiles = (kInter + plan.block_n_first - 1) / plan.block_n_first;
-      grp.c_half_stride = plan.block_n_first > 128 ? 128 : 0;
-      grp.alpha[0] = grp.alpha[1] = alpha_of(proj);
-      grp.channel_alpha = nv ? nullptr : info.channel_alpha[proj];
-      grp.out_row0 = first;
-      grp.out_col0 = proj * kInter;
-      items_first[g] = grp.l_tiles * grp.c_tiles;
-      first_groups[g] = grp;
-    } else {
-      const int proj = part;
-      grp.sf_l = info.scales[proj];
-      grp.map_l = map_base + proj;
-      grp.l_row0 = 0;
-      grp.l_rows = kInter;
-      grp.l_tiles = runs_here(proj) ? (kInter + 127) / 128 : 0;
-      grp.sf_c[0] = grp.sf_c[1] = in_scales;
-      grp.map_c[0] = grp.map_c[1] = -1;
-      grp.c_row0 = src_part * int32_t(plan.n) + first;
-      grp.c_rows = count;
-      grp.c_tiles = token_tiles_swap;
-      grp.c_half_stride = 0;
-      grp.alpha[0] = grp.alpha[1] = alpha_of(proj);
-      grp.channel_alpha = nv ? nullptr : info.channel_alpha[proj];
-      grp.out_row0 = first;
-      grp.out_col0 = proj * kInter;
-      items_first[g] = grp.l_tiles * grp.c_tiles;
-      first_groups[g] = grp;
-    }
-  }
-  if (part == 0) {
-    GemmGroup grp{};
-    const bool active = runs_here(2);
-    if (plan.form == kMoeFormSwap) {
-      grp.sf_l = info.scales[2];
-      grp.map_l = map_base + 2;
-      grp.l_row0 = 0;
-      grp.l_rows = kHidden;
-      grp.l_tiles = active ? kHidden / 128 : 0;
-      grp.sf_c[0] = grp.sf_c[1] = act_scales;
-      grp.map_c[0] = grp.map_c[1] = -1;
-      grp.c_row0 = first;
-      grp.c_rows = count;
-      grp.c_tiles = (count + plan.block_n_down - 1) / plan.block_n_down;
-      grp.c_half_stride = 0;
-    } else {
-      grp.sf_l = act_scales;
-      grp.map_l = -1;
-      grp.l_row0 = first;
-      grp.l_rows = count;
-      grp.l_tiles = active ? token_tiles_direct : 0;
-      grp.sf_c[0] = grp.sf_c[1] = info.scales[2];
-      grp.map_c[0] = grp.map_c[1] = map_base + 2;
-      grp.c_row0 = 0;
-      grp.c_rows = kHidden;
-      grp.c_tiles = kHidden / plan.block_n_down;
-      grp.c_half_stride = plan.block_n_down > 128 ? 128 : 0;
-    }
-    grp.alpha[0] = grp.alpha[1] = alpha_of(2);
-    grp.channel_alpha = nv ? nullptr : info.channel_alpha[2];
-    grp.out_row0 = first;
-    grp.out_col0 = 0;
-    items_down[e] = grp.l_tiles * grp.c_tiles;
-    down_groups[e] = grp;
-  }
-  // work_begin: exclusive sums of the work items, by warp shuffles (one thread adding them up took 5 us)
-  __shared__ int32_t warp_sums[2][8];
-  __syncthreads();
-  const unsigned lane = g % 32, warp = g / 32;
-  const bool fused = plan.form == kMoeFormFused;
-  const int32_t mine[2] = {items_first[g], g < unsigned(kExperts) ? items_down[g] : 0};
-  int32_t below[2];
-#pragma unroll
-  for (int which = 0; which < 2; ++which) {
-    int32_t scan = mine[which];
-#pragma unroll
-    for (int step = 1; step < 32; step *= 2) {
-      const int32_t other = __shfl_up_sync(0xffffffffu, scan, step);
-      if (lane >= unsigned(step)) scan += other;
-    }
-    below[which] = scan - mine[which];
-    if (lane == 31) warp_sums[which][warp] = scan;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int which = 0; which < 2; ++which)
-    for (unsigned v = 0; v < warp; ++v) below[which] += warp_sums[which][v];
-  // fused: items_first counts at the even entries only, one group per expert
-  if (!fused) first_groups[g].work_begin = below[0];
-  else if (part == 0) first_groups[e].work_begin = below[0];
-  if (g < unsigned(kExperts)) down_groups[g].work_begin = below[1];
-  if (g == 255) {
-    GemmGroup sentinel{};
-    sentinel.work_begin = below[0] + mine[0];
-    sentinel.l_tiles = sentinel.c_tiles = 1;
-    first_groups[fused ? kExperts : 2 * kExperts] = sentinel;
-    sentinel.work_begin = below[1] + mine[1];
-    down_groups[kExperts] = sentinel;
-  }
+  prepare_groups(plan, info, plan.offsets[threadIdx.x / 2], plan.offsets[threadIdx.x / 2 + 1], first_groups, down_groups);
 }
 
 // ---------------------------------------------------------------------------
@@ -908,29 +924,7 @@ moe_combine_token_kernel(const uint4* __restrict__ down, const int32_t* __restri
   }
   __syncthreads();
   const uint32_t v = threadIdx.x;
-  uint4 raw[kTopK];
-#pragma unroll
-  for (int j = 0; j < kTopK; ++j)          // all eight gathered loads are in flight before the fold starts
-    raw[j] = __ldcs(down + size_t(slot_row[j]) * kVectors + v);
-  __nv_bfloat162 sum[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) sum[i] = __floats2bfloat162_rn(0.0F, 0.0F);
-#pragma unroll
-  for (int j = 0; j < kTopK; ++j) {
-    const float w = slot_weight[j];
-    const uint32_t words[4] = {raw[j].x, raw[j].y, raw[j].z, raw[j].w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const __nv_bfloat162 product = __floats2bfloat162_rn(__fmul_rn(__uint_as_float(words[i] << 16), w),
-                                                           __fmul_rn(__uint_as_float(words[i] & 0xFFFF0000u), w));
-      sum[i] = __hadd2(sum[i], product);
-    }
-  }
-  uint4 result;
-  result.x = *reinterpret_cast<const uint32_t*>(&sum[0]);
-  result.y = *reinterpret_cast<const uint32_t*>(&sum[1]);
-  result.z = *reinterpret_cast<const uint32_t*>(&sum[2]);
-  result.w = *reinterpret_cast<const uint32_t*>(&sum[3]);
+  const uint4 result = combine_rows<kTopK>(down, slot_row, slot_weight, kVectors, v);
   __stcs(output + size_t(token) * kVectors + v, result);
   (void)rows;
 }
@@ -1314,12 +1308,13 @@ cudaError_t launch_moe_dispatch(const void* scores, const void* expert_scales, u
                                 float* weights, uint32_t* bitmaps, int32_t* chunk_counts, int32_t* offsets,
                                 int32_t* sorted_assignments, int32_t* sorted_keys, int32_t* inverse,
                                 uint32_t* barrier_state, uint32_t* error, int sm_count, bool one_launch,
-                                cudaStream_t stream) {
+                                cudaStream_t stream, const MoeGroupPlan* plan, GemmGroup* first_groups, GemmGroup* down_groups) {
   const uint32_t chunks = moe_chunks(rows);
   if (chunks == 1) {     // decode sizes: one block (32 warps, two tokens each) routes, scans and scatters
     launch_pdl(moe_route_kernel, chunks, 1024, stream, static_cast<const bf16*>(scores),
                static_cast<const bf16*>(expert_scales), rows, keys, weights, bitmaps, chunk_counts, offsets,
-               sorted_assignments, sorted_keys, inverse);
+               sorted_assignments, sorted_keys, inverse, plan != nullptr ? *plan : MoeGroupPlan{}, plan != nullptr ? first_groups : nullptr,
+               down_groups);
     return cudaGetLastError();
   }
   const uint32_t resident = uint32_t(sm_count) * kRouteGridBlocksPerSm;
@@ -1332,7 +1327,7 @@ cudaError_t launch_moe_dispatch(const void* scores, const void* expert_scales, u
   launch_pdl(moe_route_kernel, chunks, 256, stream, static_cast<const bf16*>(scores),
              static_cast<const bf16*>(expert_scales), rows, keys, weights, bitmaps, chunk_counts,
              static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr),
-             static_cast<int32_t*>(nullptr));
+             static_cast<int32_t*>(nullptr), MoeGroupPlan{}, static_cast<GemmGroup*>(nullptr), static_cast<GemmGroup*>(nullptr));
   launch_pdl(moe_scan_kernel, 1, kExperts, stream, chunk_counts, chunks, offsets);
   launch_pdl(moe_scatter_kernel, chunks, 256, stream, keys, bitmaps, chunk_counts, offsets, rows, sorted_assignments,
              sorted_keys, inverse);

@@ -63,7 +63,9 @@ cudaError_t launch_moe_dispatch(const void* scores, const void* expert_scales, u
                                 float* weights, uint32_t* bitmaps, int32_t* chunk_counts, int32_t* offsets,
                                 int32_t* sorted_assignments, int32_t* sorted_keys, int32_t* inverse,
                                 uint32_t* barrier_state, uint32_t* error, int sm_count, bool one_launch,
-                                cudaStream_t stream);
+                                cudaStream_t stream, const MoeGroupPlan* plan = nullptr, GemmGroup* first_groups = nullptr,
+                                GemmGroup* down_groups = nullptr);
+// plan != nullptr and moe_chunks(rows) == 1: the launch also writes the group descriptors of that plan.
 // barrier_state: two zero-initialised uint32 in device memory owned by the workspace (counter, generation)
 // for the grid-wide barrier of the one-launch form; one_launch == false keeps the three-launch form.
 cudaError_t launch_moe_keys_from_offsets(const int32_t* offsets, uint32_t first_expert, uint32_t expert_count,
@@ -133,5 +135,16 @@ cudaError_t launch_ep_combine(const int32_t* keys, const int32_t* inverse, const
                               const int32_t* offsets, const int32_t* dest_rank, const int32_t* dest_row0,
                               void* const* peer_down, uint32_t rows, uint32_t capacity_rows, uint32_t* error,
                               void* output, cudaStream_t stream);
+
+// gw_moe_run without its last step, and what that step reads (moe.cu).
+struct MoeCombineInput {
+  const void* down;            // BF16 [8 rows, hidden], sorted
+  const int32_t* inverse;      // sorted row of assignment (token, slot)
+  const float* weights;        // of the assignments
+};
+gw_status moe_run_to_down(gw_moe_workspace* workspace, const void* input_bf16, const void* scores_bf16, const void* expert_scales_bf16,
+                          const gw_expert_table* table, uint32_t rows, int has_bf16, int has_fp8, int has_nvfp4, int fp4, cudaStream_t stream,
+                          MoeCombineInput* combine);
+void moe_mark_combined(gw_moe_workspace* workspace, cudaStream_t stream);
 
 }  // namespace gw
