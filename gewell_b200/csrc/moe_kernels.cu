@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "combine.cuh"
 #include "moe_kernels.h"
+#include "pair.cuh"
 #include "ptx.cuh"
 
 namespace gw {
@@ -48,7 +49,7 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float* out) {
 //      fused   direct form with gate and up as the two halves of the column operand
 //              and GeGLU + FP4 quantisation in the epilogue: 128 groups (+128 down)
 // ---------------------------------------------------------------------------
-// The barrier of the 256 threads that run prepare_groups (a block of their own, or the first 256 of the routing block).
+// The barrier of the 256 threads that run prepare_groups (a block of their own, or the routing cluster's first).
 __device__ __forceinline__ void group_barrier() { asm volatile("bar.sync 2, 256;" ::: "memory"); }
 
 // 256 threads: thread g has part g % 2 of expert g / 2, whose sorted rows are [first, last).
@@ -229,7 +230,7 @@ __device__ __forceinline__ void load_expert_scales(const bf16* __restrict__ expe
 // kernel (models/gemma4/26b_a4b/sm120/moe.cu:104-157), so ids and FP32 weights match it bit for bit.
 __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, const float (&expert_scale)[4],
                                             uint32_t row, uint32_t local, unsigned lane, int32_t* __restrict__ keys,
-                                            float* __restrict__ weights, uint32_t (*bitmap)[2], int32_t* shared_keys) {
+                                            float* __restrict__ weights, uint32_t bitmap, uint32_t shared_keys) {
   // Softmax over the token's 128 logits; this lane owns experts lane, lane + 32, lane + 64, lane + 96.
   // The FP32 additions keep the order the reference's weights depend on: the lane's four terms in
   // ascending expert order first, then the xor butterfly 16, 8, 4, 2, 1 over the lanes.
@@ -251,29 +252,36 @@ __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, con
   }
 #pragma unroll
   for (int step = 16; step > 0; step >>= 1) denominator += __shfl_xor_sync(0xffffffffu, denominator, step);
-  // Eight winners, two hardware maxima a round: the largest probability (probabilities are not negative, so their bit
-  // patterns order like unsigned integers), then the smallest id among those that have it.  A candidate that has won
-  // drops to pattern 0, and its id out of the running.  Lane r keeps round r's winner.  The rounds stay a loop: decode
-  // steps run this code cold, and unrolled it was fetched from memory for longer than it ran (route of 64 tokens 18 us).
-  uint32_t pattern[4];
-  uint32_t live = 0xF;
+  // Eight winners, two hardware reductions a round: the largest probability (probabilities are not negative, so their bit
+  // patterns order like unsigned integers), then the smallest id among those that have it.  Every lane first puts its
+  // four candidates in that order, so that a round looks at one of them and the winner's lane moves up.  Lane r keeps
+  // round r's winner.  64 tokens on one SM are bound by the number of instructions, a cold launch by fetching them:
+  // hence the loop.
+  uint32_t pattern[4], id[4];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) pattern[q] = __float_as_uint(__fdiv_rn(prob[q], denominator));
+  for (int q = 0; q < 4; ++q) { pattern[q] = __float_as_uint(__fdiv_rn(prob[q], denominator)); id[q] = lane + 32 * q; }
+  const auto order = [&](int i, int j) {
+    if (pattern[j] > pattern[i] || (pattern[j] == pattern[i] && id[j] < id[i])) {
+      const uint32_t p = pattern[i], d = id[i];
+      pattern[i] = pattern[j]; id[i] = id[j];
+      pattern[j] = p; id[j] = d;
+    }
+  };
+  order(0, 1); order(2, 3); order(0, 2); order(1, 3); order(1, 2);
   int my_id = 0;
   float my_p = 0.0F;
 #pragma unroll 1
   for (unsigned round = 0; round < unsigned(kTopK); ++round) {
-    uint32_t best = 0;
+    // a lane whose four are gone offers pattern 0 with an id above every other
+    const uint32_t best = __reduce_max_sync(0xffffffffu, pattern[0]);
+    const uint32_t winner = __reduce_min_sync(0xffffffffu, pattern[0] == best ? id[0] : uint32_t(kExperts));
+    if (id[0] == winner) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) best = (live >> q & 1u) ? max(best, pattern[q]) : best;
-    best = __reduce_max_sync(0xffffffffu, best);
-    uint32_t id = kExperts;
-#pragma unroll
-    for (int q = 3; q >= 0; --q)
-      if ((live >> q & 1u) && pattern[q] == best) id = lane + 32 * q;
-    id = __reduce_min_sync(0xffffffffu, id);
-    if (id % 32 == lane) live &= ~(1u << (id / 32));
-    if (lane == round) { my_id = int(id); my_p = __uint_as_float(best); }
+      for (int q = 0; q < 3; ++q) { pattern[q] = pattern[q + 1]; id[q] = id[q + 1]; }
+      pattern[3] = 0;
+      id[3] = kExperts;
+    }
+    if (lane == round) { my_id = int(winner); my_p = __uint_as_float(best); }
   }
   // renormalisation: ((p0+p4)+(p2+p6)) + ((p1+p5)+(p3+p7)), the pairwise order of a stride-4/2/1 fold
   float sum = my_p + __shfl_down_sync(0xffffffffu, my_p, 4);
@@ -293,8 +301,8 @@ __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, con
     const float weight = __fmul_rn(__fdiv_rn(my_p, sum), scale);
     keys[size_t(row) * kTopK + rank] = my_id;
     weights[size_t(row) * kTopK + rank] = weight;
-    if (shared_keys != nullptr) shared_keys[local * kTopK + rank] = my_id;
-    atomicOr(&bitmap[my_id][local / 32], 1u << (local % 32));
+    if (shared_keys != 0) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(shared_keys + (local * kTopK + rank) * 4), "r"(my_id) : "memory");
+    asm volatile("red.shared::cluster.or.b32 [%0], %1;" ::"r"(bitmap + (my_id * 2 + local / 32) * 4), "r"(1u << (local % 32)) : "memory");
   }
 }
 
@@ -305,16 +313,11 @@ __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, con
 //    (models/gemma4/26b_a4b/sm120/moe.cu:104-157), so ids and FP32 weights match
 //    it bit for bit.  One warp per token, eight tokens per warp.
 // ---------------------------------------------------------------------------
-//    (route_token below; used by the single-block kernel and by the grid-wide kernel)
-//    With at most 64 tokens there is one block: it then also does the work of kernels 2
-//    and 3 (`offsets` != nullptr), which saves two dependent launches on the decode path.
-__global__ void __launch_bounds__(1024)
+//    Used by three kernels: one launch per step (this one), one cluster for at most 64 tokens, and one grid-wide launch.
+__global__ void __launch_bounds__(256)
 moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales, uint32_t rows,
                  int32_t* __restrict__ keys, float* __restrict__ weights, uint32_t* __restrict__ bitmaps,
-                 int32_t* __restrict__ chunk_counts, int32_t* __restrict__ offsets,
-                 int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
-                 int32_t* __restrict__ inverse, const __grid_constant__ MoeGroupPlan plan, GemmGroup* __restrict__ first_groups,
-                 GemmGroup* __restrict__ down_groups) {
+                 int32_t* __restrict__ chunk_counts) {
   griddep_launch();
   const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
   float expert_scale[4];
@@ -324,25 +327,60 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
   if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
   __syncthreads();
   const uint32_t chunk = blockIdx.x;
-  const int tokens_per_warp = kChunkTokens / int(blockDim.x / 32);     // 8 warps: 8 tokens each; 32 warps: 2
-  __shared__ int32_t shared_keys[kChunkTokens * kTopK];
 #pragma unroll 1
-  for (int t = 0; t < tokens_per_warp; ++t) {
-    const uint32_t local = warp + t * (blockDim.x / 32);
+  for (uint32_t local = warp; local < kChunkTokens; local += 8) {
     const uint32_t row = chunk * kChunkTokens + local;
     if (row >= rows) break;
-    route_token(scores, expert_scale, row, local, lane, keys, weights, bitmap, shared_keys);
+    route_token(scores, expert_scale, row, local, lane, keys, weights, ptx::smem_u32(bitmap), 0);
   }
   __syncthreads();
   if (threadIdx.x < kExperts) {
     const uint32_t w0 = bitmap[threadIdx.x][0], w1 = bitmap[threadIdx.x][1];
     bitmaps[(size_t(chunk) * kExperts + threadIdx.x) * 2] = w0;
     bitmaps[(size_t(chunk) * kExperts + threadIdx.x) * 2 + 1] = w1;
-    chunk_counts[size_t(chunk) * kExperts + threadIdx.x] = offsets != nullptr ? 0 : __popc(w0) + __popc(w1);
+    chunk_counts[size_t(chunk) * kExperts + threadIdx.x] = __popc(w0) + __popc(w1);
   }
-  if (offsets == nullptr) return;
-  // single block: offsets, positions, inverse (the scan and scatter steps of kernels 2 and 3)
+}
+
+// ---------------------------------------------------------------------------
+// 1a. At most 64 tokens (decode): a cluster of eight blocks routes them, a token per warp -- on one SM the
+//     instructions of 64 tokens alone took 5 us -- and the first block, whose shared memory the others wrote
+//     their bits and ids to, does the work of kernels 2 and 3 and the expert GEMMs' descriptors (`first_groups`
+//     != nullptr): one launch instead of four.  64 tokens: ROUTE_US.
+// ---------------------------------------------------------------------------
+constexpr int kRouteCluster = 8;
+__global__ void __cluster_dims__(kRouteCluster, 1, 1) __launch_bounds__(256)
+moe_route_cluster_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales, uint32_t rows,
+                         int32_t* __restrict__ keys, float* __restrict__ weights, uint32_t* __restrict__ bitmaps,
+                         int32_t* __restrict__ chunk_counts, int32_t* __restrict__ offsets,
+                         int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
+                         int32_t* __restrict__ inverse, const __grid_constant__ MoeGroupPlan plan, GemmGroup* __restrict__ first_groups,
+                         GemmGroup* __restrict__ down_groups) {
+  static_assert(kRouteCluster * 8 == kChunkTokens, "a token per warp");
+  __shared__ uint32_t bitmap[kExperts][2];
+  __shared__ int32_t shared_keys[kChunkTokens * kTopK];
   __shared__ int32_t base[kExperts];
+  griddep_launch();
+  const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32, block = pair::cluster_rank();
+  float expert_scale[4];
+  load_expert_scales(expert_scales, lane, expert_scale);
+  MoeExpertInfo info{};
+  if (block == 0) {
+    if (first_groups != nullptr) info = plan.experts[threadIdx.x / 2];   // of the expert table, written when it was created
+    if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
+  }
+  pair::cluster_sync_all();                // the first block's bitmaps are clear
+  griddep_wait();                          // results of earlier kernels in the stream are read from here on
+  const uint32_t token = block * 8 + warp;
+  if (token < rows)
+    route_token(scores, expert_scale, token, token, lane, keys, weights, pair::leader_address(bitmap), pair::leader_address(shared_keys));
+  pair::cluster_sync_all();                // every block's bits and ids are in the first one's memory
+  if (block != 0) return;
+  if (threadIdx.x < kExperts) {
+    bitmaps[size_t(threadIdx.x) * 2] = bitmap[threadIdx.x][0];
+    bitmaps[size_t(threadIdx.x) * 2 + 1] = bitmap[threadIdx.x][1];
+    chunk_counts[threadIdx.x] = 0;
+  }
   if (warp == 0) {
     // exclusive scan of the 128 expert counts in one warp: four consecutive experts per lane
     int32_t count[4], mine = 0;
@@ -367,7 +405,7 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
     if (lane == 31) offsets[kExperts] = acc;
   }
   __syncthreads();
-  for (uint32_t assignment = threadIdx.x; assignment < rows * kTopK; assignment += blockDim.x) {
+  for (uint32_t assignment = threadIdx.x; assignment < rows * kTopK; assignment += 256) {
     const uint32_t local = assignment / kTopK;
     const int32_t e = shared_keys[assignment];
     const uint32_t w0 = bitmap[e][0], w1 = bitmap[e][1];
@@ -378,11 +416,9 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
     sorted_keys[position] = e;
     inverse[assignment] = position;
   }
-  // the expert GEMMs' descriptors as well: one dependent launch less
-  if (first_groups != nullptr && threadIdx.x < 2 * kExperts) {
+  if (first_groups != nullptr) {
     const unsigned e = threadIdx.x / 2;
-    const int32_t first = base[e];
-    prepare_groups(plan, plan.experts[e], first, e + 1 < unsigned(kExperts) ? base[e + 1] : int32_t(rows * kTopK), first_groups, down_groups);
+    prepare_groups(plan, info, base[e], e + 1 < unsigned(kExperts) ? base[e + 1] : int32_t(rows * kTopK), first_groups, down_groups);
   }
 }
 
@@ -457,7 +493,7 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
     for (int t = 0; t < kTokensPerWarp; ++t) {
       const uint32_t local = warp * kTokensPerWarp + t;
       const uint32_t row = chunk * kChunkTokens + local;
-      if (row < rows) route_token(scores, expert_scale, row, local, lane, keys, weights, bitmap, shared_keys);
+      if (row < rows) route_token(scores, expert_scale, row, local, lane, keys, weights, ptx::smem_u32(bitmap), ptx::smem_u32(shared_keys));
     }
     __syncthreads();
     if (threadIdx.x < kExperts) {
@@ -655,9 +691,10 @@ moe_quantize_kernel(const uint4* __restrict__ input, const int32_t* __restrict__
                     const MoeExpertInfo* __restrict__ experts, uint32_t n, uint32_t scale_rows, int projection,
                     uint32_t gather_divisor, uint32_t* __restrict__ packed, uint8_t* __restrict__ scales,
                     uint4* __restrict__ activated) {
+  if (Gelu) griddep_launch();
   griddep_wait();     // results of earlier kernels in the stream are read from here on
-  // Only now: the GEMM that follows fills every SM, and its blocks would keep out other streams' kernels while they wait.
-  griddep_launch();
+  // The layer's first GEMM only now: it fills every SM, and its blocks would keep out other streams' kernels while they wait.
+  if (!Gelu) griddep_launch();
   constexpr uint32_t kVectors = K / 8;          // even: the two threads of a block are neighbours in a warp
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   const uint32_t part = blockIdx.y;             // gate/up copy (0 unless the scales differ)
@@ -1310,8 +1347,8 @@ cudaError_t launch_moe_dispatch(const void* scores, const void* expert_scales, u
                                 uint32_t* barrier_state, uint32_t* error, int sm_count, bool one_launch,
                                 cudaStream_t stream, const MoeGroupPlan* plan, GemmGroup* first_groups, GemmGroup* down_groups) {
   const uint32_t chunks = moe_chunks(rows);
-  if (chunks == 1) {     // decode sizes: one block (32 warps, two tokens each) routes, scans and scatters
-    launch_pdl(moe_route_kernel, chunks, 1024, stream, static_cast<const bf16*>(scores),
+  if (chunks == 1) {     // decode sizes: one cluster routes, scans and scatters
+    launch_pdl(moe_route_cluster_kernel, kRouteCluster, 256, stream, static_cast<const bf16*>(scores),
                static_cast<const bf16*>(expert_scales), rows, keys, weights, bitmaps, chunk_counts, offsets,
                sorted_assignments, sorted_keys, inverse, plan != nullptr ? *plan : MoeGroupPlan{}, plan != nullptr ? first_groups : nullptr,
                down_groups);
@@ -1325,9 +1362,7 @@ cudaError_t launch_moe_dispatch(const void* scores, const void* expert_scales, u
     return cudaGetLastError();
   }
   launch_pdl(moe_route_kernel, chunks, 256, stream, static_cast<const bf16*>(scores),
-             static_cast<const bf16*>(expert_scales), rows, keys, weights, bitmaps, chunk_counts,
-             static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr), static_cast<int32_t*>(nullptr),
-             static_cast<int32_t*>(nullptr), MoeGroupPlan{}, static_cast<GemmGroup*>(nullptr), static_cast<GemmGroup*>(nullptr));
+             static_cast<const bf16*>(expert_scales), rows, keys, weights, bitmaps, chunk_counts);
   launch_pdl(moe_scan_kernel, 1, kExperts, stream, chunk_counts, chunks, offsets);
   launch_pdl(moe_scatter_kernel, chunks, 256, stream, keys, bitmaps, chunk_counts, offsets, rows, sorted_assignments,
              sorted_keys, inverse);
