@@ -479,7 +479,7 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
     first.c_rows_per_tile = form == kMoeFormFused ? 128 : block_n_first;
     // Direct forms: two consecutive tiles per CTA (same token tile, same expert) before it strides on, measured best.
     // Swap form: one contiguous range, because its tiles are as short as a group's descriptor is late (64 tokens, down
-    // GEMM: CHUNK_US).
+    // GEMM: 43 -> 38 us).
     first.work_chunk = tune.chunk_first > 0 ? tune.chunk_first : (swap ? -1 : 2);
     first.error = device_error_word();
     if (form == kMoeFormFused) {
