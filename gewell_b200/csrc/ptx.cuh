@@ -65,15 +65,13 @@ __device__ __forceinline__ bool elect_one() {
 // and unwinds, so a protocol bug shows up as an error code instead of a hang.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   uint64_t limit_ns = 2000000000ull) {
-  // the timer is read only after many polls
-  uint64_t start = 0;
+  // Reading the timer after the first miss also keeps waiting lanes off the barrier for a moment: without it the NVFP4
+  // pair kernel's scale loaders polled so often that 4096x21504x5376 took 237 us instead of 233.
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint64_t start = global_timer_ns();
   for (uint32_t spin = 1;; ++spin) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((spin & 255u) == 0) {
-      const uint64_t now = global_timer_ns();
-      if (start == 0) start = now;
-      else if (now - start > limit_ns) return false;
-    }
+    if ((spin & 255u) == 0 && global_timer_ns() - start > limit_ns) return false;
   }
 }
 
@@ -85,15 +83,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
   uint32_t ok = 1;
   if ((threadIdx.x & 31) == 0) {
     if (!mbar_try_wait(bar, parity)) {
-      uint64_t start = 0;
+      const uint64_t start = global_timer_ns();
       for (uint32_t spin = 1;; ++spin) {
         if (backoff_ns) __nanosleep(backoff_ns);
         if (mbar_try_wait(bar, parity)) break;
-        if ((spin & 63u) == 0) {
-          const uint64_t now = global_timer_ns();
-          if (start == 0) start = now;
-          else if (now - start > limit_ns) { ok = 0; break; }
-        }
+        if ((spin & 63u) == 0 && global_timer_ns() - start > limit_ns) { ok = 0; break; }
       }
     }
   }
