@@ -8,6 +8,9 @@
 // 128x256 tile, which is what limits that kernel (shared-memory port and L2->SM
 // fill).  Roles per CTA as in gemm_tc.cu: one producer lane, one MMA lane (only
 // in the pair's leader, rank 0), four scale-loader warps, eight epilogue warps.
+// The single lanes are elected ones (2048x5376x43008 260.3 -> 254.9 us with the quantiser, 4096x21504x5376 237.2 -> 233.6);
+// repeated back to back the kernel is bound by the power limit (SM clock 1.45 GHz, 280 us).  All lanes of a loader warp
+// poll their barrier: one polling lane and a broadcast is slower (244 us).
 //
 // Cross-CTA protocol (all mbarriers sit at the same shared-memory offsets in both
 // CTAs):
@@ -65,7 +68,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty_bar + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
   const uint32_t rank = cluster_rank();           // 0 = leader of the pair
   griddep_launch();
   if (threadIdx.x == 0) {
@@ -89,7 +92,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   __syncthreads();
   cluster_sync_all();                               // both CTAs' barriers exist before anybody signals them
   ptx::tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_wait();
 
   const int total_kb = p.k / 64;
@@ -104,7 +107,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       long long prof_wait = 0;
@@ -147,7 +150,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA, one lane)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0, acc_phase = 0;
       const uint32_t idesc = idesc_pair_nvfp4(256);
