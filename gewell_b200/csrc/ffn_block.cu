@@ -369,9 +369,6 @@ struct DeviceBuffer {
   ~DeviceBuffer() { if (data) cudaFree(data); }
 };
 
-// Rows up to which the shared MLP runs beside the router and the routing; beyond, its GEMMs fill the GPU.
-constexpr uint32_t kForkRows = 128;
-
 constexpr uint32_t kHidden = 2816, kSharedMlp = 2112, kExperts = 128;   // model.h:12-13
 
 }  // namespace
@@ -382,8 +379,10 @@ struct gw_ffn_block {
   cudaStream_t stream = nullptr;
   gw_projection_workspace* projections = nullptr;
   gw_moe_workspace* moe = nullptr;
-  // Small row counts: the shared MLP on a stream of its own beside the router, the routing and the experts' input,
-  // which leave most of the GPU idle.  The router then needs a plan and scratch apart from the shared MLP's.
+  // The shared MLP runs on a stream of its own beside the router, the routing and the experts' input, which leave most of
+  // the GPU idle at small row counts, and fills the tails of the experts' GEMMs at large ones (one stream -> two, us: NVFP4
+  // 8 rows 100.7 -> 95.1, 470 rows 231.8 -> 213.1, 4000 rows 472.8 -> 445.5; BF16 8 rows 172 -> 149).  So the router has a
+  // plan and scratch apart from the shared MLP's.
   cudaStream_t side = nullptr;
   cudaEvent_t forked = nullptr, joined = nullptr;
   gw_bf16_plan* router_plan = nullptr;
@@ -527,12 +526,6 @@ gw_status gw_ffn_block_create(const gw_ffn_block_weights* layers, uint32_t count
     bindings.push_back(w.gate);
     bindings.push_back(w.up);
     bindings.push_back(w.down);
-    gw_projection router{};
-    router.storage = GW_STORAGE_BF16;
-    router.input = kHidden;
-    router.output = router.physical_output = kExperts;
-    router.bf16 = w.router_proj;
-    bindings.push_back(router);
   }
   auto b = std::unique_ptr<gw_ffn_block>(new (std::nothrow) gw_ffn_block());
   if (!b) return fail(GW_CUDA_ERROR, "out of host memory");
@@ -585,10 +578,7 @@ gw_status gw_ffn_block_prepare(gw_ffn_block* b, uint32_t rows, int phase) {
   if (status != GW_OK) return status;
   if (b->rows != rows) {
     gw_bf16_plan* plan = nullptr;
-    if (rows <= kForkRows) {
-      const gw_status created = gw_bf16_plan_create(rows, kHidden, kExperts, &plan);
-      if (created != GW_OK) return created;
-    }
+    if (const gw_status created = gw_bf16_plan_create(rows, kHidden, kExperts, &plan); created != GW_OK) return created;
     if (b->router_plan) gw_bf16_plan_destroy(b->router_plan);
     b->router_plan = plan;
   }
@@ -613,50 +603,33 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
                                                   b->expert_input, rows, kHidden, s);
   if (status != GW_OK) return status;
   // shared MLP (batched_executor.cu:256-259)
-  const bool fork = b->router_plan != nullptr;
-  cudaStream_t shared = as_stream(s);
-  if (fork) {
-    GW_CUDA_CHECK(cudaEventRecord(b->forked, as_stream(s)), "feed-forward block fork");
-    GW_CUDA_CHECK(cudaStreamWaitEvent(b->side, b->forked, 0), "feed-forward block fork");
-    shared = b->side;
-  }
+  GW_CUDA_CHECK(cudaEventRecord(b->forked, as_stream(s)), "feed-forward block fork");
+  GW_CUDA_CHECK(cudaStreamWaitEvent(b->side, b->forked, 0), "feed-forward block fork");
   const auto shared_mlp = [&]() {
     bool product_done = false;
-    gw_status st = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, shared, &product_done);
+    gw_status st = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, b->side, &product_done);
     if (st == GW_OK && !product_done) {
-      st = projection_workspace_run_on(b->projections, &w.gate, b->normalized, b->gate, shared);
-      if (st == GW_OK) st = projection_workspace_run_on(b->projections, &w.up, b->normalized, b->up, shared);
-      if (st == GW_OK) st = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, shared);
+      st = projection_workspace_run_on(b->projections, &w.gate, b->normalized, b->gate, b->side);
+      if (st == GW_OK) st = projection_workspace_run_on(b->projections, &w.up, b->normalized, b->up, b->side);
+      if (st == GW_OK) st = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, b->side);
     }
-    return st == GW_OK ? projection_workspace_run_on(b->projections, &w.down, b->product, b->shared_mlp, shared) : st;
+    return st == GW_OK ? projection_workspace_run_on(b->projections, &w.down, b->product, b->shared_mlp, b->side) : st;
   };
   status = shared_mlp();
   // a failed call still brings its side stream back
-  if (fork) {
-    const cudaError_t recorded = cudaEventRecord(b->joined, b->side);
-    if (status != GW_OK) {
-      (void)cudaStreamWaitEvent(as_stream(s), b->joined, 0);
-      return status;
-    }
-    GW_CUDA_CHECK(recorded, "feed-forward block join");
+  const cudaError_t recorded = cudaEventRecord(b->joined, b->side);
+  if (status != GW_OK) {
+    (void)cudaStreamWaitEvent(as_stream(s), b->joined, 0);
+    return status;
   }
-  if (status != GW_OK) return status;
+  GW_CUDA_CHECK(recorded, "feed-forward block join");
   // router logits and the experts (batched_executor.cu:262-266)
-  if (fork) {
-    status = gw_bf16_plan_run(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes, s);
-  } else {
-    gw_projection router{};
-    router.storage = GW_STORAGE_BF16;
-    router.input = kHidden;
-    router.output = router.physical_output = kExperts;
-    router.bf16 = w.router_proj;
-    status = gw_projection_workspace_run(b->projections, &router, b->router_input, b->logits);
-  }
+  status = gw_bf16_plan_run(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes, s);
   MoeCombineInput combine;
   if (status == GW_OK)
     status = moe_run_to_down(b->moe, b->expert_input, b->logits, w.router_per_expert_scale, w.experts, rows, w.has_bf16, w.has_fp8,
                              w.has_nvfp4, gw_nvfp4_fp4_activations(b->policy, b->phase), as_stream(s), &combine);
-  if (fork) GW_CUDA_CHECK(cudaStreamWaitEvent(as_stream(s), b->joined, 0), "feed-forward block join");
+  GW_CUDA_CHECK(cudaStreamWaitEvent(as_stream(s), b->joined, 0), "feed-forward block join");
   if (status != GW_OK) return status;
   // the experts' weighted sum and the block's tail in one launch
   const NormArgs a = norm_args(b->shared_mlp, rows, kHidden);
