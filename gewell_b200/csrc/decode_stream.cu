@@ -10,6 +10,9 @@
 // are added through shared memory at the end, those that several SMs share through L2 by the one that
 // arrives last at the block's counter -- always in range order, so results do not depend on who comes last.
 //
+// Measured on cold weights (us, with everything a call does; activation quantiser + tcgen05 kernel in brackets): NVFP4
+// 1x2816x2816 5.4 (7.1), FP8 8x2816x2816 6.4 (8.1); W4A16 MLP of five rows 66 against 330 with dequantised weights.
+//
 // Token values live in shared memory in the order the tensor instruction wants them.  When all of K does
 // not fit there, K is cut into slabs, the flat sequence walks slab by slab and every row block has one sum
 // per slab.
@@ -372,16 +375,18 @@ cudaError_t launch_instance(const StreamArgs& args, const StreamPlan& plan, cuda
 
 template <StreamKind KIND>
 cudaError_t launch_kind(const StreamArgs& args, const StreamPlan& plan, bool pair, cudaStream_t stream) {
-  if (pair) return plan.tiles == 1 ? launch_instance<KIND, 1, true>(args, plan, stream) : launch_instance<KIND, 2, true>(args, plan, stream);
-  return plan.tiles == 1 ? launch_instance<KIND, 1, false>(args, plan, stream) : launch_instance<KIND, 2, false>(args, plan, stream);
+  if constexpr (KIND == StreamKind::w4a16)
+    if (plan.tiles == 2) return pair ? launch_instance<KIND, 2, true>(args, plan, stream) : launch_instance<KIND, 2, false>(args, plan, stream);
+  return pair ? launch_instance<KIND, 1, true>(args, plan, stream) : launch_instance<KIND, 1, false>(args, plan, stream);
 }
 
 struct Sizes { uint32_t warps, fixed, chunk; };
 template <StreamKind KIND>
 Sizes sizes_of(bool two, bool pair) {
   const auto of = [](auto layout) { using L = decltype(layout); return Sizes{L::kWarps, L::kFixedBytes, L::kChunkBytes}; };
-  if (pair) return two ? of(Layout<KIND, 2, true>{}) : of(Layout<KIND, 1, true>{});
-  return two ? of(Layout<KIND, 2, false>{}) : of(Layout<KIND, 1, false>{});
+  if constexpr (KIND == StreamKind::w4a16)
+    if (two) return pair ? of(Layout<KIND, 2, true>{}) : of(Layout<KIND, 2, false>{});
+  return pair ? of(Layout<KIND, 1, true>{}) : of(Layout<KIND, 1, false>{});
 }
 
 uint32_t row_bytes_of(StreamKind kind, uint32_t k) { return nvfp4_weights(kind) ? k / 2 : kind == StreamKind::w8a8 ? k : 2 * k; }
@@ -393,6 +398,9 @@ StreamPlan plan_stream(StreamKind kind, uint32_t rows, uint32_t k, uint32_t n, b
   const bool nvfp4 = nvfp4_weights(kind);
   // rows come in groups of 32 (the tensor map must not reach past the matrix), tokens in groups of sixteen values
   if (rows == 0 || rows > kStreamMaxRows || k % (nvfp4 ? 64 : 16) != 0 || n % 32 != 0 || n == 0 || k == 0) return p;
+  // A second group of eight tokens costs half as many instructions again per weight byte; where another kernel runs the same
+  // projection, it is the faster one from nine rows on.
+  if (rows > 8 && kind != StreamKind::w4a16) return p;
   p.physical_n = n;
   p.tiles = rows <= 8 ? 1 : 2;
   p.blocks = int((n + 127) / 128 * 4);

@@ -16,7 +16,7 @@ namespace gw {
 // w8a8: E4M3 weights and activations; w16a16: BF16 both.
 enum class StreamKind { w4a4, w4a16, w8a8, w16a16 };
 
-constexpr uint32_t kStreamMaxRows = 16;
+constexpr uint32_t kStreamMaxRows = 16;   // W4A16; the other kinds take eight
 
 struct StreamMatrix {
   const void* data = nullptr;            // [n, k] row-major, packed as the kind says

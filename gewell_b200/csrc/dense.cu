@@ -46,7 +46,7 @@ size_t split_counter_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n)
 // W4A16 has no other kernel that reads the packed weights.
 bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
   if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
-  return plan.tiles == 1 && n <= 5376 && k <= 16384 && size_t(rows) * k <= 24 * 1024;
+  return n <= 5376 && k <= 16384 && size_t(rows) * k <= 24 * 1024;
 }
 
 // Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each.
@@ -61,7 +61,7 @@ bool stream_pair_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, ui
   if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
   const size_t bytes = 2 * n * k * (kind == StreamKind::w4a4 ? 9 : kind == StreamKind::w8a8 ? 16 : 32) / 16;
   const size_t values = size_t(rows) * k;
-  return plan.tiles == 1 && (n <= 4224 ? values <= 24 * 1024 : bytes >= (size_t(96) << 20) && values <= 8192);
+  return n <= 4224 ? values <= 24 * 1024 : bytes >= (size_t(96) << 20) && values <= 8192;
 }
 
 namespace {
