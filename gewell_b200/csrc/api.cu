@@ -247,6 +247,15 @@ void gw_nvfp4_plan_destroy(gw_nvfp4_plan* plan) { delete plan; }
 gw_status gw_nvfp4_plan_run(gw_nvfp4_plan* plan, const void* input_bf16, const uint8_t* weight_data,
                             const uint8_t* weight_scales, float input_scale, float weight_scale, void* output_bf16,
                             void* scratch, size_t scratch_capacity, void* stream, int transform) {
+  return run_nvfp4_plan(plan, input_bf16, weight_data, weight_scales, input_scale, weight_scale, output_bf16, scratch, scratch_capacity,
+                        as_stream(stream), transform, false);
+}
+
+}  // extern "C"
+
+gw_status gw::run_nvfp4_plan(gw_nvfp4_plan* plan, const void* input_bf16, const uint8_t* weight_data, const uint8_t* weight_scales,
+                             float input_scale, float weight_scale, void* output_bf16, void* scratch, size_t scratch_capacity,
+                             cudaStream_t s, int transform, bool weights_settled) {
   clear_error();
   if (!plan) return fail(GW_INVALID_ARGUMENT, "NVFP4 run requires a plan");
   const float alpha = input_scale * weight_scale;
@@ -259,7 +268,6 @@ gw_status gw_nvfp4_plan_run(gw_nvfp4_plan* plan, const void* input_bf16, const u
                 "scales");
   if (!aligned(input_bf16, 16) || !aligned(weight_data, 16) || !aligned(weight_scales, 16) || !aligned(output_bf16, 2))
     return fail(GW_INVALID_ARGUMENT, "NVFP4 run requires 16-byte aligned input, weights and weight scales");
-  cudaStream_t s = as_stream(stream);
   auto* packed = static_cast<uint8_t*>(scratch);
   uint8_t* scales = packed + plan->scale_offset;
   {
@@ -274,6 +282,7 @@ gw_status gw_nvfp4_plan_run(gw_nvfp4_plan* plan, const void* input_bf16, const u
     q.workspace = packed + plan->split_offset;
     q.counters = plan->descriptors.split_counters;
     q.error = device_error_word();
+    q.weights_settled = weights_settled;
     bool done = false;
     const gw_status status = launch_dense_stream(q, &plan->descriptors, s, &done);
     if (status != GW_OK || done) return status;
@@ -284,8 +293,11 @@ gw_status gw_nvfp4_plan_run(gw_nvfp4_plan* plan, const void* input_bf16, const u
   DenseProblem problem{GemmKind::nvfp4, plan->rows, plan->input_width, plan->output_width, weight_data, weight_scales,
                        packed, scales, alpha, nullptr, output_bf16, device_error_word()};
   if (plan->total_bytes != plan->split_offset) problem.split_workspace = packed + plan->split_offset;
+  problem.weights_settled = weights_settled;
   return launch_dense(problem, &plan->descriptors, s);
 }
+
+extern "C" {
 
 // --------------------------------------------------------------------------- FP8
 
@@ -363,6 +375,15 @@ void gw_fp8_plan_destroy(gw_fp8_plan* plan) { delete plan; }
 gw_status gw_fp8_plan_run(gw_fp8_plan* plan, const void* input_bf16, const uint8_t* weight_data, float input_scale,
                           float weight_scale, const float* channel_scales, void* output_bf16, void* scratch,
                           size_t scratch_capacity, void* stream, int transform) {
+  return run_fp8_plan(plan, input_bf16, weight_data, input_scale, weight_scale, channel_scales, output_bf16, scratch, scratch_capacity,
+                      as_stream(stream), transform, false);
+}
+
+}  // extern "C"
+
+gw_status gw::run_fp8_plan(gw_fp8_plan* plan, const void* input_bf16, const uint8_t* weight_data, float input_scale, float weight_scale,
+                           const float* channel_scales, void* output_bf16, void* scratch, size_t scratch_capacity, cudaStream_t s,
+                           int transform, bool weights_settled) {
   clear_error();
   if (!plan) return fail(GW_INVALID_ARGUMENT, "FP8 run requires a plan");
   const float alpha = input_scale * weight_scale;
@@ -375,7 +396,6 @@ gw_status gw_fp8_plan_run(gw_fp8_plan* plan, const void* input_bf16, const uint8
     return fail(GW_INVALID_ARGUMENT,
                 "FP8 run requires valid aligned device buffers, sufficient scratch, and finite positive global "
                 "scales with a finite positive product and finite input-scale reciprocal");
-  cudaStream_t s = as_stream(stream);
   auto* packed = static_cast<uint8_t*>(scratch);
   if (plan->gemv_rows == 0) {
     StreamProblem q{StreamKind::w8a8, plan->rows, plan->input_width, plan->output_width, input_bf16};
@@ -387,6 +407,7 @@ gw_status gw_fp8_plan_run(gw_fp8_plan* plan, const void* input_bf16, const uint8
     q.workspace = packed + plan->split_offset;
     q.counters = plan->descriptors.split_counters;
     q.error = device_error_word();
+    q.weights_settled = weights_settled;
     bool done = false;
     const gw_status status = launch_dense_stream(q, &plan->descriptors, s, &done);
     if (status != GW_OK || done) return status;
@@ -410,8 +431,11 @@ gw_status gw_fp8_plan_run(gw_fp8_plan* plan, const void* input_bf16, const uint8
                        packed, nullptr, alpha, plan->channel_scales ? channel_scales : nullptr, output_bf16,
                        device_error_word()};
   if (plan->total_bytes != plan->split_offset) problem.split_workspace = packed + plan->split_offset;
+  problem.weights_settled = weights_settled;
   return launch_dense(problem, &plan->descriptors, s);
 }
+
+extern "C" {
 
 // --------------------------------------------------------------------------- BF16
 
@@ -453,6 +477,13 @@ void gw_bf16_plan_destroy(gw_bf16_plan* plan) { delete plan; }
 
 gw_status gw_bf16_plan_run(gw_bf16_plan* plan, const void* input_bf16, const void* weight_bf16, void* output_bf16,
                            void* scratch, size_t scratch_capacity, void* stream) {
+  return run_bf16_plan(plan, input_bf16, weight_bf16, output_bf16, scratch, scratch_capacity, as_stream(stream), false);
+}
+
+}  // extern "C"
+
+gw_status gw::run_bf16_plan(gw_bf16_plan* plan, const void* input_bf16, const void* weight_bf16, void* output_bf16, void* scratch,
+                            size_t scratch_capacity, cudaStream_t s, bool weights_settled) {
   clear_error();
   if (!plan) return fail(GW_INVALID_ARGUMENT, "BF16 run requires a plan");
   // scratch == NULL is allowed: decode-shaped plans then keep whole tiles per CTA instead of the K split
@@ -468,15 +499,19 @@ gw_status gw_bf16_plan_run(gw_bf16_plan* plan, const void* input_bf16, const voi
     q.workspace = scratch;
     q.counters = plan->descriptors.split_counters;
     q.error = device_error_word();
+    q.weights_settled = weights_settled;
     bool done = false;
-    const gw_status status = launch_dense_stream(q, &plan->descriptors, as_stream(stream), &done);
+    const gw_status status = launch_dense_stream(q, &plan->descriptors, s, &done);
     if (status != GW_OK || done) return status;
   }
   DenseProblem problem{GemmKind::bf16, plan->rows, plan->input_width, plan->output_width, weight_bf16, nullptr,
                        input_bf16, nullptr, 1.0F, nullptr, output_bf16, device_error_word()};
   if (plan->total_bytes != 0 && scratch) problem.split_workspace = scratch;
-  return launch_dense(problem, &plan->descriptors, as_stream(stream));
+  problem.weights_settled = weights_settled;
+  return launch_dense(problem, &plan->descriptors, s);
 }
+
+extern "C" {
 
 // --------------------------------------------------------------------------- weight QDQ
 

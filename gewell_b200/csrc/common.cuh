@@ -79,18 +79,36 @@ struct Divisor {
 // Programmatic dependent launch.  A kernel launched with the programmatic-
 // serialisation attribute may start while its predecessor in the stream still
 // runs; griddep_wait() blocks until that predecessor has completed and its
-// writes are visible (no-op for a normal launch).  griddep_launch() lets the
-// successor start being scheduled.  Every kernel that can be launched that way
-// calls griddep_wait() in all threads before touching global memory, so the
-// usual stream order still holds transitively.
+// writes are visible (no-op for a normal launch).  griddep_enter() waits and
+// then lets the successor start being scheduled: so when a kernel starts,
+// everything before its direct predecessor is complete and visible, and only
+// what that one predecessor writes is not.  The activation quantisers alone
+// let the successor start first (griddep_enter_first): they are short, and the
+// GEMM behind them gets its weights under way at the end of the kernel in
+// front of them.  Before its wait a kernel may
+//   - read the launch's parameters and what the host wrote before the launch,
+//   - bring weights into L2 (ptx::tma_prefetch_*), whoever writes them,
+//   - read weights that are settled: in front of the launch, or of the
+//     quantiser before it, the same call launched another kernel, which is no
+//     quantiser and writes no weights (weights_settled in StreamProblem and
+//     DenseProblem).  Of what runs in front of a public entry point's first
+//     launch nothing is known; it may have produced the weights.
+// Everything else in global memory is touched after the wait.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void griddep_enter() {
+  griddep_wait();
+  griddep_launch();
+}
+__device__ __forceinline__ void griddep_enter_first() {
+  griddep_launch();
+  griddep_wait();
+}
 
 #endif  // __CUDACC__
 
 // Launch with the programmatic-serialisation attribute: the kernel may be scheduled while
-// its predecessor in the stream drains; it must call griddep_wait() before it touches global
-// memory (every kernel launched through this helper does so first thing).
+// its predecessor in the stream drains, and keeps to the rule above.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl_shared(void (*kernel)(Params...), dim3 grid, dim3 block, size_t shared_bytes, cudaStream_t stream,
                                      Args&&... args) {

@@ -39,6 +39,8 @@ struct StreamProblem {
   void* workspace = nullptr;   // StreamPlan::workspace_bytes, 16-byte aligned
   int32_t* counters = nullptr; // StreamPlan::counter_count zeroed ints; left zero
   bool reread = false;         // another launch reads the same weights soon
+  bool weights_settled = false;   // the same call launched the kernel before this one, which does not write the weights: the first
+                                  // pieces are read while it still runs.  Otherwise they wait in L2 meanwhile
   uint32_t* error = nullptr;   // device error word
 };
 

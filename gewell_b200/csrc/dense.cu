@@ -200,7 +200,7 @@ gw_status StreamBook::prepare(uint32_t new_rows, const std::vector<std::pair<uin
 }
 
 gw_status StreamBook::run(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4,
-                          void* workspace, cudaStream_t s, bool* done) {
+                          void* workspace, bool weights_settled, cudaStream_t s, bool* done) {
   *done = false;
   if (second && (second->storage != first.storage || second->input != first.input || second->output != first.output ||
                  second->physical_output != first.physical_output)) return GW_OK;
@@ -248,6 +248,7 @@ gw_status StreamBook::run(const gw_projection& first, const gw_projection* secon
   for (uint32_t row = 0; row < rows; row += kStreamMaxRows) {
     q.rows = std::min(rows - row, kStreamMaxRows);
     q.reread = rows - row > kStreamMaxRows;
+    q.weights_settled = weights_settled || row != 0;      // of this projection's launches only the first follows another's
     q.input = static_cast<const bf16*>(input) + size_t(row) * q.k;
     q.output = static_cast<bf16*>(output) + size_t(row) * q.ld_out;
     GW_CUDA_CHECK(launch_stream(q, with.plan, with.maps[0], with.maps[1], s), "weight-streaming projection");
@@ -320,7 +321,7 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
   g.map_l = -1;
   g.map_c[0] = g.map_c[1] = -1;
   if (swap) {
-    params.early_weights = 1;   // weights are never written by the activation-quantise kernel before this launch
+    params.weights_settled = q.weights_settled ? 1 : 0;
     params.map_l = cache->weight_map;
     params.map_c = cache->activation_map;
     params.c_rows_per_tile = block_n;

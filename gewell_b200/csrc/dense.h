@@ -64,6 +64,9 @@ struct DenseProblem {
   // partial tiles.  With it (and the plan's counters) the K loop of the weight tiles is
   // divided evenly over the SMs (see GemmParams).
   void* split_workspace = nullptr;
+  // In front of this launch, or of the quantiser of its activations, the same call launched a kernel that does not write the
+  // weights: the swap form reads its first weight tiles while that kernel still runs.  Otherwise they wait in L2 meanwhile.
+  bool weights_settled = false;
 };
 
 // true: weights on the 128-lane operand and tokens on the column operand.
@@ -98,17 +101,28 @@ struct StreamBook {
   // The projection `first` -- or, with `second`, GeGLU of both -- into [rows, first.output]; *done = false when the shape,
   // the storage or the pointers keep it off the kernel.
   gw_status run(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4, void* workspace,
-                cudaStream_t stream, bool* done);
+                bool weights_settled, cudaStream_t stream, bool* done);
 };
 
 gw_status launch_dense(const DenseProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
+// gw_*_plan_run as a step of a longer call (api.cu): `weights_settled` as in DenseProblem.  The public entry points pass
+// false.
+gw_status run_nvfp4_plan(gw_nvfp4_plan* plan, const void* input, const uint8_t* weight_data, const uint8_t* weight_scales, float input_scale,
+                         float weight_scale, void* output, void* scratch, size_t scratch_capacity, cudaStream_t stream, int transform,
+                         bool weights_settled);
+gw_status run_fp8_plan(gw_fp8_plan* plan, const void* input, const uint8_t* weight_data, float input_scale, float weight_scale,
+                       const float* channel_scales, void* output, void* scratch, size_t scratch_capacity, cudaStream_t stream, int transform,
+                       bool weights_settled);
+gw_status run_bf16_plan(gw_bf16_plan* plan, const void* input, const void* weight, void* output, void* scratch, size_t scratch_capacity,
+                        cudaStream_t stream, bool weights_settled);
+
 // gw_projection_workspace_run on a stream of the caller's choice (projection.cu).
 gw_status projection_workspace_run_on(gw_projection_workspace* workspace, const gw_projection* projection, const void* input, void* output,
-                                      cudaStream_t stream);
+                                      cudaStream_t stream, bool weights_settled);
 // product = GeGLU of both projections of a prepared workspace in one launch; *done = false when that is not the faster
 // way here.
 gw_status projection_workspace_run_geglu(gw_projection_workspace* workspace, const gw_projection& gate, const gw_projection& up,
-                                         const void* input, void* product, cudaStream_t stream, bool* done);
+                                         const void* input, void* product, cudaStream_t stream, bool weights_settled, bool* done);
 
 }  // namespace gw

@@ -161,11 +161,10 @@ __global__ void __launch_bounds__(kNormThreads) rms_norm_kernel(NormArgs a, cons
   bf16* row = reinterpret_cast<bf16*>(norm_smem);
   float* totals = reinterpret_cast<float*>(norm_smem + size_t(a.width) * sizeof(bf16));
   const uint32_t vectors = a.width / 8;
-  griddep_launch();
+  griddep_enter();
   RowPart<NV> x, w;
-  if (weight) w.load_any(weight, vectors);
-  griddep_wait();
   x.load(a.input + size_t(blockIdx.x) * a.width, vectors);
+  if (weight) w.load_any(weight, vectors);
   x.store(row, vectors);
   float inv[1];
   inverse_rms<1>(a, {row}, totals, inv);
@@ -193,13 +192,12 @@ __global__ void __launch_bounds__(kNormThreads) rms_norm_feedforward_kernel(Norm
   bf16* row = reinterpret_cast<bf16*>(norm_smem);
   float* totals = reinterpret_cast<float*>(norm_smem + size_t(a.width) * sizeof(bf16));
   const uint32_t vectors = a.width / 8;
-  griddep_launch();
+  griddep_enter();
   RowPart<NV> x, shared, expert, router;
+  x.load(a.input + size_t(blockIdx.x) * a.width, vectors);
   shared.load_any(f.shared_weight, vectors);
   expert.load_any(f.expert_weight, vectors);
   router.load_any(f.router_weight, vectors);
-  griddep_wait();
-  x.load(a.input + size_t(blockIdx.x) * a.width, vectors);
   x.store(row, vectors);
   float inv[1];
   inverse_rms<1>(a, {row}, totals, inv);
@@ -243,13 +241,14 @@ __global__ void __launch_bounds__(kNormThreads) ffn_tail_kernel(NormArgs a, Tail
   float* totals = reinterpret_cast<float*>(norm_smem + size_t(2) * a.width * sizeof(bf16));
   const size_t base = size_t(blockIdx.x) * a.width;
   const uint32_t vectors = a.width / 8;
-  griddep_launch();
+  // inside a block the launch before is the experts' down GEMM, which writes none of the four weights below
+  if constexpr (!COMBINE) griddep_enter();
   RowPart<NV> shared, branch, norm_shared, norm_routed, norm_sum, hidden;
   norm_shared.load_any(t.norm_shared, vectors);
   norm_routed.load_any(t.norm_routed, vectors);
   norm_sum.load_any(t.norm_sum, vectors);
   const float scalar = as_float(*t.layer_scalar);
-  griddep_wait();
+  if constexpr (COMBINE) griddep_enter();
   shared.load(t.shared_mlp + base, vectors);
   if constexpr (COMBINE) {
     __shared__ int32_t slot_row[kTopK];
@@ -295,8 +294,7 @@ __global__ void __launch_bounds__(kNormThreads) ffn_tail_kernel(NormArgs a, Tail
 // VECTOR: every buffer 16-byte aligned, a thread has eight values
 template <bool VECTOR>
 __global__ void add_kernel(const bf16* a, const bf16* b, bf16* y, size_t n) {
-  griddep_launch();
-  griddep_wait();
+  griddep_enter();
   const size_t i = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * (VECTOR ? 8 : 1);
   if (VECTOR && i + 8 <= n) {
     Vec u, v;
@@ -313,8 +311,7 @@ __global__ void add_kernel(const bf16* a, const bf16* b, bf16* y, size_t n) {
 // x = bf16(x * scalar[0])                                               (batched_executor.cu:30-33)
 template <bool VECTOR>
 __global__ void scale_kernel(bf16* x, const bf16* scalar, size_t n) {
-  griddep_launch();
-  griddep_wait();
+  griddep_enter();
   const float s = as_float(*scalar);
   const size_t i = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) * (VECTOR ? 8 : 1);
   if (VECTOR && i + 8 <= n) {
@@ -605,15 +602,17 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
   // shared MLP (batched_executor.cu:256-259)
   GW_CUDA_CHECK(cudaEventRecord(b->forked, as_stream(s)), "feed-forward block fork");
   GW_CUDA_CHECK(cudaStreamWaitEvent(b->side, b->forked, 0), "feed-forward block fork");
+  // in front of every launch of both streams is one of this call's own, which writes no weights
   const auto shared_mlp = [&]() {
     bool product_done = false;
-    gw_status st = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, b->side, &product_done);
+    gw_status st = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, b->side, true,
+                                                  &product_done);
     if (st == GW_OK && !product_done) {
-      st = projection_workspace_run_on(b->projections, &w.gate, b->normalized, b->gate, b->side);
-      if (st == GW_OK) st = projection_workspace_run_on(b->projections, &w.up, b->normalized, b->up, b->side);
+      st = projection_workspace_run_on(b->projections, &w.gate, b->normalized, b->gate, b->side, true);
+      if (st == GW_OK) st = projection_workspace_run_on(b->projections, &w.up, b->normalized, b->up, b->side, true);
       if (st == GW_OK) st = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, b->side);
     }
-    return st == GW_OK ? projection_workspace_run_on(b->projections, &w.down, b->product, b->shared_mlp, b->side) : st;
+    return st == GW_OK ? projection_workspace_run_on(b->projections, &w.down, b->product, b->shared_mlp, b->side, true) : st;
   };
   status = shared_mlp();
   // a failed call still brings its side stream back
@@ -624,7 +623,8 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
   }
   GW_CUDA_CHECK(recorded, "feed-forward block join");
   // router logits and the experts (batched_executor.cu:262-266)
-  status = gw_bf16_plan_run(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes, s);
+  status = run_bf16_plan(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes,
+                         as_stream(s), true);
   MoeCombineInput combine;
   if (status == GW_OK)
     status = moe_run_to_down(b->moe, b->expert_input, b->logits, w.router_per_expert_scale, w.experts, rows, w.has_bf16, w.has_fp8,

@@ -70,7 +70,6 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
   const uint32_t rank = cluster_rank();           // 0 = leader of the pair
-  griddep_launch();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(full_bar + s, 1);
@@ -93,7 +92,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   cluster_sync_all();                               // both CTAs' barriers exist before anybody signals them
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  griddep_wait();
+  griddep_enter();
 
   const int total_kb = p.k / 64;
   const int k_stages = (total_kb + kKBlocks - 1) / kKBlocks;

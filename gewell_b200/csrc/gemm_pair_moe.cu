@@ -165,7 +165,6 @@ pair_moe_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
   const uint32_t rank = cluster_rank();           // 0 = leader of the pair
-  griddep_launch();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(full_bar + s, 1);
@@ -188,7 +187,7 @@ pair_moe_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
   cluster_sync_all();                               // both CTAs' barriers exist before anybody signals them
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  griddep_wait();                                   // the offsets and the quantised rows come from earlier kernels
+  griddep_enter();                                  // the offsets and the quantised rows come from earlier kernels
   build_work_table(p, table, kCTiles);
 
   const int total = table->prefix[kExperts];
@@ -565,7 +564,6 @@ pair_moe_down_kernel(const __grid_constant__ PairMoeParams p) {
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
   const uint32_t rank = cluster_rank();
-  griddep_launch();
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(a_full_bar + b, 1);
@@ -593,7 +591,7 @@ pair_moe_down_kernel(const __grid_constant__ PairMoeParams p) {
   cluster_sync_all();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  griddep_wait();
+  griddep_enter();
   build_work_table(p, table, kChunks);
 
   const int total = table->prefix[kExperts];

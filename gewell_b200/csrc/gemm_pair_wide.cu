@@ -102,7 +102,6 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
   const uint32_t rank = cluster_rank();           // 0 = leader of the pair
-  griddep_launch();
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
       ptx::mbar_init(full_bar + s, 1);
@@ -125,7 +124,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
   cluster_sync_all();                               // both CTAs' barriers exist before anybody signals them
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
-  griddep_wait();
+  griddep_enter();
   const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
   const int total_work = p.channel_tiles * p.token_tiles;
 

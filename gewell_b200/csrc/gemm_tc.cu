@@ -176,7 +176,6 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* split_flag = reinterpret_cast<volatile int*>(tmem_slot + 2);
   int32_t* prefix = reinterpret_cast<int32_t*>(tmem_slot + 4);   // work_begin of every group (+ sentinel)
-  griddep_launch();
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0);
   const int lane = threadIdx.x % 32;
@@ -205,8 +204,8 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // Everything above is independent of earlier kernels in the stream and may overlap
   // them (programmatic dependent launch); from here on their results are read.
-  const bool early_weights = EPI == GemmEpilogue::swap_store && p.groups == nullptr && p.early_weights != 0;
-  if (!(early_weights && warp == 0)) griddep_wait();
+  const bool ahead_of_wait = EPI == GemmEpilogue::swap_store && p.groups == nullptr;      // the producer begins before its wait
+  if (!(ahead_of_wait && warp == 0)) griddep_enter();
   if (p.groups != nullptr) {
     for (int i = threadIdx.x; i <= p.num_groups; i += kThreads) prefix[i] = p.groups[i].work_begin;
     __syncthreads();
@@ -248,7 +247,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
     uint32_t phase = 0;
     int fetched = -1;                    // group whose descriptor has been asked for
     const uint64_t evict_first = ptx::l2_evict_first(), evict_normal = ptx::l2_evict_normal();
-    bool waited = !early_weights;        // this warp defers its wait for the previous kernel (see below)
+    bool waited = !ahead_of_wait;        // this warp defers its wait for the previous kernel (see below)
     WorkItem item;
     SegmentWalk walk(int(blockIdx.x), int(gridDim.x), split, total_work, k_stages, p.work_chunk);
     int tile, ks0, ks1;
@@ -340,15 +339,27 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
         }
       };
       int ks_begin = ks0;
-      if (early_weights && !waited) {
-        // Decode shapes: the weights (L side) do not depend on the kernel that quantises the
+      if (ahead_of_wait && !waited) {
+        // Decode shapes: the weights (L side) do not depend on a kernel that quantises the
         // activations, so the first ring of weight copies is issued before waiting for it;
-        // the token-side copies of those stages follow once it has finished.
+        // the token-side copies of those stages follow once it has finished.  Weights that the
+        // previous kernel may have written come as far as L2 meanwhile.
         const int ahead = min(C::kStages, ks1 - ks0);
-        for (int i = 0; i < ahead; ++i) issue(ks0 + i, i, true, false);
+        const bool settled = p.weights_settled != 0;
+        for (int i = 0; i < ahead; ++i) {
+          if (settled) {
+            issue(ks0 + i, i, true, false);
+            continue;
+          }
+#pragma unroll
+          for (int slab = 0; slab < kSlabs; ++slab) {
+            const int x = ((ks0 + i) * kSlabs + slab) * kStageRowBytes;
+            if (x < k_bytes) ptx::tma_prefetch_2d(map_l, x, l_row, l_policy);
+          }
+        }
         griddep_wait();
         waited = true;
-        for (int i = 0; i < ahead; ++i) issue(ks0 + i, i, false, true);
+        for (int i = 0; i < ahead; ++i) issue(ks0 + i, i, !settled, true);
         stage = ahead == C::kStages ? 0 : ahead;
         phase = ahead == C::kStages ? 1 : 0;
         ks_begin = ks0 + ahead;

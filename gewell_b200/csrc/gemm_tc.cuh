@@ -72,7 +72,7 @@ struct GemmParams {
   float* split_partials;          // [2 * grid][128 * BLOCK_N] FP32, or nullptr (whole tiles per CTA)
   int32_t* split_counters;        // [work items], zero at launch; left zero by the kernel
   int32_t work_chunk;             // consecutive work items a CTA takes before it strides on (0 or 1: one; -1: one contiguous range)
-  int32_t early_weights;          // swap form, groups == nullptr: the L operand (weights, weight scales) does not
+  int32_t weights_settled;        // swap form, groups == nullptr: the L operand (weights, weight scales) does not
                                   // depend on the previous kernel in the stream, so its first copies may be
                                   // issued before that kernel has finished (programmatic dependent launch)
   uint32_t* error;                // device error word (0 = fine)

@@ -140,9 +140,9 @@ struct PlanBook {
   }
 
   // `first` or GeGLU of `first` and `second` on the weight-streaming kernel, if that is the faster one here
-  gw_status stream(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4, cudaStream_t s,
-                   bool* done) {
-    return streaming.run(first, second, input, output, fp4, scratch.data, s, done);
+  gw_status stream(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4,
+                   bool weights_settled, cudaStream_t s, bool* done) {
+    return streaming.run(first, second, input, output, fp4, scratch.data, weights_settled, s, done);
   }
 };
 
@@ -244,13 +244,15 @@ gw_status gw_qkv_projector_prepare(gw_qkv_projector* q, uint32_t rows) {
 namespace {
 
 // projection_linear (executor.cuh:1187-1215): FP8 -> NVFP4 with FP4 activations -> BF16 GEMM (on the
-// BF16 weight, or on the NVFP4 weight dequantised into the book's buffer)
+// BF16 weight, or on the NVFP4 weight dequantised into the book's buffer).  `first`: the call's first projection, in front of
+// which anything may run; in front of every later one is a launch of the call itself, which writes no weights.
 gw_status run_linear(PlanBook& book, const gw_projection& p, const void* input, void* output, bool fp4, int transform,
-                     cudaStream_t s) {
+                     cudaStream_t s, bool first = false) {
+  bool settled = !first;
   const uint32_t n = p.storage == GW_STORAGE_NVFP4_W4A4 ? p.physical_output : p.output;
   if (p.storage == GW_STORAGE_NVFP4_W4A4 && !fp4 && transform == GW_TRANSFORM_IDENTITY && n == p.output) {
     bool done = false;
-    const gw_status status = book.stream(p, nullptr, input, output, fp4, s, &done);
+    const gw_status status = book.stream(p, nullptr, input, output, fp4, settled, s, &done);
     if (status != GW_OK || done) return status;
   }
   const auto plan = [&](int kind) -> const PlanSet* {
@@ -260,14 +262,14 @@ gw_status run_linear(PlanBook& book, const gw_projection& p, const void* input, 
   if (p.storage == GW_STORAGE_FP8_W8A8) {
     const PlanSet* set = plan(p.fp8_channel_scales ? kFp8Channel : kFp8);
     if (!set) return fail(GW_INVALID_ARGUMENT, "projection shape is not one of the object's shapes");
-    return gw_fp8_plan_run(set->fp8, input, p.fp8_data, p.fp8_input_scale, p.fp8_weight_scale, p.fp8_channel_scales, output,
-                           book.scratch.data, book.scratch.bytes, s, transform);
+    return run_fp8_plan(set->fp8, input, p.fp8_data, p.fp8_input_scale, p.fp8_weight_scale, p.fp8_channel_scales, output,
+                        book.scratch.data, book.scratch.bytes, s, transform, settled);
   }
   if (p.storage == GW_STORAGE_NVFP4_W4A4 && fp4) {
     const PlanSet* set = plan(kNvfp4);
     if (!set) return fail(GW_INVALID_ARGUMENT, "projection shape is not one of the object's shapes");
-    return gw_nvfp4_plan_run(set->nvfp4, input, p.nvfp4_data, p.nvfp4_scales, p.nvfp4_input_scale, p.nvfp4_weight_scale,
-                             output, book.scratch.data, book.scratch.bytes, s, transform);
+    return run_nvfp4_plan(set->nvfp4, input, p.nvfp4_data, p.nvfp4_scales, p.nvfp4_input_scale, p.nvfp4_weight_scale, output,
+                          book.scratch.data, book.scratch.bytes, s, transform, settled);
   }
   if (transform != GW_TRANSFORM_IDENTITY) return fail(GW_INVALID_ARGUMENT, "the BF16 path has no fused input transform");
   const PlanSet* set = plan(kBf16);
@@ -280,8 +282,9 @@ gw_status run_linear(PlanBook& book, const gw_projection& p, const void* input, 
                                                  book.dequantized.data, s);
     if (status != GW_OK) return status;
     weights = book.dequantized.data;
+    settled = false;
   }
-  return gw_bf16_plan_run(set->bf16, input, weights, output, book.scratch.data, book.scratch.bytes, s);
+  return run_bf16_plan(set->bf16, input, weights, output, book.scratch.data, book.scratch.bytes, s, settled);
 }
 
 gw_projection widened(const gw_projection& first, uint32_t output) {
@@ -312,14 +315,14 @@ gw_status gw_mlp_chain_run(gw_mlp_chain* c, const gw_projection* gate, const gw_
   auto* gate_out = static_cast<bf16*>(gate_up_bf16);
   gw_status status = GW_OK;
   bool paired = false;
-  if (status = c->book.stream(*gate, up, input_bf16, product_bf16, fp4, s, &paired); status != GW_OK) return status;
+  if (status = c->book.stream(*gate, up, input_bf16, product_bf16, fp4, false, s, &paired); status != GW_OK) return status;
   if (paired)                    // one launch: gate, up and GeGLU
     return run_linear(c->book, *down, product_bf16, output_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
   bool interleaved = true;       // gate_up holds [rows, gate | up]; otherwise gate rows, then up rows
   if ((nvfp4_joined(*gate, *up) && fp4) || fp8_joined(*gate, *up) || bf16_joined(*gate, *up)) {
-    status = run_linear(c->book, widened(*gate, 2 * m), input_bf16, gate_out, fp4, GW_TRANSFORM_IDENTITY, s);
+    status = run_linear(c->book, widened(*gate, 2 * m), input_bf16, gate_out, fp4, GW_TRANSFORM_IDENTITY, s, true);
   } else {
-    status = run_linear(c->book, *gate, input_bf16, gate_out, fp4, GW_TRANSFORM_IDENTITY, s);
+    status = run_linear(c->book, *gate, input_bf16, gate_out, fp4, GW_TRANSFORM_IDENTITY, s, true);
     if (status == GW_OK)
       status = run_linear(c->book, *up, input_bf16, gate_out + size_t(rows) * m, fp4, GW_TRANSFORM_IDENTITY, s);
     interleaved = false;
@@ -356,8 +359,8 @@ gw_status gw_qkv_projector_run(gw_qkv_projector* q, const gw_projection* query, 
   const bool fp8_run = fp8_joined(*query, *key) && (!value || fp8_joined(*key, *value));
   if (joined) *joined = (bf16_run || fp8_run) ? 1 : 0;
   if (bf16_run || fp8_run)      // one GEMM; the caller reads [rows, Q | K | V] from q_bf16
-    return run_linear(q->book, widened(*query, width), input_bf16, q_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
-  gw_status status = run_linear(q->book, *query, input_bf16, q_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
+    return run_linear(q->book, widened(*query, width), input_bf16, q_bf16, fp4, GW_TRANSFORM_IDENTITY, s, true);
+  gw_status status = run_linear(q->book, *query, input_bf16, q_bf16, fp4, GW_TRANSFORM_IDENTITY, s, true);
   if (status == GW_OK) status = run_linear(q->book, *key, input_bf16, k_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
   if (status == GW_OK && value) status = run_linear(q->book, *value, input_bf16, v_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
   return status;

@@ -219,7 +219,7 @@ __device__ __forceinline__ void prepare_groups(const MoeGroupPlan& plan, const M
   }
 }
 
-// The scales of this lane's experts (lane, lane + 32, ...): weights, so they are read while the kernel before still runs.
+// The scales of this lane's experts (lane, lane + 32, ...); needed last, so their loads overlap the softmax.
 __device__ __forceinline__ void load_expert_scales(const bf16* __restrict__ expert_scales, unsigned lane, float (&scale)[4]) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) scale[q] = __bfloat162float(expert_scales[lane + 32 * q]);
@@ -318,11 +318,10 @@ __global__ void __launch_bounds__(256)
 moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales, uint32_t rows,
                  int32_t* __restrict__ keys, float* __restrict__ weights, uint32_t* __restrict__ bitmaps,
                  int32_t* __restrict__ chunk_counts) {
-  griddep_launch();
   const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   float expert_scale[4];
   load_expert_scales(expert_scales, lane, expert_scale);
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
   __shared__ uint32_t bitmap[kExperts][2];
   if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
   __syncthreads();
@@ -360,17 +359,16 @@ moe_route_cluster_kernel(const bf16* __restrict__ scores, const bf16* __restrict
   __shared__ uint32_t bitmap[kExperts][2];
   __shared__ int32_t shared_keys[kChunkTokens * kTopK];
   __shared__ int32_t base[kExperts];
-  griddep_launch();
   const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32, block = pair::cluster_rank();
-  float expert_scale[4];
-  load_expert_scales(expert_scales, lane, expert_scale);
   MoeExpertInfo info{};
   if (block == 0) {
     if (first_groups != nullptr) info = plan.experts[threadIdx.x / 2];   // of the expert table, written when it was created
     if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
   }
   pair::cluster_sync_all();                // the first block's bitmaps are clear
-  griddep_wait();                          // results of earlier kernels in the stream are read from here on
+  griddep_enter();                         // results of earlier kernels in the stream are read from here on
+  float expert_scale[4];
+  load_expert_scales(expert_scales, lane, expert_scale);
   const uint32_t token = block * 8 + warp;
   if (token < rows)
     route_token(scores, expert_scale, token, token, lane, keys, weights, pair::leader_address(bitmap), pair::leader_address(shared_keys));
@@ -472,11 +470,10 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
                       uint32_t* __restrict__ bitmaps, int32_t* __restrict__ chunk_counts, int32_t* __restrict__ offsets,
                       int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
                       int32_t* __restrict__ inverse, uint32_t* __restrict__ barrier_state, uint32_t* __restrict__ error) {
-  griddep_launch();
   const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   float expert_scale[4];
   load_expert_scales(expert_scales, lane, expert_scale);
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
   __shared__ uint32_t bitmap[kExperts][2];
   __shared__ int32_t own_base[kRouteOwnChunks][kExperts];
   __shared__ int32_t part_sum[kRouteParts][kExperts];
@@ -584,8 +581,7 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kExperts)
 moe_scan_kernel(int32_t* __restrict__ chunk_counts, uint32_t chunks, int32_t* __restrict__ offsets) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   __shared__ int32_t totals[kExperts];
   const unsigned e = threadIdx.x;
   int32_t running = 0;
@@ -613,8 +609,7 @@ moe_scatter_kernel(const int32_t* __restrict__ keys, const uint32_t* __restrict_
                    const int32_t* __restrict__ chunk_base, const int32_t* __restrict__ offsets, uint32_t rows,
                    int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
                    int32_t* __restrict__ inverse) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   __shared__ uint32_t bitmap[kExperts][2];
   __shared__ int32_t base[kExperts];
   const uint32_t chunk = blockIdx.x;
@@ -644,8 +639,7 @@ moe_scatter_kernel(const int32_t* __restrict__ keys, const uint32_t* __restrict_
 __global__ void __launch_bounds__(256)
 moe_keys_from_offsets_kernel(const int32_t* __restrict__ offsets, uint32_t first_expert, uint32_t expert_count,
                              uint32_t rows, int32_t* __restrict__ sorted_keys, int32_t* __restrict__ full_offsets) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (blockIdx.x == 0 && threadIdx.x <= kExperts) {
     // offsets over all 128 experts: empty outside [first, first+count)
@@ -667,9 +661,8 @@ moe_keys_from_offsets_kernel(const int32_t* __restrict__ offsets, uint32_t first
 
 __global__ void __launch_bounds__(256)
 moe_prepare_groups_kernel(MoeGroupPlan plan, GemmGroup* __restrict__ first_groups, GemmGroup* __restrict__ down_groups) {
-  griddep_launch();
   const MoeExpertInfo info = plan.experts[threadIdx.x / 2];   // of the expert table, written when it was created
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   prepare_groups(plan, info, plan.offsets[threadIdx.x / 2], plan.offsets[threadIdx.x / 2 + 1], first_groups, down_groups);
 }
 
@@ -691,10 +684,7 @@ moe_quantize_kernel(const uint4* __restrict__ input, const int32_t* __restrict__
                     const MoeExpertInfo* __restrict__ experts, uint32_t n, uint32_t scale_rows, int projection,
                     uint32_t gather_divisor, uint32_t* __restrict__ packed, uint8_t* __restrict__ scales,
                     uint4* __restrict__ activated) {
-  if (Gelu) griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
-  // The layer's first GEMM only now: it fills every SM, and its blocks would keep out other streams' kernels while they wait.
-  if (!Gelu) griddep_launch();
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   constexpr uint32_t kVectors = K / 8;          // even: the two threads of a block are neighbours in a warp
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   const uint32_t part = blockIdx.y;             // gate/up copy (0 unless the scales differ)
@@ -764,9 +754,7 @@ moe_quantize_tokens_kernel(const uint4* __restrict__ input, const int32_t* __res
                            const int32_t* __restrict__ inverse, const int32_t* __restrict__ offsets,
                            const MoeExpertInfo* __restrict__ experts, uint32_t tokens, uint32_t scale_rows, int parts,
                            uint2* __restrict__ packed, uint8_t* __restrict__ scales) {
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
-  // Only now: the GEMM that follows fills every SM, and its blocks would keep out other streams' kernels while they wait.
-  griddep_launch();
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   // Two warps per token, each with one half of the row (88 K16 blocks, three per lane): half the
   // registers of a whole row per warp, so twice as many warps are resident to cover the loads.
   constexpr uint32_t kBlocks = kHidden / 16;            // 176
@@ -856,8 +844,7 @@ moe_quantize_fp8_kernel(const uint4* __restrict__ input, const int32_t* __restri
                         uint32_t gather_divisor, const int32_t* __restrict__ sorted_keys,
                         const int32_t* __restrict__ offsets, const MoeExpertInfo* __restrict__ experts, uint32_t n,
                         uint32_t vectors, int first_projection, uint2* __restrict__ packed) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   const uint32_t part = blockIdx.y;
   if (index >= size_t(n) * vectors) return;
@@ -879,8 +866,7 @@ moe_quantize_fp8_kernel(const uint4* __restrict__ input, const int32_t* __restri
 __global__ void __launch_bounds__(256)
 moe_activate_kernel(const uint4* __restrict__ gate_up, const int32_t* __restrict__ offsets, uint32_t n,
                     uint4* __restrict__ activated) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   constexpr uint32_t kVectors = kInter / 8;
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   if (index >= size_t(n) * kVectors) return;
@@ -906,8 +892,7 @@ moe_activate_kernel(const uint4* __restrict__ gate_up, const int32_t* __restrict
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const uint4* __restrict__ down, const int32_t* __restrict__ inverse,
                    const float* __restrict__ weights, uint32_t rows, uint32_t width, uint4* __restrict__ output) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   const uint32_t vectors = width / 8;
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   if (index >= size_t(rows) * vectors) return;
@@ -949,8 +934,7 @@ moe_combine_kernel(const uint4* __restrict__ down, const int32_t* __restrict__ i
 __global__ void __launch_bounds__(kHidden / 8)
 moe_combine_token_kernel(const uint4* __restrict__ down, const int32_t* __restrict__ inverse,
                          const float* __restrict__ weights, uint32_t rows, uint4* __restrict__ output) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   constexpr uint32_t kVectors = kHidden / 8;
   __shared__ int32_t slot_row[kTopK];
   __shared__ float slot_weight[kTopK];
@@ -969,8 +953,7 @@ moe_combine_token_kernel(const uint4* __restrict__ down, const int32_t* __restri
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ input, const int32_t* __restrict__ index, uint32_t divisor,
                    uint32_t rows, uint32_t vectors, uint4* __restrict__ output) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   const size_t i = size_t(blockIdx.x) * 256 + threadIdx.x;
   if (i >= size_t(rows) * vectors) return;
   const uint32_t row = i / vectors, v = i % vectors;
@@ -1060,8 +1043,7 @@ ep_dispatch_kernel(const uint4* __restrict__ input, const int32_t* __restrict__ 
   // The eight records of a token are built in shared memory and leave as eight bulk copies of 1584 bytes
   // each: the copy engine keeps the NVLink writes in flight, the warps do not wait on remote stores.
   __shared__ __align__(16) uint8_t staged[kDispatchTokensPerBlock][kTopK][kRecordBytes];
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   // token-major like kernel 5b: two warps per token, each with one half of the row (88 K16 blocks, three
   // per lane), read once for the token's eight records
   constexpr uint32_t kBlocks = kHidden / 16;            // 176
@@ -1147,8 +1129,7 @@ __global__ void __launch_bounds__(kExperts)
 ep_tables_kernel(const int32_t* __restrict__ counts, const int32_t* __restrict__ physical, uint32_t rank,
                  uint32_t world, int32_t* __restrict__ dest_row0, int32_t* __restrict__ local_offsets,
                  int32_t* __restrict__ segment_start, int32_t* __restrict__ home_base) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   __shared__ int32_t total_at[kExperts];       // rows of the expert at a physical position, over all sources
   __shared__ int32_t sorted_base[8][kExperts]; // a source rank's own offsets: rows of experts with a lower id
   const uint32_t e = threadIdx.x, per_rank = kExperts / world;
@@ -1193,8 +1174,7 @@ ep_row_home_kernel(const int32_t* __restrict__ sorted_keys, const int32_t* __res
                    uint8_t* const* __restrict__ peer_returned, uint32_t first_expert, uint32_t per_rank,
                    uint32_t world, uint32_t n, uint32_t home_capacity_rows, uint32_t* __restrict__ error,
                    uint64_t* __restrict__ row_home) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   const uint32_t row = blockIdx.x * 256 + threadIdx.x;
   if (row >= n || row >= uint32_t(offsets[kExperts])) return;
   const uint32_t slot = uint32_t(sorted_keys[row]) - first_expert;
@@ -1214,8 +1194,7 @@ ep_row_home_kernel(const int32_t* __restrict__ sorted_keys, const int32_t* __res
 __global__ void __launch_bounds__(256)
 ep_retile_scales_kernel(const uint8_t* __restrict__ records, const int32_t* __restrict__ sorted_keys,
                         const int32_t* __restrict__ offsets, uint32_t n, uint8_t* __restrict__ scales) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   constexpr uint32_t kWords = kHidden / 64;        // 44 four-byte words of scales per row
   const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
   if (index >= size_t(n) * kWords) return;
@@ -1237,8 +1216,7 @@ __global__ void __launch_bounds__(256)
 ep_export_activations_kernel(const uint4* __restrict__ packed, const uint8_t* __restrict__ scales,
                              const int32_t* __restrict__ sorted_keys, const int32_t* __restrict__ offsets, uint32_t rows,
                              uint4* __restrict__ records) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   const uint32_t row = (blockIdx.x * 256 + threadIdx.x) / 32, lane = threadIdx.x % 32;
   if (row >= rows || row >= uint32_t(offsets[kExperts])) return;      // `rows` may be an upper bound
   constexpr uint32_t kPackedVectors = kInter / 2 / 16;                // 22
@@ -1264,8 +1242,7 @@ ep_import_activations_kernel(const int32_t* __restrict__ keys, const int32_t* __
                              const int32_t* __restrict__ dest_row0, const uint4* const* __restrict__ peer_records,
                              uint32_t assignments, uint32_t capacity_rows, uint32_t* __restrict__ error,
                              uint4* __restrict__ packed, uint8_t* __restrict__ scales) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   const uint32_t assignment = (blockIdx.x * 128 + threadIdx.x) / 32, lane = threadIdx.x % 32;
   if (assignment >= assignments) return;
   constexpr uint32_t kPackedVectors = kInter / 2 / 16, kScaleWords = kInter / 16 / 4;
@@ -1294,8 +1271,7 @@ ep_combine_kernel(const int32_t* __restrict__ keys, const int32_t* __restrict__ 
                   const int32_t* __restrict__ dest_rank, const int32_t* __restrict__ dest_row0,
                   const uint4* const* __restrict__ peer_down, uint32_t rows, uint32_t capacity_rows,
                   uint32_t* __restrict__ error, uint4* __restrict__ output) {
-  griddep_launch();
-  griddep_wait();     // results of earlier kernels in the stream are read from here on
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
   constexpr uint32_t kVectors = kHidden / 8;
   const size_t index = size_t(blockIdx.x) * 128 + threadIdx.x;
   if (index >= size_t(rows) * kVectors) return;

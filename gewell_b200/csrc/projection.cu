@@ -33,8 +33,7 @@ namespace {
 template <bool VECTOR>
 __global__ void __launch_bounds__(256)
 compact_rows_kernel(const bf16* __restrict__ input, bf16* __restrict__ output, uint32_t rows, uint32_t logical, uint32_t physical) {
-  griddep_launch();
-  griddep_wait();
+  griddep_enter();
   const uint32_t c = (blockIdx.x * 256 + threadIdx.x) * (VECTOR ? 8 : 1);
   if (c >= logical) return;
   for (size_t row = blockIdx.y; row < rows; row += gridDim.y) {
@@ -295,7 +294,7 @@ gw_status gw_projection_workspace_prepare(gw_projection_workspace* w, uint32_t r
 
 gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_projection* projection,
                                       const void* input_bf16, void* output_bf16) {
-  return gw::projection_workspace_run_on(w, projection, input_bf16, output_bf16, w ? w->stream : nullptr);
+  return gw::projection_workspace_run_on(w, projection, input_bf16, output_bf16, w ? w->stream : nullptr, false);
 }
 
 }  // extern "C"
@@ -303,7 +302,7 @@ gw_status gw_projection_workspace_run(gw_projection_workspace* w, const gw_proje
 namespace gw {
 
 gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_projection* projection, const void* input_bf16,
-                                      void* output_bf16, cudaStream_t stream) {
+                                      void* output_bf16, cudaStream_t stream, bool weights_settled) {
   clear_error();
   if (!w || !projection || w->rows == 0 || !input_bf16 || !output_bf16)
     return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
@@ -314,7 +313,8 @@ gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_proje
   // NVFP4 at small row counts: into the caller's rows at once, and with BF16 activations from the packed weights
   if (p.storage == GW_STORAGE_NVFP4_W4A4 && (padded || !w->fp4)) {
     bool done = false;
-    const gw_status status = w->streaming.run(p, nullptr, input_bf16, output_bf16, w->fp4, w->scratch.data, stream, &done);
+    const gw_status status = w->streaming.run(p, nullptr, input_bf16, output_bf16, w->fp4, w->scratch.data, weights_settled, stream,
+                                             &done);
     if (status != GW_OK || done) return status;
   }
   void* destination = padded ? w->padded.data : output_bf16;
@@ -326,13 +326,12 @@ gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_proje
   gw_status status = GW_OK;
   if (kind == kPlanFp8) {
     if (!plans.fp8) return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
-    status = gw_fp8_plan_run(plans.fp8, input_bf16, p.fp8_data, p.fp8_input_scale, p.fp8_weight_scale, nullptr,
-                             destination, w->scratch.data, w->scratch.bytes, stream, GW_TRANSFORM_IDENTITY);
+    status = run_fp8_plan(plans.fp8, input_bf16, p.fp8_data, p.fp8_input_scale, p.fp8_weight_scale, nullptr, destination,
+                          w->scratch.data, w->scratch.bytes, stream, GW_TRANSFORM_IDENTITY, weights_settled);
   } else if (kind == kPlanNvfp4) {
     if (!plans.nvfp4) return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
-    status = gw_nvfp4_plan_run(plans.nvfp4, input_bf16, p.nvfp4_data, p.nvfp4_scales, p.nvfp4_input_scale,
-                               p.nvfp4_weight_scale, destination, w->scratch.data, w->scratch.bytes, stream,
-                               GW_TRANSFORM_IDENTITY);
+    status = run_nvfp4_plan(plans.nvfp4, input_bf16, p.nvfp4_data, p.nvfp4_scales, p.nvfp4_input_scale, p.nvfp4_weight_scale,
+                            destination, w->scratch.data, w->scratch.bytes, stream, GW_TRANSFORM_IDENTITY, weights_settled);
   } else {
     if (!plans.bf16) return fail(GW_INVALID_ARGUMENT, "prepare 26B projections before run");
     const void* weights = p.bf16;
@@ -343,10 +342,11 @@ gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_proje
                                    w->dequantized.data, stream);
       if (status != GW_OK) return status;
       weights = w->dequantized.data;
+      weights_settled = false;
     }
     const bool split = w->scratch.data && w->scratch.bytes >= gw_bf16_plan_scratch_bytes(plans.bf16);
-    status = gw_bf16_plan_run(plans.bf16, input_bf16, weights, destination, split ? w->scratch.data : nullptr,
-                              split ? w->scratch.bytes : 0, stream);
+    status = run_bf16_plan(plans.bf16, input_bf16, weights, destination, split ? w->scratch.data : nullptr,
+                           split ? w->scratch.bytes : 0, stream, weights_settled);
   }
   if (status != GW_OK) return status;
   if (padded) {
@@ -361,10 +361,10 @@ gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_proje
 }
 
 gw_status projection_workspace_run_geglu(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up, const void* input,
-                                         void* product, cudaStream_t stream, bool* done) {
+                                         void* product, cudaStream_t stream, bool weights_settled, bool* done) {
   *done = false;
   if (w->rows == 0) return GW_OK;
-  return w->streaming.run(gate, &up, input, product, w->fp4, w->scratch.data, stream, done);
+  return w->streaming.run(gate, &up, input, product, w->fp4, w->scratch.data, weights_settled, stream, done);
 }
 
 }  // namespace gw

@@ -144,6 +144,16 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, 
       ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(gmem_src)), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
       : "memory");
 }
+// The same boxes into L2 alone.  Safe before griddep_wait() whoever wrote or still writes the bytes: L2 is where every SM's
+// stores meet, so a copy issued after the wait reads what was written, prefetched or not.
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int32_t x, int32_t y, uint64_t policy) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.L2::cache_hint [%0, {%1, %2}], %3;"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int32_t x, int32_t y, int32_t z, uint64_t policy) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.L2::cache_hint [%0, {%1, %2, %3}], %4;"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 // Untiled bulk copy global -> shared; both addresses 16-byte aligned, size a
 // multiple of 16 bytes.

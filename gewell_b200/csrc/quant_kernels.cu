@@ -129,8 +129,7 @@ nvfp4_quantize_kernel(const uint4* __restrict__ input, uint32_t rows, uint32_t w
                       uint32_t* __restrict__ packed, uint8_t* __restrict__ scales, Divisor padded_items_per_row, uint32_t slab_rows) {
   constexpr int kWords = Gelu ? 4 : 8;          // packed BF16 pairs per thread
   constexpr int kShare = 8 / kWords;            // threads per K16 block
-  griddep_launch();   // the GEMM that follows may set itself up while this kernel runs
-  griddep_wait();
+  griddep_enter_first();   // the GEMM that follows may set itself up while this kernel waits
   // items of a row: a multiple of 4 * kShare, so whole K64 groups are inside or outside and sit in one warp
   const uint32_t index = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t local = padded_items_per_row.quotient(index), item = index - local * padded_items_per_row.value;
@@ -209,8 +208,7 @@ __global__ void __launch_bounds__(kThreads)
 fp8_quantize_kernel(const bf16* __restrict__ input, uint32_t rows, uint32_t width, Divisor items_per_row, uint32_t slab_rows,
                     float inverse_scale, uint8_t* __restrict__ packed) {
   constexpr uint32_t kValues = Gelu ? 8 : 16;
-  griddep_launch();   // the GEMM that follows may set itself up while this kernel runs
-  griddep_wait();
+  griddep_enter_first();   // the GEMM that follows may set itself up while this kernel waits
   const uint32_t row0 = blockIdx.y * slab_rows;
   const uint32_t index = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t local = items_per_row.quotient(index), col = (index - local * items_per_row.value) * kValues;
@@ -364,8 +362,7 @@ __device__ __forceinline__ uint4 geglu8(const uint4& g, const uint4& u) {
 // VECTOR: 16-byte aligned buffers, eight values a thread (the last thread takes what is left)
 template <bool VECTOR>
 __global__ void geglu_kernel(const bf16* gate, const bf16* up, bf16* out, size_t n) {
-  griddep_launch();
-  griddep_wait();
+  griddep_enter();
   const size_t i = (size_t(blockIdx.x) * kThreads + threadIdx.x) * (VECTOR ? 8 : 1);
   if (VECTOR && i + 8 <= n) {
     *reinterpret_cast<uint4*>(out + i) = geglu8(*reinterpret_cast<const uint4*>(gate + i), *reinterpret_cast<const uint4*>(up + i));
@@ -379,8 +376,7 @@ __global__ void geglu_kernel(const bf16* gate, const bf16* up, bf16* out, size_t
 // [rows, gate | up] -> [rows, width]: eight channels per thread, 16-byte loads and stores
 __global__ void geglu_interleaved_kernel(const uint4* __restrict__ gate_up, uint4* __restrict__ out, Divisor row_vectors,
                                          uint32_t slab_rows, uint32_t rows) {
-  griddep_launch();
-  griddep_wait();
+  griddep_enter();
   const uint32_t row0 = blockIdx.y * slab_rows, index = blockIdx.x * kThreads + threadIdx.x;
   const uint32_t local = row_vectors.quotient(index), v = index - local * row_vectors.value;
   if (local >= min(slab_rows, rows - row0)) return;

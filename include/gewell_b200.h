@@ -12,6 +12,8 @@
  * Unless stated otherwise a call neither allocates device memory nor
  * synchronises, and is ordered on `stream` only, so it may be captured in a
  * CUDA graph (plan / workspace construction must happen outside capture).
+ * Stream order covers every buffer a call is given, weights, scales and norm
+ * vectors included: they may be written by earlier work of the same stream.
  */
 #ifndef GEWELL_B200_H_
 #define GEWELL_B200_H_
