@@ -166,37 +166,44 @@ StreamBook::~StreamBook() {
   if (counters != nullptr) cudaFree(counters);
 }
 
-gw_status StreamBook::prepare(uint32_t new_rows, const std::vector<std::pair<uint32_t, uint32_t>>& shapes, size_t workspace_bytes) {
-  rows = new_rows;
-  entries.clear();
+StreamBook::Staged::~Staged() {
+  if (counters != nullptr) cudaFree(counters);
+}
+
+gw_status StreamBook::stage(uint32_t new_rows, const std::vector<std::pair<uint32_t, uint32_t>>& shapes, size_t workspace_bytes,
+                            Staged* staged) const {
+  staged->rows = new_rows;
   size_t most = 0;
   const bool allowed = DenseTuning::from_environment().streams();
   for (const auto& [k, n] : shapes)
     for (StreamKind kind : {StreamKind::w4a4, StreamKind::w4a16, StreamKind::w8a8, StreamKind::w16a16})
       for (bool pair : {false, true}) {
         // W4A16 beyond one launch's rows: several launches, each of them reads the packed weights once
-        const uint32_t tile = kind == StreamKind::w4a16 && rows <= kW4a16Rows ? std::min(rows, kStreamMaxRows) : rows;
+        const uint32_t tile = kind == StreamKind::w4a16 && new_rows <= kW4a16Rows ? std::min(new_rows, kStreamMaxRows) : new_rows;
         Entry s;
         s.plan = plan_stream(kind, tile, k, n, pair, sm_count());
         s.plan.usable = allowed && (pair ? stream_pair_pays(kind, s.plan, tile, k, n) : stream_pays(kind, s.plan, tile, k, n));
         if (!s.plan.usable || s.plan.workspace_bytes > workspace_bytes) continue;
         most = std::max(most, s.plan.counter_count);
-        entries[Key{int(kind), k, n, pair}] = s;
+        staged->entries[Key{int(kind), k, n, pair}] = s;
       }
   if (most * sizeof(int32_t) > counter_bytes) {
-    int32_t* larger = nullptr;
-    cudaError_t status = cudaMalloc(&larger, most * sizeof(int32_t));
-    if (status == cudaSuccess) status = cudaMemset(larger, 0, most * sizeof(int32_t));
-    if (status != cudaSuccess) {
-      if (larger != nullptr) cudaFree(larger);
-      entries.clear();
+    cudaError_t status = cudaMalloc(&staged->counters, most * sizeof(int32_t));
+    if (status == cudaSuccess) status = cudaMemset(staged->counters, 0, most * sizeof(int32_t));
+    if (status != cudaSuccess)
       return fail(GW_CUDA_ERROR, std::string("counters of the weight-streaming kernel: ") + cudaGetErrorString(status));
-    }
-    if (counters != nullptr) cudaFree(counters);
-    counters = larger;
-    counter_bytes = most * sizeof(int32_t);
+    staged->counter_bytes = most * sizeof(int32_t);
   }
   return GW_OK;
+}
+
+void StreamBook::publish(Staged* staged) {
+  entries.swap(staged->entries);
+  rows = staged->rows;
+  if (staged->counters != nullptr) {          // the former ones go with `staged`
+    std::swap(counters, staged->counters);
+    std::swap(counter_bytes, staged->counter_bytes);
+  }
 }
 
 gw_status StreamBook::run(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4,

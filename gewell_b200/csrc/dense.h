@@ -96,8 +96,21 @@ struct StreamBook {
   StreamBook(const StreamBook&) = delete;
   StreamBook& operator=(const StreamBook&) = delete;
   ~StreamBook();
-  // shapes: (K, physical N); `workspace_bytes`: of the workspace that run() will be given
-  gw_status prepare(uint32_t rows, const std::vector<std::pair<uint32_t, uint32_t>>& shapes, size_t workspace_bytes);
+  // What another row count needs, built beside what run() uses; publish() puts it in its place and cannot fail, so that an
+  // object publishes all of its parts or none.  shapes: (K, physical N); `workspace_bytes`: of the workspace that run() will
+  // be given.
+  struct Staged {
+    std::map<Key, Entry> entries;
+    int32_t* counters = nullptr;       // larger ones, where the present ones do not suffice
+    size_t counter_bytes = 0;
+    uint32_t rows = 0;
+    Staged() = default;
+    Staged(const Staged&) = delete;
+    Staged& operator=(const Staged&) = delete;
+    ~Staged();
+  };
+  gw_status stage(uint32_t rows, const std::vector<std::pair<uint32_t, uint32_t>>& shapes, size_t workspace_bytes, Staged* staged) const;
+  void publish(Staged* staged);
   // The projection `first` -- or, with `second`, GeGLU of both -- into [rows, first.output]; *done = false when the shape,
   // the storage or the pointers keep it off the kernel.
   gw_status run(const gw_projection& first, const gw_projection* second, const void* input, void* output, bool fp4, void* workspace,

@@ -118,8 +118,9 @@ struct PlanBook {
     if (new_rows == 0 || new_rows > max_rows)
       return fail(GW_INVALID_ARGUMENT, "prepare requires 0 < rows <= the object's max_rows");
     if (rows == new_rows) return GW_OK;
+    StreamBook::Staged next_streaming;
     std::map<Key, PlanSet> next;
-    gw_status status = GW_OK;
+    gw_status status = streaming.stage(new_rows, shapes, scratch.bytes, &next_streaming);
     for (int kind : {kNvfp4, kFp8, kFp8Channel, kBf16})
       for (const auto& [k, n] : shapes) {
         if (status != GW_OK) break;
@@ -135,8 +136,9 @@ struct PlanBook {
     }
     for (auto& entry : plans) entry.second.reset();
     plans = std::move(next);
+    streaming.publish(&next_streaming);
     rows = new_rows;
-    return streaming.prepare(rows, shapes, scratch.bytes);
+    return GW_OK;
   }
 
   // `first` or GeGLU of `first` and `second` on the weight-streaming kernel, if that is the faster one here

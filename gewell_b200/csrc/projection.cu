@@ -252,13 +252,14 @@ gw_status gw_projection_workspace_prepare(gw_projection_workspace* w, uint32_t r
     return fail(GW_INVALID_ARGUMENT, "invalid 26B projection rows/phase");
   const bool fp4 = gw_nvfp4_fp4_activations(w->policy, phase) != 0;
   if (w->rows == rows && w->fp4 == fp4) return GW_OK;
-  if (w->streaming.rows != rows) {
+  // Keep a plan when only the phase changes; rebuild on a new row count, outside the layer loop.
+  // Everything is built first and published only when all of it exists.
+  StreamBook::Staged streaming;
+  if (w->rows != rows) {
     std::vector<std::pair<uint32_t, uint32_t>> shapes;
     for (const auto& entry : w->plans) shapes.emplace_back(std::get<1>(entry.first), std::get<2>(entry.first));
-    if (const gw_status status = w->streaming.prepare(rows, shapes, w->scratch.bytes); status != GW_OK) return status;
+    if (const gw_status status = w->streaming.stage(rows, shapes, w->scratch.bytes, &streaming); status != GW_OK) return status;
   }
-  // Keep a plan when only the phase changes; rebuild on a new row count, outside the layer loop.
-  // Every requested plan is built first and published only when all of them exist.
   std::map<Shape, Plans> replacements;
   gw_status status = GW_OK;
   for (const auto& entry : w->plans) {
@@ -287,6 +288,7 @@ gw_status gw_projection_workspace_prepare(gw_projection_workspace* w, uint32_t r
       current.nvfp4 = nullptr;
     }
   }
+  if (w->rows != rows) w->streaming.publish(&streaming);
   w->rows = rows;
   w->fp4 = fp4;
   return GW_OK;

@@ -1,0 +1,55 @@
+// A CUDA runtime for host tests, put in front of the real one with LD_PRELOAD: allocations are addresses that nothing
+// touches, launches are counted, and the n-th allocation from now can be made to fail.  It needs no GPU and no CUDA headers.
+#include <atomic>
+#include <cstddef>
+#include <cstdint>
+
+namespace {
+std::atomic<long> g_fail_in{0};             // 1: the next allocation fails; 0: none does
+std::atomic<long> g_launches{0};
+std::atomic<long> g_unfinished{0};          // fills and copies queued on the default stream that nothing has waited for
+uintptr_t g_next = uintptr_t(1) << 44;
+int encode(...) { return 0; }
+}  // namespace
+
+extern "C" {
+
+void fake_fail_allocation(long in) { g_fail_in = in; }
+long fake_allocations_left() { return g_fail_in; }
+long fake_launches() { return g_launches; }
+long fake_unfinished() { return g_unfinished; }
+
+int cudaMalloc(void** p, size_t bytes) {
+  if (g_fail_in > 0 && --g_fail_in == 0) return 2;         // cudaErrorMemoryAllocation
+  *p = reinterpret_cast<void*>(g_next);
+  g_next += (bytes + 511) / 512 * 512 + 512;
+  return 0;
+}
+int cudaFree(void*) { return 0; }
+int cudaMemset(void*, int, size_t) { ++g_unfinished; return 0; }
+int cudaMemsetAsync(void*, int, size_t, void* stream) { if (stream == nullptr) ++g_unfinished; return 0; }
+int cudaMemcpy(void*, const void*, size_t, int) { ++g_unfinished; return 0; }
+int cudaMemcpyAsync(void*, const void*, size_t, int, void* stream) { if (stream == nullptr) ++g_unfinished; return 0; }
+int cudaDeviceSynchronize() { g_unfinished = 0; return 0; }
+int cudaStreamSynchronize(void* stream) { if (stream == nullptr) g_unfinished = 0; return 0; }
+
+int cudaGetDevice(int* device) { *device = 0; return 0; }
+int cudaDeviceGetAttribute(int* value, int, int) { *value = 148; return 0; }      // asked for the number of SMs only
+int cudaGetLastError() { return 0; }
+int cudaFuncSetAttribute(const void*, int, int) { return 0; }
+int cudaLaunchKernelExC(const void*, const void*, void**) { ++g_launches; return 0; }
+struct Dim3 { unsigned x, y, z; };
+int cudaLaunchKernel(const void*, Dim3, Dim3, void**, size_t, void*) { ++g_launches; return 0; }
+int cudaGetDriverEntryPoint(const char*, void** entry, unsigned long long, int* result) {
+  *entry = reinterpret_cast<void*>(&encode);
+  if (result) *result = 0;
+  return 0;
+}
+int cudaStreamCreateWithFlags(void** stream, unsigned) { *stream = reinterpret_cast<void*>(uintptr_t(0x1000)); return 0; }
+int cudaStreamDestroy(void*) { return 0; }
+int cudaStreamWaitEvent(void*, void*, unsigned) { return 0; }
+int cudaEventCreateWithFlags(void** event, unsigned) { *event = reinterpret_cast<void*>(uintptr_t(0x2000)); return 0; }
+int cudaEventDestroy(void*) { return 0; }
+int cudaEventRecord(void*, void*) { return 0; }
+
+}  // extern "C"
