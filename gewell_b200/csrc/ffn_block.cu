@@ -571,11 +571,16 @@ size_t gw_ffn_block_bytes(const gw_ffn_block* b) {
 gw_status gw_ffn_block_prepare(gw_ffn_block* b, uint32_t rows, int phase) {
   clear_error();
   if (!b || rows == 0 || rows > b->capacity) return fail(GW_INVALID_ARGUMENT, "feed-forward block: invalid rows");
-  const gw_status status = gw_projection_workspace_prepare(b->projections, rows, phase);
-  if (status != GW_OK) return status;
-  if (b->rows != rows) {
-    gw_bf16_plan* plan = nullptr;
+  // The router's plan first, beside the present one: what follows either prepares the projections too or leaves all as it was.
+  gw_bf16_plan* plan = nullptr;
+  if (b->rows != rows)
     if (const gw_status created = gw_bf16_plan_create(rows, kHidden, kExperts, &plan); created != GW_OK) return created;
+  const gw_status status = gw_projection_workspace_prepare(b->projections, rows, phase);
+  if (status != GW_OK) {
+    if (plan) gw_bf16_plan_destroy(plan);
+    return status;
+  }
+  if (plan) {
     if (b->router_plan) gw_bf16_plan_destroy(b->router_plan);
     b->router_plan = plan;
   }

@@ -79,6 +79,30 @@ for small, large in ((200, 5), (5, 40), (40, 5), (200, 40)):
     each_allocation_fails(prepare, run, small, large)
 '''
 
+BLOCK = CHILD + r'''
+NV = _lib.STORAGE_NVFP4_W4A4
+experts = (_lib.ExpertWeights * 128)()
+for e in experts:
+    e.gate = e.up = projection(NV, 2816, 704, 768)
+    e.down = projection(NV, 704, 2816)
+table = ctypes.c_void_p()
+check(lib.gw_moe_expert_table_create(experts, 128, ctypes.byref(table)))
+w = _lib.FfnBlockWeights()
+for name in ("pre_feedforward_norm", "router_scale", "pre_feedforward_norm_2", "post_feedforward_norm_1", "post_feedforward_norm_2",
+             "post_feedforward_norm", "layer_scalar", "router_proj", "router_per_expert_scale"):
+    setattr(w, name, A)
+w.gate = w.up = projection(NV, 2816, 2112, 2176)
+w.down = projection(NV, 2112, 2816)
+w.experts, w.has_nvfp4 = table, 1
+block = ctypes.c_void_p()
+check(lib.gw_ffn_block_create(ctypes.byref(w), 1, 256, _lib.POLICY_ALWAYS, 0, None, ctypes.byref(block)))
+prepare = lambda rows: lib.gw_ffn_block_prepare(block, rows, _lib.PHASE_DECODE)
+run = lambda: lib.gw_ffn_block_run(block, ctypes.byref(w), A)
+for small, large in ((8, 40), (40, 8)):
+    each_allocation_fails(prepare, run, small, large)
+'''
+
+
 @pytest.fixture(scope="module")
 def fake_runtime(tmp_path_factory):
     if shutil.which("g++") is None:
@@ -95,6 +119,6 @@ def run_child(fake_runtime, script):
     assert done.returncode == 0, done.stdout + done.stderr
 
 
-@pytest.mark.parametrize("script", [PROJECTIONS, CHAIN], ids=["projections", "mlp chain"])
+@pytest.mark.parametrize("script", [PROJECTIONS, CHAIN, BLOCK], ids=["projections", "mlp chain", "feed-forward block"])
 def test_failed_prepare_leaves_the_row_count(fake_runtime, script):
     run_child(fake_runtime, script)
