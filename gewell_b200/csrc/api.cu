@@ -41,6 +41,34 @@ int current_device_slot() {
   return device % kMaxDeviceSlots;
 }
 
+namespace {
+// One stream per GPU for set-up, ordered with no other.
+cudaError_t setup_stream(cudaStream_t* stream) {
+  static cudaStream_t streams[kMaxDeviceSlots] = {};
+  static std::mutex mutex;
+  const int slot = current_device_slot();
+  std::lock_guard<std::mutex> lock(mutex);
+  cudaError_t status = cudaSuccess;
+  if (streams[slot] == nullptr) status = cudaStreamCreateWithFlags(&streams[slot], cudaStreamNonBlocking);
+  *stream = streams[slot];
+  return status;
+}
+}  // namespace
+
+cudaError_t zero_now(void* device, size_t bytes) {
+  cudaStream_t s = nullptr;
+  cudaError_t status = setup_stream(&s);
+  if (status == cudaSuccess) status = cudaMemsetAsync(device, 0, bytes, s);
+  return status == cudaSuccess ? cudaStreamSynchronize(s) : status;
+}
+
+cudaError_t upload_now(void* device, const void* host, size_t bytes) {
+  cudaStream_t s = nullptr;
+  cudaError_t status = setup_stream(&s);
+  if (status == cudaSuccess) status = cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, s);
+  return status == cudaSuccess ? cudaStreamSynchronize(s) : status;
+}
+
 uint32_t* device_error_word() {
   static uint32_t* words[kMaxDeviceSlots] = {};
   static std::mutex mutex;
@@ -48,7 +76,7 @@ uint32_t* device_error_word() {
   std::lock_guard<std::mutex> lock(mutex);
   if (words[slot] == nullptr) {
     uint32_t* word = nullptr;
-    if (cudaMalloc(&word, sizeof(uint32_t)) == cudaSuccess && cudaMemset(word, 0, sizeof(uint32_t)) == cudaSuccess)
+    if (cudaMalloc(&word, sizeof(uint32_t)) == cudaSuccess && zero_now(word, sizeof(uint32_t)) == cudaSuccess)
       words[slot] = word;
     else
       (void)cudaGetLastError();
@@ -104,7 +132,7 @@ uint32_t gw_debug_kernel_error(void) {
   if (word == nullptr) return 0xFFFFFFFFu;
   if (cudaDeviceSynchronize() != cudaSuccess) return 0xFFFFFFFEu;
   cudaMemcpy(&value, word, sizeof(value), cudaMemcpyDeviceToHost);
-  if (value != 0) cudaMemset(word, 0, sizeof(value));
+  if (value != 0) zero_now(word, sizeof(value));
   // the allocation-free linear reports into a word of its own (it may not use the allocated one)
   const uint32_t built_in = take_static_scratch_error();
   return value != 0 ? value : built_in;

@@ -39,6 +39,10 @@ constexpr int kMaxDeviceSlots = 64;
 int current_device_slot();
 // Error word written by bounded waits (0 = no error): lazily allocated, one per GPU.
 uint32_t* device_error_word();
+// Set-up of device memory, complete when these return.  cudaMemset and a cudaMemcpy to the device may return earlier, and the
+// streams that use the memory need not be ordered behind the default stream they run on.
+cudaError_t zero_now(void* device, size_t bytes);
+cudaError_t upload_now(void* device, const void* host, size_t bytes);
 int sm_count();
 // Counts the kernels this library launches (read by gw_debug_launch_count); every launch site calls it.
 void note_launch(unsigned kernels = 1);

@@ -106,7 +106,7 @@ cudaError_t DenseDescriptors::allocate_split_counters(GemmKind kind, uint32_t ro
     if (stream.usable) bytes = std::max(bytes, align_up(stream.counter_count * sizeof(int32_t), 256));
   }
   cudaError_t status = cudaMalloc(&split_counters, bytes);
-  if (status == cudaSuccess) status = cudaMemset(split_counters, 0, bytes);
+  if (status == cudaSuccess) status = zero_now(split_counters, bytes);
   return status;
 }
 
@@ -189,7 +189,7 @@ gw_status StreamBook::stage(uint32_t new_rows, const std::vector<std::pair<uint3
       }
   if (most * sizeof(int32_t) > counter_bytes) {
     cudaError_t status = cudaMalloc(&staged->counters, most * sizeof(int32_t));
-    if (status == cudaSuccess) status = cudaMemset(staged->counters, 0, most * sizeof(int32_t));
+    if (status == cudaSuccess) status = zero_now(staged->counters, most * sizeof(int32_t));
     if (status != cudaSuccess)
       return fail(GW_CUDA_ERROR, std::string("counters of the weight-streaming kernel: ") + cudaGetErrorString(status));
     staged->counter_bytes = most * sizeof(int32_t);

@@ -207,9 +207,9 @@ gw_status gw_moe_expert_table_create(const gw_expert_weights* experts, uint32_t 
   cudaError_t status = t->maps.allocate(maps.size() * sizeof(CUtensorMap));
   if (status == cudaSuccess) status = t->info.allocate(info.size() * sizeof(MoeExpertInfo));
   if (status == cudaSuccess)
-    status = cudaMemcpy(t->maps.data, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
+    status = upload_now(t->maps.data, maps.data(), maps.size() * sizeof(CUtensorMap));
   if (status == cudaSuccess)
-    status = cudaMemcpy(t->info.data, info.data(), info.size() * sizeof(MoeExpertInfo), cudaMemcpyHostToDevice);
+    status = upload_now(t->info.data, info.data(), info.size() * sizeof(MoeExpertInfo));
   if (status != cudaSuccess) {
     delete t;
     return fail(GW_CUDA_ERROR, std::string("expert table upload: ") + cudaGetErrorString(status));
@@ -290,7 +290,7 @@ gw_status gw_moe_create_ex(uint32_t max_rows, uint32_t flags, gw_moe_workspace**
   if (status == cudaSuccess) status = w->down.allocate(n * kHidden * sizeof(bf16));
   if (status == cudaSuccess) status = w->row_home.allocate(n * sizeof(uint64_t));
   if (status == cudaSuccess) status = w->route_barrier.allocate(2 * sizeof(uint32_t));
-  if (status == cudaSuccess) status = cudaMemset(w->route_barrier.data, 0, 2 * sizeof(uint32_t));
+  if (status == cudaSuccess) status = zero_now(w->route_barrier.data, 2 * sizeof(uint32_t));
   if (status == cudaSuccess) status = w->kind_groups.allocate(2 * (2 * kExperts + 1 + kExperts + 1) * sizeof(GemmGroup));
   if (status == cudaSuccess && (flags & GW_MOE_FP8_EXPERTS)) {
     status = w->fp8_in.allocate(2 * n * kHidden);
@@ -298,8 +298,8 @@ gw_status gw_moe_create_ex(uint32_t max_rows, uint32_t flags, gw_moe_workspace**
   }
   // Scale regions contain rows no kernel writes (tile padding); start from zero so
   // that they never hold NaN patterns.
-  if (status == cudaSuccess) status = cudaMemset(w->scales_in.data, 0, w->scales_in.bytes);
-  if (status == cudaSuccess) status = cudaMemset(w->scales_act.data, 0, w->scales_act.bytes);
+  if (status == cudaSuccess) status = zero_now(w->scales_in.data, w->scales_in.bytes);
+  if (status == cudaSuccess) status = zero_now(w->scales_act.data, w->scales_act.bytes);
   if (status != cudaSuccess) {
     delete w;
     return fail(GW_CUDA_ERROR, std::string("MoE workspace allocation: ") + cudaGetErrorString(status));

@@ -88,7 +88,7 @@ uint32_t gw::take_static_scratch_error() {
   }
   uint32_t value = 0;
   if (cudaMemcpy(&value, word, sizeof(value), cudaMemcpyDeviceToHost) != cudaSuccess) return 0xFFFFFFFDu;
-  if (value != 0) cudaMemset(word, 0, sizeof(value));
+  if (value != 0) gw::zero_now(word, sizeof(value));
   return value;
 }
 

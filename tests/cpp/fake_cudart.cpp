@@ -3,11 +3,12 @@
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <map>
 
 namespace {
 std::atomic<long> g_fail_in{0};             // 1: the next allocation fails; 0: none does
 std::atomic<long> g_launches{0};
-std::atomic<long> g_unfinished{0};          // fills and copies queued on the default stream that nothing has waited for
+std::map<void*, long> g_unfinished;         // fills and copies to the device that nothing has waited for, by stream
 uintptr_t g_next = uintptr_t(1) << 44;
 int encode(...) { return 0; }
 }  // namespace
@@ -17,7 +18,11 @@ extern "C" {
 void fake_fail_allocation(long in) { g_fail_in = in; }
 long fake_allocations_left() { return g_fail_in; }
 long fake_launches() { return g_launches; }
-long fake_unfinished() { return g_unfinished; }
+long fake_unfinished() {
+  long sum = 0;
+  for (const auto& stream : g_unfinished) sum += stream.second;
+  return sum;
+}
 
 int cudaMalloc(void** p, size_t bytes) {
   if (g_fail_in > 0 && --g_fail_in == 0) return 2;         // cudaErrorMemoryAllocation
@@ -26,12 +31,13 @@ int cudaMalloc(void** p, size_t bytes) {
   return 0;
 }
 int cudaFree(void*) { return 0; }
-int cudaMemset(void*, int, size_t) { ++g_unfinished; return 0; }
-int cudaMemsetAsync(void*, int, size_t, void* stream) { if (stream == nullptr) ++g_unfinished; return 0; }
-int cudaMemcpy(void*, const void*, size_t, int) { ++g_unfinished; return 0; }
-int cudaMemcpyAsync(void*, const void*, size_t, int, void* stream) { if (stream == nullptr) ++g_unfinished; return 0; }
-int cudaDeviceSynchronize() { g_unfinished = 0; return 0; }
-int cudaStreamSynchronize(void* stream) { if (stream == nullptr) g_unfinished = 0; return 0; }
+// cudaMemset and a cudaMemcpy to the device return before the device has done them
+int cudaMemset(void*, int, size_t) { ++g_unfinished[nullptr]; return 0; }
+int cudaMemsetAsync(void*, int, size_t, void* stream) { ++g_unfinished[stream]; return 0; }
+int cudaMemcpy(void*, const void*, size_t, int kind) { if (kind == 1) ++g_unfinished[nullptr]; return 0; }
+int cudaMemcpyAsync(void*, const void*, size_t, int, void* stream) { ++g_unfinished[stream]; return 0; }
+int cudaDeviceSynchronize() { g_unfinished.clear(); return 0; }
+int cudaStreamSynchronize(void* stream) { g_unfinished.erase(stream); return 0; }
 
 int cudaGetDevice(int* device) { *device = 0; return 0; }
 int cudaDeviceGetAttribute(int* value, int, int) { *value = 148; return 0; }      // asked for the number of SMs only

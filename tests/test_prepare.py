@@ -1,6 +1,7 @@
 """A prepare() that fails leaves its object as it was: the next run() works on the row count of the last prepare() that
 succeeded, in every part of it.  Every allocation of a prepare() fails in turn, on a CUDA runtime that only counts
-(tests/cpp/fake_cudart.cpp); the number of launches of a run tells the row count each part works on.  No GPU."""
+(tests/cpp/fake_cudart.cpp); the number of launches of a run tells the row count each part works on.  A prepare() that
+succeeds has waited for what it filled: streams need not be ordered behind the default one.  No GPU."""
 import os
 import shutil
 import subprocess
@@ -42,6 +43,7 @@ def launches(run):
 def each_allocation_fails(prepare, run, small, large):
     """From `small` rows, prepare(large) fails at its 1st, 2nd, ... allocation until it has no more."""
     check(prepare(small))
+    assert fake.fake_unfinished() == 0, "set-up that a run on another stream may overtake"
     at_small = launches(run)
     failures = 0
     while True:
@@ -55,6 +57,7 @@ def each_allocation_fails(prepare, run, small, large):
         failures += 1
         assert launches(run) == at_small, f"allocation {failures} of prepare({large}) from {small} rows"
     check(status)
+    assert fake.fake_unfinished() == 0
     assert launches(run) != at_small and failures >= 1
 '''
 
