@@ -202,6 +202,62 @@ def test_ffn_block_stage_by_stage(gw, experts_shared, rows, storage, policy, pha
           f"MoE {m_moe['rel_fro']:.2e}")
 
 
+def block_layer(gw, table, storage, seed):
+    device_mlp, _ = shared_mlp_weights(gw, storage)
+    layer = {name: norm_weight(seed + i).cuda() for i, name in enumerate(
+        ("pre_feedforward_norm", "router_scale", "pre_feedforward_norm_2", "post_feedforward_norm_1", "post_feedforward_norm_2",
+         "post_feedforward_norm"))}
+    layer.update(layer_scalar=torch.tensor([0.75 + seed / 512], dtype=torch.bfloat16).cuda(),
+                 router_proj=bf16_normal((E, H), seed + 7, 0.5).cuda(), router_per_expert_scale=norm_weight(seed + 8, E).cuda(),
+                 gate=device_mlp[0], up=device_mlp[1], down=device_mlp[2], experts=table)
+    return layer
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("rows,storage,phase", [(8, "nvfp4", "decode"), (24, "bf16", "decode"), (300, "nvfp4", "prefill")])
+def test_ffn_block_back_to_back(gw, experts_shared, rows, storage, phase, graph):
+    """Two layers in a row, pass after pass on a stream of the caller's without a wait between them, against the same passes
+    with a wait after every layer; eagerly and as a replayed graph.  The block's second stream, its fork and join and the
+    early start of the next launch have to leave the bits as they are."""
+    from gewell_b200 import _lib
+    table, _ = experts_shared
+    layers = [block_layer(gw, table, storage, 80), block_layer(gw, table, storage, 100)]
+    inputs = [bf16_normal((rows, H), 200 + i, 1.0 + i % 3).cuda() for i in range(6)]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        block = gw.FfnBlock(layers, rows, _lib.POLICY_ALWAYS)
+        block.prepare(rows, getattr(_lib, "PHASE_" + phase.upper()))
+        expected = []
+        for x in inputs:
+            hidden = x.clone()
+            for layer in (0, 1):
+                block.run(layer, hidden)
+                torch.cuda.synchronize()
+            expected.append(hidden)
+        hidden = torch.empty_like(inputs[0])
+
+        def both_layers():
+            block.run(0, hidden)
+            block.run(1, hidden)
+        if graph:
+            recorded = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(recorded, stream=stream, capture_error_mode="thread_local"):
+                both_layers()
+            both_layers = recorded.replay
+        results = []
+        for _ in range(3):
+            for x in inputs:
+                hidden.copy_(x)
+                both_layers()
+                results.append(hidden.clone())
+        stream.synchronize()
+    assert gw.kernel_error() == 0
+    for i, result in enumerate(results):
+        assert torch.equal(result, expected[i % len(inputs)]), f"pass {i}"
+    assert not torch.equal(expected[0], expected[1])
+
+
 def test_ffn_block_validation(gw, experts_shared):
     from gewell_b200 import _lib
     table, _ = experts_shared
