@@ -25,14 +25,15 @@ __device__ __forceinline__ void unpack8(const uint4& raw, float* out) {
   }
 }
 
-// 128-row groups per slab, so that `per_row` items of each of its rows number less than 2^31
+// 128-row groups per slab, so that `per_row` items of each of its rows number less than 2^31.  `padding`: rows up to the next
+// multiple of 128 have items too (scale tiles); without it a matrix of one slab has blocks for its own rows alone.
 struct Slabs {
   uint32_t rows, count;
-  Slabs(uint32_t total_rows, uint32_t per_row) {
+  Slabs(uint32_t total_rows, uint32_t per_row, bool padding) {
     const uint64_t fit = ((1ull << 31) - 1) / (uint64_t(per_row ? per_row : 1) * 128) * 128;
-    const uint64_t padded = (uint64_t(total_rows) + 127) / 128 * 128;
-    rows = uint32_t(fit == 0 ? 128 : fit < padded ? fit : padded);
-    count = uint32_t((padded + rows - 1) / rows);
+    const uint64_t all = padding ? (uint64_t(total_rows) + 127) / 128 * 128 : total_rows;
+    rows = uint32_t(fit == 0 ? 128 : fit < all ? fit : all);
+    count = uint32_t((all + rows - 1) / rows);
   }
 };
 
@@ -402,7 +403,7 @@ dim3 slab_grid(const Slabs& slabs, uint32_t per_row) {
 cudaError_t launch_nvfp4_dequantize(const uint8_t* data, const uint8_t* scales, float weight_scale,
                                     uint32_t width, uint32_t rows, void* output, cudaStream_t stream) {
   const uint32_t per_row = width / 16;
-  const Slabs slabs(rows, per_row);
+  const Slabs slabs(rows, per_row, false);
   nvfp4_dequantize_kernel<<<slab_grid(slabs, per_row), kThreads, 0, stream>>>(data, scales, weight_scale, width, Divisor::of(per_row),
                                                                              slabs.rows, rows, static_cast<uint4*>(output));
   note_launch();
@@ -413,7 +414,7 @@ cudaError_t launch_nvfp4_pack_weights(const void* weights, uint32_t rows, uint32
                                       float weight_scale, uint8_t* data, uint8_t* scales,
                                       cudaStream_t stream) {
   const uint32_t per_row = (width + 63) / 64 * 4;
-  const Slabs slabs(rows, per_row);
+  const Slabs slabs(rows, per_row, true);
   nvfp4_pack_weights_kernel<<<slab_grid(slabs, per_row), kThreads, 0, stream>>>(
       static_cast<const uint4*>(weights), rows, width, weight_scale, reinterpret_cast<uint2*>(data), scales, Divisor::of(per_row), slabs.rows);
   note_launch();
@@ -424,7 +425,7 @@ cudaError_t launch_nvfp4_quantize(const void* input, uint32_t rows, uint32_t wid
                                   float inverse_global_scale, bool gelu, uint8_t* packed,
                                   uint8_t* scales, cudaStream_t stream) {
   const uint32_t per_row = (width + 63) / 64 * (gelu ? 8 : 4);
-  const Slabs slabs(rows, per_row);
+  const Slabs slabs(rows, per_row, true);
   return launch_pdl(gelu ? nvfp4_quantize_kernel<true> : nvfp4_quantize_kernel<false>, slab_grid(slabs, per_row), kThreads, stream,
                     static_cast<const uint4*>(input), rows, width, inverse_global_scale, reinterpret_cast<uint32_t*>(packed), scales,
                     Divisor::of(per_row), slabs.rows);
@@ -434,7 +435,7 @@ cudaError_t launch_fp8_quantize(const void* input, uint32_t rows, uint32_t width
                                 bool gelu, uint8_t* packed, cudaStream_t stream) {
   const bool vector = reinterpret_cast<uintptr_t>(input) % 16 == 0;
   const uint32_t per_row = width / (gelu ? 8 : 16);
-  const Slabs slabs(rows, per_row);
+  const Slabs slabs(rows, per_row, false);
   const auto kernel = gelu ? (vector ? fp8_quantize_kernel<true, true> : fp8_quantize_kernel<true, false>)
                            : (vector ? fp8_quantize_kernel<false, true> : fp8_quantize_kernel<false, false>);
   return launch_pdl(kernel, slab_grid(slabs, per_row), kThreads, stream, static_cast<const bf16*>(input), rows, width, Divisor::of(per_row),
@@ -464,7 +465,7 @@ cudaError_t launch_geglu(const void* gate, const void* up, void* out, size_t n, 
 }
 
 cudaError_t launch_geglu_interleaved(const void* gate_up, void* out, uint32_t rows, uint32_t width, cudaStream_t stream) {
-  const Slabs slabs(rows, width / 8);
+  const Slabs slabs(rows, width / 8, false);
   return launch_pdl(geglu_interleaved_kernel, slab_grid(slabs, width / 8), kThreads, stream, static_cast<const uint4*>(gate_up),
                     static_cast<uint4*>(out), Divisor::of(width / 8), slabs.rows, rows);
 }
