@@ -264,7 +264,7 @@ gw_status gw_nvfp4_plan_create(uint32_t rows, uint32_t input_width, uint32_t out
       return fail(GW_CUDA_ERROR, std::string("plan: tile counters of the K split: ") + cudaGetErrorString(counters));
     }
   }
-  p->total_bytes += p->descriptors.split_bytes(rows, output_width);
+  p->total_bytes += p->descriptors.split_bytes(rows);
   *plan = p;
   return GW_OK;
 }
@@ -392,7 +392,7 @@ gw_status gw_fp8_plan_create(uint32_t rows, uint32_t input_width, uint32_t outpu
       return fail(GW_CUDA_ERROR, std::string("plan: tile counters of the K split: ") + cudaGetErrorString(counters));
     }
   }
-  p->total_bytes += p->descriptors.split_bytes(rows, output_width);
+  p->total_bytes += p->descriptors.split_bytes(rows);
   *plan = p;
   return GW_OK;
 }
@@ -488,7 +488,7 @@ gw_status gw_bf16_plan_create(uint32_t rows, uint32_t input_width, uint32_t outp
   p->total_bytes = 0;
   const cudaError_t status = p->descriptors.allocate_split_counters(GemmKind::bf16, rows, input_width, output_width);
   if (status == cudaSuccess) {
-    p->total_bytes = p->descriptors.split_bytes(rows, output_width);
+    p->total_bytes = p->descriptors.split_bytes(rows);
   } else if (status != cudaSuccess) {
     (void)cudaGetLastError();
     if (status != cudaErrorNoDevice && status != cudaErrorInsufficientDriver) {

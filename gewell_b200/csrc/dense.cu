@@ -85,19 +85,18 @@ int swap_split_grid(GemmKind kind, int tiles, int stages, int block_n) {
 }
 }  // namespace
 
-size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n) {
-  (void)n;
+size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows) {
   if (!dense_uses_swap_form(tuning, rows) || tuning.no_split) return 0;
   return size_t(2) * sm_count() * 128 * dense_block_n(tuning, rows) * sizeof(float);
 }
 
-size_t DenseDescriptors::split_bytes(uint32_t rows, uint32_t n) const {
+size_t DenseDescriptors::split_bytes(uint32_t rows) const {
   if (split_counters == nullptr) return 0;
-  return align_up(std::max(dense_split_bytes(tuning, rows, n), stream.usable ? stream.workspace_bytes : 0), 256);
+  return align_up(std::max(dense_split_bytes(tuning, rows), stream.usable ? stream.workspace_bytes : 0), 256);
 }
 
 cudaError_t DenseDescriptors::allocate_split_counters(GemmKind kind, uint32_t rows, uint32_t k, uint32_t n) {
-  if (dense_split_bytes(tuning, rows, n) == 0) return cudaSuccess;
+  if (dense_split_bytes(tuning, rows) == 0) return cudaSuccess;
   size_t bytes = split_counter_bytes(tuning, rows, n);
   if (tuning.streams()) {
     const StreamKind as = kind == GemmKind::nvfp4 ? StreamKind::w4a4 : kind == GemmKind::fp8 ? StreamKind::w8a8 : StreamKind::w16a16;

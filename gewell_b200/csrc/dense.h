@@ -45,7 +45,7 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   StreamMaps stream_maps;
   cudaError_t allocate_split_counters(GemmKind kind, uint32_t rows, uint32_t k, uint32_t n);
   // Scratch for FP32 partial sums of either form (0: none), once the counters exist.
-  size_t split_bytes(uint32_t rows, uint32_t n) const;
+  size_t split_bytes(uint32_t rows) const;
   ~DenseDescriptors();
 };
 
@@ -73,8 +73,8 @@ struct DenseProblem {
 bool dense_uses_swap_form(const DenseTuning& tuning, uint32_t rows);
 int dense_block_n(const DenseTuning& tuning, uint32_t rows);
 
-// Bytes of split workspace a projection of this shape can use (0: none).
-size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n);
+// Bytes of split workspace a projection of so many rows can use (0: none).
+size_t dense_split_bytes(const DenseTuning& tuning, uint32_t rows);
 
 // Whether the weight-streaming kernel is the faster one for this shape (n: output channels of all matrices together).
 bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n);

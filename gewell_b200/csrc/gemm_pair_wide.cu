@@ -193,7 +193,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
           __syncwarp();
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
-        if (!failed && ptx::elect_one()) commit_pair(acc_full_bar + acc);;
+        if (!failed && ptx::elect_one()) commit_pair(acc_full_bar + acc);
       }
     }
     __syncwarp();
