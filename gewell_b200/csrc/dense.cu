@@ -38,25 +38,55 @@ size_t split_counter_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n)
 }
 }  // namespace
 
-// Where the weight-streaming kernel is the faster one (B200, cold weights, us; streamed against activation quantiser +
-// tcgen05 swap form): NVFP4 1x2816x2816 5.4 / 7.1, 8x2816x2816 6.8 / 7.3, 2x8192x5376 13.1 / 14.4, but 16x2816x2816 9.6 / 7.3,
-// 4x2816x8192 9.8 / 8.2, 8x5376x4096 10.1 / 10.4, 1x21504x5376 22.1 / 19.9; FP8 8x2816x2816 6.4 / 8.1, 16x4096x2816 10.1 / 8.6;
-// BF16 8x2816x2816 7.0 / 8.7, 4x5376x16384 33.0 / 30.2.  It saves the quantiser's launch and the tensor-memory prologue and
-// uses every SM where there are few tiles; what it pays is that every SM reads and quantises all of the activations.
+// Where the weight-streaming kernel is the faster one.  It saves the quantiser's launch and the tensor-memory prologue; what it
+// pays is that every SM reads and quantises all of the activations, and about 2 us where SMs share row blocks and add their
+// sums in a second pass (StreamPlan::needs_workspace).  Measured against activation quantiser + tcgen05 swap form over K 1024 ..
+// 16384, N 512 .. 5376, 1 to 8 rows, rows * K up to 24 K (B200, cold weights; time of the streaming kernel over the other's,
+// passes of a CUDA graph | launched one by one from Python, where small shapes wait for the second launch):
+//   whole row blocks for every SM (N 2368 .. 4736), one slab        NVFP4 0.75 .. 1.10 | 0.72 .. 1.01, FP8 0.68 .. 1.01 | 0.58 .. 0.89,
+//                                                                   BF16 0.62 .. 0.89 | 0.65 .. 1.08
+//   shared, one slab    FP8 0.76 .. 1.27 | 0.71 .. 1.06, NVFP4 0.74 .. 1.37 | 0.70 .. 1.11, but with N above 4736, K from 4096 on
+//                       and several rows 0.88 .. 1.26 | 0.87 .. 1.12; BF16 0.80 .. 1.17 | 0.80 .. 1.16, K 1024 0.97 .. 1.19 | 0.87 .. 1.19
+//   several slabs       NVFP4 and FP8 up to N 512 0.84 .. 0.97 | 0.84 .. 0.91, beyond 0.92 .. 1.41 | 0.89 .. 1.49; BF16 up to N 2048
+//                       0.78 .. 1.16 | 0.79 .. 1.16, beyond 0.88 .. 1.22 | 0.89 .. 1.26
+// In us (graph): NVFP4 1x2816x2816 5.3 / 6.9, 8x2816x2816 6.7 / 7.0, 1x1408x5376 6.8 / 5.7, 1x16384x2816 18.2 / 13.4; FP8
+// 1x5376x5376 9.2 / 12.2; BF16 8x2816x4096 7.2 / 9.2, 1x8192x2816 16.4 / 13.9.
 // W4A16 has no other kernel that reads the packed weights.
 bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
   if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
-  return n <= 5376 && k <= 16384 && size_t(rows) * k <= 24 * 1024;
+  if (n > 5376 || k > 16384 || size_t(rows) * k > 24 * 1024) return false;
+  if (!plan.needs_workspace()) return true;
+  if (plan.slabs > 1) return n <= (kind == StreamKind::w16a16 ? 2048 : 512);
+  if (kind == StreamKind::w16a16) return k >= 1408;
+  return kind == StreamKind::w8a8 || n <= 4736 || rows == 1 || k < 4096;
 }
 
-// Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each.
-constexpr uint32_t kW4a16Rows = 48;
+namespace {
+// With GeGLU in front of the quantiser every SM computes all of it.  Over GeGLU + quantiser + swap form (as above): one slab and
+// at most 12 K values in whole row blocks or 8 K in shared ones 0.80 .. 1.44 | 0.66 .. 1.16; more values 0.88 .. 1.86 |
+// 0.82 .. 1.46, several slabs 0.90 .. 1.80 | 0.91 .. 1.72.
+bool stream_gelu_pays(const StreamPlan& plan, uint32_t rows, uint32_t k) {
+  return plan.slabs == 1 && size_t(rows) * k <= (plan.needs_workspace() ? 8 : 12) * 1024;
+}
+}  // namespace
 
-// Gate, up and GeGLU as one streaming launch (n: channels of each) against the joined GEMM whose GeGLU rides in the next
-// quantiser (whole chains of hidden -> n -> hidden, us, streamed / joined): NVFP4 4 rows 1408 -> 4096 18.0 / 20.7, 8 rows of
-// the feed-forward block (2816 -> 2112) 94 / 97.5, 4 rows 2816 -> 8192 28.4 / 23.0; 5376 -> 21504 1 row 51.6 / 53.9, 8 rows
-// 55.1 / 54.2; FP8 1 row 68.4 / 69.0, 8 rows 71.5 / 69.8.  So: small matrices, whose joined GEMM leaves SMs idle, and
-// large ones for one token, where the launches it saves are all there is to gain.
+// Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each, instead of dequantising the
+// weights for a BF16 GEMM (MLP of hidden -> n -> hidden, us, streamed / dequantised):
+//   5376 -> 21504     16 rows 100 / 285    32 rows 200 / 287    48 rows 300 / 291
+//   4096 -> 11008              57 / 126             113 / 126             169 / 130
+//   2816 -> 8192               48 / 83               93 / 84              137 / 87
+//   2816 -> 2176               23 / 48               45 / 49               68 / 54
+//   1408 -> 4096               27 / 47               54 / 48               80 / 50
+constexpr uint32_t kW4a16Rows = 32;
+
+// Gate, up and GeGLU as one streaming launch (n: channels of each).  Where the two matrices lie apart it stands against two
+// projections and a GeGLU kernel, where they are joined against one GEMM whose GeGLU rides in the next quantiser (BF16: a kernel
+// of its own).  Whole chains of hidden -> n -> hidden, hidden 1408 .. 5376, n 1024 .. 21504, 1 to 8 rows, time over the other way
+// (as above):
+//   n up to 4224, rows * K up to 24 K          apart 0.63 .. 0.88 | 0.64 .. 1.04; joined 0.80 .. 1.40 | 0.60 .. 1.10
+//   96 MiB and more, rows * K up to 8 K        apart 0.78 .. 0.95 | 0.79 .. 0.94; joined 0.91 .. 1.00 | 0.91 .. 1.00
+//   the rest                                   apart 0.68 .. 1.06 | 0.64 .. 1.01; joined 0.82 .. 1.39 | 0.61 .. 1.35
+// In us (graph): NVFP4 1x5376x21504 joined 48.4 / 48.2, apart 48.1 / 59.3; FP8 1x5376x21504 joined 65.3 / 66.0.
 bool stream_pair_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
   if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
   const size_t bytes = 2 * n * k * (kind == StreamKind::w4a4 ? 9 : kind == StreamKind::w8a8 ? 16 : 32) / 16;
@@ -114,7 +144,7 @@ DenseDescriptors::~DenseDescriptors() {
 }
 
 gw_status launch_dense_stream(const StreamProblem& q, DenseDescriptors* cache, cudaStream_t stream, bool* done) {
-  *done = cache->stream.usable && stream_aligned(q);
+  *done = cache->stream.usable && stream_aligned(q) && (!q.gelu || stream_gelu_pays(cache->stream, q.rows, q.k));
   if (!*done) return GW_OK;
   std::string error;
   if (!cache->stream_maps.get(q.kind, q.first, cache->stream.physical_n, q.k, &error))

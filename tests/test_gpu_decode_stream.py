@@ -1,6 +1,7 @@
 """The weight-streaming projections of small row counts (decode_stream.cu) at the edges of their division of the work:
-K of one partial chunk, a chunk, whole and ragged slabs; row blocks shared by warps and by SMs; one and two token
-groups; two matrices with GeGLU; W4A16 over several launches."""
+K of one partial chunk, a chunk, whole and ragged slabs; row blocks shared by warps and by SMs; one group of eight tokens, and
+two for W4A16; two matrices with GeGLU; W4A16 over several launches.  Row counts above the kernel's (8; W4A16: 32) and shapes
+where it does not pay run on the kernels beside it."""
 import numpy as np
 import pytest
 import torch
@@ -67,7 +68,8 @@ def test_bf16(gw, rows, k, n):
 @pytest.mark.parametrize("hidden,mlp", [(128, 128), (640, 1408)])
 @pytest.mark.parametrize("policy", ["always", "prefill"])
 def test_nvfp4_pair_and_w4a16(gw, rows, hidden, mlp, policy):
-    """Gate and up with scales of their own (one launch with GeGLU up to 16 rows), W4A16 up to 48 rows and beyond."""
+    """Gate and up with scales of their own: one launch with GeGLU for up to eight rows (W4A16: sixteen a launch, up to 32
+    rows), projections one by one beyond."""
     from gewell_b200 import _lib
     gate, up = (gw.nvfp4_pack_weights(bf16_normal((mlp, hidden), s, 0.05).cuda(), 0.002) for s in (1, 2))
     down = gw.nvfp4_pack_weights(bf16_normal((hidden, mlp), 3, 0.05).cuda(), 0.004)
@@ -85,3 +87,35 @@ def test_nvfp4_pair_and_w4a16(gw, rows, hidden, mlp, policy):
         g, u = (C.bf16_to_f32(onv.linear_w4a16(to_f32(x), h)) for h in (hg, hu))
         expected = onv.linear_w4a16(C.gelu_tanh_multiply_bf16(g, u), hd)
     assert_gemm_close(y, expected, f"chain rows={rows} {hidden}/{mlp} {policy}")
+
+
+@pytest.mark.parametrize("rows", [32, 33])
+def test_w4a16_last_streamed_rows(gw, rows):
+    """Two launches of the packed weights, and the first row count that dequantises them."""
+    test_nvfp4_pair_and_w4a16(gw, rows, 640, 1408, "prefill")
+
+
+@pytest.mark.parametrize("rows,k,n", [(1, 8192, 2048), (1, 8448, 2048), (4, 3072, 2816), (4, 3136, 2816), (8, 1088, 256)])
+@pytest.mark.parametrize("storage", ["nvfp4", "fp8"])
+def test_geglu_inputs_around_their_limit(gw, storage, rows, k, n):
+    """A plan that streams plain inputs hands GeGLU inputs above a size to the quantiser and the tensor-core kernel; the two
+    take turns on one plan and its scratch, whose counters have to come back to zero."""
+    x, gate_up = bf16_normal((rows, k), 61), bf16_normal((rows, 2 * k), 62)
+    values = to_f32(bf16_normal((n, k), 63, 0.02))
+    if storage == "nvfp4":
+        w = onv.pack_weights(values, 0.01)
+        dev, plan, linear = oracle_weight_to_device(w), gw.Nvfp4Plan(rows, k, n), lambda a: onv.linear_w4a4(a, w, rcp_fn=gw.rcp_approx)
+    else:
+        w = ofp8.pack_weights(values, 0.01)
+        dev = gw.Fp8Weight(torch.from_numpy(w.data.copy()).cuda(), w.input_scale, w.weight_scale)
+        plan, linear = gw.Fp8Plan(rows, k, n), lambda a: ofp8.linear_w8a8(a, w)
+    scratch = torch.full((plan.scratch_bytes(),), 0xCD, dtype=torch.uint8, device="cuda")
+    product = gw.geglu_bf16(to_f32(gate_up[:, :k]), to_f32(gate_up[:, k:]))
+    for _ in range(2):
+        for source, transform, expected in ((x, gw.TRANSFORM_IDENTITY, linear(to_f32(x))),
+                                            (gate_up, gw.TRANSFORM_GELU_TANH_MULTIPLY, linear(product))):
+            y = torch.full((rows, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+            plan.run(source.cuda(), dev, y, scratch, transform=transform)
+            torch.cuda.synchronize()
+            assert gw.kernel_error() == 0
+            assert_gemm_close(bits(y), expected, f"{storage} rows={rows} K={k} N={n} transform={transform}")

@@ -68,7 +68,7 @@ ws = ctypes.c_void_p()
 check(lib.gw_projection_workspace_create((_lib.Projection * 2)(p, q), 2, 256, _lib.POLICY_PREFILL, None, ctypes.byref(ws)))
 prepare = lambda rows: lib.gw_projection_workspace_prepare(ws, rows, _lib.PHASE_DECODE)
 run = lambda: lib.gw_projection_workspace_run(ws, ctypes.byref(p), A, A)
-for small, large in ((200, 5), (5, 40), (40, 5), (200, 40)):
+for small, large in ((200, 5), (5, 24), (24, 5), (40, 5)):
     each_allocation_fails(prepare, run, small, large)
 '''
 
@@ -78,7 +78,7 @@ chain = ctypes.c_void_p()
 check(lib.gw_mlp_chain_create(640, 1408, 256, _lib.POLICY_PREFILL, ctypes.byref(chain)))
 prepare = lambda rows: lib.gw_mlp_chain_prepare(chain, rows)
 run = lambda: lib.gw_mlp_chain_run(chain, *map(ctypes.byref, (gate, up, down)), A, A, A, A, _lib.PHASE_DECODE, None)
-for small, large in ((200, 5), (5, 40), (40, 5), (200, 40)):
+for small, large in ((200, 5), (5, 24), (24, 5), (40, 5)):
     each_allocation_fails(prepare, run, small, large)
 '''
 
