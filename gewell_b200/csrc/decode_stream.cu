@@ -4,14 +4,15 @@
 // What bounds it: the weight bytes from HBM.  So the work is divided by bytes: the flat sequence of
 // (block of 32 weight rows, 128-byte chunk of K) pieces is cut into equal ranges, one per SM and inside
 // it one per warp, at any piece.  A warp walks its range alone: it has a ring of two pieces of its own that it
-// refills itself by tensor copies as soon as it has multiplied one (148 KB per SM on their way), and it stores the
-// row blocks that are wholly its own straight from registers.  Nothing synchronises while weights stream; the
+// refills itself by tensor copies as soon as it has multiplied one (144 KB per SM on their way for W4A4, 128 for W8A8,
+// 108 for W4A16, 96 for BF16), and it stores the row blocks that are wholly its own straight from registers.  Nothing synchronises while weights stream; the
 // first pieces are asked for before the kernel waits for its predecessor.  Row blocks that several warps share
 // are added through shared memory at the end, those that several SMs share through L2 by the one that
 // arrives last at the block's counter -- always in range order, so results do not depend on who comes last.
 //
 // Measured on cold weights (us, with everything a call does; activation quantiser + tcgen05 kernel in brackets): NVFP4
-// 1x2816x2816 5.4 (7.1), FP8 8x2816x2816 6.4 (8.1); W4A16 MLP of five rows 66 against 330 with dequantised weights.
+// 1x2816x2816 5.3 (6.9), FP8 8x2816x2816 6.5 (7.6); W4A16 MLP of eight rows, 5376 -> 21504, 70 against 285 with dequantised
+// weights.
 //
 // Token values live in shared memory in the order the tensor instruction wants them.  When all of K does
 // not fit there, K is cut into slabs, the flat sequence walks slab by slab and every row block has one sum

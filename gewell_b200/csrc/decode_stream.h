@@ -1,5 +1,5 @@
 // Launch description of the weight-streaming projections for small row counts
-// (decode_stream.cu): Y[rows, n] = bf16(alpha * Xq . Wq^T) for 1..16 rows, the
+// (decode_stream.cu): Y[rows, n] = bf16(alpha * Xq . Wq^T) for 1..8 rows (W4A16: 1..16), the
 // activations quantised (or copied) by every thread block itself, every weight brought
 // into shared memory once and contracted with warp-level tensor instructions.
 #pragma once

@@ -71,7 +71,8 @@ bool stream_gelu_pays(const StreamPlan& plan, uint32_t rows, uint32_t k) {
 }  // namespace
 
 // Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each, instead of dequantising the
-// weights for a BF16 GEMM (MLP of hidden -> n -> hidden, us, streamed / dequantised):
+// weights for a BF16 GEMM.  The streamed product does not round the weights to BF16, the dequantised one does, as the reference
+// does it: the line changes results within that rounding.  (MLP of hidden -> n -> hidden, us, streamed / dequantised):
 //   5376 -> 21504     16 rows 100 / 285    32 rows 200 / 287    48 rows 300 / 291
 //   4096 -> 11008              57 / 126             113 / 126             169 / 130
 //   2816 -> 8192               48 / 83               93 / 84              137 / 87

@@ -17,8 +17,8 @@
 // registers between the reduction and the output, and the row sits in shared memory for the fixed-order sums
 // only.  What bounds these kernels at decode sizes is the chain of memory latency, barriers and adds, not
 // bytes: all loads of a thread are 16 bytes wide and issued before the first barrier (2816 wide, 8 rows, weights
-// not in L2: norm 16.9 -> 3.9 us, tail 18.8 -> 4.5 us, with the launch, against element-wise loads in the output loop and a
-// block barrier for every level of the sum).  The block's tail -- two post norms, add, the third norm, residual
+// not in L2, launches of a graph behind one another: norm 4.5 -> 2.2 us, three outputs 8.6 -> 2.7, tail 9.6 -> 4.1 us, against
+// element-wise loads in the output loop and a block barrier for every level of the sum).  The block's tail -- two post norms, add, the third norm, residual
 // add, layer scalar: seven launches in the reference -- is one kernel with one block per row.
 #include <algorithm>
 #include <cmath>

@@ -9,10 +9,11 @@
 //               FP8 with per-channel scales, or BF16; otherwise two separate projections
 //   GeGLU       fused into the activation quantiser of the down projection when that one runs
 //               quantised on a joined [rows, gate | up] tensor; an element-wise kernel otherwise
-//               (rows <= 16: gate, up and GeGLU are one launch of the weight-streaming kernel, and W4A16
-//               reads the packed weights, rows <= 48)
-//   down        FP8, NVFP4 (W4A4) or BF16 GEMM; NVFP4 weights with BF16 activations are
-//               dequantised into the chain's scratch first (W4A16)
+//               (small row counts, where that is the faster way: gate, up and GeGLU are one launch of the
+//               weight-streaming kernel, see stream_pair_pays)
+//   down        FP8, NVFP4 (W4A4) or BF16 GEMM.  NVFP4 weights with BF16 activations (W4A16) are read packed by the
+//               weight-streaming kernel up to 32 rows, for gate and up too, and dequantised into the chain's scratch
+//               for a BF16 GEMM beyond
 //
 // prepare(rows) builds the plans outside the layer loop; run() allocates nothing.
 //

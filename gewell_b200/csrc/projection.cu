@@ -6,7 +6,8 @@
 // A bound projection is run by storage type, activation policy and phase:
 //   FP8                         -> fp8 plan (W8A8)
 //   NVFP4, FP4 activations      -> nvfp4 plan (W4A4)
-//   NVFP4, BF16 activations     -> dequantise the whole weight to BF16 scratch, BF16 GEMM (W4A16)
+//   NVFP4, BF16 activations     -> (W4A16) up to 32 rows the packed weights on the weight-streaming kernel, else the whole
+//                                  weight dequantised to BF16 scratch and a BF16 GEMM
 //   BF16                        -> BF16 GEMM
 // and, when the NVFP4 output dimension was padded to 128 rows, the padded
 // result is compacted to the logical width.  Plans are (re)built in prepare(),
@@ -216,7 +217,7 @@ gw_status gw_projection_workspace_create(const gw_projection* projections, uint3
       scratch_bytes = std::max(scratch_bytes, gw_nvfp4_scratch_upper_bound_bytes(max_rows, p.input, p.physical_output));
       if (p.output != p.physical_output)
         padded_bytes = std::max(padded_bytes, size_t(max_rows) * p.physical_output * sizeof(bf16));
-      if (policy == GW_POLICY_PREFILL) {     // decode keeps BF16 activations: whole-weight dequantisation + BF16 GEMM
+      if (policy == GW_POLICY_PREFILL) {     // decode keeps BF16 activations: beyond 32 rows dequantisation + BF16 GEMM
         dequantized_bytes = std::max(dequantized_bytes, size_t(p.physical_output) * p.input * sizeof(bf16));
         w->plans.emplace(Shape{kPlanBf16, p.input, p.physical_output}, Plans{});
         scratch_bytes = std::max(scratch_bytes, bf16_scratch);

@@ -8,9 +8,9 @@
 //
 // The tensor instruction is mma.sync m16n8k16 with FP32 accumulation.  Which sixteen K values make up
 // a step is free as long as both operands agree: a step takes four consecutive values of every lane's
-// own 32 bytes, so no value changes lanes.  With one to sixteen token columns the weights are used
-// once; tcgen05 reads its lane operand from shared memory at 32-38 B/clk per SM whatever the column count,
-// which is below what HBM delivers in FP4, and cannot take NVFP4 weights with BF16 activations at all.
+// own 32 bytes, so no value changes lanes.  With one to sixteen token columns the tensor instruction is not
+// what bounds a launch; tcgen05 would want quantised tokens from a launch before and a tensor-memory prologue,
+// and cannot take NVFP4 weights with BF16 activations at all.
 //
 // Both operands are exact: E2M1 x E4M3 block scale has six significant bits and fits FP16 (range
 // 2^-10 .. 2688) as well as BF16, E4M3 fits FP16.  FP4 and FP8 activations are quantised by the same

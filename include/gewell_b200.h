@@ -267,8 +267,11 @@ void gw_artifact_close(gw_artifact* artifact);
  * sequential projections on ONE stream, bound at construction.  create() sizes the scratch for
  * max_rows and the given bindings and allocates it; prepare(rows, phase) builds the plans for a row
  * count before the layer loop (it allocates small per-plan state: not capturable); run() allocates
- * nothing and picks the path by storage, policy and phase (W8A8, W4A4, or BF16 GEMM on BF16 weights /
- * on the NVFP4 weight dequantised to BF16), then strips NVFP4 output padding.  The reference's
+ * nothing and picks the path by storage, policy and phase (W8A8, W4A4, BF16, or W4A16: NVFP4 weights with
+ * BF16 activations), and leaves NVFP4 output padding out.  W4A16 multiplies the packed weights up to 32
+ * rows: products and sums of the exact e2m1 * e4m3 with BF16 activations in FP32, times weight_scale at the
+ * end.  Beyond, it dequantises the weight first, bf16(e2m1 * (e4m3 * weight_scale)) as the reference does,
+ * and its BF16 GEMM multiplies the rounded values.  _bytes counts what create allocates.  The reference's
  * cublasHandle_t argument of run has no counterpart (no library GEMM). */
 typedef struct gw_projection_workspace gw_projection_workspace;
 gw_status gw_projection_workspace_create(const gw_projection* projections, uint32_t count, uint32_t max_rows,
@@ -298,13 +301,14 @@ gw_status gw_gelu_tanh_multiply_interleaved_bf16(const void* gate_up_bf16, void*
  * globals, 31b/sm120/nvfp4_projections.h:21-33; FP8: adjacent with per-channel scales,
  * fp8_projections.h:20-50; BF16: adjacent); GeGLU is fused into the down projection's activation
  * quantiser whenever that one runs quantised on the joined tensor.  policy / phase as in
- * nvfp4_policy.h: with policy "prefill" decode keeps BF16 activations (NVFP4 weights are dequantised
- * into the chain's scratch, W4A16).
+ * nvfp4_policy.h: with policy "prefill" decode keeps BF16 activations (W4A16, as in ProjectionWorkspace:
+ * packed weights up to 32 rows, dequantised into the chain's scratch beyond).
  *   create    allocates the shared scratch for max_rows (set-up time)
  *   prepare   builds the plans for a row count, outside the layer loop
  *   run       gate_up_bf16: [rows, 2 * mlp] scratch of the caller ([rows, gate | up] when joined, gate
- *             rows then up rows otherwise), product_bf16: [rows, mlp] scratch (used by the unfused
- *             GeGLU), output_bf16: [rows, hidden]; allocates nothing */
+ *             rows then up rows otherwise; not written where gate, up and GeGLU are one launch),
+ *             product_bf16: [rows, mlp] scratch (GeGLU of the two, where it is not fused into the down
+ *             projection's quantiser), output_bf16: [rows, hidden]; allocates nothing */
 typedef struct gw_mlp_chain gw_mlp_chain;
 gw_status gw_mlp_chain_create(uint32_t hidden, uint32_t mlp, uint32_t max_rows, int policy, gw_mlp_chain** chain);
 gw_status gw_mlp_chain_prepare(gw_mlp_chain* chain, uint32_t rows);

@@ -119,3 +119,34 @@ def test_geglu_inputs_around_their_limit(gw, storage, rows, k, n):
             torch.cuda.synchronize()
             assert gw.kernel_error() == 0
             assert_gemm_close(bits(y), expected, f"{storage} rows={rows} K={k} N={n} transform={transform}")
+
+
+@pytest.mark.parametrize("rows", [1, 16, 32, 33, 64])
+def test_w4a16_arithmetic(gw, rows):
+    """Up to 32 rows the products of exact weights, beyond of weights rounded to BF16; each against the FP64 sum over its own
+    operands: one BF16 rounding (2^-8 relative) and FP32 sums of K terms ((K + 4) 2^-24 of the magnitudes' sum).  Sums that
+    cancel tell the two apart."""
+    from gewell_b200 import _lib
+    k, n = 1408, 640
+    w = onv.pack_weights(to_f32(bf16_normal((n, k), 71, 0.02)))
+    x = bf16_normal((rows, k), 72)
+    dev = oracle_weight_to_device(w)
+    p = gw.make_projection(dev, k, n)
+    ws = gw.ProjectionWorkspace([p], 64, _lib.POLICY_PREFILL)
+    ws.prepare(rows, _lib.PHASE_DECODE)
+    y = torch.empty((rows, n), dtype=torch.bfloat16, device="cuda")
+    ws.run(p, x.cuda(), y)
+    torch.cuda.synchronize()
+    assert gw.kernel_error() == 0
+    values, scales = onv.decoded_weight_values(w)
+    unrounded = (values.reshape(n, -1, 16).astype(np.float64) * scales.astype(np.float64)[:, :, None]).reshape(n, k) * float(w.weight_scale)
+    rounded = C.bf16_to_f32(onv.dequantize(w)).astype(np.float64)
+    a, got = to_f32(x).astype(np.float64), to_f32(y).astype(np.float64)
+
+    def outside(weights):
+        reference = a @ weights.T
+        bound = 2.0 ** -8 * np.abs(reference) + (k + 4) * 2.0 ** -24 * (np.abs(a) @ np.abs(weights).T)
+        return int((np.abs(got - reference) > bound).sum())
+    own, other = (unrounded, rounded) if rows <= 32 else (rounded, unrounded)
+    assert outside(own) == 0
+    assert outside(other) > 0
