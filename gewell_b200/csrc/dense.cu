@@ -301,7 +301,9 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
   const bool fp4 = q.kind == GemmKind::nvfp4;
   const uint64_t row_bytes = fp4 ? q.k / 2 : (q.kind == GemmKind::bf16 ? uint64_t(2) * q.k : q.k);
   std::string error;
-  // Outputs of these kinds are 16-byte aligned and a multiple of 8 wide (plan creation and the run check it).
+  // FP8 and BF16 beyond the swap form's rows, narrow ones too (BF16, K 2816, N 128, us, CTA pairs / single CTAs with 128- and
+  // 256-wide tiles: 129 rows 11.5 / 13.2 / 15.6, 777 rows 11.7 / 13.5 / 16.2, 8192 rows 13.9 / 14.2 / 17.8; N 512 129 rows 12.1 /
+  // 13.7 / 20.6).  Outputs of these kinds are 16-byte aligned and a multiple of 8 wide (plan creation and the run check it).
   if (!fp4 && !swap && tuning.form == 0 && tuning.block_n == 0 && !tuning.no_pair)
     return launch_dense_pair_wide(q, row_bytes, cache, stream);
   const bool single_box = !swap && block_n == 256;   // both column halves come from the one weight matrix
