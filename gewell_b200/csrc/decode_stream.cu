@@ -128,7 +128,6 @@ struct Layout {
   static constexpr int kWarps = NT == 1 && (KIND == StreamKind::w4a4 || KIND == StreamKind::w8a8) ? 16 : 12;
   static constexpr int kThreads = 32 * kWarps;
   static constexpr uint32_t kSlots = 2;                                                // pieces in a warp's ring
-  static constexpr uint32_t kAhead = 4;                                                // pieces a warp brings into L2 before its wait
   static constexpr uint32_t kScaleBytes = nvfp4_weights(KIND) ? kPieceScaleBytes : 0;
   static constexpr uint32_t kRingBytes = kWarps * kSlots * (kPieceBytes + kScaleBytes);
   static constexpr uint32_t kSumBytes = kWarps * unit_values<NT, PAIR>() * 4;                // a row block that the warp before began
@@ -227,7 +226,7 @@ template <StreamKind KIND, int NT, bool PAIR>
 __global__ void __launch_bounds__((Layout<KIND, NT, PAIR>::kThreads), 1)
 decode_stream_kernel(const __grid_constant__ StreamArgs a) {
   using L = Layout<KIND, NT, PAIR>;
-  constexpr uint32_t kValues = unit_values<NT, PAIR>(), kWarps = L::kWarps, kSlots = L::kSlots, kAhead = L::kAhead;
+  constexpr uint32_t kValues = unit_values<NT, PAIR>(), kWarps = L::kWarps, kSlots = L::kSlots;
   extern __shared__ uint8_t stream_smem[];
   __shared__ uint64_t full_bar[L::kWarps * L::kSlots];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(stream_smem) + 1023) & ~uintptr_t(1023));
@@ -288,11 +287,11 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
     };
     // Settled weights do not depend on the kernel before this one (it wrote activations): ask for them while it still runs.
     // Others come as far as L2 meanwhile and are asked for behind the tokens, whose loads would queue behind theirs (MLP of
-    // one NVFP4 row, us: settled 49.2, from L2 51.3, the other order 52.0, no prefetch 52.9).
+    // one NVFP4 row, us: settled 49.2, two pieces from L2 50.2, four 51.1, asked for before the tokens 52.0, no prefetch 52.9).
     const bool unsettled = !a.weights_settled && slab_begin == piece_begin;
     if (unsettled) {
 #pragma unroll 1
-      for (uint32_t s = 0; s < kAhead; ++s) request(true);
+      for (uint32_t s = 0; s < kSlots; ++s) request(true);
       next = begin; next_block = block; next_chunk = chunk; next_slot = turn % kSlots; next_matrix = 0;
     } else {
 #pragma unroll 1
