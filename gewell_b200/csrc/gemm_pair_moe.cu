@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "gemm_pair_moe.h"
+#include "moe_work.cuh"
 #include "pair.cuh"
 #include "ptx.cuh"
 
@@ -33,6 +34,9 @@ namespace gw {
 namespace {
 
 using namespace pair;
+using moe_work::Unit;
+using moe_work::WorkTable;
+using moe_work::decode_unit;
 
 constexpr int kExperts = 128;
 constexpr int kHidden = 2816;
@@ -41,75 +45,6 @@ constexpr int kScaleWarps = 4, kFirstEpilogueWarp = 2 + kScaleWarps;
 constexpr uint32_t kDescHiSw128 = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);   // SBO 1024 B, version 1, SWIZZLE_128B
 
 __device__ __forceinline__ uint64_t make_desc(uint32_t lo16) { return (uint64_t(kDescHiSw128) << 32) | lo16; }
-
-// ---------------------------------------------------------------------------
-// work table
-// ---------------------------------------------------------------------------
-struct WorkTable {
-  int32_t first[kExperts];        // first sorted row of the expert (clamped to the capacity)
-  int32_t count[kExperts];        // its rows
-  int32_t prefix[kExperts + 1];   // first work unit of the expert; [128] = all units
-};
-
-struct Unit {
-  int e, first, count;
-  int tile;      // 256-row pair tile inside the expert
-  int part;      // channel tile (gate/up) or channel chunk (down)
-};
-
-// All threads of the CTA.  units_per_tile work units for every 256-row pair tile of every expert.
-__device__ __forceinline__ void build_work_table(const PairMoeParams& p, WorkTable* t, int units_per_tile) {
-  __shared__ int32_t warp_totals[4];
-  const int e = threadIdx.x;
-  int32_t units = 0;
-  if (e < kExperts) {
-    int32_t first = p.offsets[e], last = p.offsets[e + 1];
-    const int32_t capacity = int32_t(p.capacity);
-    if (first < 0 || last < first || last > capacity) {
-      if (p.error != nullptr) atomicCAS(p.error, 0u, 0x70000100u | uint32_t(e));
-      first = min(max(first, 0), capacity);
-      last = min(max(last, first), capacity);
-    }
-    t->first[e] = first;
-    t->count[e] = last - first;
-    units = ((last - first + 255) / 256) * units_per_tile;
-  }
-  // exclusive scan over the 128 experts: shuffles inside each of the first four warps, then their totals
-  int32_t scan = units;
-  const int lane = threadIdx.x % 32;
-  if (e < kExperts) {
-#pragma unroll
-    for (int step = 1; step < 32; step *= 2) {
-      const int32_t other = __shfl_up_sync(0xffffffffu, scan, step);
-      if (lane >= step) scan += other;
-    }
-    if (lane == 31) warp_totals[e / 32] = scan;
-  }
-  __syncthreads();
-  if (e < kExperts) {
-    int32_t base = 0;
-    for (int w = 0; w < e / 32; ++w) base += warp_totals[w];
-    t->prefix[e] = base + scan - units;
-    if (e == kExperts - 1) t->prefix[kExperts] = base + scan;
-  }
-  __syncthreads();
-}
-
-__device__ __forceinline__ void decode_unit(const WorkTable* t, int w, int units_per_tile, Unit& u) {
-  if (u.e < 0 || w < t->prefix[u.e] || w >= t->prefix[u.e + 1]) {
-    int lo = 0, hi = kExperts;             // largest e with prefix[e] <= w (it has units, since w < prefix[128])
-    while (lo + 1 < hi) {
-      const int mid = (lo + hi) / 2;
-      if (t->prefix[mid] <= w) lo = mid; else hi = mid;
-    }
-    u.e = lo;
-    u.first = t->first[lo];
-    u.count = t->count[lo];
-  }
-  const int local = w - t->prefix[u.e];
-  u.part = local % units_per_tile;
-  u.tile = local / units_per_tile;
-}
 
 // ===========================================================================
 // gate/up: Y = Xq . [Wgate | Wup]^T per expert, GeGLU, FP4 quantisation of the result
@@ -188,7 +123,7 @@ pair_moe_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_enter();                                  // the offsets and the quantised rows come from earlier kernels
-  build_work_table(p, table, kCTiles);
+  moe_work::build_work_table<256, 0, 1>(p, table, kCTiles);
 
   const int total = table->prefix[kExperts];
   const int pairs = gridDim.x / 2, pair_index = blockIdx.x / 2;
@@ -592,7 +527,7 @@ pair_moe_down_kernel(const __grid_constant__ PairMoeParams p) {
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   griddep_enter();
-  build_work_table(p, table, kChunks);
+  moe_work::build_work_table<256, 2, 2>(p, table, kChunks);
 
   const int total = table->prefix[kExperts];
   const int pairs = gridDim.x / 2, pair_index = blockIdx.x / 2;

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "gemm_moe_narrow.h"
 #include "gemm_pair_moe.h"
 #include "gemm_tc.cuh"
 #include "moe_kernels.h"
@@ -159,7 +160,7 @@ gw_status gw_moe_expert_table_create(const gw_expert_weights* experts, uint32_t 
             !finite_positive(p.nvfp4_input_scale * p.nvfp4_weight_scale))
           return fail(GW_INVALID_ARGUMENT, "invalid 26B expert projection binding" + who);
         if (!encode_tensor_map_2d(slot + i, p.nvfp4_data, p.input / 2, p.physical_output, 128, &error) ||
-            (i == 2 && !encode_tensor_map_2d(slot + 3, p.nvfp4_data, p.input / 2, p.physical_output, 64, &error)))
+            !encode_tensor_map_2d(slot + (i == 2 ? 3 : kMoeMapGate64 + i), p.nvfp4_data, p.input / 2, p.physical_output, 64, &error))
           return fail(GW_CUDA_ERROR, "expert weight descriptor: " + error);
         info[e].scales[i] = p.nvfp4_scales;
         info[e].alpha[i] = p.nvfp4_input_scale * p.nvfp4_weight_scale;   // == __fmul_rn on the device
@@ -340,15 +341,28 @@ gw_status dispatch(gw_moe_workspace* w, const void* scores, const void* expert_s
 struct ExpertPlan {
   int form;
   bool pair_first, pair_down;
+  int narrow;                 // token rows of a tile of gemm_moe_narrow.cu, 0: it does not run
   MoeGroupPlan groups;
-  bool needs_groups() const { return !(pair_first && pair_down); }
+  bool needs_groups() const { return !narrow && !(pair_first && pair_down); }
 };
+// Sorted rows up to which experts that share their gate and up input scale run with their tokens on the columns, and the
+// width of a token tile.  Whole layer, us, 64- / 128-wide tiles / CTA pairs, even experts and a 1.2 power law:
+//   64 tokens 81 / 85 / 138, 45 / 47 / 72     512 113 / 115 / 151, 96 / 97 / 119      777 114 / 115 / 157, 114 / 105 / 133
+//   1500 182 / 137 / 172, 173 / 150 / 167     2048 219 / 179 / 186, 210 / 176 / 197   3000 295 / 232 / 203, 280 / 227 / 229
+constexpr uint32_t kNarrowRows = 8 * 2048, kNarrowRows64 = 8 * 512;
+constexpr uint32_t kCapturedRows = 8 * 512;   // up to here the BF16 intermediates are always written
 ExpertPlan plan_experts(gw_moe_workspace* w, const gw_expert_table* table, const int32_t* offsets, uint32_t n) {
   const MoeTuning& tune = w->tuning;
   int form = n <= 8 * 512 ? kMoeFormSwap : (table->shared_gate_up ? kMoeFormFused : kMoeFormDirect);
   if (tune.form == 's') form = kMoeFormSwap;
   if (tune.form == 'd') form = kMoeFormDirect;
   if (tune.form == 'f' && table->shared_gate_up) form = kMoeFormFused;
+  int narrow = 0;
+  if (table->shared_gate_up && (tune.form == 'n' || (tune.form == 0 && n <= kNarrowRows))) {
+    form = kMoeFormSwap;
+    narrow = n <= kNarrowRows64 ? 64 : 128;
+    if (tune.block_n == 64 || tune.block_n == 128) narrow = tune.block_n;
+  }
   // Large batches run on CTA pairs: the gate/up GEMM when one quantised copy of a row serves both
   // projections (the fused plan), the down GEMM whenever tokens sit on the lanes.
   const bool pair_first = form == kMoeFormFused && !tune.no_pair;
@@ -357,12 +371,13 @@ ExpertPlan plan_experts(gw_moe_workspace* w, const gw_expert_table* table, const
   if (form == kMoeFormSwap) {
     block_n_first = n <= 8 * 64 ? 32 : (n <= 8 * 256 ? 64 : 128);
     if (tune.block_n == 32 || tune.block_n == 64 || tune.block_n == 128) block_n_first = tune.block_n;
+    if (narrow) block_n_first = narrow;
     block_n_down = block_n_first;
   } else {
     block_n_first = form == kMoeFormFused ? 256 : (tune.block_n == 256 ? 256 : 128);
     block_n_down = tune.block_n_down == 256 ? 256 : 128;
   }
-  return ExpertPlan{form, pair_first, pair_down,
+  return ExpertPlan{form, pair_first, pair_down, narrow,
                     MoeGroupPlan{offsets, table->info.as<MoeExpertInfo>(), w->scales_in.as<uint8_t>(), w->scales_act.as<uint8_t>(), n,
                                  w->scale_rows, form, block_n_first, block_n_down, table->shared_gate_up ? 1 : 0, device_error_word(),
                                  kMoeKindNvfp4, 1}};
@@ -391,10 +406,11 @@ namespace {
 // the permutation (input row = index / gather_divisor); otherwise input row i
 // is sorted row i.
 //
-// Three plans (see moe_prepare_groups_kernel): small batches put the weights on
-// the 128-lane operand and an expert's few tokens on the column operand; large
-// batches put tokens on the lanes, and when gate and up share their input scale
-// the first GEMM's epilogue applies GeGLU and quantises the down input itself.
+// Small batches put the weights on the 128-lane operand and an expert's few tokens on
+// the column operand, large batches put tokens on the lanes.  When gate and up share
+// their input scale the first GEMM's epilogue applies GeGLU and quantises the down
+// input itself (gemm_moe_narrow.cu, gemm_pair_moe.cu); otherwise both run over group
+// descriptors (moe_prepare_groups_kernel) with a GeGLU kernel between them.
 //
 // `records` != nullptr (expert parallelism): the rows arrive already quantised as 1584-byte
 // records (packed E2M1 + K-ordered scale bytes) written by the ranks that routed them; the
@@ -417,6 +433,7 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
   const ExpertPlan plan = plan_experts(w, table, offsets, n);
   const int form = plan.form;
   const bool pair_first = plan.pair_first, pair_down = plan.pair_down;
+  const int narrow = plan.narrow;
   const int block_n_first = plan.groups.block_n_first, block_n_down = plan.groups.block_n_down;
   const int parts = table->shared_gate_up ? 1 : 2;
   w->mark(1, s);
@@ -449,7 +466,7 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
   w->mark(2, s);
   if (!(stages & kStageFirst)) {
     w->mark(3, s);
-  } else if (pair_first) {
+  } else if (pair_first || narrow) {
     PairMoeParams first{};
     first.map_tokens = w->first_map.map;
     first.map_table = table->maps.as<CUtensorMap>();
@@ -464,10 +481,12 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
       first.records_out = static_cast<uint8_t*>(activation_records);
       if (exported) *exported = true;
     }
-    first.capture_gate_up = w->capture ? w->gate_up.data : nullptr;
-    first.capture_activated = w->capture ? w->activated.data : nullptr;
+    const bool capture = w->capture || (narrow && n <= kCapturedRows);
+    first.capture_gate_up = capture ? w->gate_up.data : nullptr;
+    first.capture_activated = capture ? w->activated.data : nullptr;
     first.error = device_error_word();
-    GW_CUDA_CHECK(launch_pair_moe_gate_up(first, sm_count(), s), "MoE grouped gate/up GEMM on CTA pairs");
+    if (narrow) GW_CUDA_CHECK(launch_moe_narrow_gate_up(narrow, first, sm_count(), s), "MoE grouped gate/up GEMM");
+    else GW_CUDA_CHECK(launch_pair_moe_gate_up(first, sm_count(), s), "MoE grouped gate/up GEMM on CTA pairs");
     w->mark(3, s);
   } else {
     GemmParams first{};
@@ -508,7 +527,7 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
   w->mark(4, s);
   if (!(stages & kStageDown)) {
     // the caller takes the quantised activations from the workspace
-  } else if (pair_down) {
+  } else if (pair_down || narrow) {
     PairMoeParams down{};
     down.map_tokens = w->down_map.map;
     down.map_table = table->maps.as<CUtensorMap>();
@@ -519,7 +538,8 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
     down.out = down_out;
     down.row_dest = row_home;   // rows go to their homes (possibly on other GPUs) instead of down_out
     down.error = device_error_word();
-    GW_CUDA_CHECK(launch_pair_moe_down(down, sm_count(), s), "MoE grouped down GEMM on CTA pairs");
+    if (narrow) GW_CUDA_CHECK(launch_moe_narrow_down(narrow, down, sm_count(), s), "MoE grouped down GEMM");
+    else GW_CUDA_CHECK(launch_pair_moe_down(down, sm_count(), s), "MoE grouped down GEMM on CTA pairs");
   } else {
     GemmParams down{};
     (swap ? down.map_c : down.map_l) = w->down_map.map;
