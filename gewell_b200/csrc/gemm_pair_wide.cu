@@ -69,29 +69,6 @@ __device__ __forceinline__ Tile tile_of(const PairWideParams& p, int w) {
   return {rest / width, group * kGroupTiles + rest % width};
 }
 
-// 8 tokens of one channel per lane (w[i] = tokens 2i, 2i+1) -> 8 channels of one token per lane, inside groups of
-// eight lanes: afterwards lane j of a group holds token j of the group's eight channels.
-__device__ __forceinline__ void transpose_8x8(uint32_t* w, int lane) {
-  {
-    const bool hi = (lane & 4) != 0;
-    const uint32_t a = __shfl_xor_sync(0xffffffffu, hi ? w[0] : w[2], 4), b = __shfl_xor_sync(0xffffffffu, hi ? w[1] : w[3], 4);
-    if (hi) { w[0] = a; w[1] = b; } else { w[2] = a; w[3] = b; }
-  }
-  {
-    const bool hi = (lane & 2) != 0;
-    const uint32_t a = __shfl_xor_sync(0xffffffffu, hi ? w[0] : w[1], 2), b = __shfl_xor_sync(0xffffffffu, hi ? w[2] : w[3], 2);
-    if (hi) { w[0] = a; w[2] = b; } else { w[1] = a; w[3] = b; }
-  }
-  const bool odd = (lane & 1) != 0;
-  const uint32_t give = odd ? 0x5410u : 0x7632u;       // odd lanes give the first token of each pair, even ones the second
-  const uint32_t a = __shfl_xor_sync(0xffffffffu, __byte_perm(w[0], w[1], give), 1);
-  const uint32_t b = __shfl_xor_sync(0xffffffffu, __byte_perm(w[2], w[3], give), 1);
-  w[0] = odd ? __byte_perm(a, w[0], 0x7610u) : __byte_perm(w[0], a, 0x5410u);
-  w[1] = odd ? __byte_perm(a, w[1], 0x7632u) : __byte_perm(w[1], a, 0x7610u);
-  w[2] = odd ? __byte_perm(b, w[2], 0x7610u) : __byte_perm(w[2], b, 0x5410u);
-  w[3] = odd ? __byte_perm(b, w[3], 0x7632u) : __byte_perm(w[3], b, 0x7610u);
-}
-
 template <bool FP8>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
@@ -215,7 +192,8 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       }
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + acc * kAccCols + (uint32_t(quad * 32) << 16);
-      const int c = channel0 + (lane & ~7);                         // n % 8 == 0: eight channels are inside or outside
+      // A lane has one channel of 32 tokens and stores them one by one, the warp 64 contiguous bytes of a token.
+      const bool inside = channel0 + lane < p.n;
       for (int t0 = half * 32; t0 < p.tile_rows; t0 += 64) {
         const int token0 = tile.token * p.tile_rows + t0;
         if (token0 >= p.rows) break;                                // warp-uniform
@@ -223,15 +201,12 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         ptx::tmem_load16(taddr + t0, r);
         ptx::tmem_load16(taddr + t0 + 16, r + 16);
         ptx::tmem_load_wait();
+        bf16* dst = out + size_t(token0) * p.ld_out + channel0 + lane;
+        const int left = inside ? p.rows - token0 : 0;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          uint32_t v[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            v[i] = pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * g + 2 * i]), scale), __fmul_rn(__uint_as_float(r[8 * g + 2 * i + 1]), scale));
-          transpose_8x8(v, lane);
-          const int token = token0 + 8 * g + (lane & 7);
-          if (token < p.rows && c < p.n) *reinterpret_cast<uint4*>(out + size_t(token) * p.ld_out + c) = make_uint4(v[0], v[1], v[2], v[3]);
+        for (int i = 0; i < 32; ++i) {
+          if (i < left) *dst = __float2bfloat16_rn(__fmul_rn(__uint_as_float(r[i]), scale));
+          dst += p.ld_out;
         }
       }
       ptx::tc_fence_before_sync();
