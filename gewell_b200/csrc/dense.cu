@@ -322,8 +322,10 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
       return fail(GW_CUDA_ERROR, "activation descriptor: " + error);
     cache->activations = q.activations;
   }
-  // NVFP4 prefill: the CTA-pair kernel (each CTA stages half of the weight tile) unless disabled
-  if (fp4 && single_box && q.rows >= 256 && !tuning.no_pair) {
+  // NVFP4 prefill: the CTA-pair kernel (each CTA stages half of the weight tile) unless disabled; also where one pair tile holds
+  // all rows (us, with the quantiser, single CTAs / pairs: 130x2816x4096 13.8 / 10.7, 200x5376x16384 24.5 / 19.8, MLP of 200 rows
+  // 117 / 84).
+  if (fp4 && single_box && !tuning.no_pair) {
     if (cache->weight_half != q.weight) {
       if (!encode_tensor_map_2d(&cache->weight_half_map, q.weight, row_bytes, q.n, 128, &error))
         return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
