@@ -31,17 +31,12 @@
 namespace gw {
 namespace {
 
-using moe_work::Unit;
-using moe_work::WorkTable;
-using moe_work::decode_unit;
+using namespace moe_work;
 using pair::report;
 
 constexpr int kHidden = 2816;
 constexpr int kInter = 704;
 constexpr int kScaleWarps = 4, kFirstEpilogueWarp = 2 + kScaleWarps;
-// A tile of 128 tokens keeps sixteen epilogue warps busy; with 64 the wider launch costs more than it gives (MoE layer of
-// 64 tokens, us, 8 / 16 warps: 81.7 / 86.5; 1500 tokens with popular experts on 128-wide tiles 181 / 170).
-template <int TILE> constexpr int kEpilogueWarps = TILE == 128 ? 16 : 8;
 template <int TILE> constexpr int kThreads = 32 * (kFirstEpilogueWarp + kEpilogueWarps<TILE>);
 constexpr int kTmemCols = 512;
 constexpr uint32_t kDescHiSw128 = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);   // SBO 1024 B, version 1, SWIZZLE_128B
@@ -54,32 +49,12 @@ __device__ __forceinline__ uint2 lds64(uint32_t address) {
   asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(address));
   return v;
 }
-template <int THREADS>
-__device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
-// The same with a vote: every epilogue thread learns whether one of them gave up, so that all of them leave together.
-template <int THREADS>
-__device__ __forceinline__ bool epilogue_barrier_any(bool failed) {
-  uint32_t any;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-               : "=r"(any) : "r"(uint32_t(failed)), "n"(THREADS) : "memory");
-  return any != 0;
-}
-
 // The four 32-row words of a lane in a 128-row scale atom, so that the tile's first 32-row group comes first.
 __device__ __forceinline__ uint4 rotated(uint4 v, uint32_t sub) {
   if (sub & 1) v = make_uint4(v.y, v.z, v.w, v.x);
   if (sub & 2) v = make_uint4(v.z, v.w, v.x, v.y);
   return v;
 }
-
-// This CTA's contiguous share of the units.
-struct Range { int begin, end; };
-__device__ __forceinline__ Range my_range(int total) {
-  return {int((long long)(total) * blockIdx.x / gridDim.x), int((long long)(total) * (blockIdx.x + 1) / gridDim.x)};
-}
-// Token columns of a tile that hold rows of the expert, and the MMA's N.
-__device__ __forceinline__ int valid_columns(const Unit& u, int tile_rows) { return min(tile_rows, u.count - u.tile * tile_rows); }
-__device__ __forceinline__ int mma_columns(int valid) { return (valid + 15) & ~15; }
 
 // ===========================================================================
 // gate/up: Y = Xq . [Wgate | Wup]^T per expert, GeGLU, FP4 quantisation of the result
@@ -153,18 +128,10 @@ moe_narrow_gate_up_kernel(const __grid_constant__ PairMoeParams p) {
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   // The kernel in front quantised the rows; the offsets were written before it and the weights by no kernel of this call
   // (see common.cuh).  So the work is found and the first ring of weights is on its way before the wait.
-  moe_work::build_work_table<TILE, 0, 1>(p, table, C::kCTiles);
+  build_work_table<TILE, 0, 1>(p, table, C::kCTiles);
   if (warp != 0) griddep_enter();
-  const Range range = my_range(table->prefix[moe_work::kExperts]);
-  // Units of an expert: its token tiles under one channel tile follow one another, so that the second one finds the
-  // weights in L2.
-  const auto place = [&](int w, Unit& u) {
-    decode_unit(table, w, C::kCTiles, u);
-    const int local = u.tile * C::kCTiles + u.part, tiles = (u.count + TILE - 1) / TILE;
-    u.part = local / tiles;
-    u.tile = local - u.part * tiles;
-    return tiles;
-  };
+  const Range range = my_range(table->prefix[kExperts]);
+  const auto place = [&](int w, Unit& u) { return place_unit<TILE>(table, w, C::kCTiles, u); };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
@@ -502,9 +469,9 @@ moe_narrow_down_kernel(const __grid_constant__ PairMoeParams p) {
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  moe_work::build_work_table<TILE, 2, 2>(p, table, C::kCTiles);       // before the wait, as above
+  build_work_table<TILE, 2, 2>(p, table, C::kCTiles);       // before the wait, as above
   if (warp != 0) griddep_enter();
-  const Range range = my_range(table->prefix[moe_work::kExperts]);
+  const Range range = my_range(table->prefix[kExperts]);
   // A ring position and the parity of its turn.
   struct Cursor {
     int at = 0;

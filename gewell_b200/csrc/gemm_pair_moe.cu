@@ -38,7 +38,8 @@ using moe_work::Unit;
 using moe_work::WorkTable;
 using moe_work::decode_unit;
 
-constexpr int kExperts = 128;
+using moe_work::kExperts;
+
 constexpr int kHidden = 2816;
 constexpr int kInter = 704;
 constexpr int kScaleWarps = 4, kFirstEpilogueWarp = 2 + kScaleWarps;

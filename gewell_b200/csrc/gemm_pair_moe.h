@@ -26,6 +26,7 @@ struct PairMoeParams {
   const int32_t* offsets;          // [129] first sorted row of every expert
   const uint8_t* sf_tokens;        // tiled scales of the token rows, expert e's region at row (first/128 + e) * 128
   uint32_t capacity;               // rows the token buffers hold
+  int32_t kind = kMoeKindNvfp4, fp4 = 1;   // projections that run as this kind get work (see moe_effective_kind)
   // gate/up: packed E2M1 [capacity, 352] + tiled scales (same regions, K = 704), optional BF16 captures
   uint8_t* packed_out;
   uint8_t* scales_out;

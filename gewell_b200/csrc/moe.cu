@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "gemm_moe_narrow.h"
+#include "gemm_moe_plain.h"
 #include "gemm_pair_moe.h"
 #include "gemm_tc.cuh"
 #include "moe_kernels.h"
@@ -26,6 +27,12 @@ constexpr uint32_t kInter = 704;
 constexpr uint32_t kMaxRows = 65536;
 
 bool finite_positive(float v) { return v > 0.0F && std::isfinite(v); }
+
+// The maps of projection i (0 gate, 1 up, 2 down) in its 8- or 16-bit form.
+bool encode_wide_maps(CUtensorMap* slot, int i, const void* data, size_t row_bytes, uint32_t rows, std::string* error) {
+  return encode_tensor_map_2d(slot + 4 + i, data, row_bytes, rows, 128, error) &&
+         (i == 2 || encode_tensor_map_2d(slot + kMoeMapWideGate64 + i, data, row_bytes, rows, 64, error));
+}
 
 struct DeviceBuffer {
   void* data = nullptr;
@@ -48,6 +55,7 @@ struct gw_expert_table {
   std::vector<MoeExpertInfo> host_info;
   std::vector<gw_expert_weights> bound;   // the bindings as given
   bool shared_gate_up = false;   // every expert quantises gate and up inputs with one scale
+  bool all_bf16 = false, all_fp8_shared = false;   // one kind of weights only; FP8: and one input scale for gate and up
   bool all_nvfp4 = false;        // every present projection is NVFP4
   bool any_nvfp4 = false, any_bf16 = false, any_fp8 = false;
   bool w4a16 = false;            // BF16 copies exist
@@ -130,7 +138,7 @@ gw_status gw_moe_expert_table_create(const gw_expert_weights* experts, uint32_t 
     return fail(GW_INVALID_ARGUMENT, "expert table requires 128 host-resident entries");
   std::vector<CUtensorMap> maps(kExperts * kMoeMapsPerExpert);
   std::vector<MoeExpertInfo> info(kExperts);
-  bool shared = true, all_nvfp4 = true, any_nvfp4 = false, any_bf16 = false, any_fp8 = false;
+  bool shared = true, shared_fp8 = true, all_nvfp4 = true, any_nvfp4 = false, any_bf16 = false, any_fp8 = false;
   std::string error;
   const auto address = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
   for (uint32_t e = 0; e < kExperts; ++e) {
@@ -169,7 +177,7 @@ gw_status gw_moe_expert_table_create(const gw_expert_weights* experts, uint32_t 
       } else if (p.storage == GW_STORAGE_BF16) {
         if (!p.bf16 || address(p.bf16) % 16 || p.physical_output != p.output)
           return fail(GW_INVALID_ARGUMENT, "invalid 26B BF16 expert projection binding" + who);
-        if (!encode_tensor_map_2d(slot + 4 + i, p.bf16, size_t(p.input) * 2, p.output, 128, &error))
+        if (!encode_wide_maps(slot, i, p.bf16, size_t(p.input) * 2, p.output, &error))
           return fail(GW_CUDA_ERROR, "expert weight descriptor: " + error);
         any_bf16 = true;
         all_nvfp4 = false;
@@ -179,7 +187,7 @@ gw_status gw_moe_expert_table_create(const gw_expert_weights* experts, uint32_t 
             !std::isfinite(1.0F / p.fp8_input_scale) || !finite_positive(p.fp8_input_scale * p.fp8_weight_scale) ||
             address(p.fp8_channel_scales) % 16)
           return fail(GW_INVALID_ARGUMENT, "invalid 26B FP8 expert projection binding" + who);
-        if (!encode_tensor_map_2d(slot + 4 + i, p.fp8_data, p.input, p.output, 128, &error))
+        if (!encode_wide_maps(slot, i, p.fp8_data, p.input, p.output, &error))
           return fail(GW_CUDA_ERROR, "expert weight descriptor: " + error);
         info[e].alpha[i] = p.fp8_input_scale * p.fp8_weight_scale;
         info[e].inverse_input_scale[i] = 1.0F / p.fp8_input_scale;
@@ -194,6 +202,7 @@ gw_status gw_moe_expert_table_create(const gw_expert_weights* experts, uint32_t 
     if (!no_first && (experts[e].gate.storage != GW_STORAGE_NVFP4_W4A4 || experts[e].up.storage != GW_STORAGE_NVFP4_W4A4 ||
                       experts[e].gate.nvfp4_input_scale != experts[e].up.nvfp4_input_scale))
       shared = false;
+    if (experts[e].gate.storage == GW_STORAGE_FP8_W8A8 && experts[e].gate.fp8_input_scale != experts[e].up.fp8_input_scale) shared_fp8 = false;
   }
   auto* t = new (std::nothrow) gw_expert_table();
   if (!t) return fail(GW_CUDA_ERROR, "out of host memory");
@@ -202,6 +211,8 @@ gw_status gw_moe_expert_table_create(const gw_expert_weights* experts, uint32_t 
   t->any_nvfp4 = any_nvfp4;
   t->any_bf16 = any_bf16;
   t->any_fp8 = any_fp8;
+  t->all_bf16 = any_bf16 && !any_nvfp4 && !any_fp8;
+  t->all_fp8_shared = any_fp8 && !any_nvfp4 && !any_bf16 && shared_fp8;
   t->host_maps = maps;
   t->host_info = info;
   t->bound.assign(experts, experts + kExperts);
@@ -242,8 +253,7 @@ gw_status gw_moe_expert_table_enable_w4a16(gw_expert_table* t, void* stream) {
       const gw_status status = gw_nvfp4_dequantize(p.nvfp4_data, p.nvfp4_scales, p.nvfp4_weight_scale, p.input,
                                                    p.physical_output, copy, s);
       if (status != GW_OK) return status;
-      if (!encode_tensor_map_2d(&t->host_maps[e * kMoeMapsPerExpert + 4 + i], copy, size_t(p.input) * 2, p.physical_output,
-                                128, &error))
+      if (!encode_wide_maps(&t->host_maps[e * kMoeMapsPerExpert], i, copy, size_t(p.input) * 2, p.physical_output, &error))
         return fail(GW_CUDA_ERROR, "expert weight descriptor: " + error);
     }
     t->host_info[e].bf16_copy = 1;
@@ -567,11 +577,60 @@ gw_status run_experts(gw_moe_workspace* w, const void* input, const int32_t* gat
 // Every kind that is present runs its own grouped gate/up and down GEMM over the projections that run as
 // that kind (the others get no work items); all of them write the shared BF16 gate_up and down buffers.
 // GeGLU runs unfused, as in the reference.
+// Tables of one kind (FP8 with one scale for gate and up) run on gemm_moe_plain.cu instead, with 64-wide token tiles up to this
+// many sorted rows and 128-wide ones beyond.  Whole layer, us, 64- / 128-wide / group descriptors and gemm_tc.cu, even experts:
+//   FP8   1 token 25 / 30 / 36    64 120 / 125 / 147    777 162 / 164 / 211    1500 232 / 195 / 247    4096 - / 405 / 473
+//   BF16  1 token 37 / 48 / 43    64 226 / 232 / 261    777 275 / 281 / 329    1500 407 / 333 / 378    4096 - / 630 / 661
+constexpr uint32_t kPlainRows64 = 8 * 512;
 gw_status run_experts_general(gw_moe_workspace* w, const void* input, uint32_t n, const gw_expert_table* table,
                               bool run_nvfp4, bool run_bf16, bool run_fp8, int fp4, cudaStream_t s) {
   const auto* info = table->info.as<MoeExpertInfo>();
   const int32_t* offsets = w->offsets;
   const MoeTuning& tune = w->tuning;
+  // Tables of one kind run without group descriptors, with GeGLU in the gate/up epilogue.
+  const bool fp8_only = run_fp8 && !run_bf16 && !run_nvfp4 && table->all_fp8_shared;
+  const bool bf16_only = run_bf16 && !run_fp8 && !run_nvfp4 && (table->all_bf16 || (table->all_nvfp4 && !fp4));
+  if ((fp8_only || bf16_only) && (tune.form == 'n' || tune.form == 0)) {
+    int tile = n <= kPlainRows64 ? 64 : 128;
+    if (tune.block_n == 64 || tune.block_n == 128) tile = tune.block_n;
+    void* rows_in = fp8_only ? w->fp8_in.data : w->down.data;          // gathered BF16 rows are dead before down rows are written
+    void* rows_act = fp8_only ? w->fp8_act.data : w->activated.data;
+    const size_t width = fp8_only ? 1 : 2;
+    std::string error;
+    w->mark(1, s);
+    if (fp8_only)
+      GW_CUDA_CHECK(launch_moe_quantize_fp8(input, w->sorted_assignments, 8, w->sorted_keys, offsets, info, n, kHidden, 0, 1,
+                                            w->fp8_in.as<uint8_t>(), s),
+                    "MoE gather + FP8 quantise");
+    else
+      GW_CUDA_CHECK(launch_gather_rows(input, w->sorted_assignments, 8, n, kHidden, rows_in, s), "MoE gather");
+    w->mark(2, s);
+    CachedMap& first_map = fp8_only ? w->fp8_first_map : w->bf16_first_map;
+    CachedMap& down_map = fp8_only ? w->fp8_down_map : w->bf16_down_map;
+    if (!first_map.get(rows_in, kHidden * width, n, uint32_t(tile), kHidden * width, &error) ||
+        !down_map.get(rows_act, kInter * width, n, uint32_t(tile), kInter * width, &error))
+      return fail(GW_CUDA_ERROR, "MoE activation descriptor: " + error);
+    PairMoeParams params{};
+    params.map_tokens = first_map.map;
+    params.map_table = table->maps.as<CUtensorMap>();
+    params.experts = info;
+    params.offsets = offsets;
+    params.capacity = n;
+    params.kind = fp8_only ? kMoeKindFp8 : kMoeKindBf16;
+    params.fp4 = fp4;
+    params.packed_out = w->fp8_act.as<uint8_t>();
+    params.capture_gate_up = w->gate_up.data;
+    params.capture_activated = w->activated.data;
+    params.out = w->down.data;
+    params.error = device_error_word();
+    GW_CUDA_CHECK(launch_moe_plain_gate_up(tile, params, sm_count(), s), "MoE grouped gate/up GEMM");
+    w->mark(3, s);
+    w->mark(4, s);
+    params.map_tokens = down_map.map;
+    GW_CUDA_CHECK(launch_moe_plain_down(tile, params, sm_count(), s), "MoE grouped down GEMM");
+    w->mark(5, s);
+    return GW_OK;
+  }
   int form = n <= 8 * 512 ? kMoeFormSwap : kMoeFormDirect;
   if (tune.form == 's') form = kMoeFormSwap;
   if (tune.form == 'd' || tune.form == 'f') form = kMoeFormDirect;

@@ -8,6 +8,8 @@
 //   offsets[e] + #tokens t' < t that chose e,
 // computed here with per-64-token bitmaps and popcounts: kernel 1 routes and
 // builds the bitmaps, kernel 2 scans the per-chunk counts, kernel 3 scatters.
+#include <algorithm>
+
 #include "common.cuh"
 #include "combine.cuh"
 #include "moe_kernels.h"
@@ -843,23 +845,25 @@ __global__ void __launch_bounds__(256)
 moe_quantize_fp8_kernel(const uint4* __restrict__ input, const int32_t* __restrict__ gather_index,
                         uint32_t gather_divisor, const int32_t* __restrict__ sorted_keys,
                         const int32_t* __restrict__ offsets, const MoeExpertInfo* __restrict__ experts, uint32_t n,
-                        uint32_t vectors, int first_projection, uint2* __restrict__ packed) {
+                        Divisor vectors, int first_projection, uint4* __restrict__ packed) {
   griddep_enter();     // results of earlier kernels in the stream are read from here on
-  const size_t index = size_t(blockIdx.x) * 256 + threadIdx.x;
+  const uint32_t index = blockIdx.x * 256 + threadIdx.x;
   const uint32_t part = blockIdx.y;
-  if (index >= size_t(n) * vectors) return;
-  const uint32_t row = index / vectors, v = index % vectors;
-  if (row >= uint32_t(offsets[kExperts])) return;       // n may be an upper bound
+  const uint32_t row = vectors.quotient(index), v = index - row * vectors.value;
+  if (row >= n || row >= uint32_t(offsets[kExperts])) return;       // n may be an upper bound
   const int32_t e = sorted_keys[row];
   const float inverse_scale = experts[e].inverse_input_scale[first_projection + part];
   const size_t source_row = gather_index ? size_t(uint32_t(gather_index[row]) / gather_divisor) : row;
-  float x[8];
-  unpack8(input[source_row * vectors + v], x);
-  uint32_t words[2] = {0, 0};
+  const uint4* source = input + 2 * (source_row * vectors.value + v);
+  const uint4 lo = source[0], hi = source[1];
+  float x[16];
+  unpack8(lo, x);
+  unpack8(hi, x + 8);
+  uint32_t words[4] = {0, 0, 0, 0};
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 16; ++i)
     words[i / 4] |= uint32_t(float_to_e4m3(__fmul_rn(x[i], inverse_scale))) << (8 * (i % 4));
-  packed[(size_t(part) * n + row) * vectors + v] = make_uint2(words[0], words[1]);
+  packed[(size_t(part) * n + row) * vectors.value + v] = make_uint4(words[0], words[1], words[2], words[3]);
 }
 
 // GeGLU alone (moe.cu:439-445) for expert tables without FP4 activations.
@@ -952,12 +956,13 @@ moe_combine_token_kernel(const uint4* __restrict__ down, const int32_t* __restri
 
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ input, const int32_t* __restrict__ index, uint32_t divisor,
-                   uint32_t rows, uint32_t vectors, uint4* __restrict__ output) {
+                   uint32_t rows, Divisor vectors, uint32_t slab_rows, uint4* __restrict__ output) {
   griddep_enter();     // results of earlier kernels in the stream are read from here on
-  const size_t i = size_t(blockIdx.x) * 256 + threadIdx.x;
-  if (i >= size_t(rows) * vectors) return;
-  const uint32_t row = i / vectors, v = i % vectors;
-  output[i] = input[size_t(uint32_t(index[row]) / divisor) * vectors + v];
+  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+  const uint32_t local = vectors.quotient(i), v = i - local * vectors.value, row0 = blockIdx.y * slab_rows;
+  if (local >= min(slab_rows, rows - row0)) return;
+  const size_t row = row0 + size_t(local);
+  output[row * vectors.value + v] = input[size_t(uint32_t(index[row]) / divisor) * vectors.value + v];
 }
 
 // ---------------------------------------------------------------------------
@@ -1394,10 +1399,11 @@ cudaError_t launch_moe_quantize_fp8(const void* input, const int32_t* gather_ind
                                     const int32_t* sorted_keys, const int32_t* offsets, const MoeExpertInfo* experts,
                                     uint32_t n, uint32_t width, int first_projection, int parts, uint8_t* packed,
                                     cudaStream_t stream) {
-  const dim3 grid(blocks_for(size_t(n) * (width / 8)), parts);
+  // sixteen values a thread; 524288 rows of 176 threads stay below the 2^31 of the division
+  const dim3 grid(blocks_for(size_t(n) * (width / 16)), parts);
   launch_pdl(moe_quantize_fp8_kernel, grid, 256, stream, static_cast<const uint4*>(input), gather_index,
-             gather_divisor ? gather_divisor : 1, sorted_keys, offsets, experts, n, width / 8, first_projection,
-             reinterpret_cast<uint2*>(packed));
+             gather_divisor ? gather_divisor : 1, sorted_keys, offsets, experts, n, Divisor::of(width / 16), first_projection,
+             reinterpret_cast<uint4*>(packed));
   return cudaGetLastError();
 }
 
@@ -1422,8 +1428,12 @@ cudaError_t launch_moe_combine(const void* down, const int32_t* inverse, const f
 
 cudaError_t launch_gather_rows(const void* input, const int32_t* index, uint32_t divisor, uint32_t rows,
                                uint32_t width, void* output, cudaStream_t stream) {
-  launch_pdl(gather_rows_kernel, blocks_for(size_t(rows) * (width / 8)), 256, stream, 
-      static_cast<const uint4*>(input), index, divisor, rows, width / 8, static_cast<uint4*>(output));
+  // slabs of rows whose vectors number less than 2^31: a multiply-high division (64-bit divisions took more issue slots than
+  // the copies: 32768 rows of 2816 68 -> 60 us)
+  const uint32_t vectors = width / 8;
+  const uint32_t slab = std::min(rows, std::max(1u, ((1u << 31) - 256) / vectors));
+  launch_pdl(gather_rows_kernel, dim3(blocks_for(size_t(slab) * vectors), (rows + slab - 1) / slab), 256, stream,
+             static_cast<const uint4*>(input), index, divisor, rows, Divisor::of(vectors), slab, static_cast<uint4*>(output));
   return cudaGetLastError();
 }
 

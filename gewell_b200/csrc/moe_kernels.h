@@ -12,8 +12,9 @@ namespace gw {
 
 // Tensor maps per expert in the table: [0..2] gate, up, down as NVFP4 (128-row boxes), [3] down as NVFP4
 // with 64-row boxes, [4..6] gate, up, down in their 8/16-bit form: the FP8 matrix, the BF16 matrix, or
-// the BF16 copy of an NVFP4 matrix (W4A16), [7], [8] gate and up as NVFP4 with 64-row boxes.
-constexpr int kMoeMapsPerExpert = 9, kMoeMapGate64 = 7, kMoeMapUp64 = 8;
+// the BF16 copy of an NVFP4 matrix (W4A16), [7], [8] gate and up as NVFP4 with 64-row boxes, [9], [10] gate and up in their
+// 8/16-bit form with 64-row boxes.
+constexpr int kMoeMapsPerExpert = 11, kMoeMapGate64 = 7, kMoeMapUp64 = 8, kMoeMapWideGate64 = 9, kMoeMapWideUp64 = 10;
 
 // How a projection's GEMM runs: which tcgen05 kind, which operand preparation.
 enum { kMoeKindNvfp4 = 0, kMoeKindBf16 = 1, kMoeKindFp8 = 2, kMoeKindNone = 3 };

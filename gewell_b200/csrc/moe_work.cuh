@@ -22,7 +22,7 @@ struct Unit {
 };
 
 // All threads of the CTA.  units_per_tile work units for every token tile (ROWS rows) of every expert whose projections
-// FIRST .. LAST (0 gate, 1 up, 2 down) are here; rows of an expert that lives on another GPU get no work.
+// FIRST .. LAST (0 gate, 1 up, 2 down) run as the launch's kind; rows of an expert that lives on another GPU get no work.
 template <int ROWS, int FIRST, int LAST>
 __device__ __forceinline__ void build_work_table(const PairMoeParams& p, WorkTable* t, int units_per_tile) {
   __shared__ int32_t warp_totals[4];
@@ -30,7 +30,8 @@ __device__ __forceinline__ void build_work_table(const PairMoeParams& p, WorkTab
   int32_t units = 0;
   if (e < kExperts) {
     int32_t first = p.offsets[e], last = p.offsets[e + 1];
-    const bool here = p.experts[e].storage[FIRST] == GW_STORAGE_NVFP4_W4A4 && p.experts[e].storage[LAST] == GW_STORAGE_NVFP4_W4A4;
+    const bool here = moe_effective_kind(p.experts[e].storage[FIRST], p.fp4) == p.kind &&
+                      moe_effective_kind(p.experts[e].storage[LAST], p.fp4) == p.kind;
     const int32_t capacity = int32_t(p.capacity);
     if (first < 0 || last < first || last > capacity) {
       if (p.error != nullptr) atomicCAS(p.error, 0u, 0x70000100u | uint32_t(e));
@@ -76,6 +77,41 @@ __device__ __forceinline__ void decode_unit(const WorkTable* t, int w, int units
   const int local = w - t->prefix[u.e];
   u.part = local % units_per_tile;
   u.tile = local / units_per_tile;
+}
+
+// The same with the token tiles of an expert fastest, so that the second one under a channel tile finds the weights in L2.
+// Returns the expert's token tiles.
+template <int ROWS>
+__device__ __forceinline__ int place_unit(const WorkTable* t, int w, int units_per_tile, Unit& u) {
+  decode_unit(t, w, units_per_tile, u);
+  const int local = u.tile * units_per_tile + u.part, tiles = (u.count + ROWS - 1) / ROWS;
+  u.part = local / tiles;
+  u.tile = local - u.part * tiles;
+  return tiles;
+}
+
+// This CTA's contiguous share of the units.
+struct Range { int begin, end; };
+__device__ __forceinline__ Range my_range(int total) {
+  return {int((long long)(total) * blockIdx.x / gridDim.x), int((long long)(total) * (blockIdx.x + 1) / gridDim.x)};
+}
+// Token columns of a tile that hold rows of the expert, and the MMA's N.
+__device__ __forceinline__ int valid_columns(const Unit& u, int tile_rows) { return min(tile_rows, u.count - u.tile * tile_rows); }
+__device__ __forceinline__ int mma_columns(int valid) { return (valid + 15) & ~15; }
+
+// ---- epilogue warps of the kernels with an expert's tokens on the columns
+// A tile of 128 tokens keeps sixteen epilogue warps busy; with 64 the wider launch costs more than it gives (MoE layer of
+// 64 tokens, us, 8 / 16 warps: 81.7 / 86.5; 1500 tokens with popular experts on 128-wide tiles 181 / 170).
+template <int TILE> constexpr int kEpilogueWarps = TILE == 128 ? 16 : 8;
+template <int THREADS>
+__device__ __forceinline__ void epilogue_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
+// The same with a vote: every epilogue thread learns whether one of them gave up, so that all of them leave together.
+template <int THREADS>
+__device__ __forceinline__ bool epilogue_barrier_any(bool failed) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(any) : "r"(uint32_t(failed)), "n"(THREADS) : "memory");
+  return any != 0;
 }
 
 }  // namespace gw::moe_work

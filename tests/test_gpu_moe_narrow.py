@@ -1,4 +1,4 @@
-"""The grouped GEMMs with an expert's tokens on the columns (gemm_moe_narrow.cu) where a tile, a scale atom or an MMA
+"""The grouped GEMMs with an expert's tokens on the columns (gemm_moe_narrow.cu, gemm_moe_plain.cu) where a tile, a scale atom or an MMA
 width ends, against the group-descriptor plan (compared with the oracle in test_gpu_moe.py) and against the oracle."""
 import numpy as np
 import pytest
@@ -59,3 +59,56 @@ def test_layer_vs_oracle(gw, experts_shared, monkeypatch, rows, mode, tile):
     assert_gemm_close(bits(ws.activated_capture()), C.bf16_bits(capture["activated"]), "activated capture")
     assert_gemm_close(bits(ws.down_capture()), C.bf16_bits(capture["down"]), "down capture")
     assert_gemm_close(bits(y), expected, f"MoE rows={rows} {mode} tile={tile}")
+
+
+@pytest.fixture(scope="module", params=["fp8", "fp8 channel", "bf16", "w4a16"])
+def plain_table(gw, request):
+    """Tables of one kind (FP8 with one input scale for gate and up), as gemm_moe_plain.cu takes them."""
+    kind = request.param
+    g = torch.Generator(device="cuda").manual_seed(21)
+    triples = []
+    for e in range(E):
+        row = []
+        for n, k in ((I, H), (I, H), (H, I)):
+            w = (torch.randn((n, k), generator=g, device="cuda") * 0.02).bfloat16()
+            scale = (0.004 if k == H else 0.001) * (1 + (e % 4) / 16)
+            if kind == "bf16":
+                row.append(w)
+            elif kind == "w4a16":
+                padded = torch.zeros(((n + 127) // 128 * 128, k), dtype=torch.bfloat16, device="cuda")
+                padded[:n] = w
+                row.append(gw.nvfp4_pack_weights(padded, scale))
+            elif kind == "fp8":
+                amax = float(w.float().abs().max() / 448)
+                row.append(gw.Fp8Weight(gw.fp8_pack_weights(w, amax), 5 * scale, amax))
+            else:
+                rows = (w.float().abs().amax(dim=1) / 448).contiguous()
+                row.append(gw.Fp8Weight(gw.fp8_pack_weights(w, 0.0, rows), 5 * scale, 1.0, (rows * (5 * scale)).contiguous()))
+        triples.append(tuple(row))
+    table = gw.ExpertTable(triples)
+    if kind == "w4a16":
+        table.enable_w4a16()
+    return kind, table
+
+
+@pytest.mark.parametrize("tile", [64, 128])
+@pytest.mark.parametrize("rows,mode", [(1, "hot"), (15, "hot"), (17, "distributed"), (64, "hot"), (65, "hot"), (128, "hot"), (129, "uneven"), (300, "normal")])
+def test_plain_kinds(gw, plain_table, monkeypatch, tile, rows, mode):
+    """Against the group-descriptor plan: same operands and K order, so the captures agree to the GEMM gate; after the
+    second quantisation (FP8) a last-bit difference may become a step, which the gate covers too."""
+    kind, table = plain_table
+    x, scores = bf16_normal((rows, H), 400 + rows).cuda(), make_scores(rows, mode, rows).cuda()
+    one = torch.ones(E, dtype=torch.bfloat16, device="cuda")
+    flags = {"has_fp8": kind.startswith("fp8"), "has_bf16": kind == "bf16", "has_nvfp4": kind == "w4a16", "fp4": False}
+    results = {}
+    for form in ("narrow", "swap"):
+        monkeypatch.setenv("GW_MOE_FORM", form)
+        monkeypatch.setenv("GW_MOE_BLOCK_N", str(tile) if form == "narrow" else "32")
+        ws = gw.MoeWorkspace(max(64, rows), fp8_experts=kind.startswith("fp8"))
+        y = torch.empty((rows, H), dtype=torch.bfloat16, device="cuda")
+        ws.run(x, scores, one, table, y, rows, **flags)
+        torch.cuda.synchronize()
+        assert gw.kernel_error() == 0
+        results[form] = [bits(t) for t in (ws.gate_up_capture(), ws.activated_capture(), ws.down_capture(), y)]
+    for got, expected, what in zip(results["narrow"], results["swap"], ("gate_up", "activated", "down", "layer")):
+        assert_gemm_close(got, expected, f"{kind} {what} rows={rows} {mode} tile={tile}")
