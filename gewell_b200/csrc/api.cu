@@ -325,6 +325,42 @@ gw_status gw::run_nvfp4_plan(gw_nvfp4_plan* plan, const void* input_bf16, const 
   return launch_dense(problem, &plan->descriptors, s);
 }
 
+gw_status gw::run_nvfp4_geglu(gw_nvfp4_plan* gate_plan, gw_nvfp4_plan* down_plan, const gw_projection& gate, const gw_projection& up,
+                              const gw_projection& down, const void* input, void* buffer, void* output, void* scratch,
+                              size_t scratch_capacity, cudaStream_t s, bool* done) {
+  *done = false;
+  const auto usable = [](const gw_projection& p) {
+    return p.storage == GW_STORAGE_NVFP4_W4A4 && p.nvfp4_data && p.nvfp4_scales && aligned(p.nvfp4_data, 16) && aligned(p.nvfp4_scales, 16) &&
+           finite_positive(p.nvfp4_input_scale) && finite_positive(p.nvfp4_weight_scale) && std::isfinite(1.0F / p.nvfp4_input_scale) &&
+           finite_positive(p.nvfp4_input_scale * p.nvfp4_weight_scale);
+  };
+  // what is wrong with the arguments is said by the plans, one after another
+  if (!gate_plan || !down_plan || !usable(gate) || !usable(up) || !usable(down) || gate.nvfp4_input_scale != up.nvfp4_input_scale ||
+      gate.input != up.input || gate.output != up.output || gate.physical_output != up.physical_output || down.input != gate.output ||
+      gate.physical_output != align_up(gate.output, 128) || gate.output % 64 != 0 || gate_plan->input_width != gate.input ||
+      down_plan->rows != gate_plan->rows || down_plan->input_width != down.input || down_plan->output_width != down.physical_output ||
+      !dense_has_geglu(gate_plan->descriptors.tuning, gate_plan->rows) || !dense_has_geglu(down_plan->descriptors.tuning, gate_plan->rows) ||
+      !input || !output || !aligned(input, 16) || !aligned(output, 2) || !aligned(buffer, 256) || !aligned(scratch, 256) ||
+      scratch_capacity < gate_plan->split_offset || down_plan->split_offset > size_t(down_plan->rows) * down.input * sizeof(bf16))
+    return GW_OK;
+  *done = true;
+  const uint32_t rows = gate_plan->rows;
+  auto* packed_in = static_cast<uint8_t*>(scratch);
+  uint8_t* scales_in = packed_in + gate_plan->scale_offset;
+  GW_CUDA_CHECK(launch_nvfp4_quantize(input, rows, gate.input, 1.0F / gate.nvfp4_input_scale, false, packed_in, scales_in, s),
+                "NVFP4 quantize activations");
+  auto* packed = static_cast<uint8_t*>(buffer);
+  uint8_t* scales = packed + down_plan->scale_offset;
+  const GegluProblem q{rows, gate.input, gate.output, {gate.nvfp4_data, up.nvfp4_data}, {gate.nvfp4_scales, up.nvfp4_scales},
+                       {gate.nvfp4_input_scale * gate.nvfp4_weight_scale, up.nvfp4_input_scale * up.nvfp4_weight_scale},
+                       packed_in, scales_in, 1.0F / down.nvfp4_input_scale, packed, scales, device_error_word()};
+  const gw_status status = launch_dense_geglu(q, &gate_plan->descriptors, s);
+  if (status != GW_OK) return status;
+  const DenseProblem problem{GemmKind::nvfp4, rows, down.input, down.physical_output, down.nvfp4_data, down.nvfp4_scales, packed, scales,
+                             down.nvfp4_input_scale * down.nvfp4_weight_scale, nullptr, output, device_error_word()};
+  return launch_dense(problem, &down_plan->descriptors, s);
+}
+
 extern "C" {
 
 // --------------------------------------------------------------------------- FP8

@@ -406,4 +406,48 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
   return GW_OK;
 }
 
+bool dense_has_geglu(const DenseTuning& tuning, uint32_t rows) {
+  return !dense_uses_swap_form(tuning, rows) && dense_block_n(tuning, rows) == 256 && !tuning.no_pair;
+}
+
+gw_status launch_dense_geglu(const GegluProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
+  std::string error;
+  const uint32_t physical = (q.n + 127) / 128 * 128;
+  if (cache->weight_half != q.weight[0]) {
+    if (!encode_tensor_map_2d(&cache->weight_half_map, q.weight[0], q.k / 2, physical, 128, &error))
+      return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
+    cache->weight_half = q.weight[0];
+  }
+  if (cache->up != q.weight[1]) {
+    if (!encode_tensor_map_2d(&cache->up_map, q.weight[1], q.k / 2, physical, 128, &error))
+      return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
+    cache->up = q.weight[1];
+  }
+  if (cache->activations != q.activations) {
+    if (!encode_tensor_map_2d(&cache->activation_map, q.activations, q.k / 2, q.rows, 128, &error))
+      return fail(GW_CUDA_ERROR, "activation descriptor: " + error);
+    cache->activations = q.activations;
+  }
+  PairGemmParams pair{};
+  pair.map_tokens = cache->activation_map;
+  pair.map_weights = cache->weight_half_map;
+  pair.map_up = cache->up_map;
+  pair.sf_tokens = q.activation_scales;
+  pair.token_row_blocks = int32_t((q.rows + 127) / 128);
+  pair.k = int32_t(q.k);
+  pair.rows = int32_t(q.rows);
+  pair.n = int32_t(q.n);
+  pair.l_tiles = int32_t((q.rows + 255) / 256);
+  pair.c_tiles = int32_t(physical / 128);
+  pair.out = q.packed;
+  pair.scales_out = q.scales;
+  pair.alpha = q.alpha[0];
+  pair.alpha_up = q.alpha[1];
+  pair.inverse_scale = q.inverse_scale;
+  for (int i = 0; i < 2; ++i) pair.sf_gate_up[i] = q.weight_scales[i];
+  pair.error = q.error;
+  GW_CUDA_CHECK(launch_gemm_pair_geglu(pair, sm_count(), stream), "NVFP4 CTA-pair gate/up GEMM with GeGLU + quantise");
+  return GW_OK;
+}
+
 }  // namespace gw

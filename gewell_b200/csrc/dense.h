@@ -36,6 +36,8 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   CUtensorMap weight_map{}, activation_map{}, weight_scale_map{};
   const void* weight_half = nullptr;
   CUtensorMap weight_half_map{};     // 128-row box over the weights (CTA-pair kernel: each CTA stages half a tile)
+  const void* up = nullptr;
+  CUtensorMap up_map{};              // the up projection beside `weight_half`, the gate (launch_dense_geglu)
   int token_tile = 0;                // FP8 / BF16 CTA-pair kernel: token columns per tile
   // Split mode: one arrival counter per weight tile, owned by the plan (device memory,
   // zeroed at creation; the kernel leaves every counter at zero again).
@@ -119,6 +121,20 @@ struct StreamBook {
 
 gw_status launch_dense(const DenseProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
+// GeGLU of two projections of the same rows, quantised for the projection that takes it, in one launch.
+struct GegluProblem {
+  uint32_t rows, k, n;                       // n: channels of each projection; their matrices have whole 128-row tiles
+  const uint8_t *weight[2], *weight_scales[2];   // gate, up
+  float alpha[2];
+  const uint8_t *activations, *activation_scales;
+  float inverse_scale;                       // 1 / input scale of the projection that takes the result
+  uint8_t *packed, *scales;                  // [rows, n / 2] and its tiled scales
+  uint32_t* error;
+};
+// Whether a projection of so many rows runs on the kernel that has this form.
+bool dense_has_geglu(const DenseTuning& tuning, uint32_t rows);
+gw_status launch_dense_geglu(const GegluProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
+
 // gw_*_plan_run as a step of a longer call (api.cu): `weights_settled` as in DenseProblem.  The public entry points pass
 // false.
 gw_status run_nvfp4_plan(gw_nvfp4_plan* plan, const void* input, const uint8_t* weight_data, const uint8_t* weight_scales, float input_scale,
@@ -130,6 +146,13 @@ gw_status run_fp8_plan(gw_fp8_plan* plan, const void* input, const uint8_t* weig
 gw_status run_bf16_plan(gw_bf16_plan* plan, const void* input, const void* weight, void* output, void* scratch, size_t scratch_capacity,
                         cudaStream_t stream, bool weights_settled);
 
+// Gate, up, GeGLU and the quantiser of `down` into `buffer` (packed rows and their tiled scales, as in a plan's
+// scratch), then down over them; *done = false when shape, storage or pointers keep the three off that way.  `gate_plan`,
+// `down_plan`: of the gate's and of down's shape; `buffer`: room for BF16 [rows, n], n = down.input.
+gw_status run_nvfp4_geglu(gw_nvfp4_plan* gate_plan, gw_nvfp4_plan* down_plan, const gw_projection& gate, const gw_projection& up,
+                          const gw_projection& down, const void* input, void* buffer, void* output, void* scratch, size_t scratch_capacity,
+                          cudaStream_t stream, bool* done);
+
 // gw_projection_workspace_run on a stream of the caller's choice (projection.cu).
 gw_status projection_workspace_run_on(gw_projection_workspace* workspace, const gw_projection* projection, const void* input, void* output,
                                       cudaStream_t stream, bool weights_settled);
@@ -137,5 +160,8 @@ gw_status projection_workspace_run_on(gw_projection_workspace* workspace, const 
 // way here.
 gw_status projection_workspace_run_geglu(gw_projection_workspace* workspace, const gw_projection& gate, const gw_projection& up,
                                          const void* input, void* product, cudaStream_t stream, bool weights_settled, bool* done);
+// Gate, up, GeGLU and down of a prepared workspace by run_nvfp4_geglu; `buffer`: BF16 [rows, down.input].
+gw_status projection_workspace_run_mlp(gw_projection_workspace* workspace, const gw_projection& gate, const gw_projection& up,
+                                       const gw_projection& down, const void* input, void* buffer, void* output, cudaStream_t stream, bool* done);
 
 }  // namespace gw

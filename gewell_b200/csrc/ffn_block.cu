@@ -613,6 +613,9 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
     gw_status st = projection_workspace_run_geglu(b->projections, w.gate, w.up, b->normalized, b->product, b->side, true,
                                                   &product_done);
     if (st == GW_OK && !product_done) {
+      bool done = false;
+      st = projection_workspace_run_mlp(b->projections, w.gate, w.up, w.down, b->normalized, b->product, b->shared_mlp, b->side, &done);
+      if (st != GW_OK || done) return st;
       st = projection_workspace_run_on(b->projections, &w.gate, b->normalized, b->gate, b->side, true);
       if (st == GW_OK) st = projection_workspace_run_on(b->projections, &w.up, b->normalized, b->up, b->side, true);
       if (st == GW_OK) st = gw_gelu_tanh_multiply_bf16(b->gate, b->up, b->product, uint64_t(rows) * kSharedMlp, b->side);

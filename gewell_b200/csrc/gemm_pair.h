@@ -20,6 +20,12 @@ struct PairGemmParams {
   void* out;                       // BF16 [rows, ld_out]
   int64_t ld_out;
   float alpha;
+  // launch_gemm_pair_geglu: map_weights and the scales below are the gate's, map_up the up projection's; n: channels of each;
+  // out is the quantised GeGLU of the two, packed E2M1 [rows, n / 2], and scales_out its tiled scales
+  CUtensorMap map_up;
+  const uint8_t* sf_gate_up[2];
+  float alpha_up, inverse_scale;   // inverse_scale: 1 / input scale of the projection that takes the result
+  uint8_t* scales_out;
   uint32_t* error;                 // device error word (0 = fine)
   long long* profile;              // optional [grid][8] cycle counters (debug aid)
 };
@@ -31,5 +37,7 @@ struct PairGemmParams {
 void set_pair_profile_buffer(long long* device_buffer);
 
 cudaError_t launch_gemm_pair(const PairGemmParams& params, int sm_count, cudaStream_t stream);
+// Gate, up, GeGLU and the FP4 quantiser of the next projection in one launch.  n is a multiple of 32, c_tiles counts 128 channels.
+cudaError_t launch_gemm_pair_geglu(const PairGemmParams& params, int sm_count, cudaStream_t stream);
 
 }  // namespace gw

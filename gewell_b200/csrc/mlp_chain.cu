@@ -7,6 +7,8 @@
 //   gate + up   one joined GEMM over [gate | up] when the loader laid the two matrices out back to
 //               back: NVFP4 with FP4 activations (contiguous rows and scale tiles, equal globals),
 //               FP8 with per-channel scales, or BF16; otherwise two separate projections
+//               (NVFP4 from 129 rows on: gate, up, GeGLU and the down projection's quantiser are one launch of the CTA-pair
+//               kernel, joined or not)
 //   GeGLU       fused into the activation quantiser of the down projection when that one runs
 //               quantised on a joined [rows, gate | up] tensor; an element-wise kernel otherwise
 //               (small row counts, where that is the faster way: gate, up and GeGLU are one launch of the
@@ -321,6 +323,16 @@ gw_status gw_mlp_chain_run(gw_mlp_chain* c, const gw_projection* gate, const gw_
   if (status = c->book.stream(*gate, up, input_bf16, product_bf16, fp4, false, s, &paired); status != GW_OK) return status;
   if (paired)                    // one launch: gate, up and GeGLU
     return run_linear(c->book, *down, product_bf16, output_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
+  if (fp4) {                     // prefill on NVFP4: GeGLU and the down projection's quantiser in the gate/up epilogue
+    const auto nvfp4_plan = [&](uint32_t k, uint32_t n) {
+      const auto found = c->book.plans.find(Key{kNvfp4, k, n});
+      return found == c->book.plans.end() ? nullptr : found->second.nvfp4;
+    };
+    bool done = false;
+    status = run_nvfp4_geglu(nvfp4_plan(h, m), nvfp4_plan(m, h), *gate, *up, *down, input_bf16, product_bf16, output_bf16,
+                             c->book.scratch.data, c->book.scratch.bytes, s, &done);
+    if (status != GW_OK || done) return status;
+  }
   bool interleaved = true;       // gate_up holds [rows, gate | up]; otherwise gate rows, then up rows
   if ((nvfp4_joined(*gate, *up) && fp4) || fp8_joined(*gate, *up) || bf16_joined(*gate, *up)) {
     status = run_linear(c->book, widened(*gate, 2 * m), input_bf16, gate_out, fp4, GW_TRANSFORM_IDENTITY, s, true);

@@ -363,6 +363,17 @@ gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_proje
   return GW_OK;
 }
 
+gw_status projection_workspace_run_mlp(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up,
+                                       const gw_projection& down, const void* input, void* buffer, void* output, cudaStream_t stream, bool* done) {
+  *done = false;
+  if (w->rows == 0 || !w->fp4 || down.output != down.physical_output) return GW_OK;
+  const auto plan = [&](const gw_projection& p) {
+    const auto found = w->plans.find(Shape{kPlanNvfp4, p.input, p.physical_output});
+    return found == w->plans.end() ? nullptr : found->second.nvfp4;
+  };
+  return run_nvfp4_geglu(plan(gate), plan(down), gate, up, down, input, buffer, output, w->scratch.data, w->scratch.bytes, stream, done);
+}
+
 gw_status projection_workspace_run_geglu(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up, const void* input,
                                          void* product, cudaStream_t stream, bool weights_settled, bool* done) {
   *done = false;

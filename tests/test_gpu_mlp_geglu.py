@@ -1,0 +1,49 @@
+"""Gate, up and GeGLU in one prefill launch of the MLP chain, where a tile of tokens or channels ends, against the chain of
+separate launches (GW_DENSE_NO_PAIR keeps the pair kernels out), which test_gpu_mlp_chain.py compares with the oracle."""
+import pytest
+import torch
+
+from tests.gpu_helpers import assert_gemm_close, bf16_normal, bits
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gw():
+    import gewell_b200
+    return gewell_b200
+
+
+def projections(gw, storage, hidden, mlp, joined):
+    both = (bf16_normal((2 * mlp, hidden), 1) * 0.02).cuda()
+    down = (bf16_normal((hidden, mlp), 2) * 0.02).cuda()
+    packed = gw.nvfp4_pack_weights(both, 6 / 2688)
+    if joined:
+        split = gw.nvfp4_scale_storage_bytes(mlp, hidden)
+        gate = gw.Nvfp4Weight(packed.data[:mlp], packed.scales[:split], packed.input_scale, packed.weight_scale)
+        up = gw.Nvfp4Weight(packed.data[mlp:], packed.scales[split:], packed.input_scale, packed.weight_scale)
+    else:
+        gate, up = gw.nvfp4_pack_weights(both[:mlp].contiguous(), 6 / 2688), gw.nvfp4_pack_weights(both[mlp:].contiguous(), 6 / 2688)
+    return gate, up, gw.nvfp4_pack_weights(down, 16 / 2688)
+
+
+@pytest.mark.parametrize("storage,joined", [("nvfp4", True), ("nvfp4", False)])
+@pytest.mark.parametrize("rows,hidden,mlp", [(129, 128, 128), (255, 256, 384), (256, 640, 128), (257, 384, 1152), (513, 1024, 256), (300, 2816, 2176)])
+def test_fused_equals_separate_launches(gw, monkeypatch, storage, joined, rows, hidden, mlp):
+    from gewell_b200 import _lib
+    weights = projections(gw, storage, hidden, mlp, joined)
+    bound = [gw.make_projection(w, i, o) for w, i, o in zip(weights, (hidden, hidden, mlp), (mlp, mlp, hidden))]
+    x = bf16_normal((rows, hidden), rows).cuda()
+    results = []
+    for apart in (False, True):
+        if apart:
+            monkeypatch.setenv("GW_DENSE_NO_PAIR", "1")
+        else:
+            monkeypatch.delenv("GW_DENSE_NO_PAIR", raising=False)
+        chain = gw.MlpChain(hidden, mlp, rows, _lib.POLICY_ALWAYS)
+        chain.prepare(rows)
+        y = chain.run(*bound, x, _lib.PHASE_PREFILL)
+        torch.cuda.synchronize()
+        assert gw.kernel_error() == 0
+        results.append(bits(y))
+    assert_gemm_close(results[0], results[1], f"{storage} {rows}x{hidden}->{mlp}")
