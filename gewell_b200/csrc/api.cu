@@ -575,6 +575,62 @@ gw_status gw::run_bf16_plan(gw_bf16_plan* plan, const void* input_bf16, const vo
   return launch_dense(problem, &plan->descriptors, s);
 }
 
+namespace {
+// An FP8 projection whose arguments are in order, for the entry points that leave it to the plans to say what is not.
+bool usable_fp8(const gw_projection& p) {
+  return p.storage == GW_STORAGE_FP8_W8A8 && p.fp8_data && aligned(p.fp8_data, 16) && aligned(p.fp8_channel_scales, 16) &&
+         finite_positive(p.fp8_input_scale) && finite_positive(p.fp8_weight_scale) && std::isfinite(1.0F / p.fp8_input_scale) &&
+         finite_positive(p.fp8_input_scale * p.fp8_weight_scale);
+}
+bool same_shape(const gw_projection& gate, const gw_projection& up) {
+  return gate.storage == up.storage && gate.input == up.input && gate.output == up.output && gate.physical_output == gate.output &&
+         up.physical_output == up.output && gate.output % 64 == 0;
+}
+}  // namespace
+
+gw_status gw::run_fp8_geglu(gw_fp8_plan* gate_plan, const gw_projection& gate, const gw_projection& up, const gw_projection& down,
+                            const void* input, void* product, void* scratch, size_t scratch_capacity, cudaStream_t s, bool* packed, bool* done) {
+  *done = false;
+  if (!gate_plan || !same_shape(gate, up) || !usable_fp8(gate) || !usable_fp8(up) || gate.fp8_input_scale != up.fp8_input_scale ||
+      gate_plan->input_width != gate.input || gate_plan->output_width != gate.output ||
+      !dense_has_geglu_wide(gate_plan->descriptors.tuning, gate_plan->rows) || !input || !aligned(input, 2) || !product ||
+      !aligned(product, 16) || !scratch || !aligned(scratch, 256) || scratch_capacity < gate_plan->split_offset)
+    return GW_OK;
+  *done = true;
+  *packed = usable_fp8(down);
+  const uint32_t rows = gate_plan->rows;
+  GW_CUDA_CHECK(launch_fp8_quantize(input, rows, gate.input, 1.0F / gate.fp8_input_scale, false, static_cast<uint8_t*>(scratch), s),
+                "FP8 quantize activations");
+  const WideGegluProblem q{GemmKind::fp8, rows, gate.input, gate.output, scratch, {gate.fp8_data, up.fp8_data},
+                           {gate.fp8_input_scale * gate.fp8_weight_scale, up.fp8_input_scale * up.fp8_weight_scale},
+                           {gate.fp8_channel_scales, up.fp8_channel_scales}, *packed ? 1.0F / down.fp8_input_scale : 0.0F, product,
+                           device_error_word()};
+  return launch_dense_geglu_wide(q, &gate_plan->descriptors, s);
+}
+
+gw_status gw::run_bf16_geglu(gw_bf16_plan* gate_plan, const gw_projection& gate, const gw_projection& up, const gw_projection& down,
+                             const void* input, void* product, cudaStream_t s, bool* packed, bool* done) {
+  *done = false;
+  if (!gate_plan || !same_shape(gate, up) || gate.storage != GW_STORAGE_BF16 || !gate.bf16 || !up.bf16 || !aligned(gate.bf16, 16) ||
+      !aligned(up.bf16, 16) || gate_plan->input_width != gate.input || gate_plan->output_width != gate.output ||
+      !dense_has_geglu_wide(gate_plan->descriptors.tuning, gate_plan->rows) || !input || !aligned(input, 16) || !product || !aligned(product, 16))
+    return GW_OK;
+  *done = true;
+  *packed = usable_fp8(down);
+  const WideGegluProblem q{GemmKind::bf16, gate_plan->rows, gate.input, gate.output, input, {gate.bf16, up.bf16}, {1.0F, 1.0F}, {nullptr, nullptr},
+                           *packed ? 1.0F / down.fp8_input_scale : 0.0F, product, device_error_word()};
+  return launch_dense_geglu_wide(q, &gate_plan->descriptors, s);
+}
+
+gw_status gw::run_fp8_plan_packed(gw_fp8_plan* plan, const void* packed, const gw_projection& p, void* output, cudaStream_t s) {
+  if (!plan || !usable_fp8(p) || !packed || !output || !aligned(packed, 16) || !aligned(output, 16) || (plan->channel_scales && !p.fp8_channel_scales))
+    return fail(GW_INVALID_ARGUMENT, "FP8 run requires a plan, valid aligned device buffers and finite positive global scales");
+  const DenseProblem problem{GemmKind::fp8, plan->rows, plan->input_width, plan->output_width, p.fp8_data, nullptr, packed, nullptr,
+                             p.fp8_input_scale * p.fp8_weight_scale, plan->channel_scales ? p.fp8_channel_scales : nullptr, output,
+                             device_error_word()};
+  return launch_dense(problem, &plan->descriptors, s);
+}
+
 extern "C" {
 
 // --------------------------------------------------------------------------- weight QDQ

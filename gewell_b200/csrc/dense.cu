@@ -450,4 +450,43 @@ gw_status launch_dense_geglu(const GegluProblem& q, DenseDescriptors* cache, cud
   return GW_OK;
 }
 
+bool dense_has_geglu_wide(const DenseTuning& tuning, uint32_t rows) {
+  return !dense_uses_swap_form(tuning, rows) && tuning.form == 0 && tuning.block_n == 0 && !tuning.no_pair;
+}
+
+gw_status launch_dense_geglu_wide(const WideGegluProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
+  std::string error;
+  const uint64_t row_bytes = q.kind == GemmKind::bf16 ? uint64_t(2) * q.k : q.k;
+  if (cache->geglu_tile == 0) cache->geglu_tile = pair_wide_tile_rows(q.rows, 2 * q.n, sm_count());
+  const void* from[3] = {q.activations, q.weight[0], q.weight[1]};
+  for (int i = 0; i < 3; ++i)
+    if (cache->geglu_from[i] != from[i]) {
+      if (!encode_tensor_map_2d(&cache->geglu_maps[i], from[i], row_bytes, i == 0 ? q.rows : q.n, i == 0 ? uint32_t(cache->geglu_tile / 2) : 64, &error))
+        return fail(GW_CUDA_ERROR, "gate/up descriptor: " + error);
+      cache->geglu_from[i] = from[i];
+    }
+  PairWideParams pair{};
+  pair.map_tokens = cache->geglu_maps[0];
+  pair.map_weights = cache->geglu_maps[1];
+  pair.map_up = cache->geglu_maps[2];
+  pair.k_stages = int32_t((row_bytes + 127) / 128);
+  pair.last_kb = int32_t((row_bytes - uint64_t(pair.k_stages - 1) * 128 + 31) / 32);
+  pair.rows = int32_t(q.rows);
+  pair.n = int32_t(q.n);
+  pair.channel_tiles = int32_t((q.n + 127) / 128);
+  pair.token_tiles = int32_t((q.rows + cache->geglu_tile - 1) / cache->geglu_tile);
+  pair.tile_rows = cache->geglu_tile;
+  pair.out = q.output;
+  pair.ld_out = q.n;
+  pair.alpha = q.alpha[0];
+  pair.alpha_up = q.alpha[1];
+  pair.channel_alpha = q.channel_alpha[0];
+  pair.channel_alpha_up = q.channel_alpha[1];
+  pair.inverse_scale = q.inverse_scale;
+  pair.error = q.error;
+  GW_CUDA_CHECK(launch_gemm_pair_wide_geglu(q.kind == GemmKind::fp8, q.inverse_scale != 0.0F, pair, sm_count(), stream),
+                "CTA-pair gate/up GEMM with GeGLU");
+  return GW_OK;
+}
+
 }  // namespace gw

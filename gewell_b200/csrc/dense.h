@@ -39,6 +39,10 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   const void* up = nullptr;
   CUtensorMap up_map{};              // the up projection beside `weight_half`, the gate (launch_dense_geglu)
   int token_tile = 0;                // FP8 / BF16 CTA-pair kernel: token columns per tile
+  // its GeGLU form (launch_dense_geglu_wide): token columns per tile, the activations, gate and up in 64-row boxes
+  int geglu_tile = 0;
+  const void* geglu_from[3] = {};
+  CUtensorMap geglu_maps[3]{};
   // Split mode: one arrival counter per weight tile, owned by the plan (device memory,
   // zeroed at creation; the kernel leaves every counter at zero again).
   int32_t* split_counters = nullptr;
@@ -135,6 +139,20 @@ struct GegluProblem {
 bool dense_has_geglu(const DenseTuning& tuning, uint32_t rows);
 gw_status launch_dense_geglu(const GegluProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
+// The same of FP8 or BF16 projections; the result is E4M3 (inverse_scale != 0) or BF16.
+struct WideGegluProblem {
+  GemmKind kind;
+  uint32_t rows, k, n;
+  const void *activations, *weight[2];       // gate, up
+  float alpha[2];
+  const float* channel_alpha[2];
+  float inverse_scale;                       // 1 / input scale of the FP8 projection that takes the result, or 0
+  void* output;                              // [rows, n]
+  uint32_t* error;
+};
+bool dense_has_geglu_wide(const DenseTuning& tuning, uint32_t rows);
+gw_status launch_dense_geglu_wide(const WideGegluProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
+
 // gw_*_plan_run as a step of a longer call (api.cu): `weights_settled` as in DenseProblem.  The public entry points pass
 // false.
 gw_status run_nvfp4_plan(gw_nvfp4_plan* plan, const void* input, const uint8_t* weight_data, const uint8_t* weight_scales, float input_scale,
@@ -152,6 +170,15 @@ gw_status run_bf16_plan(gw_bf16_plan* plan, const void* input, const void* weigh
 gw_status run_nvfp4_geglu(gw_nvfp4_plan* gate_plan, gw_nvfp4_plan* down_plan, const gw_projection& gate, const gw_projection& up,
                           const gw_projection& down, const void* input, void* buffer, void* output, void* scratch, size_t scratch_capacity,
                           cudaStream_t stream, bool* done);
+
+// GeGLU of FP8 or BF16 gate and up projections of a prefill pass into `product`: E4M3 for `down_plan` and `down` where that is FP8, and
+// *packed = true, else BF16.  *done = false when shape, storage or pointers keep them off that way.  run_fp8_plan_packed runs
+// down over the former.
+gw_status run_fp8_geglu(gw_fp8_plan* gate_plan, const gw_projection& gate, const gw_projection& up, const gw_projection& down, const void* input,
+                        void* product, void* scratch, size_t scratch_capacity, cudaStream_t stream, bool* packed, bool* done);
+gw_status run_bf16_geglu(gw_bf16_plan* gate_plan, const gw_projection& gate, const gw_projection& up, const gw_projection& down,
+                         const void* input, void* product, cudaStream_t stream, bool* packed, bool* done);
+gw_status run_fp8_plan_packed(gw_fp8_plan* plan, const void* packed, const gw_projection& p, void* output, cudaStream_t stream);
 
 // gw_projection_workspace_run on a stream of the caller's choice (projection.cu).
 gw_status projection_workspace_run_on(gw_projection_workspace* workspace, const gw_projection* projection, const void* input, void* output,

@@ -11,6 +11,9 @@
 //
 // Roles per CTA: warp 0 = producer (one lane), warp 1 = MMA issuer (one lane, only in the pair's leader), warps
 // 4..11 = epilogue.
+// The GeGLU form computes gate and up of 64 channels per CTA and writes their GeGLU, as E4M3 where an FP8 projection takes it:
+// BF16 [rows, gate | up] is neither written nor read.  MLP, us, before / after: FP8 5376 -> 21504 276 rows 139 / 134, 2048 673 /
+// 607, 2560 -> 7040 1923 rows 123 / 105; BF16 5376 -> 21504 1024 rows 626 / 591.
 // Cross-CTA protocol (barriers at the same offsets in both CTAs):
 //   full[s]   in the leader; the operand tiles of both CTAs complete on it (the peer's copies into the peer's own
 //             shared memory may count there before the leader expects them: only its arrival closes the phase)
@@ -33,8 +36,12 @@ constexpr int kWgtBytes = 128 * 128;
 constexpr int kEpilogueWarps = 8, kFirstEpilogueWarp = 4;
 constexpr int kThreads = 32 * (kFirstEpilogueWarp + kEpilogueWarps);
 constexpr int kAccCols = 256, kTmemCols = 512;
-constexpr int kRingBytes = 221 * 1024;
-constexpr int kSmemBytes = kRingBytes + 1024;
+// The GeGLU form's epilogue transposes through shared memory: each half of its warps 32 tokens of [gate 64 | up 64] BF16 values,
+// 16 bytes more against bank conflicts.
+constexpr int kPitch = 256 + 16, kStagingBytes = 32 * kPitch;
+constexpr int ring_bytes(bool geglu) { return 221 * 1024 - (geglu ? 2 * kStagingBytes : 0); }
+constexpr int kSmemBytes = 221 * 1024 + 1024;
+enum class WideOut { store, geglu, geglu_fp8 };
 constexpr int kGroupTiles = 8;                     // token tiles that are walked together
 constexpr uint32_t kDescHiSw128 = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);   // SBO 1024 B, version 1, SWIZZLE_128B
 
@@ -69,9 +76,19 @@ __device__ __forceinline__ Tile tile_of(const PairWideParams& p, int w) {
   return {rest / width, group * kGroupTiles + rest % width};
 }
 
-template <bool FP8>
+// barrier of one half of the epilogue warps with a vote: whether one of its threads gave up, so that all of them leave together
+__device__ __forceinline__ bool half_barrier_any(int half, bool failed) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(any) : "r"(uint32_t(failed)), "r"(1 + half) : "memory");
+  return any != 0;
+}
+__device__ __forceinline__ void half_barrier(int half) { asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory"); }
+
+template <bool FP8, WideOut OUT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
+  constexpr bool kGeglu = OUT != WideOut::store;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_full_bar[2], acc_empty_bar[2];
   __shared__ uint32_t tmem_slot;
@@ -115,7 +132,8 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       const uint32_t leader_full = leader_address(full_bar);
       for (int w = pair; w < total_work && !abort_flag; w += pairs) {
         const Tile tile = tile_of(p, w);
-        const int weight_row = (tile.channel * 2 + int(rank)) * 128;
+        // GeGLU: 64 gate rows, then the up rows of the same channels
+        const int weight_row = (tile.channel * 2 + int(rank)) * (kGeglu ? 64 : 128);
         const int token_row = tile.token * p.tile_rows + int(rank) * token_half;
         bool failed = false;
         for (int ks = 0; ks < p.k_stages; ++ks) {
@@ -127,6 +145,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
           uint8_t* base = smem + stage * p.stage_bytes;
           if (rank == 0) ptx::mbar_expect_tx(full_bar + stage, bytes);       // rows beyond a matrix arrive as zeros
           tma_load_pair(base, &p.map_weights, ks * 128, weight_row, leader_full + stage * 8);
+          if constexpr (kGeglu) tma_load_pair(base + kWgtBytes / 2, &p.map_up, ks * 128, weight_row, leader_full + stage * 8);
           tma_load_pair(base + kWgtBytes, &p.map_tokens, ks * 128, token_row, leader_full + stage * 8);
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
@@ -174,6 +193,74 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       }
     }
     __syncwarp();
+  } else if (kGeglu && warp >= kFirstEpilogueWarp) {
+    // ------------------------------------------------------------------ epilogue: GeGLU (own 64 channels x tile_rows tokens)
+    // The gate lanes (0..63) and the up lanes (64..127) of a channel belong to different warps: the scaled accumulators, rounded
+    // to BF16, which is what GeGLU consumes, go through shared memory; then a thread has sixteen channels of a token.
+    const int quad = warp % 4;
+    const int half = (warp - kFirstEpilogueWarp) / 4;            // takes every other 32-token chunk
+    const uint32_t leader_acc_empty = leader_address(acc_empty_bar);
+    uint8_t* staging = smem + ring_bytes(true) + half * kStagingBytes;
+    const int tid = (int(threadIdx.x) - 32 * kFirstEpilogueWarp) % 128;
+    const float* channel_alpha = quad < 2 ? p.channel_alpha : p.channel_alpha_up;
+    int turn = 0;
+    for (int w = pair; w < total_work; w += pairs, ++turn) {
+      const int acc = turn & 1;
+      const Tile tile = tile_of(p, w);
+      const int channel0 = (tile.channel * 2 + int(rank)) * 64;
+      const int mine = channel0 + quad % 2 * 32 + lane;
+      const float scale = channel_alpha == nullptr ? (quad < 2 ? p.alpha : p.alpha_up) : mine < p.n ? __ldg(channel_alpha + mine) : 0.0F;
+      const bool arrived = ptx::mbar_wait_warp(acc_full_bar + acc, uint32_t(turn >> 1) & 1u);
+      if (!arrived) report(p.error, 0x4b000000u | (blockIdx.x << 8) | acc, &abort_flag);
+      if (half_barrier_any(half, !arrived)) break;
+      ptx::tc_fence_after_sync();
+      const uint32_t taddr = tmem_base + acc * kAccCols + (uint32_t(quad * 32) << 16);
+      for (int t0 = half * 32; t0 < p.tile_rows; t0 += 64) {
+        const int token0 = tile.token * p.tile_rows + t0;
+        if (token0 >= p.rows) break;                                // the whole half
+        uint32_t r[32];
+        ptx::tmem_load16(taddr + t0, r);
+        ptx::tmem_load16(taddr + t0 + 16, r + 16);
+        ptx::tmem_load_wait();
+        if (t0 != half * 32) half_barrier(half);                    // the chunk before has been read
+        uint16_t* put = reinterpret_cast<uint16_t*>(staging) + quad * 32 + lane;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const bf16 v = __float2bfloat16_rn(__fmul_rn(__uint_as_float(r[i]), scale));
+          put[i * (kPitch / 2)] = *reinterpret_cast<const uint16_t*>(&v);
+        }
+        half_barrier(half);
+        const int token = token0 + tid / 4, channel = channel0 + tid % 4 * 16;
+        if (token >= p.rows || channel >= p.n) continue;
+        const uint32_t from = ptx::smem_u32(staging) + uint32_t(tid / 4) * kPitch + uint32_t(tid % 4) * 32;
+        uint32_t words[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 g = ptx::lds128(from + 16 * h), u = ptx::lds128(from + 128 + 16 * h);
+          const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float lo = gelu_tanh_multiply_bf16(__uint_as_float(gw[i] << 16), __uint_as_float(uw[i] << 16));
+            const float hi = gelu_tanh_multiply_bf16(__uint_as_float(gw[i] & 0xFFFF0000u), __uint_as_float(uw[i] & 0xFFFF0000u));
+            if constexpr (OUT == WideOut::geglu_fp8)
+              words[4 * h + i] = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(lo, p.inverse_scale), __fmul_rn(hi, p.inverse_scale)), __NV_SATFINITE, __NV_E4M3);
+            else
+              words[4 * h + i] = (__float_as_uint(lo) >> 16) | (__float_as_uint(hi) & 0xFFFF0000u);
+          }
+        }
+        if constexpr (OUT == WideOut::geglu_fp8) {
+          *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.out) + size_t(token) * p.ld_out + channel) =
+              make_uint4(words[0] | words[1] << 16, words[2] | words[3] << 16, words[4] | words[5] << 16, words[6] | words[7] << 16);
+        } else {
+          uint4* dst = reinterpret_cast<uint4*>(static_cast<bf16*>(p.out) + size_t(token) * p.ld_out + channel);
+          dst[0] = make_uint4(words[0], words[1], words[2], words[3]);
+          dst[1] = make_uint4(words[4], words[5], words[6], words[7]);
+        }
+      }
+      ptx::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) arrive_cluster(leader_acc_empty + acc * 8);
+    }
   } else if (warp >= kFirstEpilogueWarp) {
     // ------------------------------------------------------------------ epilogue (own 128 channels x tile_rows tokens)
     const int quad = warp % 4;
@@ -224,12 +311,12 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
   }
 }
 
-template <bool FP8>
+template <bool FP8, WideOut OUT>
 cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStream_t stream) {
   static bool configured_on[kMaxDeviceSlots] = {};   // the attribute is per GPU
   bool& configured = configured_on[current_device_slot()];
   if (!configured) {
-    const cudaError_t status = cudaFuncSetAttribute(gemm_pair_wide_kernel<FP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    const cudaError_t status = cudaFuncSetAttribute(gemm_pair_wide_kernel<FP8, OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (status != cudaSuccess) return status;
     configured = true;
   }
@@ -250,7 +337,7 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
   config.attrs = attributes;
   config.numAttrs = 2;
   note_launch();
-  return cudaLaunchKernelEx(&config, gemm_pair_wide_kernel<FP8>, params);
+  return cudaLaunchKernelEx(&config, gemm_pair_wide_kernel<FP8, OUT>, params);
 }
 
 }  // namespace
@@ -269,12 +356,26 @@ int pair_wide_tile_rows(uint32_t rows, uint32_t n, int sm_count) {
   return best;
 }
 
-cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& given, int sm_count, cudaStream_t stream) {
+namespace {
+PairWideParams with_ring(const PairWideParams& given, bool geglu) {
   PairWideParams params = given;
   params.stage_bytes = kWgtBytes + given.tile_rows * 64;
-  params.stages = kRingBytes / params.stage_bytes < kMaxStages ? kRingBytes / params.stage_bytes : kMaxStages;
+  const int fit = ring_bytes(geglu) / params.stage_bytes;
+  params.stages = fit < kMaxStages ? fit : kMaxStages;
+  return params;
+}
+}  // namespace
 
-  return fp8 ? launch_instance<true>(params, sm_count, stream) : launch_instance<false>(params, sm_count, stream);
+cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& given, int sm_count, cudaStream_t stream) {
+  const PairWideParams params = with_ring(given, false);
+  return fp8 ? launch_instance<true, WideOut::store>(params, sm_count, stream) : launch_instance<false, WideOut::store>(params, sm_count, stream);
+}
+
+cudaError_t launch_gemm_pair_wide_geglu(bool fp8, bool quantise, const PairWideParams& given, int sm_count, cudaStream_t stream) {
+  const PairWideParams params = with_ring(given, true);
+  if (quantise)
+    return fp8 ? launch_instance<true, WideOut::geglu_fp8>(params, sm_count, stream) : launch_instance<false, WideOut::geglu_fp8>(params, sm_count, stream);
+  return fp8 ? launch_instance<true, WideOut::geglu>(params, sm_count, stream) : launch_instance<false, WideOut::geglu>(params, sm_count, stream);
 }
 
 }  // namespace gw

@@ -21,11 +21,19 @@ struct PairWideParams {
   int64_t ld_out;
   float alpha;
   const float* channel_alpha;      // optional multiplier per output channel instead of alpha
+  // launch_gemm_pair_wide_geglu: map_weights (box 64 rows) and the multipliers above are the gate's, these the up projection's
+  CUtensorMap map_up;
+  float alpha_up, inverse_scale;   // inverse_scale: 1 / input scale of the FP8 projection that takes the result
+  const float* channel_alpha_up;
   uint32_t* error;
 };
 
 // Tokens per tile for this shape: the number whose whole waves of pair tiles take least.
 int pair_wide_tile_rows(uint32_t rows, uint32_t n, int sm_count);
+
+// GeGLU of two projections with n channels each, as BF16 [rows, n] or (`quantise`) E4M3 [rows, n].  n is a multiple of 64,
+// channel_tiles counts 128 channels.
+cudaError_t launch_gemm_pair_wide_geglu(bool fp8, bool quantise, const PairWideParams& params, int sm_count, cudaStream_t stream);
 
 cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& params, int sm_count, cudaStream_t stream);
 

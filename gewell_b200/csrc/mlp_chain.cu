@@ -8,7 +8,7 @@
 //               back: NVFP4 with FP4 activations (contiguous rows and scale tiles, equal globals),
 //               FP8 with per-channel scales, or BF16; otherwise two separate projections
 //               (NVFP4 from 129 rows on: gate, up, GeGLU and the down projection's quantiser are one launch of the CTA-pair
-//               kernel, joined or not)
+//               kernel, joined or not; FP8 and BF16 gate, up and GeGLU too)
 //   GeGLU       fused into the activation quantiser of the down projection when that one runs
 //               quantised on a joined [rows, gate | up] tensor; an element-wise kernel otherwise
 //               (small row counts, where that is the faster way: gate, up and GeGLU are one launch of the
@@ -332,6 +332,27 @@ gw_status gw_mlp_chain_run(gw_mlp_chain* c, const gw_projection* gate, const gw_
     status = run_nvfp4_geglu(nvfp4_plan(h, m), nvfp4_plan(m, h), *gate, *up, *down, input_bf16, product_bf16, output_bf16,
                              c->book.scratch.data, c->book.scratch.bytes, s, &done);
     if (status != GW_OK || done) return status;
+  }
+  {                              // prefill on FP8 or BF16: GeGLU in the gate/up epilogue, in FP8 where down takes that
+    const auto plan = [&](int kind, uint32_t k, uint32_t n) -> const PlanSet* {
+      const auto found = c->book.plans.find(Key{kind, k, n});
+      return found == c->book.plans.end() ? nullptr : &found->second;
+    };
+    const auto fp8_plan = [&](const gw_projection& p) {
+      const PlanSet* set = plan(p.fp8_channel_scales ? kFp8Channel : kFp8, p.input, p.output);
+      return set ? set->fp8 : nullptr;
+    };
+    bool packed = false, done = false;
+    if (gate->storage == GW_STORAGE_FP8_W8A8) {
+      status = run_fp8_geglu(fp8_plan(*gate), *gate, *up, *down, input_bf16, product_bf16, c->book.scratch.data, c->book.scratch.bytes, s,
+                             &packed, &done);
+    } else if (gate->storage == GW_STORAGE_BF16) {
+      const PlanSet* set = plan(kBf16, h, m);
+      status = run_bf16_geglu(set ? set->bf16 : nullptr, *gate, *up, *down, input_bf16, product_bf16, s, &packed, &done);
+    }
+    if (status != GW_OK) return status;
+    if (done && packed) return run_fp8_plan_packed(fp8_plan(*down), product_bf16, *down, output_bf16, s);
+    if (done) return run_linear(c->book, *down, product_bf16, output_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
   }
   bool interleaved = true;       // gate_up holds [rows, gate | up]; otherwise gate rows, then up rows
   if ((nvfp4_joined(*gate, *up) && fp4) || fp8_joined(*gate, *up) || bf16_joined(*gate, *up)) {

@@ -366,12 +366,33 @@ gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_proje
 gw_status projection_workspace_run_mlp(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up,
                                        const gw_projection& down, const void* input, void* buffer, void* output, cudaStream_t stream, bool* done) {
   *done = false;
-  if (w->rows == 0 || !w->fp4 || down.output != down.physical_output) return GW_OK;
-  const auto plan = [&](const gw_projection& p) {
-    const auto found = w->plans.find(Shape{kPlanNvfp4, p.input, p.physical_output});
-    return found == w->plans.end() ? nullptr : found->second.nvfp4;
+  if (w->rows == 0 || down.output != down.physical_output) return GW_OK;
+  const auto plans = [&](int kind, const gw_projection& p) -> const Plans* {
+    const auto found = w->plans.find(Shape{kind, p.input, p.physical_output});
+    return found == w->plans.end() ? nullptr : &found->second;
   };
-  return run_nvfp4_geglu(plan(gate), plan(down), gate, up, down, input, buffer, output, w->scratch.data, w->scratch.bytes, stream, done);
+  if (gate.storage == GW_STORAGE_NVFP4_W4A4) {
+    const Plans *first = plans(kPlanNvfp4, gate), *second = plans(kPlanNvfp4, down);
+    if (!w->fp4 || !first || !second) return GW_OK;
+    return run_nvfp4_geglu(first->nvfp4, second->nvfp4, gate, up, down, input, buffer, output, w->scratch.data, w->scratch.bytes, stream, done);
+  }
+  bool packed = false;
+  gw_status status = GW_OK;
+  // the workspace's FP8 plans take one scale per matrix
+  if (gate.fp8_channel_scales || up.fp8_channel_scales || down.fp8_channel_scales) return GW_OK;
+  if (gate.storage == GW_STORAGE_FP8_W8A8) {
+    const Plans* first = plans(kPlanFp8, gate);
+    if (!first) return GW_OK;
+    status = run_fp8_geglu(first->fp8, gate, up, down, input, buffer, w->scratch.data, w->scratch.bytes, stream, &packed, done);
+  } else if (gate.storage == GW_STORAGE_BF16) {
+    const Plans* first = plans(kPlanBf16, gate);
+    if (!first) return GW_OK;
+    status = run_bf16_geglu(first->bf16, gate, up, down, input, buffer, stream, &packed, done);
+  }
+  if (status != GW_OK || !*done) return status;
+  if (!packed) return projection_workspace_run_on(w, &down, buffer, output, stream, true);
+  const Plans* second = plans(kPlanFp8, down);
+  return run_fp8_plan_packed(second ? second->fp8 : nullptr, buffer, down, output, stream);
 }
 
 gw_status projection_workspace_run_geglu(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up, const void* input,

@@ -17,6 +17,26 @@ def gw():
 def projections(gw, storage, hidden, mlp, joined):
     both = (bf16_normal((2 * mlp, hidden), 1) * 0.02).cuda()
     down = (bf16_normal((hidden, mlp), 2) * 0.02).cuda()
+    gate, up = (both[:mlp], both[mlp:]) if joined else (both[:mlp].clone(), both[mlp:].clone())
+
+    def fp8(w, input_scale, channel):
+        rows = (w.float().abs().amax(dim=1) / 448).contiguous()
+        if channel is not None:
+            return gw.Fp8Weight(gw.fp8_pack_weights(w, 0.0, rows), input_scale, 1.0, (rows * input_scale).contiguous())
+        return gw.Fp8Weight(gw.fp8_pack_weights(w, float(rows.max())), input_scale, float(rows.max()))
+
+    if storage == "bf16":
+        return gate, up, down
+    if storage == "bf16 fp8":
+        return gate, up, fp8(down, 16 / 448, None)
+    if storage == "fp8":
+        return fp8(gate.contiguous(), 6 / 448, None), fp8(up.contiguous(), 6 / 448, None), fp8(down, 16 / 448, None)
+    if storage in ("fp8 channel", "fp8 bf16"):
+        rows = (both.float().abs().amax(dim=1) / 448).contiguous()
+        scales = (rows * (6 / 448)).contiguous()
+        data = gw.fp8_pack_weights(both, 0.0, rows)
+        pair = [gw.Fp8Weight(data[s], 6 / 448, 1.0, scales[s]) for s in (slice(0, mlp), slice(mlp, 2 * mlp))]
+        return (*pair, down if storage == "fp8 bf16" else fp8(down, 16 / 448, rows))
     packed = gw.nvfp4_pack_weights(both, 6 / 2688)
     if joined:
         split = gw.nvfp4_scale_storage_bytes(mlp, hidden)
@@ -27,7 +47,8 @@ def projections(gw, storage, hidden, mlp, joined):
     return gate, up, gw.nvfp4_pack_weights(down, 16 / 2688)
 
 
-@pytest.mark.parametrize("storage,joined", [("nvfp4", True), ("nvfp4", False)])
+@pytest.mark.parametrize("storage,joined", [("nvfp4", True), ("nvfp4", False), ("fp8", False), ("fp8 channel", True), ("fp8 bf16", True),
+                                            ("bf16", True), ("bf16", False), ("bf16 fp8", True)])
 @pytest.mark.parametrize("rows,hidden,mlp", [(129, 128, 128), (255, 256, 384), (256, 640, 128), (257, 384, 1152), (513, 1024, 256), (300, 2816, 2176)])
 def test_fused_equals_separate_launches(gw, monkeypatch, storage, joined, rows, hidden, mlp):
     from gewell_b200 import _lib
