@@ -1,9 +1,9 @@
 // Weight-streaming projections for small row counts (decode): one launch quantises the
 // activations, reads every weight once and writes the BF16 result.
 //
-// What bounds it: the weight bytes from HBM.  So the work is divided by bytes: the flat sequence of
-// (block of 32 weight rows, 128-byte chunk of K) pieces is cut into equal ranges, one per SM and inside
-// it one per warp, at any piece.  A warp walks its range alone: it has a ring of two pieces of its own that it
+// What bounds it: the weight bytes from HBM, and at small sizes latency.  The flat sequence of (block of 32 weight rows, 128-byte
+// chunk of K) pieces is cut into ranges, one per SM -- whole row blocks where all of K is one slab, equal ranges cut at any piece
+// otherwise -- and inside it one per warp, at any piece.  A warp walks its range alone: it has a ring of two pieces of its own that it
 // refills itself by tensor copies as soon as it has multiplied one (144 KB per SM on their way for W4A4, 128 for W8A8,
 // 108 for W4A16, 96 for BF16), and it stores the row blocks that are wholly its own straight from registers.  Nothing synchronises while weights stream; the
 // first pieces are asked for before the kernel waits for its predecessor.  Row blocks that several warps share
@@ -17,6 +17,7 @@
 // Token values live in shared memory in the order the tensor instruction wants them.  When all of K does
 // not fit there, K is cut into slabs, the flat sequence walks slab by slab and every row block has one sum
 // per slab.
+#include <algorithm>
 #include <string>
 
 #include "common.cuh"
@@ -49,15 +50,15 @@ struct StreamArgs {
   float inverse_scale;
   uint32_t rows, k, n, gelu;
   uint32_t blocks, chunks, chunks_per_slab, slabs, max_units;
-  uint32_t range, longer;                // pieces per SM; the first `longer` SMs have one more
+  uint32_t range, longer, step;          // steps per SM, of `step` pieces each; the first `longer` SMs have one more
   Divisor by_range, by_range1;           // range, range + 1
   Divisor by_slab, by_chunks, by_last_chunks, by_blocks;   // pieces of a whole slab; chunks of a whole and of the last slab; blocks
 };
 
 constexpr int kSharedLimit = 226 * 1024;
 
-// Where the piece ranges lie: piece x of the launch belongs to thread block cta_of(x).
-__device__ __forceinline__ uint32_t range_begin(const StreamArgs& a, uint32_t cta) { return cta * a.range + min(cta, a.longer); }
+// Where the piece ranges lie.  Where they cut row blocks (a step is one piece), piece x belongs to thread block cta_of(x).
+__device__ __forceinline__ uint32_t range_begin(const StreamArgs& a, uint32_t cta) { return (cta * a.range + min(cta, a.longer)) * a.step; }
 __device__ __forceinline__ uint32_t cta_of(const StreamArgs& a, uint32_t x) {
   const uint32_t cut = a.longer * (a.range + 1);
   return x < cut ? a.by_range1.quotient(x) : a.longer + a.by_range.quotient(x - cut);
@@ -436,17 +437,23 @@ StreamPlan plan_stream(StreamKind kind, uint32_t rows, uint32_t k, uint32_t n, b
   p.slabs = (p.chunks + p.chunks_per_slab - 1) / p.chunks_per_slab;
   const uint64_t pieces = uint64_t(p.blocks) * p.chunks;
   if (pieces >= (1u << 30) || p.slabs > 32) return p;          // one lane per slab when the sums are added
+  // Whole row blocks for every SM, where all of K fits: the sums of a block that SMs share cost a pass through L2, 2 us, more than
+  // some SMs with one block more than others do.  (Shared / whole, us: NVFP4 1x2816x2048 7.5 / 5.3, 1x2816x8192 9.1 / 6.9, 1x5376x21504
+  // 17.3 / 15.2, FP8 8x2816x4096 9.7 / 6.6, 4x5376x43008 38.6 / 36.4, BF16 8x2816x1024 7.9 / 6.2; with K 1024 and N 8192, where a
+  // block does not feed the warps, NVFP4 5.2 / 5.8 and FP8 4.8 / 4.8.)
+  p.whole = p.slabs == 1;
+  if (p.whole) p.grid = std::min(p.blocks, sm_count);
   // at least one piece per warp
-  p.grid = int(pieces / size.warps < uint64_t(sm_count) ? (pieces + size.warps - 1) / size.warps : sm_count);
-  // Row blocks that are whole need no second pass over their sums: when every SM can have one of its own, it does.
-  if (p.slabs == 1 && p.blocks <= sm_count && 2 * p.blocks >= sm_count) p.grid = p.blocks;
+  else p.grid = int(pieces / size.warps < uint64_t(sm_count) ? (pieces + size.warps - 1) / size.warps : sm_count);
   const int per_cta = int(pieces / p.grid);
-  if (p.chunks_per_slab / per_cta + 2 > 32) return p;          // one lane per part of a slab's row block
+  if (!p.whole && p.chunks_per_slab / per_cta + 2 > 32) return p;          // one lane per part of a slab's row block
   const int shortest = p.chunks - (p.slabs - 1) * p.chunks_per_slab;
   p.max_units = per_cta / shortest + 3;
   p.shared_bytes = size_t(p.chunks_per_slab) * size.chunk + size.fixed;
-  p.workspace_bytes = size_t(p.grid) * p.max_units * p.tiles * (pair ? 512 : 256) * sizeof(float);
-  p.counter_count = size_t(p.blocks);
+  if (!p.whole) {
+    p.workspace_bytes = size_t(p.grid) * p.max_units * p.tiles * (pair ? 512 : 256) * sizeof(float);
+    p.counter_count = size_t(p.blocks);
+  }
   p.usable = p.workspace_bytes <= (size_t(16) << 20);          // callers size their scratch by upper bounds above this
   return p;
 }
@@ -500,9 +507,10 @@ cudaError_t launch_stream(const StreamProblem& q, const StreamPlan& plan, const 
   a.chunks_per_slab = uint32_t(plan.chunks_per_slab);
   a.slabs = uint32_t(plan.slabs);
   a.max_units = uint32_t(plan.max_units);
-  const uint32_t pieces = a.blocks * a.chunks;
-  a.range = pieces / uint32_t(plan.grid);
-  a.longer = pieces % uint32_t(plan.grid);
+  const uint32_t steps = plan.whole ? a.blocks : a.blocks * a.chunks;
+  a.step = plan.whole ? a.chunks : 1;
+  a.range = steps / uint32_t(plan.grid);
+  a.longer = steps % uint32_t(plan.grid);
   a.by_range = Divisor::of(a.range);
   a.by_range1 = Divisor::of(a.range + 1);
   a.by_slab = Divisor::of(a.blocks * a.chunks_per_slab);

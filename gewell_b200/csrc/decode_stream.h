@@ -46,6 +46,7 @@ struct StreamProblem {
 
 // How a problem of this shape is divided over the GPU.
 struct StreamPlan {
+  bool whole = false;          // every SM's range is whole row blocks: no sums to add up across SMs
   bool usable = false;         // the shape can run here (widths a piece can walk, row count)
   uint32_t physical_n = 0;     // rows of each weight matrix in memory
   int tiles = 0;               // groups of eight token rows: 1 or 2
@@ -53,7 +54,7 @@ struct StreamPlan {
   size_t workspace_bytes = 0;  // FP32 partial sums
   size_t counter_count = 0;
   size_t shared_bytes = 0;
-  bool needs_workspace() const { return slabs > 1 || grid != blocks; }
+  bool needs_workspace() const { return !whole; }
 };
 // `n`: rows of each weight matrix in memory; `pair`: two matrices.
 StreamPlan plan_stream(StreamKind kind, uint32_t rows, uint32_t k, uint32_t n, bool pair, int sm_count);

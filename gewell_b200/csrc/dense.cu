@@ -39,35 +39,32 @@ size_t split_counter_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n)
 }  // namespace
 
 // Where the weight-streaming kernel is the faster one.  It saves the quantiser's launch and the tensor-memory prologue; what it
-// pays is that every SM reads and quantises all of the activations, and about 2 us where SMs share row blocks and add their
-// sums in a second pass (StreamPlan::needs_workspace).  Measured against activation quantiser + tcgen05 swap form over K 1024 ..
-// 16384, N 512 .. 5376, 1 to 8 rows, rows * K up to 24 K (B200, cold weights; time of the streaming kernel over the other's,
-// passes of a CUDA graph | launched one by one from Python, where small shapes wait for the second launch):
-//   whole row blocks for every SM (N 2368 .. 4736), one slab        NVFP4 0.75 .. 1.10 | 0.72 .. 1.01, FP8 0.68 .. 1.01 | 0.58 .. 0.89,
-//                                                                   BF16 0.62 .. 0.89 | 0.65 .. 1.08
-//   shared, one slab    FP8 0.76 .. 1.27 | 0.71 .. 1.06, NVFP4 0.74 .. 1.37 | 0.70 .. 1.11, but with N above 4736, K from 4096 on
-//                       and several rows 0.88 .. 1.26 | 0.87 .. 1.12; BF16 0.80 .. 1.17 | 0.80 .. 1.16, K 1024 0.97 .. 1.19 | 0.87 .. 1.19
-//   several slabs       NVFP4 and FP8 up to N 512 0.84 .. 0.97 | 0.84 .. 0.91, beyond 0.92 .. 1.41 | 0.89 .. 1.49; BF16 up to N 2048
-//                       0.78 .. 1.16 | 0.79 .. 1.16, beyond 0.88 .. 1.22 | 0.89 .. 1.26
-// In us (graph): NVFP4 1x2816x2816 5.3 / 6.9, 8x2816x2816 6.7 / 7.0, 1x1408x5376 6.8 / 5.7, 1x16384x2816 18.2 / 13.4; FP8
-// 1x5376x5376 9.2 / 12.2; BF16 8x2816x4096 7.2 / 9.2, 1x8192x2816 16.4 / 13.9.
-// W4A16 has no other kernel that reads the packed weights.
+// pays is that every SM reads and quantises all of the activations, that some SMs have one row block more than others, and, with
+// several slabs (!StreamPlan::whole), 2 us for adding sums in a second pass.  Measured against activation quantiser + tcgen05 swap form
+// (B200, rotating weights, passes of a CUDA graph; time of the streaming kernel over the other's):
+//   whole row blocks    FP8, 1 to 8 rows, K 1024 .. 8192, N 512 .. 43008, rows * K up to 44 K    0.58 .. 1.02, 8x5376x16384 1.06
+//                       BF16 the same                                                            0.55 .. 1.01, 8x5376x16384 1.05
+//                       NVFP4, N up to 4736 (one block an SM), rows * K up to 24 K   0.67 .. 1.04; more 0.97 .. 1.09
+//                              N up to 9472, rows * K up to 6 K      0.89 .. 0.98; more 0.98 .. 1.21
+//                              N up to 18944 (one wave of the swap form's tiles)  0.94 .. 1.22
+//                              beyond, rows * K up to 24 K           0.68 .. 1.00; 8x5376x43008 1.04
+//   several slabs       NVFP4 and FP8 up to N 512 0.84 .. 0.97, beyond 0.82 .. 1.41; BF16 up to N 2048 0.78 .. 1.16, beyond 0.88 .. 1.65
+// In us: NVFP4 1x2816x2816 5.3 / 6.9, 1x5376x21504 15.2 / 18.2, 8x2816x8192 8.3 / 7.6; FP8 1x5376x5376 6.7 / 11.5 (K 4096), 4x5376x43008 36.4 /
+// 40.6; BF16 8x2816x4096 7.3 / 9.2.  W4A16 has no other kernel that reads the packed weights.
 bool stream_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
   if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
-  if (n > 5376 || k > 16384 || size_t(rows) * k > 24 * 1024) return false;
-  if (!plan.needs_workspace()) return true;
-  if (plan.slabs > 1) return n <= (kind == StreamKind::w16a16 ? 2048 : 512);
-  if (kind == StreamKind::w16a16) return k >= 1408;
-  return kind == StreamKind::w8a8 || n <= 4736 || rows == 1 || k < 4096;
+  const size_t values = size_t(rows) * k, sms = size_t(sm_count());
+  if (!plan.whole) return k <= 16384 && values <= 24 * 1024 && n <= (kind == StreamKind::w16a16 ? 2048 : 512);
+  if (kind != StreamKind::w4a4) return values <= 44 * 1024;
+  if (n <= 32 * sms || n > 128 * sms) return values <= 24 * 1024;
+  return n <= 64 * sms && values <= 6 * 1024;
 }
 
 namespace {
-// With GeGLU in front of the quantiser every SM computes all of it.  Over GeGLU + quantiser + swap form (as above): one slab and
-// at most 12 K values in whole row blocks or 8 K in shared ones 0.80 .. 1.44 | 0.66 .. 1.16; more values 0.88 .. 1.86 |
-// 0.82 .. 1.46, several slabs 0.90 .. 1.80 | 0.91 .. 1.72.
-bool stream_gelu_pays(const StreamPlan& plan, uint32_t rows, uint32_t k) {
-  return plan.slabs == 1 && size_t(rows) * k <= (plan.needs_workspace() ? 8 : 12) * 1024;
-}
+// With GeGLU in front of the quantiser every SM computes all of it.  Over GeGLU + quantiser + swap form (passes of a graph |
+// launched one by one): one slab and at most 12 K values 0.80 .. 1.44 | 0.66 .. 1.16; more values 0.88 .. 1.86 | 0.82 .. 1.46, several
+// slabs 0.90 .. 1.80 | 0.91 .. 1.72.
+bool stream_gelu_pays(const StreamPlan& plan, uint32_t rows, uint32_t k) { return plan.whole && size_t(rows) * k <= 12 * 1024; }
 }  // namespace
 
 // Rows up to which W4A16 runs as launches of the weight-streaming kernel, sixteen rows each, instead of dequantising the
@@ -82,17 +79,21 @@ constexpr uint32_t kW4a16Rows = 32;
 
 // Gate, up and GeGLU as one streaming launch (n: channels of each).  Where the two matrices lie apart it stands against two
 // projections and a GeGLU kernel, where they are joined against one GEMM whose GeGLU rides in the next quantiser (BF16: a kernel
-// of its own).  Whole chains of hidden -> n -> hidden, hidden 1408 .. 5376, n 1024 .. 21504, 1 to 8 rows, time over the other way
-// (as above):
-//   n up to 4224, rows * K up to 24 K          apart 0.63 .. 0.88 | 0.64 .. 1.04; joined 0.80 .. 1.40 | 0.60 .. 1.10
-//   96 MiB and more, rows * K up to 8 K        apart 0.78 .. 0.95 | 0.79 .. 0.94; joined 0.91 .. 1.00 | 0.91 .. 1.00
-//   the rest                                   apart 0.68 .. 1.06 | 0.64 .. 1.01; joined 0.82 .. 1.39 | 0.61 .. 1.35
-// In us (graph): NVFP4 1x5376x21504 joined 48.4 / 48.2, apart 48.1 / 59.3; FP8 1x5376x21504 joined 65.3 / 66.0.
+// of its own).  Whole chains of hidden -> n -> hidden with joined matrices, hidden 1152 .. 5376, 1 to 8 rows, time over the other way
+// (passes of a graph):
+//   n up to 4224, rows * K up to 24 K   NVFP4 0.98 .. 1.11, FP8 0.96 .. 1.13, BF16 0.90 .. 1.14; apart 0.64 .. 1.04 (launched one by one)
+//   BF16 beyond                         0.89 .. 0.99
+//   FP8, matrices of 64 MB and more     0.92 .. 1.00; less: one row 0.92 .. 0.98, more 0.97 .. 1.27
+//   NVFP4, 48 MB and more, rows * K up to 22 K   0.86 .. 0.99, more 1.00 .. 1.02; less: one row 0.92 .. 1.05, more 0.99 .. 1.25
+// In us: NVFP4 1x5376x21504 47.9 / 51.5, 1x4096x11008 24.6 / 28.7; FP8 1x5376x21504 63.5 / 65.9; BF16 4x3584x12544 49.4 / 55.6.
 bool stream_pair_pays(StreamKind kind, const StreamPlan& plan, uint32_t rows, uint32_t k, size_t n) {
   if (!plan.usable || kind == StreamKind::w4a16) return plan.usable;
   const size_t bytes = 2 * n * k * (kind == StreamKind::w4a4 ? 9 : kind == StreamKind::w8a8 ? 16 : 32) / 16;
   const size_t values = size_t(rows) * k;
-  return n <= 4224 ? values <= 24 * 1024 : bytes >= (size_t(96) << 20) && values <= 8192;
+  if (n <= 4224) return values <= 24 * 1024;
+  if (!plan.whole) return bytes >= (size_t(96) << 20) && values <= 8192;
+  if (kind == StreamKind::w16a16 || rows == 1) return true;
+  return kind == StreamKind::w8a8 ? bytes >= (size_t(64) << 20) : bytes >= (size_t(48) << 20) && values <= 22 * 1024;
 }
 
 namespace {
