@@ -119,22 +119,45 @@ __device__ __forceinline__ void inverse_rms(const NormArgs& a, const bf16* const
   __shared__ float result[ROWS];
   __syncthreads();                                     // the rows are complete; `totals` is free
   const uint32_t lanes = a.lanes;                      // a power of two; 4 * lanes <= width
-  for (uint32_t item = threadIdx.x; item < ROWS * lanes; item += blockDim.x) {
-    const uint32_t which = ROWS == 1 ? 0 : item / lanes, l = ROWS == 1 ? item : item % lanes;
-    const bf16* row = rows[0];
+  if (lanes >= 8 && lanes <= 64) {
+    // Launches of many rows have few logical lanes, which walk far: a thread per accumulator, so that 32 lanes keep 128 threads
+    // busy (feed-forward block of 4000 rows, with three blocks of the tail an SM: 403 -> 369 us).
+    const uint32_t shift = 31 - __clz(4 * lanes);
+    for (uint32_t item = threadIdx.x; item < ROWS * 4 * lanes; item += blockDim.x) {      // whole warps
+      const uint32_t which = ROWS == 1 ? 0 : item >> shift, l = item & (4 * lanes - 1);
+      const bf16* row = rows[0];
 #pragma unroll
-    for (int r = 1; r < ROWS; ++r)
-      if (which == r) row = rows[r];
-    float sum[4] = {0.F, 0.F, 0.F, 0.F};
+      for (int r = 1; r < ROWS; ++r)
+        if (which == uint32_t(r)) row = rows[r];
+      float sum = 0.F;
 #pragma unroll 4
-    for (uint32_t i = 4 * l; i < a.width; i += 4 * lanes) {
-      const uint2 bits = *reinterpret_cast<const uint2*>(row + i);
-      const float v[4] = {bf16_bits_to_float(bits.x & 0xffff), bf16_bits_to_float(bits.x >> 16), bf16_bits_to_float(bits.y & 0xffff),
-                          bf16_bits_to_float(bits.y >> 16)};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) sum[e] = __fadd_rn(sum[e], __fmul_rn(v[e], v[e]));
+      for (uint32_t i = l; i < a.width; i += 4 * lanes) {
+        const float v = as_float(row[i]);
+        sum = __fadd_rn(sum, __fmul_rn(v, v));
+      }
+      float total = __fadd_rn(sum, __shfl_down_sync(0xffffffffu, sum, 1));
+      total = __fadd_rn(total, __shfl_down_sync(0xffffffffu, sum, 2));
+      total = __fadd_rn(total, __shfl_down_sync(0xffffffffu, sum, 3));
+      if (l % 4 == 0) totals[item / 4] = total;
     }
-    totals[item] = __fadd_rn(__fadd_rn(__fadd_rn(sum[0], sum[1]), sum[2]), sum[3]);
+  } else {
+    for (uint32_t item = threadIdx.x; item < ROWS * lanes; item += blockDim.x) {
+      const uint32_t which = ROWS == 1 ? 0 : item / lanes, l = ROWS == 1 ? item : item % lanes;
+      const bf16* row = rows[0];
+#pragma unroll
+      for (int r = 1; r < ROWS; ++r)
+        if (which == r) row = rows[r];
+      float sum[4] = {0.F, 0.F, 0.F, 0.F};
+#pragma unroll 4
+      for (uint32_t i = 4 * l; i < a.width; i += 4 * lanes) {
+        const uint2 bits = *reinterpret_cast<const uint2*>(row + i);
+        const float v[4] = {bf16_bits_to_float(bits.x & 0xffff), bf16_bits_to_float(bits.x >> 16), bf16_bits_to_float(bits.y & 0xffff),
+                            bf16_bits_to_float(bits.y >> 16)};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[e] = __fadd_rn(sum[e], __fmul_rn(v[e], v[e]));
+      }
+      totals[item] = __fadd_rn(__fadd_rn(__fadd_rn(sum[0], sum[1]), sum[2]), sum[3]);
+    }
   }
   __syncthreads();
   const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, warps = blockDim.x / 32;
@@ -229,11 +252,12 @@ struct TailArgs {
   const float* weights;
 };
 constexpr int kTopK = 8;
+constexpr int kBlockThreads = 2816 / 8;     // COMBINE: of the block's own width.  Three of its launch's blocks fit an SM (56 registers, not 63)
 
 // shared = norm1(shared_mlp); branch = norm2(routed); sum = bf16(shared + branch); branch = norm3(sum);
 // hidden = bf16(hidden + branch); hidden = bf16(hidden * scalar)        (batched_executor.cu:260,278-285)
 template <int NV, bool COMBINE>
-__global__ void __launch_bounds__(kNormThreads) ffn_tail_kernel(NormArgs a, TailArgs t) {
+__global__ void __launch_bounds__((COMBINE ? kBlockThreads : kNormThreads), (COMBINE ? 3 : 1)) ffn_tail_kernel(NormArgs a, TailArgs t) {
   static_assert(!COMBINE || NV == 1, "one vector a thread");
   extern __shared__ __align__(16) unsigned char norm_smem[];
   bf16* first = reinterpret_cast<bf16*>(norm_smem);
@@ -288,6 +312,52 @@ __global__ void __launch_bounds__(kNormThreads) ffn_tail_kernel(NormArgs a, Tail
       hidden.part[j].v[e] = rounded(__fmul_rn(as_float(updated), scalar));
     }
   hidden.store_any(t.hidden + base, vectors);
+}
+
+// Router logits of few rows: bf16(x . Wrouter^T) for 128 experts.  What bounds it is latency, 720 KB and two to eight
+// microseconds of dependent steps; so a block takes sixteen experts and eight rows over all of K, its weights are on their way
+// before the wait, every load of a thread is in flight at once and nothing passes through global memory but the
+// logits.  (8 rows, alone: weight-streaming kernel 8.7 us, this 4.8.)
+// mma.sync: sixteen experts are no tcgen05 tile, and the tensor pipe is idle.  A K step takes any values as long as both
+// operands agree: lane 4 * g + t has the same eight consecutive values of expert g, expert g + 8 and row g.
+constexpr int kRouterThreads = 256, kRouterSteps = 2816 / 32 / (kRouterThreads / 32);     // of 32 values, each warp
+static_assert(kRouterSteps * 32 * (kRouterThreads / 32) == 2816, "whole steps for every warp");
+constexpr uint32_t kRouterRows = 128, kRouterExperts = 128;
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__global__ void __launch_bounds__(kRouterThreads)
+router_logits_kernel(const uint4* __restrict__ input, const uint4* __restrict__ weights, bf16* __restrict__ logits, uint32_t rows) {
+  constexpr uint32_t kVectors = 2816 / 8;
+  __shared__ float sums[kRouterThreads / 32][16][8];
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane / 4, t = lane % 4;
+  const uint32_t first = warp * kRouterSteps * 4 + t, expert = blockIdx.x * 16, row = blockIdx.y * 8 + g;
+  uint4 lo[kRouterSteps], hi[kRouterSteps], x[kRouterSteps];
+#pragma unroll
+  for (int i = 0; i < kRouterSteps; ++i) {
+    lo[i] = weights[size_t(expert + g) * kVectors + first + 4 * i];
+    hi[i] = weights[size_t(expert + g + 8) * kVectors + first + 4 * i];
+  }
+  griddep_enter();
+#pragma unroll
+  for (int i = 0; i < kRouterSteps; ++i)
+    x[i] = row < rows ? input[size_t(row) * kVectors + first + 4 * i] : make_uint4(0, 0, 0, 0);
+  float even[4] = {0.F, 0.F, 0.F, 0.F}, odd[4] = {0.F, 0.F, 0.F, 0.F};
+#pragma unroll
+  for (int i = 0; i < kRouterSteps; ++i) {
+    mma_bf16(even, lo[i].x, hi[i].x, lo[i].y, hi[i].y, x[i].x, x[i].y);
+    mma_bf16(odd, lo[i].z, hi[i].z, lo[i].w, hi[i].w, x[i].z, x[i].w);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) sums[warp][g + 8 * (j / 2)][2 * t + j % 2] = even[j] + odd[j];
+  __syncthreads();
+  const uint32_t e = threadIdx.x % 16, r = threadIdx.x / 16;
+  if (r >= 8 || blockIdx.y * 8 + r >= rows) return;
+  float sum = 0.F;
+#pragma unroll
+  for (int w = 0; w < kRouterThreads / 32; ++w) sum += sums[w][e][r];
+  logits[size_t(blockIdx.y * 8 + r) * kRouterExperts + expert + e] = rounded(sum);
 }
 
 // y = bf16(a + b)                                                       (bf16_math.cuh:109-112)
@@ -631,8 +701,15 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
   }
   GW_CUDA_CHECK(recorded, "feed-forward block join");
   // router logits and the experts (batched_executor.cu:262-266)
-  status = run_bf16_plan(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes,
-                         as_stream(s), true);
+  if (rows <= kRouterRows && aligned16(w.router_proj)) {
+    status = GW_OK;
+    GW_CUDA_CHECK(launch_pdl(router_logits_kernel, dim3(kRouterExperts / 16, (rows + 7) / 8), kRouterThreads, as_stream(s),
+                             reinterpret_cast<const uint4*>(b->router_input), static_cast<const uint4*>(w.router_proj), b->logits, rows),
+                  "router logits");
+  } else {
+    status = run_bf16_plan(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes,
+                           as_stream(s), true);
+  }
   MoeCombineInput combine;
   if (status == GW_OK)
     status = moe_run_to_down(b->moe, b->expert_input, b->logits, w.router_per_expert_scale, w.experts, rows, w.has_bf16, w.has_fp8,
@@ -645,7 +722,7 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
                    static_cast<const bf16*>(w.post_feedforward_norm_2), static_cast<const bf16*>(w.post_feedforward_norm),
                    static_cast<const bf16*>(w.layer_scalar), static_cast<bf16*>(hidden_bf16), static_cast<const uint4*>(combine.down),
                    combine.inverse, combine.weights};
-  static_assert(kHidden / 8 <= kNormThreads, "one vector a thread");
+  static_assert(kHidden / 8 == kBlockThreads, "one vector a thread");
   GW_CUDA_CHECK(launch_pdl_shared(ffn_tail_kernel<1, true>, rows, norm_threads(kHidden), norm_shared_bytes(kHidden, a.lanes, 2), as_stream(s), a, t),
                 "feed-forward tail");
   moe_mark_combined(b->moe, as_stream(s));
