@@ -339,7 +339,7 @@ gw_status gw::run_nvfp4_geglu(gw_nvfp4_plan* gate_plan, gw_nvfp4_plan* down_plan
       gate.input != up.input || gate.output != up.output || gate.physical_output != up.physical_output || down.input != gate.output ||
       gate.physical_output != align_up(gate.output, 128) || gate.output % 64 != 0 || gate_plan->input_width != gate.input ||
       down_plan->rows != gate_plan->rows || down_plan->input_width != down.input || down_plan->output_width != down.physical_output ||
-      !dense_has_geglu(gate_plan->descriptors.tuning, gate_plan->rows) || !dense_has_geglu(down_plan->descriptors.tuning, gate_plan->rows) ||
+      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::nvfp4, gate_plan->rows, gate.output) ||
       !input || !output || !aligned(input, 16) || !aligned(output, 2) || !aligned(buffer, 256) || !aligned(scratch, 256) ||
       scratch_capacity < gate_plan->split_offset || down_plan->split_offset > size_t(down_plan->rows) * down.input * sizeof(bf16))
     return GW_OK;
@@ -356,8 +356,12 @@ gw_status gw::run_nvfp4_geglu(gw_nvfp4_plan* gate_plan, gw_nvfp4_plan* down_plan
                        packed_in, scales_in, 1.0F / down.nvfp4_input_scale, packed, scales, device_error_word()};
   const gw_status status = launch_dense_geglu(q, &gate_plan->descriptors, s);
   if (status != GW_OK) return status;
-  const DenseProblem problem{GemmKind::nvfp4, rows, down.input, down.physical_output, down.nvfp4_data, down.nvfp4_scales, packed, scales,
-                             down.nvfp4_input_scale * down.nvfp4_weight_scale, nullptr, output, device_error_word()};
+  DenseProblem problem{GemmKind::nvfp4, rows, down.input, down.physical_output, down.nvfp4_data, down.nvfp4_scales, packed, scales,
+                       down.nvfp4_input_scale * down.nvfp4_weight_scale, nullptr, output, device_error_word()};
+  problem.weights_settled = true;
+  // the quantised input is dead when down's partial sums are written
+  const size_t split = down_plan->total_bytes - down_plan->split_offset;
+  if (split != 0 && split <= scratch_capacity) problem.split_workspace = scratch;
   return launch_dense(problem, &down_plan->descriptors, s);
 }
 
@@ -593,7 +597,7 @@ gw_status gw::run_fp8_geglu(gw_fp8_plan* gate_plan, const gw_projection& gate, c
   *done = false;
   if (!gate_plan || !same_shape(gate, up) || !usable_fp8(gate) || !usable_fp8(up) || gate.fp8_input_scale != up.fp8_input_scale ||
       gate_plan->input_width != gate.input || gate_plan->output_width != gate.output ||
-      !dense_has_geglu_wide(gate_plan->descriptors.tuning, gate_plan->rows) || !input || !aligned(input, 2) || !product ||
+      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::fp8, gate_plan->rows, gate.output) || !input || !aligned(input, 2) || !product ||
       !aligned(product, 16) || !scratch || !aligned(scratch, 256) || scratch_capacity < gate_plan->split_offset)
     return GW_OK;
   *done = true;
@@ -613,7 +617,7 @@ gw_status gw::run_bf16_geglu(gw_bf16_plan* gate_plan, const gw_projection& gate,
   *done = false;
   if (!gate_plan || !same_shape(gate, up) || gate.storage != GW_STORAGE_BF16 || !gate.bf16 || !up.bf16 || !aligned(gate.bf16, 16) ||
       !aligned(up.bf16, 16) || gate_plan->input_width != gate.input || gate_plan->output_width != gate.output ||
-      !dense_has_geglu_wide(gate_plan->descriptors.tuning, gate_plan->rows) || !input || !aligned(input, 16) || !product || !aligned(product, 16))
+      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::bf16, gate_plan->rows, gate.output) || !input || !aligned(input, 16) || !product || !aligned(product, 16))
     return GW_OK;
   *done = true;
   *packed = usable_fp8(down);
@@ -622,12 +626,16 @@ gw_status gw::run_bf16_geglu(gw_bf16_plan* gate_plan, const gw_projection& gate,
   return launch_dense_geglu_wide(q, &gate_plan->descriptors, s);
 }
 
-gw_status gw::run_fp8_plan_packed(gw_fp8_plan* plan, const void* packed, const gw_projection& p, void* output, cudaStream_t s) {
+gw_status gw::run_fp8_plan_packed(gw_fp8_plan* plan, const void* packed, const gw_projection& p, void* output, void* scratch,
+                                  size_t scratch_capacity, cudaStream_t s) {
   if (!plan || !usable_fp8(p) || !packed || !output || !aligned(packed, 16) || !aligned(output, 16) || (plan->channel_scales && !p.fp8_channel_scales))
     return fail(GW_INVALID_ARGUMENT, "FP8 run requires a plan, valid aligned device buffers and finite positive global scales");
-  const DenseProblem problem{GemmKind::fp8, plan->rows, plan->input_width, plan->output_width, p.fp8_data, nullptr, packed, nullptr,
-                             p.fp8_input_scale * p.fp8_weight_scale, plan->channel_scales ? p.fp8_channel_scales : nullptr, output,
-                             device_error_word()};
+  DenseProblem problem{GemmKind::fp8, plan->rows, plan->input_width, plan->output_width, p.fp8_data, nullptr, packed, nullptr,
+                       p.fp8_input_scale * p.fp8_weight_scale, plan->channel_scales ? p.fp8_channel_scales : nullptr, output,
+                       device_error_word()};
+  problem.weights_settled = true;
+  const size_t split = plan->total_bytes - plan->split_offset;
+  if (split != 0 && split <= scratch_capacity && aligned(scratch, 256)) problem.split_workspace = scratch;
   return launch_dense(problem, &plan->descriptors, s);
 }
 

@@ -407,32 +407,30 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
   return GW_OK;
 }
 
-bool dense_has_geglu(const DenseTuning& tuning, uint32_t rows) {
-  return !dense_uses_swap_form(tuning, rows) && dense_block_n(tuning, rows) == 256 && !tuning.no_pair;
+// Beyond the swap form's rows always; with fewer where one wave of pair tiles (NVFP4: half of one) holds all channels, so that
+// three launches stand against the swap form's four to nine.  MLP, us, swap form / this: NVFP4 2816 -> 2176 16 rows 22.8 / 20.3,
+// 2816 -> 4096 100 rows 22.9 / 21.6, 4096 -> 8192 40 rows 27.2 / 29.7; FP8 2816 -> 4096 20 rows 22.8 / 20.6, 4096 -> 8192 100 rows
+// 38.5 / 37.6; BF16 3200 -> 4224 53 rows 30.3 / 29.5.
+bool dense_geglu_pays(const DenseTuning& tuning, GemmKind kind, uint32_t rows, uint32_t n) {
+  if (tuning.form != 0 || tuning.block_n != 0 || tuning.no_pair) return false;
+  if (!dense_uses_swap_form(tuning, rows)) return true;
+  return rows > 8 && int((n + 127) / 128) <= sm_count() / (kind == GemmKind::nvfp4 ? 4 : 2);
 }
 
 gw_status launch_dense_geglu(const GegluProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
   std::string error;
   const uint32_t physical = (q.n + 127) / 128 * 128;
-  if (cache->weight_half != q.weight[0]) {
-    if (!encode_tensor_map_2d(&cache->weight_half_map, q.weight[0], q.k / 2, physical, 128, &error))
-      return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
-    cache->weight_half = q.weight[0];
-  }
-  if (cache->up != q.weight[1]) {
-    if (!encode_tensor_map_2d(&cache->up_map, q.weight[1], q.k / 2, physical, 128, &error))
-      return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
-    cache->up = q.weight[1];
-  }
-  if (cache->activations != q.activations) {
-    if (!encode_tensor_map_2d(&cache->activation_map, q.activations, q.k / 2, q.rows, 128, &error))
-      return fail(GW_CUDA_ERROR, "activation descriptor: " + error);
-    cache->activations = q.activations;
-  }
+  const void* from[3] = {q.activations, q.weight[0], q.weight[1]};
+  for (int i = 0; i < 3; ++i)
+    if (cache->geglu_from[i] != from[i]) {
+      if (!encode_tensor_map_2d(&cache->geglu_maps[i], from[i], q.k / 2, i == 0 ? q.rows : physical, 128, &error))
+        return fail(GW_CUDA_ERROR, "gate/up descriptor: " + error);
+      cache->geglu_from[i] = from[i];
+    }
   PairGemmParams pair{};
-  pair.map_tokens = cache->activation_map;
-  pair.map_weights = cache->weight_half_map;
-  pair.map_up = cache->up_map;
+  pair.map_tokens = cache->geglu_maps[0];
+  pair.map_weights = cache->geglu_maps[1];
+  pair.map_up = cache->geglu_maps[2];
   pair.sf_tokens = q.activation_scales;
   pair.token_row_blocks = int32_t((q.rows + 127) / 128);
   pair.k = int32_t(q.k);
@@ -449,10 +447,6 @@ gw_status launch_dense_geglu(const GegluProblem& q, DenseDescriptors* cache, cud
   pair.error = q.error;
   GW_CUDA_CHECK(launch_gemm_pair_geglu(pair, sm_count(), stream), "NVFP4 CTA-pair gate/up GEMM with GeGLU + quantise");
   return GW_OK;
-}
-
-bool dense_has_geglu_wide(const DenseTuning& tuning, uint32_t rows) {
-  return !dense_uses_swap_form(tuning, rows) && tuning.form == 0 && tuning.block_n == 0 && !tuning.no_pair;
 }
 
 gw_status launch_dense_geglu_wide(const WideGegluProblem& q, DenseDescriptors* cache, cudaStream_t stream) {

@@ -36,10 +36,8 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   CUtensorMap weight_map{}, activation_map{}, weight_scale_map{};
   const void* weight_half = nullptr;
   CUtensorMap weight_half_map{};     // 128-row box over the weights (CTA-pair kernel: each CTA stages half a tile)
-  const void* up = nullptr;
-  CUtensorMap up_map{};              // the up projection beside `weight_half`, the gate (launch_dense_geglu)
   int token_tile = 0;                // FP8 / BF16 CTA-pair kernel: token columns per tile
-  // its GeGLU form (launch_dense_geglu_wide): token columns per tile, the activations, gate and up in 64-row boxes
+  // the GeGLU forms (launch_dense_geglu, launch_dense_geglu_wide): token columns per tile; the activations, gate and up
   int geglu_tile = 0;
   const void* geglu_from[3] = {};
   CUtensorMap geglu_maps[3]{};
@@ -135,8 +133,8 @@ struct GegluProblem {
   uint8_t *packed, *scales;                  // [rows, n / 2] and its tiled scales
   uint32_t* error;
 };
-// Whether a projection of so many rows runs on the kernel that has this form.
-bool dense_has_geglu(const DenseTuning& tuning, uint32_t rows);
+// Whether that is the faster way for gate and up projections of n channels each.
+bool dense_geglu_pays(const DenseTuning& tuning, GemmKind kind, uint32_t rows, uint32_t n);
 gw_status launch_dense_geglu(const GegluProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
 // The same of FP8 or BF16 projections; the result is E4M3 (inverse_scale != 0) or BF16.
@@ -150,7 +148,6 @@ struct WideGegluProblem {
   void* output;                              // [rows, n]
   uint32_t* error;
 };
-bool dense_has_geglu_wide(const DenseTuning& tuning, uint32_t rows);
 gw_status launch_dense_geglu_wide(const WideGegluProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
 // gw_*_plan_run as a step of a longer call (api.cu): `weights_settled` as in DenseProblem.  The public entry points pass
@@ -172,13 +169,14 @@ gw_status run_nvfp4_geglu(gw_nvfp4_plan* gate_plan, gw_nvfp4_plan* down_plan, co
                           cudaStream_t stream, bool* done);
 
 // GeGLU of FP8 or BF16 gate and up projections of a prefill pass into `product`: E4M3 for `down_plan` and `down` where that is FP8, and
-// *packed = true, else BF16.  *done = false when shape, storage or pointers keep them off that way.  run_fp8_plan_packed runs
-// down over the former.
+// *packed = true, else BF16.  *done = false when shape, storage or pointers keep them off that way.  run_fp8_plan_packed, with the same
+// scratch, runs down over the former.
 gw_status run_fp8_geglu(gw_fp8_plan* gate_plan, const gw_projection& gate, const gw_projection& up, const gw_projection& down, const void* input,
                         void* product, void* scratch, size_t scratch_capacity, cudaStream_t stream, bool* packed, bool* done);
 gw_status run_bf16_geglu(gw_bf16_plan* gate_plan, const gw_projection& gate, const gw_projection& up, const gw_projection& down,
                          const void* input, void* product, cudaStream_t stream, bool* packed, bool* done);
-gw_status run_fp8_plan_packed(gw_fp8_plan* plan, const void* packed, const gw_projection& p, void* output, cudaStream_t stream);
+gw_status run_fp8_plan_packed(gw_fp8_plan* plan, const void* packed, const gw_projection& p, void* output, void* scratch,
+                              size_t scratch_capacity, cudaStream_t stream);
 
 // gw_projection_workspace_run on a stream of the caller's choice (projection.cu).
 gw_status projection_workspace_run_on(gw_projection_workspace* workspace, const gw_projection* projection, const void* input, void* output,

@@ -351,7 +351,7 @@ gw_status gw_mlp_chain_run(gw_mlp_chain* c, const gw_projection* gate, const gw_
       status = run_bf16_geglu(set ? set->bf16 : nullptr, *gate, *up, *down, input_bf16, product_bf16, s, &packed, &done);
     }
     if (status != GW_OK) return status;
-    if (done && packed) return run_fp8_plan_packed(fp8_plan(*down), product_bf16, *down, output_bf16, s);
+    if (done && packed) return run_fp8_plan_packed(fp8_plan(*down), product_bf16, *down, output_bf16, c->book.scratch.data, c->book.scratch.bytes, s);
     if (done) return run_linear(c->book, *down, product_bf16, output_bf16, fp4, GW_TRANSFORM_IDENTITY, s);
   }
   bool interleaved = true;       // gate_up holds [rows, gate | up]; otherwise gate rows, then up rows

@@ -392,7 +392,7 @@ gw_status projection_workspace_run_mlp(gw_projection_workspace* w, const gw_proj
   if (status != GW_OK || !*done) return status;
   if (!packed) return projection_workspace_run_on(w, &down, buffer, output, stream, true);
   const Plans* second = plans(kPlanFp8, down);
-  return run_fp8_plan_packed(second ? second->fp8 : nullptr, buffer, down, output, stream);
+  return run_fp8_plan_packed(second ? second->fp8 : nullptr, buffer, down, output, w->scratch.data, w->scratch.bytes, stream);
 }
 
 gw_status projection_workspace_run_geglu(gw_projection_workspace* w, const gw_projection& gate, const gw_projection& up, const void* input,
