@@ -744,93 +744,69 @@ moe_quantize_kernel(const uint4* __restrict__ input, const int32_t* __restrict__
 }
 
 // ---------------------------------------------------------------------------
-// 5b. The same quantisation, token-major: two warps read a token's row once
-//     (a lane keeps three K16 blocks as packed BF16 and their maxima) and write
-//     the token's eight quantised copies, one per chosen expert, each with that
-//     expert's input scale, at the copy's sorted position.  Arithmetic per
-//     value is that of kernel 5, so the bytes are identical; the input is read
-//     from memory once instead of eight times.
+// 5b. The same quantisation, token-major: a block reads a token's row once (a thread has one K16 block) and writes the token's
+//     eight quantised copies, one per chosen expert, each with that expert's input scale, at the copy's sorted position.
+//     Arithmetic per value is that of kernel 5, so the bytes are identical.  Bound by the store path at large sizes and by the
+//     chain of dependent loads at small ones, hence a block per token (alone, us: 300 tokens 5.4, where
+//     kernel 5 took 8.5; 775 9.6 and 8192 37.0, where two warps a token with three blocks a lane took 10.0 and 40.5).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+constexpr int kTokenThreads = kHidden / 16;        // 176
+__global__ void __launch_bounds__(kTokenThreads)
 moe_quantize_tokens_kernel(const uint4* __restrict__ input, const int32_t* __restrict__ keys,
                            const int32_t* __restrict__ inverse, const int32_t* __restrict__ offsets,
                            const MoeExpertInfo* __restrict__ experts, uint32_t tokens, uint32_t scale_rows, int parts,
                            uint2* __restrict__ packed, uint8_t* __restrict__ scales) {
   griddep_enter();     // results of earlier kernels in the stream are read from here on
-  // Two warps per token, each with one half of the row (88 K16 blocks, three per lane): half the
-  // registers of a whole row per warp, so twice as many warps are resident to cover the loads.
-  constexpr uint32_t kBlocks = kHidden / 16;            // 176
-  constexpr uint32_t kHalfBlocks = kBlocks / 2;         // 88
-  constexpr int kPerLane = (kHalfBlocks + 31) / 32;     // 3
-  const uint32_t warp_index = (blockIdx.x * 256 + threadIdx.x) / 32, lane = threadIdx.x % 32;
-  const uint32_t token = warp_index / 2, half = warp_index % 2;
-  if (token >= tokens) return;
-  const uint32_t n = tokens * kTopK;
-  // Lane j < 8 fetches what copy j needs (expert, destination row, the expert's first row and input
-  // scales): one round of dependent loads for the token instead of one per copy.
-  int32_t copy_expert = 0, copy_first = 0;
-  uint32_t copy_row = 0;
-  float copy_scale[2] = {0.0F, 0.0F};
-  if (lane < kTopK) {
-    copy_expert = keys[token * kTopK + lane];
-    copy_row = uint32_t(inverse[token * kTopK + lane]);
-    copy_first = offsets[copy_expert];
-    copy_scale[0] = experts[copy_expert].inverse_input_scale[0];
-    if (parts > 1) copy_scale[1] = experts[copy_expert].inverse_input_scale[1];
+  __shared__ uint32_t copy_row[kTopK], copy_local[kTopK], copy_region[kTopK];
+  __shared__ float copy_scale[2][kTopK];
+  const uint32_t token = blockIdx.x, kb = threadIdx.x, n = tokens * kTopK;
+  const uint4 a = input[2 * (size_t(token) * kTokenThreads + kb)], b = input[2 * (size_t(token) * kTokenThreads + kb) + 1];
+  if (kb < kTopK) {
+    const int32_t e = keys[token * kTopK + kb], first = offsets[e], row = inverse[token * kTopK + kb];
+    copy_row[kb] = uint32_t(row);
+    copy_local[kb] = uint32_t(row - first);
+    copy_region[kb] = uint32_t(first / 128 + e);
+    copy_scale[0][kb] = experts[e].inverse_input_scale[0];
+    copy_scale[1][kb] = experts[e].inverse_input_scale[1];
   }
-  uint32_t raw[kPerLane][8];
-  float amax[kPerLane];
+  const uint32_t raw[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  float amax = 0.0F;
 #pragma unroll
-  for (int i = 0; i < kPerLane; ++i) {
-    const uint32_t local = lane + 32 * i;
-    const uint32_t kb = half * kHalfBlocks + local;
-    amax[i] = 0.0F;
-    if (local < kHalfBlocks) {
-      const uint4 a = input[2 * (size_t(token) * kBlocks + kb)], b = input[2 * (size_t(token) * kBlocks + kb) + 1];
-      raw[i][0] = a.x; raw[i][1] = a.y; raw[i][2] = a.z; raw[i][3] = a.w;
-      raw[i][4] = b.x; raw[i][5] = b.y; raw[i][6] = b.z; raw[i][7] = b.w;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        amax[i] = fmaxf(amax[i], fabsf(__uint_as_float(raw[i][k] << 16)));
-        amax[i] = fmaxf(amax[i], fabsf(__uint_as_float(raw[i][k] & 0xFFFF0000u)));
-      }
-    }
+  for (int k = 0; k < 8; ++k) {
+    amax = fmaxf(amax, fabsf(__uint_as_float(raw[k] << 16)));
+    amax = fmaxf(amax, fabsf(__uint_as_float(raw[k] & 0xFFFF0000u)));
   }
+  __syncthreads();
+  const uint32_t warp_mask = kb / 32 == kTokenThreads / 32 ? (1u << (kTokenThreads % 32)) - 1u : 0xffffffffu;
   // The quantised row depends on the input scale only: consecutive copies with the same scale (experts
   // calibrated together, or one scale for the whole layer) reuse the codes of the copy before them.
-  uint32_t out[kPerLane][2];
-  uint8_t scale_code[kPerLane];
+  uint2 out = make_uint2(0, 0);
+  uint32_t scale_word = 0;             // of the four K16 blocks of a scale atom, in the first one's thread
   float quantised_with = -1.0F;        // input scales are positive
+#pragma unroll 1
   for (int j = 0; j < kTopK; ++j) {
-    const int32_t e = __shfl_sync(0xffffffffu, copy_expert, j);
-    const uint32_t row = __shfl_sync(0xffffffffu, copy_row, j);
-    const int32_t first = __shfl_sync(0xffffffffu, copy_first, j);
-    const float scale_of_part[2] = {__shfl_sync(0xffffffffu, copy_scale[0], j), __shfl_sync(0xffffffffu, copy_scale[1], j)};
+    const uint32_t row = copy_row[j], local = copy_local[j];
     for (int part = 0; part < parts; ++part) {
-      const float inverse_scale = scale_of_part[part];
-      const size_t region = (size_t(part) * scale_rows + size_t(first / 128 + e) * 128) * kBlocks;
-      if (inverse_scale != quantised_with) {     // the same for every lane of the warp
+      const float inverse_scale = copy_scale[part][j];
+      if (inverse_scale != quantised_with) {     // the same for the whole block
         quantised_with = inverse_scale;
+        scale_word = float_to_e4m3(inverse_scale * (amax * rcp_approx_ftz(6.0F)));
+        const float block_scale = e4m3_to_float(uint8_t(scale_word));
+        const float factor =
+            block_scale == 0.0F ? 0.0F : rcp_approx_ftz(block_scale * rcp_approx_ftz(inverse_scale));
+        uint32_t words[2] = {0, 0};
 #pragma unroll
-        for (int i = 0; i < kPerLane; ++i) {
-          scale_code[i] = float_to_e4m3(inverse_scale * (amax[i] * rcp_approx_ftz(6.0F)));
-          const float block_scale = e4m3_to_float(scale_code[i]);
-          const float factor =
-              block_scale == 0.0F ? 0.0F : rcp_approx_ftz(block_scale * rcp_approx_ftz(inverse_scale));
-          out[i][0] = out[i][1] = 0;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            out[i][k / 4] |= uint32_t(float2_to_e2m1x2(__uint_as_float(raw[i][k] << 16) * factor,
-                                                       __uint_as_float(raw[i][k] & 0xFFFF0000u) * factor)) << (8 * (k % 4));
-        }
+        for (int k = 0; k < 8; ++k)
+          words[k / 4] |= uint32_t(float2_to_e2m1x2(__uint_as_float(raw[k] << 16) * factor,
+                                                    __uint_as_float(raw[k] & 0xFFFF0000u) * factor)) << (8 * (k % 4));
+        out = make_uint2(words[0], words[1]);
+        scale_word |= __shfl_down_sync(warp_mask, scale_word, 1) << 8;
+        scale_word |= __shfl_down_sync(warp_mask, scale_word, 2) << 16;
       }
-#pragma unroll
-      for (int i = 0; i < kPerLane; ++i) {
-        const uint32_t local = lane + 32 * i;
-        const uint32_t kb = half * kHalfBlocks + local;
-        if (local >= kHalfBlocks) continue;
-        packed[(size_t(part) * n + row) * kBlocks + kb] = make_uint2(out[i][0], out[i][1]);
-        scales[region + scale_offset(row - first, kb, kHidden)] = scale_code[i];
+      packed[(size_t(part) * n + row) * kTokenThreads + kb] = out;
+      if (kb % 4 == 0) {
+        const size_t region = (size_t(part) * scale_rows + size_t(copy_region[j]) * 128) * kTokenThreads;
+        *reinterpret_cast<uint32_t*>(scales + region + scale_offset(local, kb, kHidden)) = scale_word;
       }
     }
   }
@@ -1379,7 +1355,7 @@ cudaError_t launch_moe_quantize_tokens(const void* input, const int32_t* keys, c
                                        const int32_t* offsets, const MoeExpertInfo* experts, uint32_t tokens,
                                        uint32_t scale_rows, int parts, uint8_t* packed, uint8_t* scales,
                                        cudaStream_t stream) {
-  launch_pdl(moe_quantize_tokens_kernel, blocks_for(size_t(tokens) * 64), 256, stream, 
+  launch_pdl(moe_quantize_tokens_kernel, tokens, kTokenThreads, stream,
       static_cast<const uint4*>(input), keys, inverse, offsets, experts, tokens, scale_rows, parts,
       reinterpret_cast<uint2*>(packed), scales);
   return cudaGetLastError();
