@@ -74,17 +74,19 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 
 // W4A16.  An E2M1 code's three magnitude bits, put at bits 8..6 of a BF16 pattern, are the value times
 // 2^-126 (the code for 0.5 lands on a subnormal, as it is one in E2M1 too); multiplying by the block scale
-// times 2^118 gives value x scale x 2^-8 exactly, and the epilogue's multiplier carries the 2^8.  Nibbles j
+// times 2^118 gives value x scale x 2^-8 exactly, and the epilogue's multiplier carries the 2^8.  A multiplication puts the
+// sign and the magnitude of a pair of nibbles in their places at once, which leaves nine instructions of eight codes to the
+// ALU, the pipe that bounds the kernel, instead of twelve (MLP of one row 63.0 -> 59.8 us).  Nibbles j
 // and j + 4 of a word share their shifts, so a pair holds values j and j + 4 (the tokens are stored in the
 // same order).
 constexpr float kW4a16Exponent = 0x1p118F;
 constexpr float kW4a16Alpha = 256.0F;
 __device__ __forceinline__ void e2m1x8_to_bf16(uint32_t word, uint32_t* r) {
-  const uint32_t b = word * 16u, c = word * 256u, d = word * 4096u;
-  r[0] = (d & 0x80008000u) | ((d >> 6) & 0x01C001C0u);
-  r[1] = (c & 0x80008000u) | ((c >> 6) & 0x01C001C0u);
-  r[2] = (b & 0x80008000u) | ((b >> 6) & 0x01C001C0u);
-  r[3] = (word & 0x80008000u) | ((word >> 6) & 0x01C001C0u);
+  const uint32_t high = word >> 8;
+  r[0] = ((word & 0x000F000Fu) * 0x1040u) & 0x81C081C0u;       // x << 12 for the sign, x << 6 for the magnitude
+  r[1] = ((word & 0x00F000F0u) * 0x0104u) & 0x81C081C0u;
+  r[2] = ((high & 0x000F000Fu) * 0x1040u) & 0x81C081C0u;
+  r[3] = ((high & 0x00F000F0u) * 0x0104u) & 0x81C081C0u;
 }
 
 // two E4M3 block scales (the low half of the word) -> one pair (s, s) per scale, in the format of the kind's multiplication
