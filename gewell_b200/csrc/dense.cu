@@ -160,27 +160,27 @@ namespace {
 // FP8 and BF16 with more rows than the swap form takes: channels on the lanes of a CTA pair.
 gw_status launch_dense_pair_wide(const DenseProblem& q, uint64_t row_bytes, DenseDescriptors* cache, cudaStream_t stream) {
   std::string error;
-  if (cache->token_tile == 0) cache->token_tile = pair_wide_tile_rows(q.rows, q.n, sm_count());
+  if (cache->wide.tile_rows == 0) cache->wide = pair_wide_tiles(q.rows, q.n, sm_count());
   if (cache->weight_half != q.weight) {
     if (!encode_tensor_map_2d(&cache->weight_half_map, q.weight, row_bytes, q.n, 128, &error))
       return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
     cache->weight_half = q.weight;
   }
   if (cache->activations != q.activations) {
-    if (!encode_tensor_map_2d(&cache->activation_map, q.activations, row_bytes, q.rows, uint32_t(cache->token_tile / 2), &error))
+    if (!encode_tensor_map_2d(&cache->activation_map, q.activations, row_bytes, q.rows, uint32_t(cache->wide.tile_rows / 2), &error) ||
+        !encode_tensor_map_2d(&cache->piece_map, q.activations, row_bytes, q.rows, uint32_t(cache->wide.piece_rows / 2), &error))
       return fail(GW_CUDA_ERROR, "activation descriptor: " + error);
     cache->activations = q.activations;
   }
   PairWideParams pair{};
   pair.map_weights = cache->weight_half_map;
   pair.map_tokens = cache->activation_map;
+  pair.map_piece = cache->piece_map;
   pair.k_stages = int32_t((row_bytes + 127) / 128);
   pair.last_kb = int32_t((row_bytes - uint64_t(pair.k_stages - 1) * 128 + 31) / 32);
   pair.rows = int32_t(q.rows);
   pair.n = int32_t(q.n);
-  pair.channel_tiles = int32_t((q.n + 255) / 256);
-  pair.token_tiles = int32_t((q.rows + cache->token_tile - 1) / cache->token_tile);
-  pair.tile_rows = cache->token_tile;
+  pair.tiles = cache->wide;
   pair.out = q.output;
   pair.ld_out = q.n;
   pair.alpha = q.alpha;
@@ -452,25 +452,26 @@ gw_status launch_dense_geglu(const GegluProblem& q, DenseDescriptors* cache, cud
 gw_status launch_dense_geglu_wide(const WideGegluProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
   std::string error;
   const uint64_t row_bytes = q.kind == GemmKind::bf16 ? uint64_t(2) * q.k : q.k;
-  if (cache->geglu_tile == 0) cache->geglu_tile = pair_wide_tile_rows(q.rows, 2 * q.n, sm_count());
+  if (cache->geglu_wide.tile_rows == 0) cache->geglu_wide = pair_wide_tiles(q.rows, 2 * q.n, sm_count());
   const void* from[3] = {q.activations, q.weight[0], q.weight[1]};
   for (int i = 0; i < 3; ++i)
     if (cache->geglu_from[i] != from[i]) {
-      if (!encode_tensor_map_2d(&cache->geglu_maps[i], from[i], row_bytes, i == 0 ? q.rows : q.n, i == 0 ? uint32_t(cache->geglu_tile / 2) : 64, &error))
+      if (!encode_tensor_map_2d(&cache->geglu_maps[i], from[i], row_bytes, i == 0 ? q.rows : q.n, i == 0 ? uint32_t(cache->geglu_wide.tile_rows / 2) : 64, &error))
+        return fail(GW_CUDA_ERROR, "gate/up descriptor: " + error);
+      if (i == 0 && !encode_tensor_map_2d(&cache->geglu_piece_map, from[0], row_bytes, q.rows, uint32_t(cache->geglu_wide.piece_rows / 2), &error))
         return fail(GW_CUDA_ERROR, "gate/up descriptor: " + error);
       cache->geglu_from[i] = from[i];
     }
   PairWideParams pair{};
   pair.map_tokens = cache->geglu_maps[0];
+  pair.map_piece = cache->geglu_piece_map;
   pair.map_weights = cache->geglu_maps[1];
   pair.map_up = cache->geglu_maps[2];
   pair.k_stages = int32_t((row_bytes + 127) / 128);
   pair.last_kb = int32_t((row_bytes - uint64_t(pair.k_stages - 1) * 128 + 31) / 32);
   pair.rows = int32_t(q.rows);
   pair.n = int32_t(q.n);
-  pair.channel_tiles = int32_t((q.n + 127) / 128);
-  pair.token_tiles = int32_t((q.rows + cache->geglu_tile - 1) / cache->geglu_tile);
-  pair.tile_rows = cache->geglu_tile;
+  pair.tiles = cache->geglu_wide;
   pair.out = q.output;
   pair.ld_out = q.n;
   pair.alpha = q.alpha[0];

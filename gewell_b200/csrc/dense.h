@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "decode_stream.h"
+#include "gemm_pair_wide.h"
 #include "gemm_tc.cuh"
 
 namespace gw {
@@ -36,9 +37,11 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   CUtensorMap weight_map{}, activation_map{}, weight_scale_map{};
   const void* weight_half = nullptr;
   CUtensorMap weight_half_map{};     // 128-row box over the weights (CTA-pair kernel: each CTA stages half a tile)
-  int token_tile = 0;                // FP8 / BF16 CTA-pair kernel: token columns per tile
-  // the GeGLU forms (launch_dense_geglu, launch_dense_geglu_wide): token columns per tile; the activations, gate and up
-  int geglu_tile = 0;
+  PairWideTiles wide;                // FP8 / BF16 CTA-pair kernel: division of the work
+  CUtensorMap piece_map{};           // and its box over the activations for the pieces of tiles
+  // the GeGLU forms (launch_dense_geglu, launch_dense_geglu_wide): division; the activations (and pieces of them), gate and up
+  PairWideTiles geglu_wide;
+  CUtensorMap geglu_piece_map{};
   const void* geglu_from[3] = {};
   CUtensorMap geglu_maps[3]{};
   // Split mode: one arrival counter per weight tile, owned by the plan (device memory,

@@ -68,12 +68,26 @@ __device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uin
 
 // Work item -> tile.  Eight token tiles at a time go through all channels, token tile fastest: the pairs that run
 // together (74) then read 8 token tiles and about 9 weight tiles, whatever the larger side of the problem is.
-struct Tile { int channel, token; };
-__device__ __forceinline__ Tile tile_of(const PairWideParams& p, int w) {
-  const int group = w / (kGroupTiles * p.channel_tiles);
-  const int rest = w - group * kGroupTiles * p.channel_tiles;
-  const int width = min(kGroupTiles, p.token_tiles - group * kGroupTiles);
-  return {rest / width, group * kGroupTiles + rest % width};
+// The tiles behind the last whole wave are divided into pieces of fewer tokens, so that all pairs have one.
+struct Tile { int channel, token0, width, end; };      // first token, token columns, end of the tokens that it stores
+__device__ __forceinline__ Tile tile_of(const PairWideTiles& t, int rows, int w) {
+  int index = w, piece = 0;
+  const bool whole = w < t.whole;
+  if (!whole) {
+    const int behind = w - t.whole;
+    index = t.whole + behind / t.pieces;
+    piece = behind % t.pieces;
+  }
+  const int group = index / (kGroupTiles * t.channel_tiles);
+  const int rest = index - group * kGroupTiles * t.channel_tiles;
+  const int across = min(kGroupTiles, t.token_tiles - group * kGroupTiles);
+  const int tile0 = (group * kGroupTiles + rest % across) * t.tile_rows;
+  const int width = whole ? t.tile_rows : t.piece_rows;
+  const int token0 = tile0 + piece * width;
+  return {rest / across, token0, width, min(min(token0 + width, tile0 + t.tile_rows), rows)};
+}
+__host__ __device__ __forceinline__ int work_items(const PairWideTiles& t) {
+  return t.whole + (t.channel_tiles * t.token_tiles - t.whole) * t.pieces;
 }
 
 // barrier of one half of the epilogue warps with a vote: whether one of its threads gave up, so that all of them leave together
@@ -120,21 +134,21 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   griddep_enter();
   const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
-  const int total_work = p.channel_tiles * p.token_tiles;
+  const int total_work = work_items(p.tiles);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
     if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      const int token_half = p.tile_rows / 2;
-      const uint32_t bytes = 2 * (kWgtBytes + uint32_t(token_half) * 128);      // of both CTAs
       const uint32_t leader_full = leader_address(full_bar);
       for (int w = pair; w < total_work && !abort_flag; w += pairs) {
-        const Tile tile = tile_of(p, w);
+        const Tile tile = tile_of(p.tiles, p.rows, w);
         // GeGLU: 64 gate rows, then the up rows of the same channels
         const int weight_row = (tile.channel * 2 + int(rank)) * (kGeglu ? 64 : 128);
-        const int token_row = tile.token * p.tile_rows + int(rank) * token_half;
+        const int token_row = tile.token0 + int(rank) * (tile.width / 2);
+        const uint32_t bytes = 2 * (kWgtBytes + uint32_t(tile.width / 2) * 128);  // of both CTAs
+        const CUtensorMap* map_tokens = w < p.tiles.whole ? &p.map_tokens : &p.map_piece;
         bool failed = false;
         for (int ks = 0; ks < p.k_stages; ++ks) {
           if (!ptx::mbar_wait_bounded(empty_bar + stage, phase ^ 1)) {
@@ -146,7 +160,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
           if (rank == 0) ptx::mbar_expect_tx(full_bar + stage, bytes);       // rows beyond a matrix arrive as zeros
           tma_load_pair(base, &p.map_weights, ks * 128, weight_row, leader_full + stage * 8);
           if constexpr (kGeglu) tma_load_pair(base + kWgtBytes / 2, &p.map_up, ks * 128, weight_row, leader_full + stage * 8);
-          tma_load_pair(base + kWgtBytes, &p.map_tokens, ks * 128, token_row, leader_full + stage * 8);
+          tma_load_pair(base + kWgtBytes, map_tokens, ks * 128, token_row, leader_full + stage * 8);
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
         if (failed) break;
@@ -159,7 +173,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       int stage = 0, turn = 0;
       uint32_t phase = 0;
       // FP32 accumulator, E4M3 or BF16 operands, M = 256 across the pair
-      const uint32_t idesc = (1u << 4) | (FP8 ? 0u : (1u << 7) | (1u << 10)) | ((uint32_t(p.tile_rows) >> 3) << 17) | ((256u >> 4) << 24);
+      const uint32_t idesc_of_width = (1u << 4) | (FP8 ? 0u : (1u << 7) | (1u << 10)) | ((256u >> 4) << 24);
       const uint32_t smem_base16 = ptx::smem_u32(smem) >> 4;
       bool failed = false;
       for (int w = pair; w < total_work && !failed; w += pairs, ++turn) {
@@ -170,6 +184,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         }
         ptx::tc_fence_after_sync();
         const uint32_t d = tmem_base + acc * kAccCols;
+        const uint32_t idesc = idesc_of_width | ((uint32_t(w < p.tiles.whole ? p.tiles.tile_rows : p.tiles.piece_rows) >> 3) << 17);
         for (int ks = 0; ks < p.k_stages; ++ks) {
           if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(full_bar + stage, phase))) {
             report(p.error, 0x35000000u | (blockIdx.x << 8) | stage, &abort_flag);
@@ -206,7 +221,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
     int turn = 0;
     for (int w = pair; w < total_work; w += pairs, ++turn) {
       const int acc = turn & 1;
-      const Tile tile = tile_of(p, w);
+      const Tile tile = tile_of(p.tiles, p.rows, w);
       const int channel0 = (tile.channel * 2 + int(rank)) * 64;
       const int mine = channel0 + quad % 2 * 32 + lane;
       const float scale = channel_alpha == nullptr ? (quad < 2 ? p.alpha : p.alpha_up) : mine < p.n ? __ldg(channel_alpha + mine) : 0.0F;
@@ -215,9 +230,9 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       if (half_barrier_any(half, !arrived)) break;
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + acc * kAccCols + (uint32_t(quad * 32) << 16);
-      for (int t0 = half * 32; t0 < p.tile_rows; t0 += 64) {
-        const int token0 = tile.token * p.tile_rows + t0;
-        if (token0 >= p.rows) break;                                // the whole half
+      for (int t0 = half * 32; t0 < tile.width; t0 += 64) {
+        const int token0 = tile.token0 + t0;
+        if (token0 >= tile.end) break;                                // the whole half
         uint32_t r[32];
         ptx::tmem_load16(taddr + t0, r);
         ptx::tmem_load16(taddr + t0 + 16, r + 16);
@@ -231,7 +246,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         }
         half_barrier(half);
         const int token = token0 + tid / 4, channel = channel0 + tid % 4 * 16;
-        if (token >= p.rows || channel >= p.n) continue;
+        if (token >= tile.end || channel >= p.n) continue;
         const uint32_t from = ptx::smem_u32(staging) + uint32_t(tid / 4) * kPitch + uint32_t(tid % 4) * 32;
         uint32_t words[8];
 #pragma unroll
@@ -270,7 +285,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
     int turn = 0;
     for (int w = pair; w < total_work && !abort_flag; w += pairs, ++turn) {
       const int acc = turn & 1;
-      const Tile tile = tile_of(p, w);
+      const Tile tile = tile_of(p.tiles, p.rows, w);
       const int channel0 = (tile.channel * 2 + int(rank)) * 128 + quad * 32;
       const float scale = p.channel_alpha == nullptr ? p.alpha : channel0 + lane < p.n ? __ldg(p.channel_alpha + channel0 + lane) : 0.0F;
       if (!ptx::mbar_wait_warp(acc_full_bar + acc, uint32_t(turn >> 1) & 1u)) {
@@ -281,15 +296,15 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       const uint32_t taddr = tmem_base + acc * kAccCols + (uint32_t(quad * 32) << 16);
       // A lane has one channel of 32 tokens and stores them one by one, the warp 64 contiguous bytes of a token.
       const bool inside = channel0 + lane < p.n;
-      for (int t0 = half * 32; t0 < p.tile_rows; t0 += 64) {
-        const int token0 = tile.token * p.tile_rows + t0;
-        if (token0 >= p.rows) break;                                // warp-uniform
+      for (int t0 = half * 32; t0 < tile.width; t0 += 64) {
+        const int token0 = tile.token0 + t0;
+        if (token0 >= tile.end) break;                                // warp-uniform
         uint32_t r[32];
         ptx::tmem_load16(taddr + t0, r);
         ptx::tmem_load16(taddr + t0 + 16, r + 16);
         ptx::tmem_load_wait();
         bf16* dst = out + size_t(token0) * p.ld_out + channel0 + lane;
-        const int left = inside ? p.rows - token0 : 0;
+        const int left = inside ? tile.end - token0 : 0;
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           if (i < left) *dst = __float2bfloat16_rn(__fmul_rn(__uint_as_float(r[i]), scale));
@@ -320,7 +335,7 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
     if (status != cudaSuccess) return status;
     configured = true;
   }
-  const int work = params.channel_tiles * params.token_tiles;
+  const int work = work_items(params.tiles);
   const int pairs = work < sm_count / 2 ? work : sm_count / 2;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(2 * pairs);
@@ -342,24 +357,40 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
 
 }  // namespace
 
-int pair_wide_tile_rows(uint32_t rows, uint32_t n, int sm_count) {
+PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int sm_count) {
   // A tile takes as long as its weight rows and MMA issue cost whatever its width (about 136 columns) plus its columns:
   // measured on FP8 K=5376, per wave of tiles of 64 / 128 / 192 / 256 tokens 8.9 / 11.3 / 14.3 / 17.4 us.
-  const uint64_t channel_tiles = (n + 255) / 256, pairs = uint64_t(sm_count / 2);
-  int best = 256;
+  const int channel_tiles = int((n + 255) / 256), pairs = sm_count / 2;
+  PairWideTiles t{};
   uint64_t best_cost = ~0ull;
   for (int tile = 256; tile >= 64; tile -= 32) {
-    const uint64_t tiles = channel_tiles * ((rows + tile - 1) / tile);
+    const int token_tiles = int((rows + tile - 1) / tile);
+    const uint64_t tiles = uint64_t(channel_tiles) * token_tiles;
     const uint64_t cost = (tiles + pairs - 1) / pairs * uint64_t(tile + 136);
-    if (cost < best_cost) { best_cost = cost; best = tile; }
+    if (cost < best_cost) {
+      best_cost = cost;
+      t = {tile, channel_tiles, token_tiles, int32_t(tiles), 1, tile};
+    }
   }
-  return best;
+  // A last wave for half of the pairs or fewer: its tiles in as many pieces as keep every pair at work, 32 columns or a multiple.
+  // us, whole tiles / pieces: FP8 250x5376x21504 (74 + 10 tiles) 37.2 / 32.9, 180 rows 32.5 / 30.7, BF16 200 rows 59.2 / 55.0,
+  // 4096x2816x4096 (222 + 34) 65.1 / 62.5, FP8 1025x5376x16384 (296 + 24) 76.0 / 75.5.  A wave with few tiles is quicker than a
+  // full one, so that a tile width chosen for its pieces loses (BF16 2048x2816x2816, 256 wide and four pieces against 160 wide
+  // 25.4 / 27.4).
+  const int behind = t.whole % pairs;
+  if (t.whole > pairs && behind > 0 && behind <= pairs / 2) {
+    const int most = pairs / behind;
+    t.whole -= behind;
+    t.piece_rows = ((t.tile_rows + most - 1) / most + 31) / 32 * 32;
+    t.pieces = (t.tile_rows + t.piece_rows - 1) / t.piece_rows;
+  }
+  return t;
 }
 
 namespace {
 PairWideParams with_ring(const PairWideParams& given, bool geglu) {
   PairWideParams params = given;
-  params.stage_bytes = kWgtBytes + given.tile_rows * 64;
+  params.stage_bytes = kWgtBytes + given.tiles.tile_rows * 64;
   const int fit = ring_bytes(geglu) / params.stage_bytes;
   params.stages = fit < kMaxStages ? fit : kMaxStages;
   return params;

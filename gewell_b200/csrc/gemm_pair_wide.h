@@ -9,13 +9,22 @@
 
 namespace gw {
 
+// Division of [token tiles x channel tiles] over the pairs.
+struct PairWideTiles {
+  int32_t tile_rows = 0;           // token columns per tile (0: not computed yet)
+  int32_t channel_tiles, token_tiles;
+  int32_t whole;                   // tiles that are taken whole: as many as fill waves of all pairs
+  int32_t pieces, piece_rows;      // of each tile behind them: how many pieces, and their token columns
+};
+
 struct PairWideParams {
   CUtensorMap map_weights;         // weights [n, k], box 128 rows x 128 bytes, 128-byte swizzle
   CUtensorMap map_tokens;          // activations [rows, k], box tile_rows / 2 rows
+  CUtensorMap map_piece;           // the same, box piece_rows / 2 rows
   int32_t k_stages;                // 128-byte slabs of K
   int32_t last_kb;                 // 32-byte K blocks in the last one
   int32_t rows, n;
-  int32_t channel_tiles, token_tiles, tile_rows;
+  PairWideTiles tiles;
   int32_t stages, stage_bytes;     // of the operand ring (set by the launch)
   void* out;                       // BF16 [rows, ld_out], 16-byte aligned rows
   int64_t ld_out;
@@ -28,11 +37,11 @@ struct PairWideParams {
   uint32_t* error;
 };
 
-// Tokens per tile for this shape: the number whose whole waves of pair tiles take least.
-int pair_wide_tile_rows(uint32_t rows, uint32_t n, int sm_count);
+// The division for this shape that takes least: `n` channels, 256 per tile.
+PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int sm_count);
 
-// GeGLU of two projections with n channels each, as BF16 [rows, n] or (`quantise`) E4M3 [rows, n].  n is a multiple of 64,
-// channel_tiles counts 128 channels.
+// GeGLU of two projections with n channels each, as BF16 [rows, n] or (`quantise`) E4M3 [rows, n].  n is a multiple of 64, a tile
+// has 128 channels of each.
 cudaError_t launch_gemm_pair_wide_geglu(bool fp8, bool quantise, const PairWideParams& params, int sm_count, cudaStream_t stream);
 
 cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& params, int sm_count, cudaStream_t stream);

@@ -68,3 +68,10 @@ def test_fused_equals_separate_launches(gw, monkeypatch, storage, joined, rows, 
         assert gw.kernel_error() == 0
         results.append(bits(y))
     assert_gemm_close(results[0], results[1], f"{storage} {rows}x{hidden}->{mlp}")
+
+
+@pytest.mark.parametrize("storage", ["fp8 channel", "bf16", "bf16 fp8"])
+@pytest.mark.parametrize("rows,mlp", [(250, 9728), (300, 9600)])
+def test_last_wave_in_pieces(gw, monkeypatch, storage, rows, mlp):
+    """Two or a few tiles behind the last whole wave of 148 SMs, in pieces of 32 tokens."""
+    test_fused_equals_separate_launches(gw, monkeypatch, storage, True, rows, 128, mlp)

@@ -32,3 +32,10 @@ def test_pair(kind, rows, k, n):
     torch.cuda.synchronize()
     assert gw.kernel_error() == 0 and torch.all(y[-64:] == -7.0)
     assert_gemm_close(bits(y[:-64]).reshape(rows, n), want, f"{kind} rows={rows} K={k} N={n}")
+
+
+@pytest.mark.parametrize("kind", ["fp8", "bf16"])
+@pytest.mark.parametrize("rows,n", [(250, 19456), (200, 28160), (256, 43008), (300, 19216)])
+def test_last_wave_in_pieces(kind, rows, n):
+    """Tiles behind the last whole wave (of 148 SMs), cut into eight, two, three and five pieces; the last pieces are cut short or empty."""
+    test_pair(kind, rows, 80, n)
