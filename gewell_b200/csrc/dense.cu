@@ -160,7 +160,7 @@ namespace {
 // FP8 and BF16 with more rows than the swap form takes: channels on the lanes of a CTA pair.
 gw_status launch_dense_pair_wide(const DenseProblem& q, uint64_t row_bytes, DenseDescriptors* cache, cudaStream_t stream) {
   std::string error;
-  if (cache->wide.tile_rows == 0) cache->wide = pair_wide_tiles(q.rows, q.n, sm_count());
+  if (cache->wide.tile_rows == 0) cache->wide = pair_wide_tiles(q.rows, q.n, int((row_bytes + 127) / 128), sm_count());
   if (cache->weight_half != q.weight) {
     if (!encode_tensor_map_2d(&cache->weight_half_map, q.weight, row_bytes, q.n, 128, &error))
       return fail(GW_CUDA_ERROR, "weight descriptor: " + error);
@@ -452,7 +452,7 @@ gw_status launch_dense_geglu(const GegluProblem& q, DenseDescriptors* cache, cud
 gw_status launch_dense_geglu_wide(const WideGegluProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
   std::string error;
   const uint64_t row_bytes = q.kind == GemmKind::bf16 ? uint64_t(2) * q.k : q.k;
-  if (cache->geglu_wide.tile_rows == 0) cache->geglu_wide = pair_wide_tiles(q.rows, 2 * q.n, sm_count());
+  if (cache->geglu_wide.tile_rows == 0) cache->geglu_wide = pair_wide_tiles(q.rows, 2 * q.n, 0, sm_count());
   const void* from[3] = {q.activations, q.weight[0], q.weight[1]};
   for (int i = 0; i < 3; ++i)
     if (cache->geglu_from[i] != from[i]) {

@@ -19,6 +19,8 @@
 //             shared memory may count there before the leader expects them: only its arrival closes the phase)
 //   empty[s], acc_full[a]   local; signalled in both CTAs at once by the leader's tcgen05.commit
 //   acc_empty[a]   in the leader, 16 arrivals (epilogue warps of both CTAs)
+// The split form is for a few tiles with a long K: two to four pairs in one cluster each have a part of a tile's K slabs and add
+// their FP32 sums up through each other's shared memory (BF16 401x6480x560 22.6 -> 12.1 us).
 // Every wait is bounded; the kernel ends with a cluster barrier before tensor memory is released.  No load fans
 // out to other CTAs.
 #include "common.cuh"
@@ -41,7 +43,11 @@ constexpr int kAccCols = 256, kTmemCols = 512;
 constexpr int kPitch = 256 + 16, kStagingBytes = 32 * kPitch;
 constexpr int ring_bytes(bool geglu) { return 221 * 1024 - (geglu ? 2 * kStagingBytes : 0); }
 constexpr int kSmemBytes = 221 * 1024 + 1024;
-enum class WideOut { store, geglu, geglu_fp8 };
+constexpr int kMaxSplit = 4;
+constexpr int kPartBytes = 128 * 32 * 4;             // one pair's FP32 part of 32 tokens
+static_assert(4 * kPartBytes <= ring_bytes(false) && 3 * 2 * kPartBytes <= ring_bytes(false) && 2 * 3 * kPartBytes <= ring_bytes(false),
+              "the parts that a pair sums in a split by two, three and four");
+enum class WideOut { store, split, geglu, geglu_fp8 };
 constexpr int kGroupTiles = 8;                     // token tiles that are walked together
 constexpr uint32_t kDescHiSw128 = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);   // SBO 1024 B, version 1, SWIZZLE_128B
 
@@ -102,14 +108,15 @@ __device__ __forceinline__ void half_barrier(int half) { asm volatile("bar.sync 
 template <bool FP8, WideOut OUT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
-  constexpr bool kGeglu = OUT != WideOut::store;
+  constexpr bool kGeglu = OUT == WideOut::geglu || OUT == WideOut::geglu_fp8, kSplit = OUT == WideOut::split;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], acc_full_bar[2], acc_empty_bar[2];
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
-  const uint32_t rank = cluster_rank();           // 0 = leader of the pair
+  // Rank in the pair (0 = leader) and the leader's in the cluster; a cluster is one pair, or p.tiles.split of them.
+  const uint32_t cta = cluster_rank(), rank = kSplit ? cta & 1u : cta, leader = kSplit ? cta & ~1u : 0u;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
       ptx::mbar_init(full_bar + s, 1);
@@ -133,15 +140,18 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
   griddep_enter();
-  const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
+  const int pairs = kSplit ? gridDim.x / (2 * p.tiles.split) : gridDim.x / 2, pair = kSplit ? blockIdx.x / (2 * p.tiles.split) : blockIdx.x / 2;
   const int total_work = work_items(p.tiles);
+  // Split: one tile per cluster, an even part of its K slabs per pair
+  const int first_ks = kSplit ? int(leader / 2) * p.k_stages / p.tiles.split : 0;
+  const int end_ks = kSplit ? int(leader / 2 + 1) * p.k_stages / p.tiles.split : p.k_stages;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
     if (ptx::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
-      const uint32_t leader_full = leader_address(full_bar);
+      const uint32_t leader_full = cluster_address(full_bar, leader);
       for (int w = pair; w < total_work && !abort_flag; w += pairs) {
         const Tile tile = tile_of(p.tiles, p.rows, w);
         // GeGLU: 64 gate rows, then the up rows of the same channels
@@ -150,7 +160,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         const uint32_t bytes = 2 * (kWgtBytes + uint32_t(tile.width / 2) * 128);  // of both CTAs
         const CUtensorMap* map_tokens = w < p.tiles.whole ? &p.map_tokens : &p.map_piece;
         bool failed = false;
-        for (int ks = 0; ks < p.k_stages; ++ks) {
+        for (int ks = first_ks; ks < end_ks; ++ks) {
           if (!ptx::mbar_wait_bounded(empty_bar + stage, phase ^ 1)) {
             report(p.error, 0x15000000u | (blockIdx.x << 8) | stage, &abort_flag);
             failed = true;
@@ -185,7 +195,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         ptx::tc_fence_after_sync();
         const uint32_t d = tmem_base + acc * kAccCols;
         const uint32_t idesc = idesc_of_width | ((uint32_t(w < p.tiles.whole ? p.tiles.tile_rows : p.tiles.piece_rows) >> 3) << 17);
-        for (int ks = 0; ks < p.k_stages; ++ks) {
+        for (int ks = first_ks; ks < end_ks; ++ks) {
           if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(full_bar + stage, phase))) {
             report(p.error, 0x35000000u | (blockIdx.x << 8) | stage, &abort_flag);
             failed = true;
@@ -198,13 +208,13 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
             const uint64_t a = make_desc(base16), b = make_desc(base16 + (kWgtBytes >> 4));
 #pragma unroll
             for (int kb = 0; kb < 4; ++kb)
-              if (kb < nkb) mma_pair<FP8>(d, a + 2 * kb, b + 2 * kb, idesc, (ks | kb) != 0 ? 1u : 0u);
-            commit_pair(empty_bar + stage);
+              if (kb < nkb) mma_pair<FP8>(d, a + 2 * kb, b + 2 * kb, idesc, ((ks - first_ks) | kb) != 0 ? 1u : 0u);
+            commit_pair(empty_bar + stage, leader);
           }
           __syncwarp();
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
-        if (!failed && ptx::elect_one()) commit_pair(acc_full_bar + acc);
+        if (!failed && ptx::elect_one()) commit_pair(acc_full_bar + acc, leader);
       }
     }
     __syncwarp();
@@ -276,6 +286,8 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       __syncwarp();
       if (lane == 0) arrive_cluster(leader_acc_empty + acc * 8);
     }
+  } else if (kSplit && warp >= kFirstEpilogueWarp) {
+    if (!ptx::mbar_wait_warp(acc_full_bar, 0)) report(p.error, 0x55000000u | (blockIdx.x << 8), &abort_flag);
   } else if (warp >= kFirstEpilogueWarp) {
     // ------------------------------------------------------------------ epilogue (own 128 channels x tile_rows tokens)
     const int quad = warp % 4;
@@ -317,6 +329,64 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
     }
   }
 
+  if constexpr (kSplit) {
+    // ------------------------------------------------------------------ sum of the pairs' parts
+    // Chunk c of 32 tokens is summed and stored by pair c % split: the other pairs write their 128 x 32 FP32 values of it into
+    // that pair's operand ring, [token / 4][lane][token % 4], once every pair's MMAs have read theirs.
+    __syncwarp();
+    ptx::tc_fence_before_sync();
+    cluster_sync_all();
+    ptx::tc_fence_after_sync();
+    const int split = p.tiles.split, part = int(leader / 2), quad = warp % 4, half = (warp - kFirstEpilogueWarp) / 4;
+    const Tile tile = tile_of(p.tiles, p.rows, pair);
+    const int chunks = (tile.end - tile.token0 + 31) / 32;
+    const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16);
+    const uint32_t at = uint32_t(quad * 32 + lane) * 16;
+    if (warp >= kFirstEpilogueWarp) {
+      for (int c = half; c < chunks; c += 2) {
+        const int owner = c % split;
+        if (owner == part) continue;
+        uint32_t r[32];
+        ptx::tmem_load16(taddr + 32 * c, r);
+        ptx::tmem_load16(taddr + 32 * c + 16, r + 16);
+        ptx::tmem_load_wait();
+        const int slot = c / split * (split - 1) + (part < owner ? part : part - 1);
+        const uint32_t to = cluster_address(smem + slot * kPartBytes, uint32_t(2 * owner) + rank) + at;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) store_cluster(to + i * (128 * 16), r + 4 * i);
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= kFirstEpilogueWarp && !abort_flag) {
+      const int channel = (tile.channel * 2 + int(rank)) * 128 + quad * 32 + lane;
+      const float scale = p.channel_alpha == nullptr ? p.alpha : channel < p.n ? __ldg(p.channel_alpha + channel) : 0.0F;
+      for (int k = half, c = part + half * split; c < chunks; k += 2, c += 2 * split) {
+        uint32_t r[32];
+        ptx::tmem_load16(taddr + 32 * c, r);
+        ptx::tmem_load16(taddr + 32 * c + 16, r + 16);
+        ptx::tmem_load_wait();
+        for (int other = 0; other < split - 1; ++other) {
+          const uint32_t from = ptx::smem_u32(smem + (k * (split - 1) + other) * kPartBytes) + at;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 v = ptx::lds128(from + i * (128 * 16));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[4 * i + j] = __float_as_uint(__uint_as_float(r[4 * i + j]) + __uint_as_float(w[j]));
+          }
+        }
+        bf16* dst = static_cast<bf16*>(p.out) + size_t(tile.token0 + 32 * c) * p.ld_out + channel;
+        const int left = channel < p.n ? tile.end - tile.token0 - 32 * c : 0;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          if (i < left) *dst = __float2bfloat16_rn(__fmul_rn(__uint_as_float(r[i]), scale));
+          dst += p.ld_out;
+        }
+      }
+    }
+    __syncwarp();
+  }
   ptx::tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();                               // the peer no longer reads this CTA's shared or tensor memory
@@ -335,8 +405,8 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
     if (status != cudaSuccess) return status;
     configured = true;
   }
-  const int work = work_items(params.tiles);
-  const int pairs = work < sm_count / 2 ? work : sm_count / 2;
+  const int work = work_items(params.tiles), split = params.tiles.split;
+  const int pairs = split > 1 ? work * split : work < sm_count / 2 ? work : sm_count / 2;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(2 * pairs);
   config.blockDim = dim3(kThreads);
@@ -344,7 +414,7 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
   config.stream = stream;
   cudaLaunchAttribute attributes[2]{};
   attributes[0].id = cudaLaunchAttributeClusterDimension;
-  attributes[0].val.clusterDim.x = 2;
+  attributes[0].val.clusterDim.x = 2 * split;
   attributes[0].val.clusterDim.y = 1;
   attributes[0].val.clusterDim.z = 1;
   attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -357,7 +427,35 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
 
 }  // namespace
 
-PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int sm_count) {
+namespace {
+// Clusters of 2 * split CTAs that the GPU holds at once.
+int clusters_at_once(int split) {
+  static int known[kMaxDeviceSlots][kMaxSplit + 1] = {};      // a plain int: two threads write the same
+  int& count = known[current_device_slot()][split];
+  if (count == 0) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(2 * split);
+    config.blockDim = dim3(kThreads);
+    config.dynamicSmemBytes = kSmemBytes;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = 2 * split;
+    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(gemm_pair_wide_kernel<true, WideOut::split>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, gemm_pair_wide_kernel<true, WideOut::split>, &config) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    count = clusters > 0 ? clusters : -1;
+  }
+  return count;
+}
+}  // namespace
+
+PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int k_stages, int sm_count) {
   // A tile takes as long as its weight rows and MMA issue cost whatever its width (about 136 columns) plus its columns:
   // measured on FP8 K=5376, per wave of tiles of 64 / 128 / 192 / 256 tokens 8.9 / 11.3 / 14.3 / 17.4 us.
   const int channel_tiles = int((n + 255) / 256), pairs = sm_count / 2;
@@ -372,6 +470,23 @@ PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int sm_count) {
       t = {tile, channel_tiles, token_tiles, int32_t(tiles), 1, tile};
     }
   }
+  // K shared by the pairs of a cluster, where few wide tiles leave pairs idle and narrower ones would read the weights more often: a
+  // slab of a tile costs what it did, the launch and its barriers about 900 columns more, and 20 per column whose sum another pair
+  // has.  It has to win an eighth, because pairs at work slow each other down.  us, one pair / several, quantiser included: FP8 218x16384x5376 (three pairs, 224 wide) 32.9 / 27.4, 130x21504x5376 38.9 / 29.1, 180x8192x2816 18.0 / 13.4,
+  // BF16 140x5376x2048 19.7 / 12.2, 250x5376x4096 (two, 128 wide) 20.8 / 16.4; outside of the rule BF16 200x2816x8192
+  // 14.4 / 16.7, 491x5376x4096 22.2 / 23.0, FP8 300x2816x2816 9.6 / 10.1, 800x5376x2048 16.0 / 17.2.
+  uint64_t split_cost = (best_cost * uint64_t(k_stages) + 1900) * 7 / 8;
+  for (int split = 2; split <= kMaxSplit && split <= k_stages; ++split)
+    for (int tile = 256; tile >= 64; tile -= 32) {
+      const int token_tiles = int((rows + tile - 1) / tile);
+      const uint64_t tiles = uint64_t(channel_tiles) * token_tiles;
+      const uint64_t cost = uint64_t((k_stages + split - 1) / split) * uint64_t(tile + 136) + 2800 + uint64_t(20 * tile * (split - 1) / split);
+      if (cost < split_cost && tiles * split <= uint64_t(pairs) && int64_t(tiles) <= clusters_at_once(split)) {
+        split_cost = cost;
+        t = {tile, channel_tiles, token_tiles, int32_t(tiles), 1, tile, split};
+      }
+    }
+  if (t.split > 1) return t;
   // A last wave for half of the pairs or fewer: its tiles in as many pieces as keep every pair at work, 32 columns or a multiple.
   // us, whole tiles / pieces: FP8 250x5376x21504 (74 + 10 tiles) 37.2 / 32.9, 180 rows 32.5 / 30.7, BF16 200 rows 59.2 / 55.0,
   // 4096x2816x4096 (222 + 34) 65.1 / 62.5, FP8 1025x5376x16384 (296 + 24) 76.0 / 75.5.  A wave with few tiles is quicker than a
@@ -399,6 +514,8 @@ PairWideParams with_ring(const PairWideParams& given, bool geglu) {
 
 cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& given, int sm_count, cudaStream_t stream) {
   const PairWideParams params = with_ring(given, false);
+  if (params.tiles.split > 1)
+    return fp8 ? launch_instance<true, WideOut::split>(params, sm_count, stream) : launch_instance<false, WideOut::split>(params, sm_count, stream);
   return fp8 ? launch_instance<true, WideOut::store>(params, sm_count, stream) : launch_instance<false, WideOut::store>(params, sm_count, stream);
 }
 

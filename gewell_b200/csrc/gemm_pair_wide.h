@@ -15,6 +15,7 @@ struct PairWideTiles {
   int32_t channel_tiles, token_tiles;
   int32_t whole;                   // tiles that are taken whole: as many as fill waves of all pairs
   int32_t pieces, piece_rows;      // of each tile behind them: how many pieces, and their token columns
+  int32_t split = 1;               // pairs that share the K loop of a tile
 };
 
 struct PairWideParams {
@@ -37,8 +38,8 @@ struct PairWideParams {
   uint32_t* error;
 };
 
-// The division for this shape that takes least: `n` channels, 256 per tile.
-PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int sm_count);
+// The division for this shape that takes least: `n` channels, 256 per tile; k_stages != 0: the K loop may be shared.
+PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int k_stages, int sm_count);
 
 // GeGLU of two projections with n channels each, as BF16 [rows, n] or (`quantise`) E4M3 [rows, n].  n is a multiple of 64, a tile
 // has 128 channels of each.

@@ -25,6 +25,15 @@ __device__ __forceinline__ uint32_t leader_address(const void* local) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"(ptx::smem_u32(local)));
   return remote;
 }
+// address of the same shared-memory location in another CTA of the cluster
+__device__ __forceinline__ uint32_t cluster_address(const void* local, uint32_t cta) {
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(ptx::smem_u32(local)), "r"(cta));
+  return remote;
+}
+__device__ __forceinline__ void store_cluster(uint32_t cluster_address, const uint32_t* v) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_address), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
 // Plain (CTA-scope release) form on purpose: measured on B200, the .release.cluster form of this arrive
 // cost the scale-loader warps about 1000 cycles per stage.  What the arrival publishes is tensor memory
 // written by tcgen05.st, which tcgen05.wait::st and the tcgen05 fences on both sides order.
@@ -50,9 +59,10 @@ __device__ __forceinline__ void mma_pair_nvfp4(uint32_t d, uint64_t a, uint64_t 
       : "memory");
 }
 // arrive on the barrier at this shared-memory offset in both CTAs of the pair once the MMAs issued so far are done
-__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+// (`leader`: the leader's rank in the cluster)
+__device__ __forceinline__ void commit_pair(uint64_t* bar, uint32_t leader = 0) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(ptx::smem_u32(bar)), "h"(uint16_t(3)) : "memory");
+               ::"r"(ptx::smem_u32(bar)), "h"(uint16_t(3u << leader)) : "memory");
 }
 // E2M1 x E2M1 with UE4M3 scales, FP32 accumulate, M = 256 across the pair, K-major operands
 __host__ __device__ constexpr uint32_t idesc_pair_nvfp4(uint32_t n) {

@@ -39,3 +39,10 @@ def test_pair(kind, rows, k, n):
 def test_last_wave_in_pieces(kind, rows, n):
     """Tiles behind the last whole wave (of 148 SMs), cut into eight, two, three and five pieces; the last pieces are cut short or empty."""
     test_pair(kind, rows, 80, n)
+
+
+@pytest.mark.parametrize("kind,rows,k,n", [("fp8", 131, 8208, 272), ("bf16", 257, 4104, 768), ("fp8 per channel", 218, 8208, 5136),
+                                           ("bf16", 300, 4104, 2576), ("fp8", 700, 8208, 272), ("bf16", 140, 4104, 8080)])
+def test_shared_k(kind, rows, k, n):
+    """K over four, four, three, three, three and two pairs (of 148 SMs); channels and tokens that end within a tile."""
+    test_pair(kind, rows, k, n)
