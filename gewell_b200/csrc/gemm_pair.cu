@@ -26,7 +26,9 @@
 // Every wait is bounded; the kernel ends with a cluster barrier before the
 // tensor memory is released.  No load fans out to other CTAs.
 //
-// The second form (kGeglu) computes gate and up of 128 channels and writes their GeGLU quantised for the down projection:
+// The split form is for tiles too few for the pairs and a long K: two to four pairs in one cluster each have a part of a tile's K
+// stages and add their FP32 sums up through each other's shared memory.
+// The GeGLU form (kGeglu) computes gate and up of 128 channels and writes their GeGLU quantised for the down projection:
 // BF16 [rows, gate | up] (86 KB a token at 5376 -> 21504) is neither written nor read, and two launches fewer stand in the
 // chain.  MLP of NVFP4 weights, us, before / after: 300 rows 124 / 114, 1186 314 / 273, 2859 720 / 626; 1000 rows of
 // 1024 -> 2048 22.7 / 20.0.
@@ -55,14 +57,57 @@ constexpr int threads(bool geglu) { return 32 * (kFirstEpilogueWarp + epilogue_w
 constexpr int kAccCols = 256;
 constexpr int kSfSlotCols = kKBlocks * (4 + 8);   // per stage: token scales 4 columns per K block, weight scales 8
 constexpr int kTmemCols = 512;
+constexpr int kMaxSplit = 4;
+constexpr int kPartBytes = 128 * 32 * 4;          // one pair's FP32 part of 32 channels; at most 4, 6, 6 of them in a split by 2, 3, 4
+static_assert(6 * kPartBytes <= kStages * kStageBytes, "the parts that a pair sums take the place of its operands");
 static_assert(kAccCols + kStages * kSfSlotCols <= kTmemCols, "tensor memory over-subscribed");
 constexpr int kBarrierBytes = (4 * kStages + 2) * 8 + 16;
 constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + 1024;
 
+// 32 columns of a lane as BF16
+__device__ __forceinline__ void to_bf16(const uint32_t* r, float alpha, uint4* u) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    u[q] = make_uint4(pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q]), alpha), __fmul_rn(__uint_as_float(r[8 * q + 1]), alpha)),
+                      pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q + 2]), alpha), __fmul_rn(__uint_as_float(r[8 * q + 3]), alpha)),
+                      pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q + 4]), alpha), __fmul_rn(__uint_as_float(r[8 * q + 5]), alpha)),
+                      pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q + 6]), alpha), __fmul_rn(__uint_as_float(r[8 * q + 7]), alpha)));
+}
+
+// A warp's 32 rows x 32 channels (from c0) into the output: four lanes exchange their rows' sixteen bytes, so that a store has 64
+// contiguous bytes of a row.  row0: first of the four lanes' rows.
+__device__ __forceinline__ void store_chunk(bf16* out, int64_t ld_out, int row0, int rows_left, int c0, int n, uint4* u, int lane) {
+  const bool hi = (lane & 2) != 0, lo = (lane & 1) != 0;
+  {
+    const uint4 send_a = hi ? u[0] : u[2], send_b = hi ? u[1] : u[3];
+    const uint4 got_a = shfl_xor_u4(send_a, 2), got_b = shfl_xor_u4(send_b, 2);
+    if (hi) { u[0] = got_a; u[1] = got_b; } else { u[2] = got_a; u[3] = got_b; }
+  }
+  {
+    const uint4 send_a = lo ? u[0] : u[1], send_b = lo ? u[2] : u[3];
+    const uint4 got_a = shfl_xor_u4(send_a, 1), got_b = shfl_xor_u4(send_b, 1);
+    if (lo) { u[0] = got_a; u[2] = got_b; } else { u[1] = got_a; u[3] = got_b; }
+  }
+  const int c = c0 + 8 * (lane & 3);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (i >= rows_left || c >= n) continue;
+    bf16* dst = out + size_t(row0 + i) * ld_out + c;
+    if (c + 8 <= n) {
+      *reinterpret_cast<uint4*>(dst) = u[i];
+    } else {
+      const uint32_t words[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+      for (int e = 0; e < 8; ++e)
+        if (c + e < n) reinterpret_cast<uint16_t*>(dst)[e] = uint16_t(words[e / 2] >> (16 * (e % 2)));
+    }
+  }
+}
+
 // kGeglu: the pair's first CTA stages the gate rows of 128 channels, its second the up rows, so that gate is in the
 // accumulator columns 0..127 and up in 128..255 for the same tokens and channels, and the epilogue writes the quantised GeGLU.
 // kProfile: cycle counters of the tuning aid live in an instantiation of their own.
-template <bool kGeglu, bool kProfile>
+// kSplit: a cluster is p.split pairs, which share the K loop of one tile.
+template <bool kGeglu, bool kProfile, bool kSplit>
 __global__ void __launch_bounds__(threads(kGeglu), 1)
 gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   constexpr int kEpilogueWarps = epilogue_warps(kGeglu);
@@ -79,7 +124,8 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x) / 32, 0), lane = threadIdx.x % 32;
-  const uint32_t rank = cluster_rank();           // 0 = leader of the pair
+  // rank in the pair (0 = leader), and the leader's in the cluster
+  const uint32_t cta = cluster_rank(), rank = kSplit ? cta & 1u : cta, leader = kSplit ? cta & ~1u : 0u;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(full_bar + s, 1);
@@ -107,7 +153,8 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   const int total_kb = p.k / 64;
   const int k_stages = (total_kb + kKBlocks - 1) / kKBlocks;
   const int k_atoms = p.k / 64;
-  const int pairs = gridDim.x / 2, pair = blockIdx.x / 2;
+  const int first_ks = kSplit ? int(leader / 2) * k_stages / p.split : 0, end_ks = kSplit ? int(leader / 2 + 1) * k_stages / p.split : k_stages;
+  const int pairs = kSplit ? gridDim.x / (2 * p.split) : gridDim.x / 2, pair = kSplit ? blockIdx.x / (2 * p.split) : blockIdx.x / 2;
   const int total_work = p.l_tiles * p.c_tiles;
   constexpr uint32_t kDescHiSw128 = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);
   auto make_desc = [](uint32_t hi, uint32_t lo) { return (uint64_t(hi) << 32) | lo; };
@@ -131,7 +178,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
         const int token_block = min(l_tile * 2 + int(rank), p.token_row_blocks - 1);
         const uint8_t* sf_tokens = p.sf_tokens + size_t(token_block) * k_atoms * 512;
         bool failed = false;
-        for (int ks = 0; ks < k_stages; ++ks) {
+        for (int ks = first_ks; ks < end_ks; ++ks) {
           const long long t0 = prof ? clock64() : 0;
           if (!ptx::mbar_wait_bounded(empty_bar + stage, phase ^ 1)) {
             report(p.error, 0x11000000u | (blockIdx.x << 8) | stage, abort_flag);
@@ -182,7 +229,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
         if (prof) prof_acc += clock64() - ta;
         ptx::tc_fence_after_sync();
         bool failed = false;
-        for (int ks = 0; ks < k_stages; ++ks) {
+        for (int ks = first_ks; ks < end_ks; ++ks) {
           const long long t0 = prof ? clock64() : 0;
           // sf_ready implies that both CTAs' operands have landed (the loader warps arrive after their
           // CTA's operand barrier), so this is the only wait of the stage
@@ -204,13 +251,13 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
             if (kb < nkb)
               mma_pair_nvfp4(tmem_base, make_desc(kDescHiSw128, base16 + 2 * kb),
                              make_desc(kDescHiSw128, base16 + (kTokBytes >> 4) + 2 * kb), idesc, sf_tok + 4 * kb,
-                             sf_wgt + 8 * kb, (ks | kb) != 0 ? 1u : 0u);
-          commit_pair(empty_bar + stage);
+                             sf_wgt + 8 * kb, ((ks - first_ks) | kb) != 0 ? 1u : 0u);
+          commit_pair(empty_bar + stage, leader);
           if (prof) prof_issue += clock64() - t2;
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
         if (failed) break;
-        commit_pair(acc_full_bar);
+        commit_pair(acc_full_bar, leader);
         acc_phase ^= 1;
       }
       if (prof) {
@@ -223,13 +270,13 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   } else if (warp < kFirstEpilogueWarp) {
     // ------------------------------------------------------------------ scale loaders
     const uint32_t quad_lane = uint32_t((warp % 4) * 32) << 16;
-    const uint32_t leader_sf_ready = leader_address(sf_ready_bar);
+    const uint32_t leader_sf_ready = cluster_address(sf_ready_bar, leader);
     int stage = 0;
     uint32_t phase = 0;
     long long prof_copy = 0, prof_arrive = 0;
     for (int w = pair; w < total_work && !*abort_flag; w += pairs) {
       bool failed = false;
-      for (int ks = 0; ks < k_stages; ++ks) {
+      for (int ks = first_ks; ks < end_ks; ++ks) {
         if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(sf_full_bar + stage, phase))) {
           report(p.error, 0x61000000u | (blockIdx.x << 8) | stage, abort_flag);
           failed = true;
@@ -348,12 +395,13 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
         *reinterpret_cast<uint16_t*>(p.scales_out + scale_offset(row, channel0 / 16, p.n)) = uint16_t(scale_pair);
       }
     }
+  } else if constexpr (kSplit) {
+    if (!ptx::mbar_wait_warp(acc_full_bar, 0)) report(p.error, 0x51000000u | (blockIdx.x << 8), abort_flag);
   } else {
     // ------------------------------------------------------------------ epilogue (own 128 rows x 256 channels)
     const int quad = warp % 4;
     const int col_half = (warp - kFirstEpilogueWarp) / 4;
     const uint32_t leader_acc_empty = leader_address(acc_empty_bar);
-    const bool hi = (lane & 2) != 0, lo = (lane & 1) != 0;
     uint32_t acc_phase = 0;
     bf16* out = static_cast<bf16*>(p.out);
     for (int w = pair; w < total_work && !*abort_flag; w += pairs) {
@@ -376,48 +424,73 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
         ptx::tmem_load16(taddr + c0, r);
         ptx::tmem_load16(taddr + c0 + 16, r + 16);
         ptx::tmem_load_wait();
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          unit[ch][q] = make_uint4(
-              pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q]), p.alpha), __fmul_rn(__uint_as_float(r[8 * q + 1]), p.alpha)),
-              pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q + 2]), p.alpha), __fmul_rn(__uint_as_float(r[8 * q + 3]), p.alpha)),
-              pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q + 4]), p.alpha), __fmul_rn(__uint_as_float(r[8 * q + 5]), p.alpha)),
-              pack_bf16x2(__fmul_rn(__uint_as_float(r[8 * q + 6]), p.alpha), __fmul_rn(__uint_as_float(r[8 * q + 7]), p.alpha)));
+        to_bf16(r, p.alpha, unit[ch]);
       }
       ptx::tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) arrive_cluster(leader_acc_empty);             // the next tile's MMAs may start
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch) {
-        const int c0 = col_half * 128 + 32 * ch;
-        uint4* u = unit[ch];
-        {
-          const uint4 send_a = hi ? u[0] : u[2], send_b = hi ? u[1] : u[3];
-          const uint4 got_a = shfl_xor_u4(send_a, 2), got_b = shfl_xor_u4(send_b, 2);
-          if (hi) { u[0] = got_a; u[1] = got_b; } else { u[2] = got_a; u[3] = got_b; }
-        }
-        {
-          const uint4 send_a = lo ? u[0] : u[1], send_b = lo ? u[2] : u[3];
-          const uint4 got_a = shfl_xor_u4(send_a, 1), got_b = shfl_xor_u4(send_b, 1);
-          if (lo) { u[0] = got_a; u[2] = got_b; } else { u[1] = got_a; u[3] = got_b; }
-        }
-        const int c = c_base + c0 + 8 * (lane & 3);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (i >= rows_left || c >= p.n) continue;
-          bf16* dst = out + size_t(row0 + i) * p.ld_out + c;
-          if (c + 8 <= p.n) {
-            *reinterpret_cast<uint4*>(dst) = u[i];
-          } else {
-            const uint32_t words[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
-            for (int e = 0; e < 8; ++e)
-              if (c + e < p.n) reinterpret_cast<uint16_t*>(dst)[e] = uint16_t(words[e / 2] >> (16 * (e % 2)));
-          }
-        }
+        store_chunk(out, p.ld_out, row0, rows_left, c_base + col_half * 128 + 32 * ch, p.n, unit[ch], lane);
       }
     }
   }
 
+  if constexpr (kSplit) {
+    // ------------------------------------------------------------------ sum of the pairs' parts
+    // As in gemm_pair_wide.cu: chunk c of 32 channels is summed and stored by pair c % split; the other pairs write their 128 x 32
+    // FP32 values of it into that pair's operand ring, [channel / 4][lane][channel % 4], once every pair's MMAs have read theirs.
+    __syncwarp();
+    ptx::tc_fence_before_sync();
+    cluster_sync_all();
+    ptx::tc_fence_after_sync();
+    const int part = int(leader / 2), quad = warp % 4, half = (warp - kFirstEpilogueWarp) / 4;
+    const int c_tile = pair % p.c_tiles, l_tile = pair / p.c_tiles;
+    const int row_of_warp = (l_tile * 2 + int(rank)) * 128 + quad * 32;
+    const int chunks = min(8, (p.n - c_tile * 256 + 31) / 32);
+    const bool active = warp >= kFirstEpilogueWarp && row_of_warp < p.rows;
+    const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16);
+    const uint32_t at = uint32_t(quad * 32 + lane) * 16;
+    if (active) {
+      for (int c = half; c < chunks; c += 2) {
+        const int owner = c % p.split;
+        if (owner == part) continue;
+        uint32_t r[32];
+        ptx::tmem_load16(taddr + 32 * c, r);
+        ptx::tmem_load16(taddr + 32 * c + 16, r + 16);
+        ptx::tmem_load_wait();
+        const int slot = c / p.split * (p.split - 1) + (part < owner ? part : part - 1);
+        const uint32_t to = cluster_address(smem + slot * kPartBytes, uint32_t(2 * owner) + rank) + at;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) store_cluster(to + i * (128 * 16), r + 4 * i);
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (active && !*abort_flag) {
+      const int row0 = row_of_warp + (lane & ~3);
+      for (int k = half, c = part + half * p.split; c < chunks; k += 2, c += 2 * p.split) {
+        uint32_t r[32];
+        ptx::tmem_load16(taddr + 32 * c, r);
+        ptx::tmem_load16(taddr + 32 * c + 16, r + 16);
+        ptx::tmem_load_wait();
+        for (int other = 0; other < p.split - 1; ++other) {
+          const uint32_t from = ptx::smem_u32(smem + (k * (p.split - 1) + other) * kPartBytes) + at;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 v = ptx::lds128(from + i * (128 * 16));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) r[4 * i + j] = __float_as_uint(__uint_as_float(r[4 * i + j]) + __uint_as_float(w[j]));
+          }
+        }
+        uint4 u[4];
+        to_bf16(r, p.alpha, u);
+        store_chunk(static_cast<bf16*>(p.out), p.ld_out, row0, p.rows - row0, c_tile * 256 + 32 * c, p.n, u, lane);
+      }
+    }
+    __syncwarp();
+  }
   ptx::tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();                               // the peer no longer reads this CTA's shared or tensor memory
@@ -434,19 +507,20 @@ long long* g_pair_profile = nullptr;
 void set_pair_profile_buffer(long long* device_buffer) { g_pair_profile = device_buffer; }
 
 namespace {
-template <bool kGeglu, bool kProfile>
+template <bool kGeglu, bool kProfile, bool kSplit>
 cudaError_t launch_pair_instance(const PairGemmParams& params, int sm_count, cudaStream_t stream) {
   static bool configured_on[kMaxDeviceSlots] = {};   // the attribute is per GPU
   bool& configured = configured_on[current_device_slot()];
   if (!configured) {
     cudaError_t status =
-        cudaFuncSetAttribute(gemm_pair_kernel<kGeglu, kProfile>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        cudaFuncSetAttribute(gemm_pair_kernel<kGeglu, kProfile, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (status != cudaSuccess) return status;
     configured = true;
   }
   const int work = params.l_tiles * params.c_tiles;
   int pairs = sm_count / 2;
-  if (work < pairs) pairs = work;
+  if (kSplit) pairs = work * params.split;
+  else if (work < pairs) pairs = work;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(2 * pairs);
   config.blockDim = dim3(threads(kGeglu));
@@ -454,7 +528,7 @@ cudaError_t launch_pair_instance(const PairGemmParams& params, int sm_count, cud
   config.stream = stream;
   cudaLaunchAttribute attributes[2]{};
   attributes[0].id = cudaLaunchAttributeClusterDimension;
-  attributes[0].val.clusterDim.x = 2;
+  attributes[0].val.clusterDim.x = kSplit ? 2 * params.split : 2;
   attributes[0].val.clusterDim.y = 1;
   attributes[0].val.clusterDim.z = 1;
   attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -462,19 +536,42 @@ cudaError_t launch_pair_instance(const PairGemmParams& params, int sm_count, cud
   config.attrs = attributes;
   config.numAttrs = 2;
   note_launch();
-  return cudaLaunchKernelEx(&config, gemm_pair_kernel<kGeglu, kProfile>, params);
+  return cudaLaunchKernelEx(&config, gemm_pair_kernel<kGeglu, kProfile, kSplit>, params);
+}
+}  // namespace
+
+namespace {
+// Pairs that share a tile's K: the number that saves most of its stages (0.36 us each), after the time that adding the parts up
+// takes, 8, 14 and 13 stages for two, three and four pairs.  us with the quantiser, one pair / two / three / four: 250x2816x2816 10.3 /
+// 11.1 / 12.0 / 11.4, 250x4096x2816 12.1 / 11.8 / 12.6 / 12.1, 250x5376x2048 13.8 / 13.0 / 13.0 / 12.6, 250x8192x2816 17.9 / 14.7 /
+// 14.4 / 13.7, 700x8192x2816 21.1 / 18.2, 250x21504x5376 39.8 / 28.5 / 25.9.
+int pair_split(const PairGemmParams& p, int sm_count) {
+  constexpr int kCost[kMaxSplit + 1] = {0, 0, 8, 14, 13};
+  const int k_stages = (p.k / 64 + kKBlocks - 1) / kKBlocks, tiles = p.l_tiles * p.c_tiles;
+  int best = 1, best_gain = 1;
+  for (int split = 2; split <= kMaxSplit; ++split) {
+    const int gain = k_stages - (k_stages + split - 1) / split - kCost[split];
+    if (gain > best_gain && tiles * split <= sm_count / 2 &&
+        tiles <= clusters_at_once<gemm_pair_kernel<false, false, true>>(split, threads(false), kSmemBytes)) {
+      best_gain = gain;
+      best = split;
+    }
+  }
+  return best;
 }
 }  // namespace
 
 cudaError_t launch_gemm_pair(const PairGemmParams& params_in, int sm_count, cudaStream_t stream) {
   PairGemmParams params = params_in;
   params.profile = g_pair_profile;
-  if (params.profile != nullptr) return launch_pair_instance<false, true>(params, sm_count, stream);
-  return launch_pair_instance<false, false>(params, sm_count, stream);
+  if (params.profile != nullptr) return launch_pair_instance<false, true, false>(params, sm_count, stream);
+  params.split = pair_split(params, sm_count);
+  if (params.split > 1) return launch_pair_instance<false, false, true>(params, sm_count, stream);
+  return launch_pair_instance<false, false, false>(params, sm_count, stream);
 }
 
 cudaError_t launch_gemm_pair_geglu(const PairGemmParams& params, int sm_count, cudaStream_t stream) {
-  return launch_pair_instance<true, false>(params, sm_count, stream);
+  return launch_pair_instance<true, false, false>(params, sm_count, stream);
 }
 
 }  // namespace gw

@@ -17,6 +17,7 @@ struct PairGemmParams {
   int32_t token_row_blocks;        // 128-row blocks the activation scale storage holds
   int32_t k, rows, n;
   int32_t l_tiles, c_tiles;        // 256-token tiles, 256-channel tiles
+  int32_t split;                   // pairs that share the K loop of a tile (set by the launch)
   void* out;                       // BF16 [rows, ld_out]
   int64_t ld_out;
   float alpha;

@@ -427,34 +427,6 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
 
 }  // namespace
 
-namespace {
-// Clusters of 2 * split CTAs that the GPU holds at once.
-int clusters_at_once(int split) {
-  static int known[kMaxDeviceSlots][kMaxSplit + 1] = {};      // a plain int: two threads write the same
-  int& count = known[current_device_slot()][split];
-  if (count == 0) {
-    cudaLaunchConfig_t config{};
-    config.gridDim = dim3(2 * split);
-    config.blockDim = dim3(kThreads);
-    config.dynamicSmemBytes = kSmemBytes;
-    cudaLaunchAttribute attribute{};
-    attribute.id = cudaLaunchAttributeClusterDimension;
-    attribute.val.clusterDim.x = 2 * split;
-    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
-    config.attrs = &attribute;
-    config.numAttrs = 1;
-    int clusters = 0;
-    if (cudaFuncSetAttribute(gemm_pair_wide_kernel<true, WideOut::split>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, gemm_pair_wide_kernel<true, WideOut::split>, &config) != cudaSuccess) {
-      cudaGetLastError();
-      clusters = 0;
-    }
-    count = clusters > 0 ? clusters : -1;
-  }
-  return count;
-}
-}  // namespace
-
 PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int k_stages, int sm_count) {
   // A tile takes as long as its weight rows and MMA issue cost whatever its width (about 136 columns) plus its columns:
   // measured on FP8 K=5376, per wave of tiles of 64 / 128 / 192 / 256 tokens 8.9 / 11.3 / 14.3 / 17.4 us.
@@ -481,7 +453,7 @@ PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int k_stages, int sm_co
       const int token_tiles = int((rows + tile - 1) / tile);
       const uint64_t tiles = uint64_t(channel_tiles) * token_tiles;
       const uint64_t cost = uint64_t((k_stages + split - 1) / split) * uint64_t(tile + 136) + 2800 + uint64_t(20 * tile * (split - 1) / split);
-      if (cost < split_cost && tiles * split <= uint64_t(pairs) && int64_t(tiles) <= clusters_at_once(split)) {
+      if (cost < split_cost && tiles * split <= uint64_t(pairs) && int64_t(tiles) <= clusters_at_once<gemm_pair_wide_kernel<true, WideOut::split>>(split, kThreads, kSmemBytes)) {
         split_cost = cost;
         t = {tile, channel_tiles, token_tiles, int32_t(tiles), 1, tile, split};
       }

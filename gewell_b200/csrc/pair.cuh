@@ -6,6 +6,7 @@
 
 #include <cstdint>
 
+#include "common.cuh"
 #include "ptx.cuh"
 
 namespace gw::pair {
@@ -95,6 +96,33 @@ __device__ __forceinline__ void transpose_units(uint4* u, int lane) {
     const uint4 got_a = shfl_xor_u4(send_a, 1), got_b = shfl_xor_u4(send_b, 1);
     if (lo) { u[0] = got_a; u[2] = got_b; } else { u[1] = got_a; u[3] = got_b; }
   }
+}
+
+// Clusters of 2 * split CTAs of a kernel that the GPU holds at once, one answer per kernel.
+template <auto* kernel>
+int clusters_at_once(int split, int threads, int smem_bytes) {
+  static int known[kMaxDeviceSlots][5] = {};      // plain ints: two threads write the same
+  int& count = known[current_device_slot()][split];
+  if (count == 0) {
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(2 * split);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem_bytes;
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = 2 * split;
+    attribute.val.clusterDim.y = attribute.val.clusterDim.z = 1;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    count = clusters > 0 ? clusters : -1;
+  }
+  return count;
 }
 
 }  // namespace gw::pair
