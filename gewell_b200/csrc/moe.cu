@@ -64,7 +64,7 @@ struct gw_expert_table {
 // Tuning overrides, read from the environment once, when a workspace is created:
 //   GW_MOE_FORM          swap / direct / fused: plan of the grouped GEMMs (default: by batch size)
 //   GW_MOE_NO_PAIR       1: never use the CTA-pair kernels (single-CTA kernels for every batch size)
-//   GW_MOE_ROUTE_THREE_LAUNCHES  1: route, scan and scatter as three launches instead of one with a grid barrier
+//   GW_MOE_ROUTE_THREE_LAUNCHES  1: route, scan and scatter as three launches, whatever the size
 //   GW_MOE_BLOCK_N, GW_MOE_BLOCK_N_DOWN, GW_MOE_CHUNK_FIRST, GW_MOE_CHUNK_DOWN: tile / schedule of the
 //                        single-CTA kernels
 struct MoeTuning {
@@ -106,7 +106,6 @@ struct gw_moe_workspace {
   MoeTuning tuning;
   CachedMap first_map, down_map;
   DeviceBuffer metadata, bitmaps, groups, packed_in, scales_in, gate_up, activated, packed_act, scales_act, down;
-  DeviceBuffer route_barrier;   // counter and generation of the routing kernel's grid-wide barrier
   DeviceBuffer row_home;   // expert parallelism: address of every produced row's home in its source rank
   DeviceBuffer fp8_in, fp8_act;   // FP8 experts (GW_MOE_FP8_EXPERTS): E4M3 gate / up inputs [2][n, 2816], down input [n, 704]
   DeviceBuffer kind_groups;       // group descriptors of the BF16 and FP8 launches of a mixed table
@@ -300,8 +299,6 @@ gw_status gw_moe_create_ex(uint32_t max_rows, uint32_t flags, gw_moe_workspace**
   if (status == cudaSuccess) status = w->scales_act.allocate(size_t(w->scale_rows) * (kInter / 16));
   if (status == cudaSuccess) status = w->down.allocate(n * kHidden * sizeof(bf16));
   if (status == cudaSuccess) status = w->row_home.allocate(n * sizeof(uint64_t));
-  if (status == cudaSuccess) status = w->route_barrier.allocate(2 * sizeof(uint32_t));
-  if (status == cudaSuccess) status = zero_now(w->route_barrier.data, 2 * sizeof(uint32_t));
   if (status == cudaSuccess) status = w->kind_groups.allocate(2 * (2 * kExperts + 1 + kExperts + 1) * sizeof(GemmGroup));
   if (status == cudaSuccess && (flags & GW_MOE_FP8_EXPERTS)) {
     status = w->fp8_in.allocate(2 * n * kHidden);
@@ -341,8 +338,7 @@ GemmGroup* down_groups_of(gw_moe_workspace* w) { return w->groups.as<GemmGroup>(
 gw_status dispatch(gw_moe_workspace* w, const void* scores, const void* expert_scales, uint32_t rows, const MoeGroupPlan* plan, cudaStream_t s) {
   GW_CUDA_CHECK(launch_moe_dispatch(scores, expert_scales, rows, w->keys, w->weights, w->bitmaps.as<uint32_t>(),
                                     w->chunk_counts, w->offsets, w->sorted_assignments, w->sorted_keys, w->inverse,
-                                    w->route_barrier.as<uint32_t>(), device_error_word(), sm_count(),
-                                    !w->tuning.route_three_launches, s, plan, first_groups_of(w), down_groups_of(w)),
+                                    sm_count(), w->tuning.route_three_launches, s, plan, first_groups_of(w), down_groups_of(w)),
                 "MoE dispatch");
   return GW_OK;
 }

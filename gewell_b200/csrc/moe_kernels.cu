@@ -7,7 +7,7 @@
 // is simply token order.  So the position of assignment (t, slot) is
 //   offsets[e] + #tokens t' < t that chose e,
 // computed here with per-64-token bitmaps and popcounts: kernel 1 routes and
-// builds the bitmaps, kernel 2 scans the per-chunk counts, kernel 3 scatters.
+// builds the bitmaps, kernel 1b scans the per-chunk counts and scatters (for very many tokens kernels 2 and 3).
 #include <algorithm>
 
 #include "common.cuh"
@@ -313,32 +313,29 @@ __device__ __forceinline__ void route_token(const bf16* __restrict__ scores, con
 //    ties), renormalise, times the per-expert scale, sort the eight by id.
 //    The FP32 operation order is that of the reference's select kernel
 //    (models/gemma4/26b_a4b/sm120/moe.cu:104-157), so ids and FP32 weights match
-//    it bit for bit.  One warp per token, eight tokens per warp.
+//    it bit for bit.  A token per warp and a chunk of 64 tokens per cluster of eight blocks, whose bits meet in the
+//    first one's shared memory: bound by latency up to some 9000 tokens, where one block per chunk was bound by the
+//    instructions of its 64 tokens.
 // ---------------------------------------------------------------------------
-//    Used by three kernels: one launch per step (this one), one cluster for at most 64 tokens, and one grid-wide launch.
-__global__ void __launch_bounds__(256)
+constexpr int kRouteCluster = 8;
+__global__ void __cluster_dims__(kRouteCluster, 1, 1) __launch_bounds__(256)
 moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales, uint32_t rows,
                  int32_t* __restrict__ keys, float* __restrict__ weights, uint32_t* __restrict__ bitmaps,
                  int32_t* __restrict__ chunk_counts) {
-  const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  griddep_enter();     // results of earlier kernels in the stream are read from here on
+  static_assert(kRouteCluster * 8 == kChunkTokens, "a token per warp");
+  __shared__ uint32_t bitmap[kExperts][2];
+  const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32, block = pair::cluster_rank();
+  if (block == 0 && threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
+  pair::cluster_sync_all();                // the first block's bitmaps are clear
+  griddep_enter();                         // results of earlier kernels in the stream are read from here on
   float expert_scale[4];
   load_expert_scales(expert_scales, lane, expert_scale);
-  __shared__ uint32_t bitmap[kExperts][2];
-  if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
-  __syncthreads();
-  const uint32_t chunk = blockIdx.x;
-#pragma unroll 1
-  for (uint32_t local = warp; local < kChunkTokens; local += 8) {
-    const uint32_t row = chunk * kChunkTokens + local;
-    if (row >= rows) break;
-    route_token(scores, expert_scale, row, local, lane, keys, weights, ptx::smem_u32(bitmap), 0);
-  }
-  __syncthreads();
-  if (threadIdx.x < kExperts) {
+  const uint32_t chunk = blockIdx.x / kRouteCluster, local = block * 8 + warp, row = chunk * kChunkTokens + local;
+  if (row < rows) route_token(scores, expert_scale, row, local, lane, keys, weights, pair::leader_address(bitmap), 0);
+  pair::cluster_sync_all();                // every block's bits are in the first one's memory
+  if (block == 0 && threadIdx.x < kExperts) {
     const uint32_t w0 = bitmap[threadIdx.x][0], w1 = bitmap[threadIdx.x][1];
-    bitmaps[(size_t(chunk) * kExperts + threadIdx.x) * 2] = w0;
-    bitmaps[(size_t(chunk) * kExperts + threadIdx.x) * 2 + 1] = w1;
+    *reinterpret_cast<uint2*>(bitmaps + (size_t(chunk) * kExperts + threadIdx.x) * 2) = make_uint2(w0, w1);
     chunk_counts[size_t(chunk) * kExperts + threadIdx.x] = __popc(w0) + __popc(w1);
   }
 }
@@ -349,7 +346,6 @@ moe_route_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ exper
 //     their bits and ids to, does the work of kernels 2 and 3 and the expert GEMMs' descriptors (`first_groups`
 //     != nullptr): one launch instead of four.  64 tokens, descriptors included: 14 -> 7.4 us.
 // ---------------------------------------------------------------------------
-constexpr int kRouteCluster = 8;
 __global__ void __cluster_dims__(kRouteCluster, 1, 1) __launch_bounds__(256)
 moe_route_cluster_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales, uint32_t rows,
                          int32_t* __restrict__ keys, float* __restrict__ weights, uint32_t* __restrict__ bitmaps,
@@ -357,7 +353,6 @@ moe_route_cluster_kernel(const bf16* __restrict__ scores, const bf16* __restrict
                          int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
                          int32_t* __restrict__ inverse, const __grid_constant__ MoeGroupPlan plan, GemmGroup* __restrict__ first_groups,
                          GemmGroup* __restrict__ down_groups) {
-  static_assert(kRouteCluster * 8 == kChunkTokens, "a token per warp");
   __shared__ uint32_t bitmap[kExperts][2];
   __shared__ int32_t shared_keys[kChunkTokens * kTopK];
   __shared__ int32_t base[kExperts];
@@ -423,110 +418,50 @@ moe_route_cluster_kernel(const bf16* __restrict__ scores, const bf16* __restrict
 }
 
 // ---------------------------------------------------------------------------
-// 1b. route + scan + scatter in ONE launch for more than 64 tokens.  At most
-//     kRouteGridBlocksPerSm blocks per SM, each walking chunks b, b + grid, ...:
-//       phase 1  route the block's chunks (bitmaps and per-chunk counts to global memory)
-//       barrier  every block has published its counts
-//       phase 2  every block walks all chunk counts once: the running sums at its own chunks are
-//                their bases, the totals give the expert offsets (block 0 stores them)
-//       phase 3  scatter the block's chunks
-//     The barrier is a counter plus a generation word in the workspace (the last block to arrive
-//     resets the counter and bumps the generation, so replays need no host-side reset).  All blocks
-//     are resident together -- the grid is sized below what the GPU holds at once -- and the wait is
-//     bounded: on a timeout the block reports through the error word and returns.
+// 1b. scan + scatter in one launch behind kernel 1, for more than 64 tokens: every block walks all chunk counts once -- the
+//     running sums at its own chunks (b, b + grid, ...) are their bases, the totals give the expert offsets (block 0 stores
+//     them) -- and scatters its chunks.
+//     Whole layer, us, route + grid barrier + scatter in one launch / kernel 1 and this one: 70 tokens 98.1 / 94.0, 191 104.8 /
+//     100.0, 777 118.6 / 114.3, 2407 188.3 / 185.3, 8192 430 / 424.
 // ---------------------------------------------------------------------------
-constexpr int kRouteGridBlocksPerSm = 1;
-constexpr int kRouteGridThreads = 1024;
-constexpr int kRouteOwnChunks = 16;     // chunks per block the launch sizes the grid for (65536 tokens / 64 / 148 < 8)
-constexpr int kRouteParts = kRouteGridThreads / kExperts;   // phase 2: eight threads share an expert's chunk list
+constexpr int kPlaceThreads = 1024;
+constexpr int kOwnChunks = 16;          // chunks per block at most (65536 tokens / 64 / 148 < 8)
+constexpr int kPlaceParts = kPlaceThreads / kExperts;   // eight threads share an expert's chunk list
 
-__device__ __forceinline__ bool route_grid_barrier(uint32_t* state, uint32_t blocks, uint32_t* error) {
-  __shared__ int passed;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();                                        // this block's counts are visible before it arrives
-    const uint32_t generation = atomicAdd(state + 1, 0u);
-    int ok = 1;
-    if (atomicAdd(state, 1u) == blocks - 1) {
-      atomicExch(state, 0u);                                // ready for the next launch
-      __threadfence();
-      atomicAdd(state + 1, 1u);
-    } else {
-      const uint64_t start = ptx_global_timer();
-      for (uint32_t spin = 1; atomicAdd(state + 1, 0u) == generation; ++spin) {
-        if ((spin & 63u) == 0 && ptx_global_timer() - start > 2000000000ull) { ok = 0; break; }
-        __nanosleep(32);
-      }
-    }
-    __threadfence();
-    if (!ok && error != nullptr) atomicCAS(error, 0u, 0x80000000u | blockIdx.x);
-    passed = ok;
-  }
-  __syncthreads();
-  return passed != 0;
-}
-
-__global__ void __launch_bounds__(kRouteGridThreads)
-moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ expert_scales, uint32_t rows,
-                      uint32_t chunks, int32_t* __restrict__ keys, float* __restrict__ weights,
-                      uint32_t* __restrict__ bitmaps, int32_t* __restrict__ chunk_counts, int32_t* __restrict__ offsets,
-                      int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys,
-                      int32_t* __restrict__ inverse, uint32_t* __restrict__ barrier_state, uint32_t* __restrict__ error) {
+__global__ void __launch_bounds__(kPlaceThreads)
+moe_place_kernel(uint32_t rows, uint32_t chunks, const int32_t* __restrict__ keys, const uint32_t* __restrict__ bitmaps,
+                 const int32_t* __restrict__ chunk_counts, int32_t* __restrict__ offsets,
+                 int32_t* __restrict__ sorted_assignments, int32_t* __restrict__ sorted_keys, int32_t* __restrict__ inverse) {
   const unsigned lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-  griddep_enter();     // results of earlier kernels in the stream are read from here on
-  float expert_scale[4];
-  load_expert_scales(expert_scales, lane, expert_scale);
   __shared__ uint32_t bitmap[kExperts][2];
-  __shared__ int32_t own_base[kRouteOwnChunks][kExperts];
-  __shared__ int32_t part_sum[kRouteParts][kExperts];
+  __shared__ int32_t own_base[kOwnChunks][kExperts];
+  __shared__ int32_t part_sum[kPlaceParts][kExperts];
   __shared__ int32_t expert_offset[kExperts];
   __shared__ int32_t warp_totals[4];
-  __shared__ int32_t shared_keys[kChunkTokens * kTopK];
-  const bool one_chunk = chunks <= gridDim.x;       // then the block's bitmaps and keys are still in shared memory in phase 3
-  constexpr int kTokensPerWarp = kChunkTokens / (kRouteGridThreads / 32);     // 2
-  // ---- phase 1: 32 warps, two tokens each, per chunk
-  for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
-    if (threadIdx.x < kExperts) { bitmap[threadIdx.x][0] = 0; bitmap[threadIdx.x][1] = 0; }
-    __syncthreads();
-#pragma unroll 1
-    for (int t = 0; t < kTokensPerWarp; ++t) {
-      const uint32_t local = warp * kTokensPerWarp + t;
-      const uint32_t row = chunk * kChunkTokens + local;
-      if (row < rows) route_token(scores, expert_scale, row, local, lane, keys, weights, ptx::smem_u32(bitmap), ptx::smem_u32(shared_keys));
-    }
-    __syncthreads();
-    if (threadIdx.x < kExperts) {
-      const uint32_t w0 = bitmap[threadIdx.x][0], w1 = bitmap[threadIdx.x][1];
-      bitmaps[(size_t(chunk) * kExperts + threadIdx.x) * 2] = w0;
-      bitmaps[(size_t(chunk) * kExperts + threadIdx.x) * 2 + 1] = w1;
-      chunk_counts[size_t(chunk) * kExperts + threadIdx.x] = __popc(w0) + __popc(w1);
-    }
-    __syncthreads();
-  }
-  if (!route_grid_barrier(barrier_state, gridDim.x, error)) return;
-  // ---- phase 2: expert e's counts summed over the chunks in order; eight threads share the list (contiguous
+  griddep_enter();     // results of earlier kernels in the stream are read from here on
+  // ---- expert e's counts summed over the chunks in order; eight threads share the list (contiguous
   // ranges of chunks), their partial sums are combined in order afterwards
   {
     const unsigned e = threadIdx.x % kExperts, part = threadIdx.x / kExperts;
-    const uint32_t per_part = (chunks + kRouteParts - 1) / kRouteParts;
+    const uint32_t per_part = (chunks + kPlaceParts - 1) / kPlaceParts;
     const uint32_t c_begin = min(part * per_part, chunks), c_end = min(c_begin + per_part, chunks);
     int32_t running = 0;
 #pragma unroll 8
-    for (uint32_t c = c_begin; c < c_end; ++c) running += __ldcg(chunk_counts + size_t(c) * kExperts + e);
+    for (uint32_t c = c_begin; c < c_end; ++c) running += __ldg(chunk_counts + size_t(c) * kExperts + e);
     part_sum[part][e] = running;
     __syncthreads();
     // bases of this block's own chunks: sum of the parts before the chunk's part plus the counts inside it
     if (part == 0) {
-      int32_t before[kRouteParts];
+      int32_t before[kPlaceParts];
       int32_t total = 0;
 #pragma unroll
-      for (int q = 0; q < kRouteParts; ++q) { before[q] = total; total += part_sum[q][e]; }
+      for (int q = 0; q < kPlaceParts; ++q) { before[q] = total; total += part_sum[q][e]; }
       uint32_t own = 0;
       for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x, ++own) {
         const uint32_t q = chunk / per_part;
         int32_t base = before[q];
 #pragma unroll 8
-        for (uint32_t c = q * per_part; c < chunk; ++c) base += __ldcg(chunk_counts + size_t(c) * kExperts + e);
+        for (uint32_t c = q * per_part; c < chunk; ++c) base += __ldg(chunk_counts + size_t(c) * kExperts + e);
         own_base[own][e] = base;
       }
       // exclusive scan of the totals over the 128 experts (threads 0..127 are four whole warps)
@@ -551,20 +486,17 @@ moe_route_grid_kernel(const bf16* __restrict__ scores, const bf16* __restrict__ 
     }
   }
   __syncthreads();
-  // ---- phase 3
+  // ---- scatter
   uint32_t own = 0;
   for (uint32_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x, ++own) {
-    if (!one_chunk && threadIdx.x < kExperts) {
-      bitmap[threadIdx.x][0] = __ldcg(bitmaps + (size_t(chunk) * kExperts + threadIdx.x) * 2);
-      bitmap[threadIdx.x][1] = __ldcg(bitmaps + (size_t(chunk) * kExperts + threadIdx.x) * 2 + 1);
-    }
+    if (threadIdx.x < 2 * kExperts) bitmap[threadIdx.x / 2][threadIdx.x % 2] = bitmaps[size_t(chunk) * kExperts * 2 + threadIdx.x];
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kChunkTokens * kTopK; i += kRouteGridThreads) {
+    for (uint32_t i = threadIdx.x; i < kChunkTokens * kTopK; i += kPlaceThreads) {
       const uint32_t local = i / kTopK;
       const uint32_t row = chunk * kChunkTokens + local;
       if (row >= rows) continue;
       const uint32_t assignment = row * kTopK + i % kTopK;
-      const int32_t e = one_chunk ? shared_keys[i] : keys[assignment];
+      const int32_t e = keys[assignment];
       const uint32_t w0 = bitmap[e][0], w1 = bitmap[e][1];
       const int rank = local < 32 ? __popc(w0 & ((1u << local) - 1u))
                                   : __popc(w0) + __popc(w1 & ((1u << (local - 32)) - 1u));
@@ -1301,8 +1233,7 @@ uint32_t moe_chunks(uint32_t rows) { return (rows + kChunkTokens - 1) / kChunkTo
 cudaError_t launch_moe_dispatch(const void* scores, const void* expert_scales, uint32_t rows, int32_t* keys,
                                 float* weights, uint32_t* bitmaps, int32_t* chunk_counts, int32_t* offsets,
                                 int32_t* sorted_assignments, int32_t* sorted_keys, int32_t* inverse,
-                                uint32_t* barrier_state, uint32_t* error, int sm_count, bool one_launch,
-                                cudaStream_t stream, const MoeGroupPlan* plan, GemmGroup* first_groups, GemmGroup* down_groups) {
+                                int sm_count, bool three_launches, cudaStream_t stream, const MoeGroupPlan* plan, GemmGroup* first_groups, GemmGroup* down_groups) {
   const uint32_t chunks = moe_chunks(rows);
   if (chunks == 1) {     // decode sizes: one cluster routes, scans and scatters
     launch_pdl(moe_route_cluster_kernel, kRouteCluster, 256, stream, static_cast<const bf16*>(scores),
@@ -1311,15 +1242,13 @@ cudaError_t launch_moe_dispatch(const void* scores, const void* expert_scales, u
                down_groups);
     return cudaGetLastError();
   }
-  const uint32_t resident = uint32_t(sm_count) * kRouteGridBlocksPerSm;
-  if (one_launch && barrier_state != nullptr && chunks <= resident * kRouteOwnChunks) {
-    launch_pdl(moe_route_grid_kernel, chunks < resident ? chunks : resident, kRouteGridThreads, stream,
-               static_cast<const bf16*>(scores), static_cast<const bf16*>(expert_scales), rows, chunks, keys, weights,
-               bitmaps, chunk_counts, offsets, sorted_assignments, sorted_keys, inverse, barrier_state, error);
+  launch_pdl(moe_route_kernel, chunks * kRouteCluster, 256, stream, static_cast<const bf16*>(scores),
+             static_cast<const bf16*>(expert_scales), rows, keys, weights, bitmaps, chunk_counts);
+  if (!three_launches && chunks <= uint32_t(sm_count) * kOwnChunks) {
+    launch_pdl(moe_place_kernel, std::min(chunks, uint32_t(sm_count)), kPlaceThreads, stream, rows, chunks, keys, bitmaps, chunk_counts,
+               offsets, sorted_assignments, sorted_keys, inverse);
     return cudaGetLastError();
   }
-  launch_pdl(moe_route_kernel, chunks, 256, stream, static_cast<const bf16*>(scores),
-             static_cast<const bf16*>(expert_scales), rows, keys, weights, bitmaps, chunk_counts);
   launch_pdl(moe_scan_kernel, 1, kExperts, stream, chunk_counts, chunks, offsets);
   launch_pdl(moe_scatter_kernel, chunks, 256, stream, keys, bitmaps, chunk_counts, offsets, rows, sorted_assignments,
              sorted_keys, inverse);

@@ -103,14 +103,13 @@ def make_scores(rows, mode, seed=0):
 @pytest.mark.parametrize("rows,mode,launches", [
     (1, "hot", 1), (17, "distributed", 1), (65, "normal", 1), (129, "uneven", 1), (257, "distributed", 1), (17, "ties", 1),
     (4096, "hot", 1), (4096, "distributed", 1), (1000, "normal", 1), (8192, "normal", 1),
-    # more chunks than resident blocks: several chunks per block of the one-launch kernel
+    # more chunks than SMs: several chunks per block of the scan + scatter kernel
     (40000, "normal", 1), (65536, "uneven", 1),
     (1000, "normal", 3), (8192, "normal", 3)])
 def test_dispatch_exact(gw, rows, mode, launches, monkeypatch):
     """Selected ids, stable permutation and offsets are bit-exact; the FP32
     routing weights agree to a few ulps (host exp vs device expf).  From 65 tokens on
-    routing, scan and scatter are one launch with a grid-wide barrier (or, on request,
-    three launches)."""
+    scan and scatter are one launch behind the routing (or, on request, two)."""
     if launches == 3:
         monkeypatch.setenv("GW_MOE_ROUTE_THREE_LAUNCHES", "1")
     scores = make_scores(rows, mode)
