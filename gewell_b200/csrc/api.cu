@@ -551,7 +551,7 @@ gw_status gw_bf16_plan_run(gw_bf16_plan* plan, const void* input_bf16, const voi
 }  // extern "C"
 
 gw_status gw::run_bf16_plan(gw_bf16_plan* plan, const void* input_bf16, const void* weight_bf16, void* output_bf16, void* scratch,
-                            size_t scratch_capacity, cudaStream_t s, bool weights_settled) {
+                            size_t scratch_capacity, cudaStream_t s, bool weights_settled, bool weights_fresh) {
   clear_error();
   if (!plan) return fail(GW_INVALID_ARGUMENT, "BF16 run requires a plan");
   // scratch == NULL is allowed: decode-shaped plans then keep whole tiles per CTA instead of the K split
@@ -576,6 +576,7 @@ gw_status gw::run_bf16_plan(gw_bf16_plan* plan, const void* input_bf16, const vo
                        input_bf16, nullptr, 1.0F, nullptr, output_bf16, device_error_word()};
   if (plan->total_bytes != 0 && scratch) problem.split_workspace = scratch;
   problem.weights_settled = weights_settled;
+  problem.weights_fresh = weights_fresh;
   return launch_dense(problem, &plan->descriptors, s);
 }
 

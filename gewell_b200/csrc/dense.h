@@ -74,6 +74,8 @@ struct DenseProblem {
   // In front of this launch, or of the quantiser of its activations, the same call launched a kernel that does not write the
   // weights: the swap form reads its first weight tiles while that kernel still runs.  Otherwise they wait in L2 meanwhile.
   bool weights_settled = false;
+  // The launch in front of this one wrote the weights (the dequantiser of the BF16 path).
+  bool weights_fresh = false;
 };
 
 // true: weights on the 128-lane operand and tokens on the column operand.
@@ -153,7 +155,7 @@ struct WideGegluProblem {
 };
 gw_status launch_dense_geglu_wide(const WideGegluProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
-// gw_*_plan_run as a step of a longer call (api.cu): `weights_settled` as in DenseProblem.  The public entry points pass
+// gw_*_plan_run as a step of a longer call (api.cu): `weights_settled`, `weights_fresh` as in DenseProblem.  The public entry points pass
 // false.
 gw_status run_nvfp4_plan(gw_nvfp4_plan* plan, const void* input, const uint8_t* weight_data, const uint8_t* weight_scales, float input_scale,
                          float weight_scale, void* output, void* scratch, size_t scratch_capacity, cudaStream_t stream, int transform,
@@ -162,7 +164,7 @@ gw_status run_fp8_plan(gw_fp8_plan* plan, const void* input, const uint8_t* weig
                        const float* channel_scales, void* output, void* scratch, size_t scratch_capacity, cudaStream_t stream, int transform,
                        bool weights_settled);
 gw_status run_bf16_plan(gw_bf16_plan* plan, const void* input, const void* weight, void* output, void* scratch, size_t scratch_capacity,
-                        cudaStream_t stream, bool weights_settled);
+                        cudaStream_t stream, bool weights_settled, bool weights_fresh = false);
 
 // Gate, up, GeGLU and the quantiser of `down` into `buffer` (packed rows and their tiled scales, as in a plan's
 // scratch), then down over them; *done = false when shape, storage or pointers keep the three off that way.  `gate_plan`,

@@ -195,6 +195,8 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         ptx::tc_fence_after_sync();
         const uint32_t d = tmem_base + acc * kAccCols;
         const uint32_t idesc = idesc_of_width | ((uint32_t(w < p.tiles.whole ? p.tiles.tile_rows : p.tiles.piece_rows) >> 3) << 17);
+        // The split form has both accumulators to itself: each takes half of the K slabs.
+        const int mid_ks = kSplit ? (first_ks + end_ks + 1) / 2 : end_ks;
         for (int ks = first_ks; ks < end_ks; ++ks) {
           if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(full_bar + stage, phase))) {
             report(p.error, 0x35000000u | (blockIdx.x << 8) | stage, &abort_flag);
@@ -208,7 +210,9 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
             const uint64_t a = make_desc(base16), b = make_desc(base16 + (kWgtBytes >> 4));
 #pragma unroll
             for (int kb = 0; kb < 4; ++kb)
-              if (kb < nkb) mma_pair<FP8>(d, a + 2 * kb, b + 2 * kb, idesc, ((ks - first_ks) | kb) != 0 ? 1u : 0u);
+              if (kb < nkb)
+                mma_pair<FP8>(kSplit && ks >= mid_ks ? d + kAccCols : d, a + 2 * kb, b + 2 * kb, idesc,
+                              ((kSplit && ks >= mid_ks ? ks - mid_ks : ks - first_ks) | kb) != 0 ? 1u : 0u);
             commit_pair(empty_bar + stage, leader);
           }
           __syncwarp();
@@ -334,22 +338,38 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
     // Chunk c of 32 tokens is summed and stored by pair c % split: the other pairs write their 128 x 32 FP32 values of it into
     // that pair's operand ring, [token / 4][lane][token % 4], once every pair's MMAs have read theirs.
     __syncwarp();
-    ptx::tc_fence_before_sync();
-    cluster_sync_all();
+    const int split = p.tiles.split;
+    if (split > 1) {
+      ptx::tc_fence_before_sync();
+      cluster_sync_all();
+    }
     ptx::tc_fence_after_sync();
-    const int split = p.tiles.split, part = int(leader / 2), quad = warp % 4, half = (warp - kFirstEpilogueWarp) / 4;
+    const int part = int(leader / 2), quad = warp % 4, half = (warp - kFirstEpilogueWarp) / 4;
     const Tile tile = tile_of(p.tiles, p.rows, pair);
     const int chunks = (tile.end - tile.token0 + 31) / 32;
     const uint32_t taddr = tmem_base + (uint32_t(quad * 32) << 16);
     const uint32_t at = uint32_t(quad * 32 + lane) * 16;
-    if (warp >= kFirstEpilogueWarp) {
+    const bool both = end_ks - first_ks > 1;           // accumulators
+    const auto load_sum = [&](int c, uint32_t* r) {
+      ptx::tmem_load16(taddr + 32 * c, r);
+      ptx::tmem_load16(taddr + 32 * c + 16, r + 16);
+      if (both) {
+        uint32_t s[32];
+        ptx::tmem_load16(taddr + kAccCols + 32 * c, s);
+        ptx::tmem_load16(taddr + kAccCols + 32 * c + 16, s + 16);
+        ptx::tmem_load_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(s[i]));
+      } else {
+        ptx::tmem_load_wait();
+      }
+    };
+    if (split > 1 && warp >= kFirstEpilogueWarp) {
       for (int c = half; c < chunks; c += 2) {
         const int owner = c % split;
         if (owner == part) continue;
         uint32_t r[32];
-        ptx::tmem_load16(taddr + 32 * c, r);
-        ptx::tmem_load16(taddr + 32 * c + 16, r + 16);
-        ptx::tmem_load_wait();
+        load_sum(c, r);
         const int slot = c / split * (split - 1) + (part < owner ? part : part - 1);
         const uint32_t to = cluster_address(smem + slot * kPartBytes, uint32_t(2 * owner) + rank) + at;
 #pragma unroll
@@ -357,15 +377,13 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
       }
     }
     __syncwarp();
-    cluster_sync_all();
+    if (split > 1) cluster_sync_all();
     if (warp >= kFirstEpilogueWarp && !abort_flag) {
       const int channel = (tile.channel * 2 + int(rank)) * 128 + quad * 32 + lane;
       const float scale = p.channel_alpha == nullptr ? p.alpha : channel < p.n ? __ldg(p.channel_alpha + channel) : 0.0F;
       for (int k = half, c = part + half * split; c < chunks; k += 2, c += 2 * split) {
         uint32_t r[32];
-        ptx::tmem_load16(taddr + 32 * c, r);
-        ptx::tmem_load16(taddr + 32 * c + 16, r + 16);
-        ptx::tmem_load_wait();
+        load_sum(c, r);
         for (int other = 0; other < split - 1; ++other) {
           const uint32_t from = ptx::smem_u32(smem + (k * (split - 1) + other) * kPartBytes) + at;
 #pragma unroll
@@ -406,7 +424,7 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
     configured = true;
   }
   const int work = work_items(params.tiles), split = params.tiles.split;
-  const int pairs = split > 1 ? work * split : work < sm_count / 2 ? work : sm_count / 2;
+  const int pairs = split > 0 ? work * split : work < sm_count / 2 ? work : sm_count / 2;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(2 * pairs);
   config.blockDim = dim3(kThreads);
@@ -414,7 +432,7 @@ cudaError_t launch_instance(const PairWideParams& params, int sm_count, cudaStre
   config.stream = stream;
   cudaLaunchAttribute attributes[2]{};
   attributes[0].id = cudaLaunchAttributeClusterDimension;
-  attributes[0].val.clusterDim.x = 2 * split;
+  attributes[0].val.clusterDim.x = split > 0 ? 2 * split : 2;
   attributes[0].val.clusterDim.y = 1;
   attributes[0].val.clusterDim.z = 1;
   attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -431,25 +449,27 @@ PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int k_stages, int sm_co
   // A tile takes as long as its weight rows and MMA issue cost whatever its width (about 136 columns) plus its columns:
   // measured on FP8 K=5376, per wave of tiles of 64 / 128 / 192 / 256 tokens 8.9 / 11.3 / 14.3 / 17.4 us.
   const int channel_tiles = int((n + 255) / 256), pairs = sm_count / 2;
+  const bool small = rows <= 128 && k_stages > 0;
   PairWideTiles t{};
   uint64_t best_cost = ~0ull;
-  for (int tile = 256; tile >= 64; tile -= 32) {
+  for (int tile = small ? 128 : 256; tile >= (small ? 32 : 64); tile -= 32) {
     const int token_tiles = int((rows + tile - 1) / tile);
     const uint64_t tiles = uint64_t(channel_tiles) * token_tiles;
     const uint64_t cost = (tiles + pairs - 1) / pairs * uint64_t(tile + 136);
-    if (cost < best_cost) {
+    if (cost < best_cost && (!small || tiles <= uint64_t(pairs))) {
       best_cost = cost;
-      t = {tile, channel_tiles, token_tiles, int32_t(tiles), 1, tile};
+      t = {tile, channel_tiles, token_tiles, int32_t(tiles), 1, tile, small ? 1 : 0};
     }
   }
   // K shared by the pairs of a cluster, where few wide tiles leave pairs idle and narrower ones would read the weights more often: a
   // slab of a tile costs what it did, the launch and its barriers about 900 columns more, and 20 per column whose sum another pair
-  // has.  It has to win an eighth, because pairs at work slow each other down.  us, one pair / several, quantiser included: FP8 218x16384x5376 (three pairs, 224 wide) 32.9 / 27.4, 130x21504x5376 38.9 / 29.1, 180x8192x2816 18.0 / 13.4,
-  // BF16 140x5376x2048 19.7 / 12.2, 250x5376x4096 (two, 128 wide) 20.8 / 16.4; outside of the rule BF16 200x2816x8192
-  // 14.4 / 16.7, 491x5376x4096 22.2 / 23.0, FP8 300x2816x2816 9.6 / 10.1, 800x5376x2048 16.0 / 17.2.
+  // has.  It has to win an eighth, because pairs at work slow each other down.  us, one pair / several, quantiser included: FP8
+  // 218x16384x5376 (three pairs, 224 wide) 32.9 / 27.4, 130x21504x5376 38.9 / 29.1, 180x8192x2816 18.0 / 13.4, BF16 140x5376x2048
+  // 19.7 / 12.2, 250x5376x4096 (two, 128 wide) 20.8 / 16.4; outside of the rule BF16 200x2816x8192 14.4 / 16.7, 491x5376x4096
+  // 22.2 / 23.0, FP8 300x2816x2816 9.6 / 10.1, 800x5376x2048 16.0 / 17.2.
   uint64_t split_cost = (best_cost * uint64_t(k_stages) + 1900) * 7 / 8;
   for (int split = 2; split <= kMaxSplit && split <= k_stages; ++split)
-    for (int tile = 256; tile >= 64; tile -= 32) {
+    for (int tile = small ? 128 : 256; tile >= (small ? 32 : 64); tile -= 32) {
       const int token_tiles = int((rows + tile - 1) / tile);
       const uint64_t tiles = uint64_t(channel_tiles) * token_tiles;
       const uint64_t cost = uint64_t((k_stages + split - 1) / split) * uint64_t(tile + 136) + 2800 + uint64_t(20 * tile * (split - 1) / split);
@@ -458,7 +478,7 @@ PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int k_stages, int sm_co
         t = {tile, channel_tiles, token_tiles, int32_t(tiles), 1, tile, split};
       }
     }
-  if (t.split > 1) return t;
+  if (t.split > 0) return t;
   // A last wave for half of the pairs or fewer: its tiles in as many pieces as keep every pair at work, 32 columns or a multiple.
   // us, whole tiles / pieces: FP8 250x5376x21504 (74 + 10 tiles) 37.2 / 32.9, 180 rows 32.5 / 30.7, BF16 200 rows 59.2 / 55.0,
   // 4096x2816x4096 (222 + 34) 65.1 / 62.5, FP8 1025x5376x16384 (296 + 24) 76.0 / 75.5.  A wave with few tiles is quicker than a
@@ -486,7 +506,7 @@ PairWideParams with_ring(const PairWideParams& given, bool geglu) {
 
 cudaError_t launch_gemm_pair_wide(bool fp8, const PairWideParams& given, int sm_count, cudaStream_t stream) {
   const PairWideParams params = with_ring(given, false);
-  if (params.tiles.split > 1)
+  if (params.tiles.split > 0)
     return fp8 ? launch_instance<true, WideOut::split>(params, sm_count, stream) : launch_instance<false, WideOut::split>(params, sm_count, stream);
   return fp8 ? launch_instance<true, WideOut::store>(params, sm_count, stream) : launch_instance<false, WideOut::store>(params, sm_count, stream);
 }

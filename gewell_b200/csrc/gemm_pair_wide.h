@@ -15,7 +15,7 @@ struct PairWideTiles {
   int32_t channel_tiles, token_tiles;
   int32_t whole;                   // tiles that are taken whole: as many as fill waves of all pairs
   int32_t pieces, piece_rows;      // of each tile behind them: how many pieces, and their token columns
-  int32_t split = 1;               // pairs that share the K loop of a tile
+  int32_t split = 0;               // split form, one tile per cluster: pairs that share its K loop
 };
 
 struct PairWideParams {
@@ -38,7 +38,8 @@ struct PairWideParams {
   uint32_t* error;
 };
 
-// The division for this shape that takes least: `n` channels, 256 per tile; k_stages != 0: the K loop may be shared.
+// The division for this shape that takes least: `n` channels, 256 per tile; k_stages != 0: the split form is possible, and for at most
+// 128 rows it is what is taken (which needs one wave of tiles).
 PairWideTiles pair_wide_tiles(uint32_t rows, uint32_t n, int k_stages, int sm_count);
 
 // GeGLU of two projections with n channels each, as BF16 [rows, n] or (`quantise`) E4M3 [rows, n].  n is a multiple of 64, a tile

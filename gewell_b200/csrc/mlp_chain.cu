@@ -289,7 +289,7 @@ gw_status run_linear(PlanBook& book, const gw_projection& p, const void* input, 
     weights = book.dequantized.data;
     settled = false;
   }
-  return run_bf16_plan(set->bf16, input, weights, output, book.scratch.data, book.scratch.bytes, s, settled);
+  return run_bf16_plan(set->bf16, input, weights, output, book.scratch.data, book.scratch.bytes, s, settled, weights != p.bf16);
 }
 
 gw_projection widened(const gw_projection& first, uint32_t output) {

@@ -349,7 +349,7 @@ gw_status projection_workspace_run_on(gw_projection_workspace* w, const gw_proje
     }
     const bool split = w->scratch.data && w->scratch.bytes >= gw_bf16_plan_scratch_bytes(plans.bf16);
     status = run_bf16_plan(plans.bf16, input_bf16, weights, destination, split ? w->scratch.data : nullptr,
-                           split ? w->scratch.bytes : 0, stream, weights_settled);
+                           split ? w->scratch.bytes : 0, stream, weights_settled, weights != p.bf16);
   }
   if (status != GW_OK) return status;
   if (padded) {

@@ -46,3 +46,10 @@ def test_last_wave_in_pieces(kind, rows, n):
 def test_shared_k(kind, rows, k, n):
     """K over four, four, three, three, three and two pairs (of 148 SMs); channels and tokens that end within a tile."""
     test_pair(kind, rows, k, n)
+
+
+@pytest.mark.parametrize("kind,rows,k,n", [("fp8", 33, 4112, 272), ("fp8", 65, 80, 784), ("fp8 per channel", 128, 8208, 5376), ("bf16", 33, 16, 16),
+                                           ("bf16", 64, 2056, 6160), ("bf16", 97, 72, 9360), ("bf16", 128, 4104, 2816)])
+def test_few_rows(kind, rows, k, n):
+    """One wave of tiles for at most 128 rows: one slab of K (one accumulator) and many, one pair to a tile and several."""
+    test_pair(kind, rows, k, n)
