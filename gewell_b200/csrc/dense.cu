@@ -325,6 +325,10 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
   const DenseTuning& tuning = cache->tuning;
   const bool small_pairs = q.rows <= 128 && small_on_pairs(tuning, q);
   const bool swap = !small_pairs && dense_uses_swap_form(tuning, q.rows);
+  if (cache->small_pairs != small_pairs) {          // the other route's maps have other boxes
+    cache->small_pairs = small_pairs;
+    cache->weight = cache->activations = nullptr;
+  }
   const int block_n = small_pairs ? 256 : dense_block_n(tuning, q.rows);
   const bool fp4 = q.kind == GemmKind::nvfp4;
   const uint64_t row_bytes = fp4 ? q.k / 2 : (q.kind == GemmKind::bf16 ? uint64_t(2) * q.k : q.k);
