@@ -299,7 +299,8 @@ gw_status gw_gelu_tanh_multiply_interleaved_bf16(const void* gate_up_bf16, void*
  * bound weights (gw_projection: BF16, FP8 or NVFP4 each; physical_output == output).  Gate and up run
  * as ONE GEMM when they are stored back to back (NVFP4: contiguous rows and scale tiles with equal
  * globals, 31b/sm120/nvfp4_projections.h:21-33; FP8: adjacent with per-channel scales,
- * fp8_projections.h:20-50; BF16: adjacent); GeGLU is fused into the down projection's activation
+ * fp8_projections.h:20-50; BF16: adjacent); GeGLU is fused into the gate/up launch beyond 128 rows, for
+ * narrow MLPs beyond 8 and where the weights stream, else into the down projection's activation
  * quantiser whenever that one runs quantised on the joined tensor.  policy / phase as in
  * nvfp4_policy.h: with policy "prefill" decode keeps BF16 activations (W4A16, as in ProjectionWorkspace:
  * packed weights up to 32 rows, dequantised into the chain's scratch beyond).
@@ -307,8 +308,8 @@ gw_status gw_gelu_tanh_multiply_interleaved_bf16(const void* gate_up_bf16, void*
  *   prepare   builds the plans for a row count, outside the layer loop
  *   run       gate_up_bf16: [rows, 2 * mlp] scratch of the caller ([rows, gate | up] when joined, gate
  *             rows then up rows otherwise; not written where gate, up and GeGLU are one launch),
- *             product_bf16: [rows, mlp] scratch (GeGLU of the two, where it is not fused into the down
- *             projection's quantiser), output_bf16: [rows, hidden]; allocates nothing */
+ *             product_bf16: [rows, mlp] scratch (GeGLU of the two, or that quantised for the down projection,
+ *             where it is not fused into the down projection's quantiser), output_bf16: [rows, hidden]; allocates nothing */
 typedef struct gw_mlp_chain gw_mlp_chain;
 gw_status gw_mlp_chain_create(uint32_t hidden, uint32_t mlp, uint32_t max_rows, int policy, gw_mlp_chain** chain);
 gw_status gw_mlp_chain_prepare(gw_mlp_chain* chain, uint32_t rows);
@@ -387,9 +388,10 @@ gw_status gw_moe_dispatch(gw_moe_workspace* workspace, const void* scores_bf16,
 /* MoeWorkspace::run (moe.cu:489-534).  has_bf16 / has_fp8 / has_nvfp4 say which kinds of expert
  * weights the table holds (a kind whose flag is 0 is not computed, as in the reference); fp4 != 0 runs
  * NVFP4 experts with FP4 activations (W4A4), fp4 == 0 with BF16 activations (W4A16, see
- * gw_moe_expert_table_enable_w4a16).  A table of NVFP4 experts only with fp4 != 0 takes the fused
- * large-batch path; every other combination runs one grouped gate/up and down GEMM per kind present
- * (tcgen05 kind::mxf4nvf4 / kind::f16 / kind::f8f6f4) with GeGLU unfused. */
+ * gw_moe_expert_table_enable_w4a16).  Tables of one kind run with GeGLU in the gate/up GEMM (NVFP4 with
+ * fp4 != 0 and FP8 where gate and up share an input scale, or NVFP4 beyond 2048 tokens; BF16; fp4 == 0);
+ * every other combination runs one grouped gate/up and down GEMM per kind present (tcgen05
+ * kind::mxf4nvf4 / kind::f16 / kind::f8f6f4) with GeGLU unfused. */
 gw_status gw_moe_run(gw_moe_workspace* workspace, const void* input_bf16, const void* scores_bf16,
                      const void* expert_scales_bf16, const gw_expert_table* table, void* output_bf16,
                      uint32_t rows, int has_bf16, int has_fp8, int has_nvfp4, int fp4, void* stream);
