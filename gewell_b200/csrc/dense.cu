@@ -306,7 +306,8 @@ namespace {
 //   BF16  33 x 2816x2816 10.4 / 9.2; 128 x 5376x2048 17.1 / 12.3, 21504x5376 52.2 / 42.0
 //   both  more than a third of the pairs' channels, 5376x8192 65 rows FP8 15.4 / 15.6, BF16 22.2 / 20.5, 128 rows 16.9 / 15.8, 23.9 / 20.8
 //   NVFP4, whose tile is 256 rows high whatever their number, long K and few channels: 65 x 8192x2816 13.9 / 11.9, 12288x4096 16.6 /
-//         16.2, 128 rows 15.0 / 12.9, 20.1 / 17.9; but 65 x 8192x5376 14.0 / 14.6, 112 x 4096x2816 10.7 / 11.9
+//         16.2, 128 rows 15.0 / 12.9, 20.1 / 17.9; but 65 x 8192x5376 14.0 / 14.6, 112 x 4096x2816 10.7 / 11.9;
+//         33 x 8192x2816 12.0 / 10.9, 8192x3072 11.9 / 11.0, 12288x2048 12.5 / 12.2, but 16384x2816 14.5 / 14.5, 21504x512 14.1 / 14.5
 // Weights that the launch before wrote, more of them than L2 holds, stay on the swap form (MLP 5376 -> 21504 with dequantised weights
 // 36 rows 286 / 292, 128 rows 312 / 312; 2816 -> 8192 86 / 84, 97 / 88).
 // The pairs' sums are of more and shorter parts of K; the error against FP64 is no larger at any of these sizes.
@@ -315,7 +316,7 @@ bool small_on_pairs(const DenseTuning& tuning, const DenseProblem& q) {
   if (!tuning.streams() || tuning.no_pair || q.rows <= 32) return false;
   const int channel_tiles = int((q.n + 255) / 256), pairs = sm_count() / 2;
   if (q.kind == GemmKind::nvfp4)
-    return q.rows > 64 && q.k >= 8192 && channel_tiles <= pairs / 4 && q.n % 8 == 0 && reinterpret_cast<uintptr_t>(q.output) % 16 == 0;
+    return q.k >= 8192 && (q.rows > 64 ? channel_tiles <= pairs / 4 : channel_tiles <= pairs / 6 && q.k <= 12288) && q.n % 8 == 0 && reinterpret_cast<uintptr_t>(q.output) % 16 == 0;
   if (q.weights_fresh && size_t(q.n) * q.k * sizeof(bf16) > kBeyondL2) return false;
   return channel_tiles <= (q.rows <= 96 ? pairs / 3 : pairs / 2) && (q.kind == GemmKind::bf16 || q.rows > 64 || q.k >= 4096);
 }

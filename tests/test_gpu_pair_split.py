@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("rows,k,n", [(129, 16448, 128), (255, 8256, 384), (257, 12352, 2560), (256, 21504, 5376), (512, 16384, 4096),
-                                      (513, 8256, 2816), (65, 8192, 128), (128, 16448, 4608), (100, 8256, 2816)])
+                                      (513, 8256, 2816), (33, 8192, 128), (64, 12288, 2816), (65, 8192, 128), (128, 16448, 4608), (100, 8256, 2816)])
 def test_shared_k(monkeypatch, rows, k, n):
     """K over two to four pairs (of 148 SMs); tokens and channels that end within a tile, K that ends within a stage."""
     import gewell_b200 as gw
