@@ -24,8 +24,12 @@ bool dense_uses_swap_form(const DenseTuning& tuning, uint32_t rows) {
   return rows <= 128;
 }
 
+namespace {
+int swap_block_n(uint32_t rows) { return rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
+}  // namespace
+
 int dense_block_n(const DenseTuning& tuning, uint32_t rows) {
-  if (dense_uses_swap_form(tuning, rows)) return rows <= 32 ? 32 : rows <= 64 ? 64 : 128;
+  if (dense_uses_swap_form(tuning, rows)) return swap_block_n(rows);
   if (tuning.block_n == 128 || tuning.block_n == 256) return tuning.block_n;
   return 256;
 }
@@ -324,13 +328,16 @@ bool small_on_pairs(const DenseTuning& tuning, const DenseProblem& q) {
 
 gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStream_t stream) {
   const DenseTuning& tuning = cache->tuning;
+  // NVFP4 outputs may lie on any 2-byte boundary.  The swap form stores two bytes at a time, all other kernels sixteen.
+  const bool unaligned = q.kind == GemmKind::nvfp4 && reinterpret_cast<uintptr_t>(q.output) % 16 != 0;
   const bool small_pairs = q.rows <= 128 && small_on_pairs(tuning, q);
-  const bool swap = !small_pairs && dense_uses_swap_form(tuning, q.rows);
-  if (cache->small_pairs != small_pairs) {          // the other route's maps have other boxes
+  const bool swap = unaligned || (!small_pairs && dense_uses_swap_form(tuning, q.rows));
+  const int block_n = small_pairs ? 256 : swap ? swap_block_n(q.rows) : dense_block_n(tuning, q.rows);
+  if (cache->small_pairs != small_pairs || cache->swap != swap) {          // another route's maps have other boxes
     cache->small_pairs = small_pairs;
+    cache->swap = swap;
     cache->weight = cache->activations = nullptr;
   }
-  const int block_n = small_pairs ? 256 : dense_block_n(tuning, q.rows);
   const bool fp4 = q.kind == GemmKind::nvfp4;
   const uint64_t row_bytes = fp4 ? q.k / 2 : (q.kind == GemmKind::bf16 ? uint64_t(2) * q.k : q.k);
   std::string error;

@@ -35,7 +35,7 @@ struct DenseDescriptors {          // re-encoded only when a pointer changes
   const void* activations = nullptr;
   const void* weight_scales = nullptr;
   CUtensorMap weight_map{}, activation_map{}, weight_scale_map{};
-  bool small_pairs = false;          // which route of few rows the maps are for
+  bool small_pairs = false, swap = false;          // which route the maps are for
   const void* weight_half = nullptr;
   CUtensorMap weight_half_map{};     // 128-row box over the weights (CTA-pair kernel: each CTA stages half a tile)
   PairWideTiles wide;                // FP8 / BF16 CTA-pair kernel: division of the work

@@ -1,0 +1,49 @@
+"""Which kernels a projection is launched on, from the host code alone: a CUDA runtime that only records
+(tests/cpp/fake_cudart.cpp, 148 SMs) names them.  No GPU."""
+import pytest
+
+from tests.test_prepare import CHILD, fake_runtime, run_child  # noqa: F401  (fixture)
+
+NAMES = CHILD + r'''
+fake.fake_launched.restype = ctypes.c_char_p
+
+
+def kernels(run):
+    """The kernels that a run launches, as the compiler mangles their names."""
+    fake.fake_launched()
+    check(run())
+    return fake.fake_launched().decode().split()
+
+
+def nvfp4_plan(rows, k, n):
+    plan = ctypes.c_void_p()
+    check(lib.gw_nvfp4_plan_create(rows, k, n, ctypes.byref(plan)))
+    return lambda output: lib.gw_nvfp4_plan_run(plan, A, A, A, 0.01, 0.01, output, A, 1 << 40, None, 0)
+'''
+
+UNALIGNED = NAMES + r'''
+swap_form = kernels(lambda: nvfp4_plan(128, 2816, 2816)(A))[-1]
+assert "gemm_tc_kernel" in swap_form
+for rows, k, n in ((128, 8192, 256), (129, 256, 128), (200, 2816, 2816), (257, 12352, 2560), (1000, 640, 384)):
+    run = nvfp4_plan(rows, k, n)
+    for offset in (0, 2, 8, 0, 14):
+        names = kernels(lambda: run(A + offset))
+        assert len(names) == 2
+        assert (names[1] == swap_form) == (offset != 0), (rows, k, n, offset, names)
+        assert ("gemm_pair" in names[1]) == (offset == 0), (rows, k, n, offset, names)
+'''
+
+
+@pytest.mark.parametrize("form", [None, "direct"])
+def test_unaligned_nvfp4_output_keeps_off_vector_stores(fake_runtime, monkeypatch, form):
+    """The kernels of more than 128 rows store sixteen bytes at a time; an output that is not 16-byte aligned takes the swap form."""
+    script = UNALIGNED
+    if form:
+        monkeypatch.setenv("GW_DENSE_FORM", form)
+        script = NAMES + r'''
+for rows in (1, 40, 128, 300):
+    run = nvfp4_plan(rows, 640, 384)
+    direct, unaligned = kernels(lambda: run(A))[-1], kernels(lambda: run(A + 2))[-1]
+    assert direct != unaligned and "gemm_tc_kernel" in unaligned, rows
+'''
+    run_child(fake_runtime, script)
