@@ -702,10 +702,10 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
   GW_CUDA_CHECK(recorded, "feed-forward block join");
   // router logits and the experts (batched_executor.cu:262-266)
   if (rows <= kRouterRows && aligned16(w.router_proj)) {
-    status = GW_OK;
-    GW_CUDA_CHECK(launch_pdl(router_logits_kernel, dim3(kRouterExperts / 16, (rows + 7) / 8), kRouterThreads, as_stream(s),
-                             reinterpret_cast<const uint4*>(b->router_input), static_cast<const uint4*>(w.router_proj), b->logits, rows),
-                  "router logits");
+    const cudaError_t launched =
+        launch_pdl(router_logits_kernel, dim3(kRouterExperts / 16, (rows + 7) / 8), kRouterThreads, as_stream(s),
+                   reinterpret_cast<const uint4*>(b->router_input), static_cast<const uint4*>(w.router_proj), b->logits, rows);
+    if (launched != cudaSuccess) status = fail(GW_CUDA_ERROR, std::string("router logits: ") + cudaGetErrorString(launched));
   } else {
     status = run_bf16_plan(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes,
                            as_stream(s), true);

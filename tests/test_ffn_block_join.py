@@ -1,0 +1,29 @@
+"""A feed-forward block whose run fails brings its side stream back: work that follows on the caller's stream does not overlap
+the shared MLP's, and a stream capture is left without a fork.  Every launch of a run fails in turn, on a CUDA runtime that only
+records (tests/cpp/fake_cudart.cpp).  No GPU."""
+import pytest
+
+from tests.test_prepare import BLOCK, fake_runtime, run_child  # noqa: F401  (fixture)
+
+JOIN = BLOCK[:BLOCK.index("for small, large")] + r'''
+fake.fake_forked.restype = fake.fake_launch_failures_left.restype = ctypes.c_long
+fake.fake_fail_launch.argtypes = [ctypes.c_long]
+for rows in ROWS:
+    check(prepare(rows))
+    total = launches(run)
+    assert fake.fake_forked() == 0
+    reported = 0
+    for n in range(1, total + 1):
+        fake.fake_fail_launch(n)
+        status = run()
+        assert fake.fake_launch_failures_left() == 0
+        assert fake.fake_forked() == 0, f"{rows} rows: launch {n} of {total} failed and the side stream was not joined"
+        reported += status == _lib.GW_CUDA_ERROR
+    assert reported >= 1
+    assert launches(run) == total
+'''
+
+
+@pytest.mark.parametrize("rows", [8, 40, 129])
+def test_failed_run_joins_the_side_stream(fake_runtime, rows):
+    run_child(fake_runtime, JOIN.replace("ROWS", f"({rows},)"))
