@@ -449,11 +449,10 @@ struct gw_ffn_block {
   // The shared MLP runs on a stream of its own beside the router, the routing and the experts' input, which leave most of
   // the GPU idle at small row counts, and fills the tails of the experts' GEMMs at large ones (one stream -> two, us: NVFP4
   // 8 rows 100.7 -> 95.1, 470 rows 231.8 -> 213.1, 4000 rows 472.8 -> 445.5; BF16 8 rows 172 -> 149).  So the router has a
-  // plan and scratch apart from the shared MLP's.
+  // plan apart from the shared MLP's, beyond the rows of router_logits_kernel; such a plan needs no scratch.
   cudaStream_t side = nullptr;
   cudaEvent_t forked = nullptr, joined = nullptr;
   gw_bf16_plan* router_plan = nullptr;
-  DeviceBuffer router_scratch;
   DeviceBuffer buffers;                  // one allocation, carved below
   bf16 *normalized = nullptr, *router_input = nullptr, *expert_input = nullptr, *gate = nullptr, *up = nullptr,
        *product = nullptr, *shared_mlp = nullptr, *logits = nullptr, *routed = nullptr;
@@ -608,8 +607,6 @@ gw_status gw_ffn_block_create(const gw_ffn_block_weights* layers, uint32_t count
   const size_t narrow = align_up(size_t(max_rows) * kSharedMlp * sizeof(bf16), 256);
   const size_t scores = align_up(size_t(max_rows) * kExperts * sizeof(bf16), 256);
   GW_CUDA_CHECK(b->buffers.allocate(5 * wide + 3 * narrow + scores), "feed-forward block buffers");
-  // FP32 partial tiles of the router's K split (<= 128 rows, 128-wide tiles)
-  GW_CUDA_CHECK(b->router_scratch.allocate(size_t(2) * size_t(sm_count()) * 128 * 128 * sizeof(float) + 256), "feed-forward block buffers");
   GW_CUDA_CHECK(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "feed-forward block stream");
   GW_CUDA_CHECK(cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming), "feed-forward block event");
   GW_CUDA_CHECK(cudaEventCreateWithFlags(&b->joined, cudaEventDisableTiming), "feed-forward block event");
@@ -635,7 +632,7 @@ gw_status gw_ffn_block_create(const gw_ffn_block_weights* layers, uint32_t count
 void gw_ffn_block_destroy(gw_ffn_block* block) { delete block; }
 
 size_t gw_ffn_block_bytes(const gw_ffn_block* b) {
-  return b ? b->buffers.bytes + b->router_scratch.bytes + gw_projection_workspace_bytes(b->projections) + gw_moe_bytes(b->moe) : 0;
+  return b ? b->buffers.bytes + gw_projection_workspace_bytes(b->projections) + gw_moe_bytes(b->moe) : 0;
 }
 
 gw_status gw_ffn_block_prepare(gw_ffn_block* b, uint32_t rows, int phase) {
@@ -643,14 +640,14 @@ gw_status gw_ffn_block_prepare(gw_ffn_block* b, uint32_t rows, int phase) {
   if (!b || rows == 0 || rows > b->capacity) return fail(GW_INVALID_ARGUMENT, "feed-forward block: invalid rows");
   // The router's plan first, beside the present one: what follows either prepares the projections too or leaves all as it was.
   gw_bf16_plan* plan = nullptr;
-  if (b->rows != rows)
+  if (b->rows != rows && rows > kRouterRows)
     if (const gw_status created = gw_bf16_plan_create(rows, kHidden, kExperts, &plan); created != GW_OK) return created;
   const gw_status status = gw_projection_workspace_prepare(b->projections, rows, phase);
   if (status != GW_OK) {
     if (plan) gw_bf16_plan_destroy(plan);
     return status;
   }
-  if (plan) {
+  if (b->rows != rows) {
     if (b->router_plan) gw_bf16_plan_destroy(b->router_plan);
     b->router_plan = plan;
   }
@@ -668,6 +665,7 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
       !w.post_feedforward_norm_2 || !w.post_feedforward_norm || !w.layer_scalar || !w.router_proj ||
       !w.router_per_expert_scale || !w.experts)
     return fail(GW_INVALID_ARGUMENT, "feed-forward block: a weight is missing");
+  if (!aligned16(w.router_proj)) return fail(GW_INVALID_ARGUMENT, "feed-forward block requires a 16-byte aligned router projection");
   const uint32_t rows = b->rows;
   void* s = b->stream;
   gw_status status = gw_rms_norm_feedforward_bf16(hidden_bf16, w.pre_feedforward_norm, w.router_scale,
@@ -701,14 +699,13 @@ gw_status gw_ffn_block_run(gw_ffn_block* b, const gw_ffn_block_weights* weights,
   }
   GW_CUDA_CHECK(recorded, "feed-forward block join");
   // router logits and the experts (batched_executor.cu:262-266)
-  if (rows <= kRouterRows && aligned16(w.router_proj)) {
+  if (rows <= kRouterRows) {
     const cudaError_t launched =
         launch_pdl(router_logits_kernel, dim3(kRouterExperts / 16, (rows + 7) / 8), kRouterThreads, as_stream(s),
                    reinterpret_cast<const uint4*>(b->router_input), static_cast<const uint4*>(w.router_proj), b->logits, rows);
     if (launched != cudaSuccess) status = fail(GW_CUDA_ERROR, std::string("router logits: ") + cudaGetErrorString(launched));
   } else {
-    status = run_bf16_plan(b->router_plan, b->router_input, w.router_proj, b->logits, b->router_scratch.data, b->router_scratch.bytes,
-                           as_stream(s), true);
+    status = run_bf16_plan(b->router_plan, b->router_input, w.router_proj, b->logits, nullptr, 0, as_stream(s), true);
   }
   MoeCombineInput combine;
   if (status == GW_OK)

@@ -27,3 +27,23 @@ for rows in ROWS:
 @pytest.mark.parametrize("rows", [8, 40, 129])
 def test_failed_run_joins_the_side_stream(fake_runtime, rows):
     run_child(fake_runtime, JOIN.replace("ROWS", f"({rows},)"))
+
+
+def test_router_memory_and_alignment(fake_runtime):
+    """Beyond the block's buffers nothing is held for the router, and a router projection that no kernel takes is refused before
+    anything is launched, at every row count."""
+    run_child(fake_runtime, BLOCK[:BLOCK.index("for small, large")] + r'''
+for name in ("gw_ffn_block_bytes", "gw_moe_bytes", "gw_projection_workspace_bytes"):
+    getattr(lib, name).restype = ctypes.c_size_t
+ws = ctypes.c_void_p()
+check(lib.gw_projection_workspace_create((_lib.Projection * 3)(w.gate, w.up, w.down), 3, 256, _lib.POLICY_ALWAYS, None, ctypes.byref(ws)))
+buffers = 256 * (5 * 2816 + 3 * 2112 + 128) * 2
+assert lib.gw_ffn_block_bytes(block) == buffers + lib.gw_projection_workspace_bytes(ws) + lib.gw_moe_bytes(lib.gw_ffn_block_moe(block))
+for rows in (8, 128, 129, 8):
+    check(prepare(rows))
+    w.router_proj = A + 8
+    before = fake.fake_launches()
+    assert run() == _lib.GW_INVALID_ARGUMENT and fake.fake_launches() == before
+    w.router_proj = A
+    check(run())
+''')
