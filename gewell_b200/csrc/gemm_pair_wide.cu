@@ -43,6 +43,8 @@ constexpr int kAccCols = 256, kTmemCols = 512;
 constexpr int kPitch = 256 + 16, kStagingBytes = 32 * kPitch;
 constexpr int ring_bytes(bool geglu) { return 221 * 1024 - (geglu ? 2 * kStagingBytes : 0); }
 constexpr int kSmemBytes = 221 * 1024 + 1024;
+constexpr int kPartCols = 128;                     // the GeGLU form's accumulators of a part of K
+static_assert(4 * kPartCols <= kTmemCols, "tensor memory over-subscribed");
 constexpr int kMaxSplit = 4;
 constexpr int kPartBytes = 128 * 32 * 4;             // one pair's FP32 part of 32 tokens
 static_assert(4 * kPartBytes <= ring_bytes(false) && 3 * 2 * kPartBytes <= ring_bytes(false) && 2 * 3 * kPartBytes <= ring_bytes(false),
@@ -145,6 +147,11 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
   // Split: one tile per cluster, an even part of its K slabs per pair
   const int first_ks = kSplit ? int(leader / 2) * p.k_stages / p.tiles.split : 0;
   const int end_ks = kSplit ? int(leader / 2 + 1) * p.k_stages / p.tiles.split : p.k_stages;
+  // GeGLU of at most one tile a pair, 128 tokens wide at most: tensor memory holds four accumulators, each for an even part of K,
+  // and the epilogue adds them up.  The swap form, which runs such rows otherwise, divides K over four CTAs, and a sum of all of K
+  // in one accumulator is further from the exact one (outputs that are not the nearest BF16, 2816 -> 2176, swap form / one
+  // accumulator: BF16 16 rows 4.1e-4 / 1.5e-3, FP8 with blocks of sixteen activations scaled by 2^-6 .. 2^6 1.7e-4 / 5.5e-4).
+  const int parts = kGeglu && total_work <= pairs && p.tiles.tile_rows <= kPartCols ? min(4, p.k_stages) : 1;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
@@ -197,7 +204,13 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         const uint32_t idesc = idesc_of_width | ((uint32_t(w < p.tiles.whole ? p.tiles.tile_rows : p.tiles.piece_rows) >> 3) << 17);
         // The split form has both accumulators to itself: each takes half of the K slabs.
         const int mid_ks = kSplit ? (first_ks + end_ks + 1) / 2 : end_ks;
+        int part = 0, part_end = kGeglu ? p.k_stages / parts : 0;
+        bool begins = true;
         for (int ks = first_ks; ks < end_ks; ++ks) {
+          if (kGeglu && ks == part_end) {
+            begins = true;
+            part_end = (++part + 1) * p.k_stages / parts;
+          }
           if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(full_bar + stage, phase))) {
             report(p.error, 0x35000000u | (blockIdx.x << 8) | stage, &abort_flag);
             failed = true;
@@ -210,12 +223,17 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
             const uint64_t a = make_desc(base16), b = make_desc(base16 + (kWgtBytes >> 4));
 #pragma unroll
             for (int kb = 0; kb < 4; ++kb)
-              if (kb < nkb)
-                mma_pair<FP8>(kSplit && ks >= mid_ks ? d + kAccCols : d, a + 2 * kb, b + 2 * kb, idesc,
-                              ((kSplit && ks >= mid_ks ? ks - mid_ks : ks - first_ks) | kb) != 0 ? 1u : 0u);
+              if (kb < nkb) {
+                if constexpr (kGeglu)
+                  mma_pair<FP8>(d + uint32_t(part * kPartCols), a + 2 * kb, b + 2 * kb, idesc, begins && kb == 0 ? 0u : 1u);
+                else
+                  mma_pair<FP8>(kSplit && ks >= mid_ks ? d + kAccCols : d, a + 2 * kb, b + 2 * kb, idesc,
+                                ((kSplit && ks >= mid_ks ? ks - mid_ks : ks - first_ks) | kb) != 0 ? 1u : 0u);
+              }
             commit_pair(empty_bar + stage, leader);
           }
           __syncwarp();
+          begins = false;
           if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
         if (!failed && ptx::elect_one()) commit_pair(acc_full_bar + acc, leader);
@@ -251,6 +269,14 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         ptx::tmem_load16(taddr + t0, r);
         ptx::tmem_load16(taddr + t0 + 16, r + 16);
         ptx::tmem_load_wait();
+        for (int part = 1; part < parts; ++part) {
+          uint32_t s[32];
+          ptx::tmem_load16(taddr + part * kPartCols + t0, s);
+          ptx::tmem_load16(taddr + part * kPartCols + t0 + 16, s + 16);
+          ptx::tmem_load_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(s[i]));
+        }
         if (t0 != half * 32) half_barrier(half);                    // the chunk before has been read
         uint16_t* put = reinterpret_cast<uint16_t*>(staging) + quad * 32 + lane;
 #pragma unroll
