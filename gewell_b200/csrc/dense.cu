@@ -107,9 +107,11 @@ namespace {
 // leaves idle.  A K stage takes 0.28 (NVFP4) / 0.5 (FP8, two slabs) / 0.2 us (BF16) of latency, and no less than its bytes
 // at 5.2 TB/s over the CTAs that run.  Measured, divided over all SMs -> whole tiles (us): NVFP4 32x2816x2816 12.8 -> 7.6,
 // 64x2816x2816 16.3 -> 8.9, 24x5376x8192 14.4 -> 10.4, FP8 64x2816x2816 15.3 -> 8.9; BF16 64x2816x128 stays divided, by
-// four: 12.4 -> 9.9.  CTAs that begin in one tile and end in another write two partial tiles, so NVFP4, whose sums are exact however
-// they are divided, takes as many for every tile: 12x21504x5376 (42 tiles, 148 -> 126 CTAs) 19.2 -> 16.9, 64x8192x5376 18.1 -> 14.4,
-// 100x21504x5376 30.8 -> 25.1.
+// four: 12.4 -> 9.9.  CTAs that begin in one tile and end in another write two partial tiles, so NVFP4 takes as many for
+// every tile: 12x21504x5376 (42 tiles, 148 -> 126 CTAs) 19.2 -> 16.9, 64x8192x5376 18.1 -> 14.4, 100x21504x5376 30.8 -> 25.1.  Their
+// parts of K are longer, and a sum of products with block scales rounds where the scales differ widely (outputs that are not the
+// nearest BF16 with blocks scaled by 2^-6 .. 2^6, 100x21504x5376, 148 / 126 CTAs 1.3e-3 / 1.6e-3; none with N(0, 1)): so each of these
+// CTAs has an accumulator for either half of its part.
 int swap_split_grid(GemmKind kind, int tiles, int stages, int block_n) {
   const int sms = sm_count();
   const double latency = kind == GemmKind::nvfp4 ? 0.28 : kind == GemmKind::fp8 ? 0.5 : 0.2;

@@ -218,6 +218,9 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
   const int k_stages = (total_kb + kKbPerStage - 1) / kKbPerStage;
   const int k_atoms = p.k / 64;                             // scale atoms per 128-row block (NVFP4)
   const bool split = p.split_partials != nullptr;
+  // As many CTAs for every tile (the host divides NVFP4 so): a CTA has one part of one tile and both accumulators to itself, each
+  // for half of its K stages.
+  const bool halved = kNvfp4 && EPI == GemmEpilogue::swap_store && C::kAccStages == 2 && split && gridDim.x % total_work == 0;
 
   // shared-memory descriptors: high words are constants, low word = address >> 4
   constexpr uint32_t kDescHiSw128 = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);   // SBO 1024 B, version 1, SWIZZLE_128B
@@ -401,6 +404,7 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
       const uint32_t idesc = kNvfp4 ? ptx::idesc_nvfp4(item.mma_n)
                              : (KIND == GemmKind::bf16 ? ptx::idesc_bf16(item.mma_n) : ptx::idesc_fp8(item.mma_n));
       bool failed = false;
+      const int mid = halved ? (ks0 + ks1 + 1) / 2 : ks1;
       for (int ks = ks0; ks < ks1; ++ks) {
         const long long t0 = prof ? clock64() : 0;
         if constexpr (kNvfp4) {
@@ -428,7 +432,8 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
           const uint32_t base16 = smem_base16 + uint32_t(stage) * uint32_t(C::kStageBytes >> 4);
           const uint32_t sfl_t = sfl_tmem + uint32_t(stage) * C::kSfSlotCols;
           const uint32_t sfc_t = sfc_tmem + uint32_t(stage) * C::kSfSlotCols;
-          const uint32_t first = ks == ks0 ? 0u : 1u;
+          const uint32_t first = ks == ks0 || ks == mid ? 0u : 1u;
+          const uint32_t d = halved && ks >= mid ? d_tmem + BLOCK_N : d_tmem;
 #pragma unroll
           for (int kb = 0; kb < kKbPerStage; ++kb) {
             if (kb < nkb) {
@@ -438,12 +443,12 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
               const uint32_t c16 = base16 + kCOff16 + uint32_t(kb / kKBlocksPerStage) * uint32_t(C::kCSlabBytes >> 4) +
                                    2 * uint32_t(kb % kKBlocksPerStage);
               if constexpr (kNvfp4)
-                ptx::tc_mma_nvfp4(d_tmem, make_desc(kDescHiSw128, l16), make_desc(kDescHiSw128, c16), idesc, sfl_t + 4 * kb,
+                ptx::tc_mma_nvfp4(d, make_desc(kDescHiSw128, l16), make_desc(kDescHiSw128, c16), idesc, sfl_t + 4 * kb,
                                   sfc_t + kb * C::kSfcColsPerKb, kb == 0 ? first : 1u);
               else if constexpr (KIND == GemmKind::bf16)
-                ptx::tc_mma_bf16(d_tmem, make_desc(kDescHiSw128, l16), make_desc(kDescHiSw128, c16), idesc, kb == 0 ? first : 1u);
+                ptx::tc_mma_bf16(d, make_desc(kDescHiSw128, l16), make_desc(kDescHiSw128, c16), idesc, kb == 0 ? first : 1u);
               else
-                ptx::tc_mma_fp8(d_tmem, make_desc(kDescHiSw128, l16), make_desc(kDescHiSw128, c16), idesc, kb == 0 ? first : 1u);
+                ptx::tc_mma_fp8(d, make_desc(kDescHiSw128, l16), make_desc(kDescHiSw128, c16), idesc, kb == 0 ? first : 1u);
             }
           }
           ptx::tc_commit(empty_bar + stage);
@@ -599,6 +604,13 @@ gemm_tc_kernel(const __grid_constant__ GemmParams p) {
             uint32_t r[16];
             ptx::tmem_load16(taddr + c0, r);
             ptx::tmem_load_wait();
+            if (halved && ks1 - ks0 > 1) {
+              uint32_t second[16];
+              ptx::tmem_load16(taddr + BLOCK_N + c0, second);
+              ptx::tmem_load_wait();
+#pragma unroll
+              for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(second[i]));
+            }
 #pragma unroll
             for (int i = 0; i < 16; ++i) __stcg(mine + (c0 + i) * kTileL + row, __uint_as_float(r[i]));
           }

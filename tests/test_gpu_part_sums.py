@@ -49,6 +49,15 @@ def projected(gw, kind, x, weight, k, n):
     return y.float()
 
 
+@pytest.mark.parametrize("rows", [12, 64, 100])
+def test_swap_form_split_sums_sixths(gw, rows):
+    """42 tiles of NVFP4 channels: three CTAs a tile, and two accumulators in each of them; the four parts between the ends are kept."""
+    k, n = 21504, 5376
+    x, weight, whole = operands(gw, "w4a4", rows, k, n)
+    kept = projected(gw, "w4a4", x, weight, k, n) / whole
+    assert kept.min() >= 4 / 6 - 0.03 and kept.max() <= 1.05, (kept.min(), kept.max())
+
+
 @pytest.mark.parametrize("kind", ["bf16", "fp8"])
 @pytest.mark.parametrize("rows,hidden,mlp", [(9, 2816, 2176), (33, 2816, 2176), (64, 5376, 2048), (128, 2816, 384)])
 def test_geglu_sums_quarters(gw, kind, rows, hidden, mlp):
