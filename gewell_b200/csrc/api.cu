@@ -339,7 +339,7 @@ gw_status gw::run_nvfp4_geglu(gw_nvfp4_plan* gate_plan, gw_nvfp4_plan* down_plan
       gate.input != up.input || gate.output != up.output || gate.physical_output != up.physical_output || down.input != gate.output ||
       gate.physical_output != align_up(gate.output, 128) || gate.output % 64 != 0 || gate_plan->input_width != gate.input ||
       down_plan->rows != gate_plan->rows || down_plan->input_width != down.input || down_plan->output_width != down.physical_output ||
-      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::nvfp4, gate_plan->rows, gate.output) ||
+      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::nvfp4, gate_plan->rows, gate.input, gate.output) ||
       !input || !output || !aligned(input, 16) || !aligned(output, 2) || !aligned(buffer, 256) || !aligned(scratch, 256) ||
       scratch_capacity < gate_plan->split_offset || down_plan->split_offset > size_t(down_plan->rows) * down.input * sizeof(bf16))
     return GW_OK;
@@ -598,7 +598,7 @@ gw_status gw::run_fp8_geglu(gw_fp8_plan* gate_plan, const gw_projection& gate, c
   *done = false;
   if (!gate_plan || !same_shape(gate, up) || !usable_fp8(gate) || !usable_fp8(up) || gate.fp8_input_scale != up.fp8_input_scale ||
       gate_plan->input_width != gate.input || gate_plan->output_width != gate.output ||
-      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::fp8, gate_plan->rows, gate.output) || !input || !aligned(input, 2) || !product ||
+      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::fp8, gate_plan->rows, gate.input, gate.output) || !input || !aligned(input, 2) || !product ||
       !aligned(product, 16) || !scratch || !aligned(scratch, 256) || scratch_capacity < gate_plan->split_offset)
     return GW_OK;
   *done = true;
@@ -618,7 +618,7 @@ gw_status gw::run_bf16_geglu(gw_bf16_plan* gate_plan, const gw_projection& gate,
   *done = false;
   if (!gate_plan || !same_shape(gate, up) || gate.storage != GW_STORAGE_BF16 || !gate.bf16 || !up.bf16 || !aligned(gate.bf16, 16) ||
       !aligned(up.bf16, 16) || gate_plan->input_width != gate.input || gate_plan->output_width != gate.output ||
-      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::bf16, gate_plan->rows, gate.output) || !input || !aligned(input, 16) || !product || !aligned(product, 16))
+      !dense_geglu_pays(gate_plan->descriptors.tuning, GemmKind::bf16, gate_plan->rows, gate.input, gate.output) || !input || !aligned(input, 16) || !product || !aligned(product, 16))
     return GW_OK;
   *done = true;
   *packed = usable_fp8(down);

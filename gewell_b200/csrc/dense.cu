@@ -452,9 +452,17 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
 // three launches stand against the swap form's four to nine.  MLP, us, swap form / this: NVFP4 2816 -> 2176 16 rows 22.8 / 20.3,
 // 2816 -> 4096 100 rows 22.9 / 21.6, 4096 -> 8192 40 rows 27.2 / 29.7; FP8 2816 -> 4096 20 rows 22.8 / 20.6, 4096 -> 8192 100 rows
 // 38.5 / 37.6; BF16 3200 -> 4224 53 rows 30.3 / 29.5.
-bool dense_geglu_pays(const DenseTuning& tuning, GemmKind kind, uint32_t rows, uint32_t n) {
+//
+// NVFP4 of few rows has one accumulator here (tensor memory is full beside the scales), so it stays on the swap form where that
+// divides K: the sums would be of longer parts, and with widely varying block scales further from the exact ones.
+bool dense_geglu_pays(const DenseTuning& tuning, GemmKind kind, uint32_t rows, uint32_t k, uint32_t n) {
   if (tuning.form != 0 || tuning.block_n != 0 || tuning.no_pair) return false;
   if (!dense_uses_swap_form(tuning, rows)) return true;
+  if (kind == GemmKind::nvfp4) {
+    const int tiles = int((n + 127) / 128), stages = gemm_tc_k_stages(kind, GemmEpilogue::swap_store, k / 2);
+    for (const int of : {tiles, 2 * tiles})          // gate and up apart, joined
+      if (swap_split_grid(kind, of, stages, swap_block_n(rows)) > 0) return false;
+  }
   return rows > 8 && int((n + 127) / 128) <= sm_count() / (kind == GemmKind::nvfp4 ? 4 : 2);
 }
 

@@ -140,7 +140,7 @@ struct GegluProblem {
   uint32_t* error;
 };
 // Whether that is the faster way for gate and up projections of n channels each.
-bool dense_geglu_pays(const DenseTuning& tuning, GemmKind kind, uint32_t rows, uint32_t n);
+bool dense_geglu_pays(const DenseTuning& tuning, GemmKind kind, uint32_t rows, uint32_t k, uint32_t n);
 gw_status launch_dense_geglu(const GegluProblem& problem, DenseDescriptors* cache, cudaStream_t stream);
 
 // The same of FP8 or BF16 projections; the result is E4M3 (inverse_scale != 0) or BF16.

@@ -47,3 +47,22 @@ for rows in (1, 40, 128, 300):
     assert direct != unaligned and "gemm_tc_kernel" in unaligned, rows
 '''
     run_child(fake_runtime, script)
+
+
+GEGLU = NAMES + r'''
+NV, F8, BF = _lib.STORAGE_NVFP4_W4A4, _lib.STORAGE_FP8_W8A8, _lib.STORAGE_BF16
+for storage, kernel in ((NV, "gemm_pair_kernelILb1E"), (F8, "gemm_pair_wide_kernelILb1ELNS0_7WideOutE3"), (BF, "gemm_pair_wide_kernelILb0ELNS0_7WideOutE2")):
+    for rows, hidden, mlp, fused in ((8, 2816, 2176, False), (9, 2816, 2176, True), (32, 256, 384, True), (33, 640, 1152, True),
+                                     (65, 2816, 256, True), (128, 384, 2176, True), (64, 2816, 9600, False), (129, 2816, 9600, True),
+                                     (16, 5376, 2048, storage != NV)):      # the swap form divides K of NVFP4 there
+        chain = ctypes.c_void_p()
+        check(lib.gw_mlp_chain_create(hidden, mlp, 256, _lib.POLICY_ALWAYS, ctypes.byref(chain)))
+        check(lib.gw_mlp_chain_prepare(chain, rows))
+        bound = [projection(storage, k, n) for k, n in ((hidden, mlp), (hidden, mlp), (mlp, hidden))]
+        names = kernels(lambda: lib.gw_mlp_chain_run(chain, *map(ctypes.byref, bound), A, A, A, A, _lib.PHASE_PREFILL, None))
+        assert any(kernel in name for name in names) == fused, (storage, rows, hidden, mlp, names)
+'''
+
+
+def test_narrow_mlps_of_few_rows_run_gate_up_and_geglu_in_one_launch(fake_runtime):
+    run_child(fake_runtime, GEGLU)
