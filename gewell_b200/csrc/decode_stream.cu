@@ -312,6 +312,10 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
     __syncthreads();
 
     constexpr int kMatrices = PAIR ? 2 : 1, kSums = lane_sums<NT, PAIR>();
+    // A warp with many pieces of a row block sums each piece by itself and adds the sums: the tensor instruction rounds at every
+    // step, and the longer it adds up the further it ends (outputs that are not the nearest BF16, BF16 1x5376x1024, equal ranges
+    // of pieces for all SMs / whole row blocks 1.0e-4 / 2.8e-4, 4x5376x2048 1.6e-4 / 3.4e-4).
+    constexpr bool kPieceSums = KIND != StreamKind::w4a16;
     float acc[kMatrices][2][NT][4] = {};
     const auto sum_at = [&](int i) -> float& { return acc[i / (NT * 8)][i / 4 % 2][i / 8 % NT][i % 4]; };
     float* mine = sums + warp * kValues + lane;
@@ -334,10 +338,22 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
           const uint4 s = ptx::lds128(ptx::smem_u32(ring_scales + place * L::kScaleBytes) + lane % 4 * 128 + lane / 4 * 16);
           scale[0] = s.x; scale[1] = s.y; scale[2] = s.z; scale[3] = s.w;
         }
-        multiply<KIND, NT>(ptx::smem_u32(ring + place * kPieceBytes) + lane / 4 * 128, lane, scale,
-                           ptx::smem_u32(tokens) + chunk * L::kChunkBytes, acc[m]);
-        __syncwarp();                                        // every lane has read the slot
-        request();
+        const auto multiply_into = [&](float (*sum)[NT][4]) {
+          multiply<KIND, NT>(ptx::smem_u32(ring + place * kPieceBytes) + lane / 4 * 128, lane, scale,
+                             ptx::smem_u32(tokens) + chunk * L::kChunkBytes, sum);
+        };
+        if constexpr (kPieceSums) {
+          float of_piece[2][NT][4] = {};
+          multiply_into(of_piece);
+          __syncwarp();                                        // every lane has read the slot
+          request();
+#pragma unroll
+          for (int i = 0; i < 8 * NT; ++i) acc[m][i / 4 % 2][i / 8][i % 4] += of_piece[i / 4 % 2][i / 8][i % 4];
+        } else {
+          multiply_into(acc[m]);
+          __syncwarp();
+          request();
+        }
       }
       if (++chunk != chunks) continue;
       // the row block ends here

@@ -49,6 +49,17 @@ def projected(gw, kind, x, weight, k, n):
     return y.float()
 
 
+@pytest.mark.parametrize("kind,piece", [("bf16", 64), ("fp8", 128)])
+@pytest.mark.parametrize("rows", [1, 8])
+def test_streaming_sums_pieces(gw, kind, piece, rows):
+    """Weight-streaming kernel, fewer row blocks than half of the SMs: all pieces of 128 bytes of K but the first and the last are
+    kept.  A piece is a whole number of units in the last place of L."""
+    k, n = 5376, 1024
+    x, weight, whole = operands(gw, kind, rows, k, n)
+    kept = projected(gw, kind, x, weight, k, n) / whole
+    assert kept.min() >= 1 - 2 * piece / k - 2.0 ** -8 and kept.max() <= 1 + 2.0 ** -8, (kept.min(), kept.max())
+
+
 @pytest.mark.parametrize("rows", [12, 64, 100])
 def test_swap_form_split_sums_sixths(gw, rows):
     """42 tiles of NVFP4 channels: three CTAs a tile, and two accumulators in each of them; the four parts between the ends are kept."""
