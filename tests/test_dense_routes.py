@@ -2,6 +2,9 @@
 (tests/cpp/fake_cudart.cpp, 148 SMs) names them.  No GPU."""
 import pytest
 
+from tests.test_gpu_pair_split import SHARED
+from tests.test_gpu_pair_wide import FEW_ROWS
+from tests.test_gpu_stream_whole import STREAMED
 from tests.test_prepare import CHILD, fake_runtime, run_child  # noqa: F401  (fixture)
 
 NAMES = CHILD + r'''
@@ -66,3 +69,35 @@ for storage, kernel in ((NV, "gemm_pair_kernelILb1E"), (F8, "gemm_pair_wide_kern
 
 def test_narrow_mlps_of_few_rows_run_gate_up_and_geglu_in_one_launch(fake_runtime):
     run_child(fake_runtime, GEGLU)
+
+
+PLANS = NAMES + r'''
+def projection_kernels(kind, rows, k, n):
+    """Of a projection by a plan of its own."""
+    plan = ctypes.c_void_p()
+    channel = kind.endswith("per channel")
+    if kind == "nvfp4":
+        run = nvfp4_plan(rows, k, n)
+    elif kind.startswith("fp8"):
+        check(lib.gw_fp8_plan_create(rows, k, n, int(channel), ctypes.byref(plan)))
+        run = lambda output: lib.gw_fp8_plan_run(plan, A, A, 0.01, 0.01, A if channel else None, output, A, 1 << 40, None, 0)
+    else:
+        check(lib.gw_bf16_plan_create(rows, k, n, ctypes.byref(plan)))
+        run = lambda output: lib.gw_bf16_plan_run(plan, A, A, output, A, 1 << 40, None)
+    return kernels(lambda: run(A))
+
+
+for kind, rows, k, n in SHAPES:
+    names = projection_kernels(kind, rows, k, n)
+    assert KERNEL in names[-1] and (not SPLIT or SPLIT in names[-1]), (kind, rows, k, n, names)
+    if KERNEL == "decode_stream_kernel":
+        assert len(names) == 1
+'''
+
+
+@pytest.mark.parametrize("shapes,kernel,split", [
+    ([(kind, *shape) for kind, of in STREAMED.items() for shape in of], "decode_stream_kernel", None),
+    ([("nvfp4", *shape) for shape in SHARED], "gemm_pair_kernel", "ILb0ELb0ELb1E"),
+    (FEW_ROWS, "gemm_pair_wide_kernel", None)], ids=["streamed", "shared K", "few rows on pairs"])
+def test_shapes_of_the_gpu_tests_take_the_route_under_test(fake_runtime, shapes, kernel, split):
+    run_child(fake_runtime, f"SHAPES, KERNEL, SPLIT = {shapes!r}, {kernel!r}, {split!r}\n" + PLANS)

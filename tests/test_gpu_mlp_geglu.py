@@ -70,6 +70,14 @@ def test_fused_equals_separate_launches(gw, monkeypatch, storage, joined, rows, 
     assert_gemm_close(results[0], results[1], f"{storage} {rows}x{hidden}->{mlp}")
 
 
+@pytest.mark.parametrize("storage,joined", [("nvfp4", True), ("nvfp4", False), ("fp8", False), ("fp8 channel", True), ("fp8 bf16", True),
+                                            ("bf16", False), ("bf16 fp8", True)])
+@pytest.mark.parametrize("rows,hidden,mlp", [(9, 2816, 2176), (32, 256, 384), (33, 640, 1152), (65, 2816, 256), (128, 384, 2176)])
+def test_few_rows(gw, monkeypatch, storage, joined, rows, hidden, mlp):
+    """Narrow MLPs from 9 rows on; test_dense_routes.py asserts the launches."""
+    test_fused_equals_separate_launches(gw, monkeypatch, storage, joined, rows, hidden, mlp)
+
+
 @pytest.mark.parametrize("storage", ["fp8 channel", "bf16", "bf16 fp8"])
 @pytest.mark.parametrize("rows,mlp", [(250, 9728), (300, 9600)])
 def test_last_wave_in_pieces(gw, monkeypatch, storage, rows, mlp):

@@ -3,13 +3,16 @@
 import pytest
 import torch
 
-from tests.gpu_helpers import assert_gemm_close, bf16_normal, bits
+from tests.gpu_helpers import assert_gemm_close, assert_reference_tolerance, bf16_normal, bits
 
 pytestmark = pytest.mark.gpu
 
+# test_dense_routes.py asserts that all of them share K
+SHARED = [(129, 16448, 128), (255, 8256, 384), (257, 12352, 2560), (256, 21504, 5376), (512, 16384, 4096),
+          (513, 8256, 2816), (33, 8192, 128), (64, 12288, 2816), (65, 8192, 128), (128, 16448, 4608), (100, 8256, 2816)]
 
-@pytest.mark.parametrize("rows,k,n", [(129, 16448, 128), (255, 8256, 384), (257, 12352, 2560), (256, 21504, 5376), (512, 16384, 4096),
-                                      (513, 8256, 2816), (33, 8192, 128), (64, 12288, 2816), (65, 8192, 128), (128, 16448, 4608), (100, 8256, 2816)])
+
+@pytest.mark.parametrize("rows,k,n", SHARED)
 def test_shared_k(monkeypatch, rows, k, n):
     """K over two to four pairs (of 148 SMs); tokens and channels that end within a tile, K that ends within a stage."""
     import gewell_b200 as gw
@@ -30,6 +33,7 @@ def test_shared_k(monkeypatch, rows, k, n):
         assert gw.kernel_error() == 0 and torch.all(y[-64:] == -7.0)
         results.append(bits(y[:-64]))
     assert_gemm_close(results[0], results[1], f"{rows}x{k}x{n}")
+    assert_reference_tolerance(results[0], results[1], f"{rows}x{k}x{n}")       # a last bit of a value
 
 
 def test_one_plan_on_both_routes():
