@@ -91,6 +91,9 @@ struct Divisor {
 // GEMM behind them gets its weights under way at the end of the kernel in
 // front of them.  Before its wait a kernel may
 //   - read the launch's parameters and what the host wrote before the launch,
+//   - read what an earlier launch than its direct predecessor wrote, if that
+//     one is none of those quantisers: so the grouped MoE GEMMs read the
+//     expert offsets, with the routing and the rows' own launch before them,
 //   - bring weights into L2 (ptx::tma_prefetch_*), whoever writes them,
 //   - read weights that are settled: in front of the launch, or of the
 //     quantiser before it, the same call launched another kernel, which is no

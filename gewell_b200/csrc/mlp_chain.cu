@@ -7,8 +7,8 @@
 //   gate + up   one joined GEMM over [gate | up] when the loader laid the two matrices out back to
 //               back: NVFP4 with FP4 activations (contiguous rows and scale tiles, equal globals),
 //               FP8 with per-channel scales, or BF16; otherwise two separate projections
-//               (NVFP4 from 129 rows on: gate, up, GeGLU and the down projection's quantiser are one launch of the CTA-pair
-//               kernel, joined or not; FP8 and BF16 gate, up and GeGLU too)
+//               (beyond 128 rows, and beyond 8 where the MLP is narrow (dense_geglu_pays): gate, up and GeGLU are one launch
+//               of the CTA-pair kernels, joined or not; with the down projection's quantiser where that is NVFP4 or FP8)
 //   GeGLU       fused into the activation quantiser of the down projection when that one runs
 //               quantised on a joined [rows, gate | up] tensor; an element-wise kernel otherwise
 //               (small row counts, where that is the faster way: gate, up and GeGLU are one launch of the
