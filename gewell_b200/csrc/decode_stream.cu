@@ -223,7 +223,9 @@ __device__ __forceinline__ void finish_unit(const StreamArgs& a, uint32_t unit, 
   store_unit<NT, PAIR>(a, block, lane, sum);
 }
 
-template <StreamKind KIND, int NT, bool PAIR>
+// PIECE_SUMS: each piece is summed by itself and the sums are added.  The tensor instruction rounds at every step, and the longer
+// it adds up the further it ends (StreamPlan::piece_sums says where that matters).
+template <StreamKind KIND, int NT, bool PAIR, bool PIECE_SUMS>
 __global__ void __launch_bounds__((Layout<KIND, NT, PAIR>::kThreads), 1)
 decode_stream_kernel(const __grid_constant__ StreamArgs a) {
   using L = Layout<KIND, NT, PAIR>;
@@ -312,10 +314,6 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
     __syncthreads();
 
     constexpr int kMatrices = PAIR ? 2 : 1, kSums = lane_sums<NT, PAIR>();
-    // A warp with many pieces of a row block sums each piece by itself and adds the sums: the tensor instruction rounds at every
-    // step, and the longer it adds up the further it ends (outputs that are not the nearest BF16, BF16 1x5376x1024, equal ranges
-    // of pieces for all SMs / whole row blocks 1.0e-4 / 2.8e-4, 4x5376x2048 1.6e-4 / 3.4e-4).
-    constexpr bool kPieceSums = KIND != StreamKind::w4a16;
     float acc[kMatrices][2][NT][4] = {};
     const auto sum_at = [&](int i) -> float& { return acc[i / (NT * 8)][i / 4 % 2][i / 8 % NT][i % 4]; };
     float* mine = sums + warp * kValues + lane;
@@ -342,7 +340,7 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
           multiply<KIND, NT>(ptx::smem_u32(ring + place * kPieceBytes) + lane / 4 * 128, lane, scale,
                              ptx::smem_u32(tokens) + chunk * L::kChunkBytes, sum);
         };
-        if constexpr (kPieceSums) {
+        if constexpr (PIECE_SUMS) {
           float of_piece[2][NT][4] = {};
           multiply_into(of_piece);
           __syncwarp();                                        // every lane has read the slot
@@ -399,23 +397,26 @@ decode_stream_kernel(const __grid_constant__ StreamArgs a) {
   }
 }
 
-template <StreamKind KIND, int NT, bool PAIR>
+template <StreamKind KIND, int NT, bool PAIR, bool PIECE_SUMS>
 cudaError_t launch_instance(const StreamArgs& args, const StreamPlan& plan, cudaStream_t stream) {
   static bool configured_on[kMaxDeviceSlots] = {};   // the attribute is per GPU
   bool& configured = configured_on[current_device_slot()];
   if (!configured) {
-    const cudaError_t status = cudaFuncSetAttribute(decode_stream_kernel<KIND, NT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit);
+    const cudaError_t status = cudaFuncSetAttribute(decode_stream_kernel<KIND, NT, PAIR, PIECE_SUMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit);
     if (status != cudaSuccess) return status;
     configured = true;
   }
-  return launch_pdl_shared(decode_stream_kernel<KIND, NT, PAIR>, plan.grid, Layout<KIND, NT, PAIR>::kThreads, plan.shared_bytes, stream, args);
+  return launch_pdl_shared(decode_stream_kernel<KIND, NT, PAIR, PIECE_SUMS>, plan.grid, Layout<KIND, NT, PAIR>::kThreads, plan.shared_bytes, stream, args);
 }
 
 template <StreamKind KIND>
 cudaError_t launch_kind(const StreamArgs& args, const StreamPlan& plan, bool pair, cudaStream_t stream) {
-  if constexpr (KIND == StreamKind::w4a16)
-    if (plan.tiles == 2) return pair ? launch_instance<KIND, 2, true>(args, plan, stream) : launch_instance<KIND, 2, false>(args, plan, stream);
-  return pair ? launch_instance<KIND, 1, true>(args, plan, stream) : launch_instance<KIND, 1, false>(args, plan, stream);
+  if constexpr (KIND == StreamKind::w4a16) {
+    if (plan.tiles == 2) return pair ? launch_instance<KIND, 2, true, false>(args, plan, stream) : launch_instance<KIND, 2, false, false>(args, plan, stream);
+  } else if (plan.piece_sums) {
+    return pair ? launch_instance<KIND, 1, true, true>(args, plan, stream) : launch_instance<KIND, 1, false, true>(args, plan, stream);
+  }
+  return pair ? launch_instance<KIND, 1, true, false>(args, plan, stream) : launch_instance<KIND, 1, false, false>(args, plan, stream);
 }
 
 struct Sizes { uint32_t warps, fixed, chunk; };
@@ -454,15 +455,26 @@ StreamPlan plan_stream(StreamKind kind, uint32_t rows, uint32_t k, uint32_t n, b
   const uint64_t pieces = uint64_t(p.blocks) * p.chunks;
   if (pieces >= (1u << 30) || p.slabs > 32) return p;          // one lane per slab when the sums are added
   // Whole row blocks for every SM, where all of K fits: the sums of a block that SMs share cost a pass through L2, 2 us, more than
-  // some SMs with one block more than others do.  (Shared / whole, us: NVFP4 1x2816x2048 7.5 / 5.3, 1x2816x8192 9.1 / 6.9, 1x5376x21504
-  // 17.3 / 15.2, FP8 8x2816x4096 9.7 / 6.6, 4x5376x43008 38.6 / 36.4, BF16 8x2816x1024 7.9 / 6.2; with K 1024 and N 8192, where a
-  // block does not feed the warps, NVFP4 5.2 / 5.8 and FP8 4.8 / 4.8.)
-  p.whole = p.slabs == 1;
-  if (p.whole) p.grid = std::min(p.blocks, sm_count);
-  // at least one piece per warp
-  else p.grid = int(pieces / size.warps < uint64_t(sm_count) ? (pieces + size.warps - 1) / size.warps : sm_count);
+  // some SMs with one block more than others do.  (Shared / whole, us: NVFP4 1x2816x2048 7.3 / 5.0, 1x2816x8192 9.1 / 6.9, 1x5376x21504
+  // 17.3 / 15.2, FP8 8x2816x4096 9.7 / 6.6, 4x5376x43008 38.6 / 36.4, BF16 8x2816x1024 7.9 / 6.1.)  Blocks of a short K come together
+  // until they feed a block's warps; an SM for each is the slower way (NVFP4 1x1024x4864 4.8 / 5.4, FP8 1x512x4864 3.7 / 4.3).
+  const auto share = [](uint64_t all, uint64_t of) { return (all + of - 1) / of; };
+  const bool one_each = p.blocks <= sm_count && 2 * p.blocks >= sm_count;
+  const int together = std::max(1, int(size.warps) / p.chunks);
+  const int whole_grid = one_each ? p.blocks : int(std::min<uint64_t>(sm_count, share(p.blocks, together)));
+  const int cut_grid = int(std::min<uint64_t>(sm_count, share(pieces, size.warps)));          // at least one piece per warp
+  const bool cuts = p.chunks_per_slab / int(pieces / cut_grid) + 2 <= 32;                     // one lane per part of a slab's row block
+  // Where a warp has more pieces than with equal ranges its sums would be longer, and further from the exact ones: each piece is
+  // then summed by itself, for 0.5 to 3 % of the time (outputs that are not the nearest BF16, shared / whole / whole with sums of pieces:
+  // BF16 1x5376x1024 9.8e-5 / 2.8e-4 / 9.8e-5, 4x5376x2048 1.6e-4 / 3.4e-4 / 1.4e-4).  W4A16, whose time goes into decoding, stays
+  // shared there (MLP of one row, whole / shared, us: 5376 -> 4864 26.5 / 23.8, 5376 -> 14336 48.1 / 46.5, 5376 -> 21504 61.4 / 61.8;
+  // but 2816 -> 6144, as many pieces, 17.2 / 20.2).
+  const bool longer = !one_each && share(share(p.blocks, whole_grid) * p.chunks, size.warps) > share(share(pieces, cut_grid), size.warps);
+  p.whole = p.slabs == 1 && (kind != StreamKind::w4a16 || !longer || !cuts);
+  p.piece_sums = p.whole && longer && kind != StreamKind::w4a16;
+  if (!p.whole && !cuts) return p;
+  p.grid = p.whole ? whole_grid : cut_grid;
   const int per_cta = int(pieces / p.grid);
-  if (!p.whole && p.chunks_per_slab / per_cta + 2 > 32) return p;          // one lane per part of a slab's row block
   const int shortest = p.chunks - (p.slabs - 1) * p.chunks_per_slab;
   p.max_units = per_cta / shortest + 3;
   p.shared_bytes = size_t(p.chunks_per_slab) * size.chunk + size.fixed;

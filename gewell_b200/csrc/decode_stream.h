@@ -47,6 +47,7 @@ struct StreamProblem {
 // How a problem of this shape is divided over the GPU.
 struct StreamPlan {
   bool whole = false;          // every SM's range is whole row blocks: no sums to add up across SMs
+  bool piece_sums = false;     // every piece of K is summed by itself
   bool usable = false;         // the shape can run here (widths a piece can walk, row count)
   uint32_t physical_n = 0;     // rows of each weight matrix in memory
   int tiles = 0;               // groups of eight token rows: 1 or 2

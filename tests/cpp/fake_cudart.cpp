@@ -12,6 +12,7 @@ std::atomic<long> g_fail_in{0};             // 1: the next allocation fails; 0: 
 std::atomic<long> g_launches{0};
 std::atomic<long> g_fail_launch_in{0};      // as g_fail_in, of launches
 std::map<const void*, std::string> g_names;      // of the registered kernels
+unsigned g_grid = 0;                        // blocks of the last launch in x
 std::string g_launched;                     // kernels launched since fake_launched(), one name a line
 std::map<void*, void*> g_recorded;          // event -> the stream it was last recorded on
 std::map<void*, bool> g_forked;             // stream of the library's -> something has waited for it since it waited
@@ -40,6 +41,7 @@ const char* fake_launched() {
   g_launched.clear();
   return last.c_str();
 }
+long fake_grid() { return g_grid; }
 // 1: the library's own stream waited for another, which has not waited for it since
 long fake_forked() { return g_forked[kOwnStream]; }
 long fake_unfinished() {
@@ -72,7 +74,10 @@ int cudaOccupancyMaxActiveClusters(int* clusters, const void*, const void* confi
   *clusters = 148 / int(*static_cast<const unsigned*>(config));
   return 0;
 }
-int cudaLaunchKernelExC(const void*, const void* kernel, void**) { return launch(kernel); }
+int cudaLaunchKernelExC(const void* config, const void* kernel, void**) {      // it begins with gridDim.x
+  g_grid = *static_cast<const unsigned*>(config);
+  return launch(kernel);
+}
 struct Dim3 { unsigned x, y, z; };
 int cudaLaunchKernel(const void* kernel, Dim3, Dim3, void**, size_t, void*) { return launch(kernel); }
 int cudaGetDriverEntryPoint(const char*, void** entry, unsigned long long, int* result) {

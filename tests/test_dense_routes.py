@@ -101,3 +101,22 @@ for kind, rows, k, n in SHAPES:
     (FEW_ROWS, "gemm_pair_wide_kernel", None)], ids=["streamed", "shared K", "few rows on pairs"])
 def test_shapes_of_the_gpu_tests_take_the_route_under_test(fake_runtime, shapes, kernel, split):
     run_child(fake_runtime, f"SHAPES, KERNEL, SPLIT = {shapes!r}, {kernel!r}, {split!r}\n" + PLANS)
+
+
+GRIDS = PLANS[:PLANS.index("for kind, rows, k, n in SHAPES")] + r'''
+fake.fake_grid.restype = ctypes.c_long
+# (kind, rows, K, N): blocks of the launch, whether pieces are summed by themselves
+for shape, grid, pieces in (
+        (("nvfp4", 1, 1024, 4864), 38, False), (("fp8", 1, 512, 4864), 38, False), (("fp8", 1, 1024, 512), 8, False),      # short K
+        (("nvfp4", 1, 2816, 512), 16, False), (("nvfp4", 1, 2816, 8192), 148, False), (("bf16", 1, 2816, 4096), 128, False),
+        (("nvfp4", 1, 5376, 1024), 32, True), (("fp8", 8, 2816, 1024), 32, True), (("bf16", 8, 5376, 2048), 64, True),       # few blocks, long K
+        (("nvfp4", 1, 5376, 4096), 128, False), (("fp8", 8, 5376, 43008), 148, True)):
+    names = projection_kernels(*shape)
+    assert len(names) == 1 and "decode_stream_kernel" in names[0], (shape, names)
+    assert fake.fake_grid() == grid and ("ELi1ELb0ELb1E" in names[0]) == pieces, (shape, fake.fake_grid(), names)
+'''
+
+
+def test_division_of_the_streaming_kernel(fake_runtime):
+    """Blocks of a short K come together; pieces are summed by themselves where a warp has more of them than equal ranges would give it."""
+    run_child(fake_runtime, GRIDS)
