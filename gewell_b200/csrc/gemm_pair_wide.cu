@@ -151,7 +151,7 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
   // and the epilogue adds them up.  The swap form, which runs such rows otherwise, divides K over four CTAs, and a sum of all of K
   // in one accumulator is further from the exact one (outputs that are not the nearest BF16, 2816 -> 2176, swap form / one
   // accumulator: BF16 16 rows 4.1e-4 / 1.5e-3, FP8 with blocks of sixteen activations scaled by 2^-6 .. 2^6 1.7e-4 / 5.5e-4).
-  const int parts = kGeglu && total_work <= pairs && p.tiles.tile_rows <= kPartCols ? min(4, p.k_stages) : 1;
+  const bool quarters = kGeglu && total_work <= pairs && p.tiles.tile_rows <= kPartCols && p.k_stages >= 4;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (one lane)
@@ -204,12 +204,12 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         const uint32_t idesc = idesc_of_width | ((uint32_t(w < p.tiles.whole ? p.tiles.tile_rows : p.tiles.piece_rows) >> 3) << 17);
         // The split form has both accumulators to itself: each takes half of the K slabs.
         const int mid_ks = kSplit ? (first_ks + end_ks + 1) / 2 : end_ks;
-        int part = 0, part_end = kGeglu ? p.k_stages / parts : 0;
+        int part = 0, part_end = quarters ? p.k_stages / 4 : p.k_stages;
         bool begins = true;
         for (int ks = first_ks; ks < end_ks; ++ks) {
           if (kGeglu && ks == part_end) {
             begins = true;
-            part_end = (++part + 1) * p.k_stages / parts;
+            part_end = (++part + 1) * p.k_stages / 4;
           }
           if (!__all_sync(0xffffffffu, ptx::mbar_wait_bounded(full_bar + stage, phase))) {
             report(p.error, 0x35000000u | (blockIdx.x << 8) | stage, &abort_flag);
@@ -266,16 +266,21 @@ gemm_pair_wide_kernel(const __grid_constant__ PairWideParams p) {
         const int token0 = tile.token0 + t0;
         if (token0 >= tile.end) break;                                // the whole half
         uint32_t r[32];
-        ptx::tmem_load16(taddr + t0, r);
-        ptx::tmem_load16(taddr + t0 + 16, r + 16);
-        ptx::tmem_load_wait();
-        for (int part = 1; part < parts; ++part) {
-          uint32_t s[32];
-          ptx::tmem_load16(taddr + part * kPartCols + t0, s);
-          ptx::tmem_load16(taddr + part * kPartCols + t0 + 16, s + 16);
-          ptx::tmem_load_wait();
+        if (quarters) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(s[i]));
+          for (int h = 0; h < 2; ++h) {
+            uint32_t q[4][16];
+#pragma unroll
+            for (int part = 0; part < 4; ++part) ptx::tmem_load16(taddr + part * kPartCols + t0 + 16 * h, q[part]);
+            ptx::tmem_load_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              r[16 * h + i] = __float_as_uint(__uint_as_float(q[0][i]) + __uint_as_float(q[1][i]) + __uint_as_float(q[2][i]) + __uint_as_float(q[3][i]));
+          }
+        } else {
+          ptx::tmem_load16(taddr + t0, r);
+          ptx::tmem_load16(taddr + t0 + 16, r + 16);
+          ptx::tmem_load_wait();
         }
         if (t0 != half * 32) half_barrier(half);                    // the chunk before has been read
         uint16_t* put = reinterpret_cast<uint16_t*>(staging) + quad * 32 + lane;
