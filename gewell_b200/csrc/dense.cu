@@ -449,16 +449,24 @@ gw_status launch_dense(const DenseProblem& q, DenseDescriptors* cache, cudaStrea
 }
 
 // Beyond the swap form's rows always; with fewer where one wave of pair tiles (NVFP4: half of one) holds all channels, so that
-// three launches stand against the swap form's four to nine.  MLP, us, swap form / this: NVFP4 2816 -> 2176 16 rows 22.8 / 20.3,
-// 2816 -> 4096 100 rows 22.9 / 21.6, 4096 -> 8192 40 rows 27.2 / 29.7; FP8 2816 -> 4096 20 rows 22.8 / 20.6, 4096 -> 8192 100 rows
-// 38.5 / 37.6; BF16 3200 -> 4224 53 rows 30.3 / 29.5.
+// three launches stand against the swap form's four to nine.  MLP of joined gate and up, us launched one by one | in a graph, swap form /
+// this:
+//   NVFP4 16x2816 -> 4096 21.8 / 20.5 | 17.1 / 19.2, 128x2048 -> 4096 22.6 / 21.6 | 21.3 / 20.5; with few channels for their K slower either
+//         way, 96x5376 -> 2048 22.2 / 24.3 | 20.5 / 23.2; 40x4096 -> 8192 27.2 / 29.7
+//   FP8   16x2816 -> 4096 22.0 / 20.3 | 16.5 / 18.9, 64x2816 -> 4096 22.6 / 21.2 | 21.4 / 19.9; apart 16x2816 -> 2176 - | 24.3 / 14.6
+//   BF16  64x2816 -> 4096 29.3 / 25.7 | 28.6 / 24.8; up to 32 rows slower, 16x2816 -> 2176 20.9 / 22.3 | 20.5 / 21.1, 16x5376 -> 2048
+//         25.7 / 30.3 | 25.2 / 29.3, and up to 64 with few channels for their K, 48x5376 -> 2048 29.3 / 31.4 | 28.9 / 30.5
 //
 // NVFP4 of few rows has one accumulator here (tensor memory is full beside the scales), so it stays on the swap form where that
-// divides K: the sums would be of longer parts, and with widely varying block scales further from the exact ones.
+// divides K: the sums would be of longer parts, and with widely varying block scales further from the exact ones (outputs of an MLP
+// that differ from those with exact gate and up, 16x5376 -> 2048: none / 2.7e-3).
 bool dense_geglu_pays(const DenseTuning& tuning, GemmKind kind, uint32_t rows, uint32_t k, uint32_t n) {
   if (tuning.form != 0 || tuning.block_n != 0 || tuning.no_pair) return false;
   if (!dense_uses_swap_form(tuning, rows)) return true;
+  const bool few_channels = 2 * size_t(n) < k;
+  if (kind == GemmKind::bf16 && (rows <= 32 || (rows <= 64 && few_channels))) return false;
   if (kind == GemmKind::nvfp4) {
+    if (few_channels) return false;
     const int tiles = int((n + 127) / 128), stages = gemm_tc_k_stages(kind, GemmEpilogue::swap_store, k / 2);
     for (const int of : {tiles, 2 * tiles})          // gate and up apart, joined
       if (swap_split_grid(kind, of, stages, swap_block_n(rows)) > 0) return false;

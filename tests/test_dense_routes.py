@@ -55,9 +55,11 @@ for rows in (1, 40, 128, 300):
 GEGLU = NAMES + r'''
 NV, F8, BF = _lib.STORAGE_NVFP4_W4A4, _lib.STORAGE_FP8_W8A8, _lib.STORAGE_BF16
 for storage, kernel in ((NV, "gemm_pair_kernelILb1E"), (F8, "gemm_pair_wide_kernelILb1ELNS0_7WideOutE3"), (BF, "gemm_pair_wide_kernelILb0ELNS0_7WideOutE2")):
-    for rows, hidden, mlp, fused in ((8, 2816, 2176, False), (9, 2816, 2176, True), (32, 256, 384, True), (33, 640, 1152, True),
-                                     (65, 2816, 256, True), (128, 384, 2176, True), (64, 2816, 9600, False), (129, 2816, 9600, True),
-                                     (16, 5376, 2048, storage != NV)):      # the swap form divides K of NVFP4 there
+    for rows, hidden, mlp, fused in ((8, 2816, 2176, False), (9, 2816, 2176, storage != BF), (32, 256, 384, storage != BF),
+                                     (33, 640, 1152, True), (41, 2816, 2176, True), (64, 256, 384, True), (65, 384, 256, True),
+                                     (128, 384, 2176, True), (64, 2816, 9600, False), (129, 2816, 9600, True),
+                                     (16, 5376, 2816, storage == F8),      # the swap form divides K of NVFP4 there
+                                     (64, 5376, 2048, storage == F8), (96, 5376, 2048, storage != NV), (129, 5376, 2048, True)):
         chain = ctypes.c_void_p()
         check(lib.gw_mlp_chain_create(hidden, mlp, 256, _lib.POLICY_ALWAYS, ctypes.byref(chain)))
         check(lib.gw_mlp_chain_prepare(chain, rows))
