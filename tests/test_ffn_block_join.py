@@ -47,3 +47,15 @@ for rows in (8, 128, 129, 8):
     w.router_proj = A
     check(run())
 ''')
+
+
+def test_shared_mlp_of_few_nvfp4_rows_stays_on_the_swap_form(fake_runtime):
+    """Gate, up and GeGLU in one launch from 65 rows on."""
+    run_child(fake_runtime, BLOCK[:BLOCK.index("for small, large")] + r'''
+fake.fake_launched.restype = ctypes.c_char_p
+for rows, one_launch in ((9, False), (64, False), (65, True), (128, True), (129, True)):
+    check(prepare(rows))
+    fake.fake_launched()
+    check(run())
+    assert ("gemm_pair_kernelILb1E" in fake.fake_launched().decode()) == one_launch, rows
+''')
