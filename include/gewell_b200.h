@@ -300,7 +300,7 @@ gw_status gw_gelu_tanh_multiply_interleaved_bf16(const void* gate_up_bf16, void*
  * as ONE GEMM when they are stored back to back (NVFP4: contiguous rows and scale tiles with equal
  * globals, 31b/sm120/nvfp4_projections.h:21-33; FP8: adjacent with per-channel scales,
  * fp8_projections.h:20-50; BF16: adjacent); GeGLU is fused into the gate/up launch beyond 128 rows, for
- * narrow MLPs beyond 8 and where the weights stream, else into the down projection's activation
+ * narrow MLPs beyond 8 (BF16: 32) and where the weights stream, else into the down projection's activation
  * quantiser whenever that one runs quantised on the joined tensor.  policy / phase as in
  * nvfp4_policy.h: with policy "prefill" decode keeps BF16 activations (W4A16, as in ProjectionWorkspace:
  * packed weights up to 32 rows, dequantised into the chain's scratch beyond).
