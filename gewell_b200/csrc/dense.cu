@@ -46,10 +46,11 @@ size_t split_counter_bytes(const DenseTuning& tuning, uint32_t rows, uint32_t n)
 // pays is that every SM reads and quantises all of the activations, that some SMs have one row block more than others, and, with
 // several slabs (!StreamPlan::whole), 2 us for adding sums in a second pass.  Measured against activation quantiser + tcgen05 swap form
 // (B200, rotating weights, passes of a CUDA graph; time of the streaming kernel over the other's):
-//   whole row blocks    FP8, 1 to 8 rows, K 1024 .. 8192, N 512 .. 43008, rows * K up to 44 K    0.58 .. 1.02, 8x5376x16384 1.06
+//   whole row blocks    FP8, 1 to 8 rows, K 1024 .. 8192, N 512 .. 43008, rows * K up to 44 K    0.58 .. 1.02, 8x5376x16384 1.06,
+//                                                                                8 rows, K up to 2048, N 6144 .. 9600 1.02 .. 1.06
 //                       BF16 the same                                                            0.55 .. 1.01, 8x5376x16384 1.05
 //                       NVFP4, N up to 4736 (one block an SM), rows * K up to 24 K   0.67 .. 1.04; more 0.97 .. 1.09
-//                              N up to 9472, rows * K up to 6 K      0.89 .. 0.98; more 0.98 .. 1.21
+//                              N up to 9472, rows * K up to 6 K      0.89 .. 0.98, K 512 1.02 .. 1.08; more 0.98 .. 1.21
 //                              N up to 18944 (one wave of the swap form's tiles)  0.94 .. 1.22
 //                              beyond, rows * K up to 24 K           0.68 .. 1.00; 8x5376x43008 1.04
 //   several slabs       NVFP4 and FP8 up to N 512 0.84 .. 0.97, beyond 0.82 .. 1.41; BF16 up to N 2048 0.78 .. 1.16, beyond 0.88 .. 1.65
